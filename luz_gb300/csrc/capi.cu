@@ -88,12 +88,52 @@ static void free_frame_buffers(luz_frame* f) {
                     f->primary_hit, f->hit_instance, f->gb_coarse, f->gb_fine, f->shadow_bits, f->ao_bits, f->ao, f->ao_denoised, f->signal,
                     f->unshadowed, f->denoised, f->surf, f->surf_mat,
                     f->features, f->lin_depth, f->taa, f->taa_next, f->compose, f->hist, f->hist_state,
-                    f->block_counts, f->lit_count, f->dn_list, f->dn_count, f->d_scene, f->d_lights, f->d_models,
-                    f->d_slot_table, f->d_light_slot, f->d_model_skip, f->work_counter, f->d_textures,
+                    f->block_counts, f->lit_count, f->dn_list, f->dn_count, f->d_upload, f->work_counter, f->d_textures,
                     f->d_texels, f->d_shadow_lights, f->d_shadow_maps, f->rays_a, f->rays_b, f->rays_c, f->beams,
                     f->beam_lists};
     for (void* p : ptrs)
         if (p) cudaFree(p);
+    if (f->h_upload) cudaFreeHost(f->h_upload);
+    if (f->upload_done) cudaEventDestroy(f->upload_done);
+}
+
+// The frame's constants (scene block, lights, slot tables, ModelBlocks) are one device
+// block with a pinned copy of the same layout, so that an upload is one copy that the host
+// does not wait for. Regions are sized by capacities that only grow, so a region keeps its
+// address while nothing outgrows its capacity.
+static luz_status reserve_upload(luz_ctx* ctx, luz_frame* f, uint32_t lights, uint32_t slots, uint32_t models) {
+    if (f->d_upload && lights <= f->lights_cap && slots <= f->slots_cap && models <= f->models_cap) return LUZ_OK;
+    auto grown = [](uint32_t need, uint32_t cap) { return need <= cap ? cap : std::max(need, std::max(cap * 2, 16u)); };
+    const uint32_t nl = grown(lights, f->lights_cap), ns = grown(slots, f->slots_cap), nm = grown(models, f->models_cap);
+    size_t bytes = 0;
+    auto region = [&](size_t n) { const size_t at = bytes; bytes += (n + 255) & ~(size_t)255; return at; };
+    const size_t scene = region(sizeof(luz_scene)), light = region((size_t)nl * sizeof(luz_light)),
+                 first = region((size_t)nl * 4), slot = region((size_t)ns * 4),
+                 model = region((size_t)nm * sizeof(luz_model)), skip = region(nm);
+    // the old block stays in place until the new one is there
+    if (!f->upload_done) LUZ_CUDA(ctx, cudaEventCreateWithFlags(&f->upload_done, cudaEventDisableTiming));
+    LUZ_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
+    void *dev = nullptr, *host = nullptr;
+    LUZ_CUDA(ctx, cudaMalloc(&dev, bytes));
+    if (cudaError_t e = cudaMallocHost(&host, bytes); e != cudaSuccess) {
+        cudaFree(dev);
+        return cuda_error(ctx, e, "cudaMallocHost(frame constants)");
+    }
+    if (f->d_upload) cudaFree(f->d_upload);
+    if (f->h_upload) cudaFreeHost(f->h_upload);
+    f->d_upload = dev;
+    f->h_upload = host;
+    f->lights_cap = nl;
+    f->slots_cap = ns;
+    f->models_cap = nm;
+    char* d = (char*)f->d_upload;
+    f->d_scene = (luz_scene*)(d + scene);
+    f->d_lights = (luz_light*)(d + light);
+    f->d_light_slot = (uint32_t*)(d + first);
+    f->d_slot_table = (uint32_t*)(d + slot);
+    f->d_models = (luz_model*)(d + model);
+    f->d_model_skip = (uint8_t*)(d + skip);
+    return LUZ_OK;
 }
 
 // (Re)allocates *p for at least `need` elements when `cap` is short; cap is updated.
@@ -488,12 +528,16 @@ luz_status luz_frame_create(luz_ctx* ctx, uint32_t width, uint32_t height, luz_f
     A((void**)&f->surf_mat, P * 16);
     A((void**)&f->block_counts, (size_t)chunks * 4);
     A((void**)&f->lit_count, 4);
-    A((void**)&f->d_scene, sizeof(luz_scene));
     A((void**)&f->work_counter, 8);
     if (e != cudaSuccess) {
         free_frame_buffers(f);
         delete f;
         return cuda_error(ctx, e, "cudaMalloc(frame)");
+    }
+    if (luz_status s = reserve_upload(ctx, f, 16, 16, 16); s != LUZ_OK) {
+        free_frame_buffers(f);
+        delete f;
+        return s;
     }
     cudaMemset(f->ao_denoised, 0, P * 4);
     cudaMemset(f->signal, 0, P * 16);
@@ -524,42 +568,40 @@ static luz_status frame_upload_body(luz_ctx* ctx, luz_frame* f, const luz_scene*
     if (scene->ao_min < 0.0f) return set_error(ctx, LUZ_ERR_INVALID, "ao_min is negative (a ray query's tMin)");
     if (light_count > 65535) return set_error(ctx, LUZ_ERR_LIMIT, "more than 65535 lights");
     // Shadow slots: Σ numShadowSamples (GPUScene.cpp:248), one bit plane each.
-    std::vector<uint32_t> slot_table, light_slot(std::max(light_count, 1u));
+    auto samples = [&](uint32_t l) {
+        return scene->shadow_type == LUZ_SHADOW_RAYTRACING ? (uint32_t)std::max(lights[l].num_shadow_samples, 0) : 0u;
+    };
+    uint64_t slots = 0;
     for (uint32_t l = 0; l < light_count; ++l) {
-        light_slot[l] = (uint32_t)slot_table.size();
-        int ns = scene->shadow_type == LUZ_SHADOW_RAYTRACING ? lights[l].num_shadow_samples : 0;
-        if (ns < 0) ns = 0;
-        if (slot_table.size() + ns > LUZ_MAX_SHADOW_SLOTS)
+        slots += samples(l);
+        if (slots > LUZ_MAX_SHADOW_SLOTS)
             return set_error(ctx, LUZ_ERR_LIMIT, "more than LUZ_MAX_SHADOW_SLOTS shadow samples per pixel");
-        for (int s = 0; s < ns; ++s) slot_table.push_back(l | ((uint32_t)s << 16));
     }
-    cudaStream_t st = ctx->stream;
-    uint32_t shadow_slots = (uint32_t)slot_table.size();
-    uint32_t ao = (uint32_t)scene->ao_num_samples;
+    const uint32_t shadow_slots = (uint32_t)slots, ao = (uint32_t)scene->ao_num_samples;
     uint32_t cap_shadow = f->shadow_planes_cap, cap_ao = f->ao_planes_cap;
     luz_status s;
     if ((s = grow(ctx, (void**)&f->shadow_bits, cap_shadow, std::max(shadow_slots, 1u), (size_t)f->words * 4)) != LUZ_OK) return s;
-    if ((s = grow(ctx, (void**)&f->ao_bits, cap_ao, std::max(ao, 1u), (size_t)f->words * 4)) != LUZ_OK) return s;
     f->shadow_planes_cap = cap_shadow;
+    if ((s = grow(ctx, (void**)&f->ao_bits, cap_ao, std::max(ao, 1u), (size_t)f->words * 4)) != LUZ_OK) return s;
     f->ao_planes_cap = cap_ao;
     static_assert(sizeof(luz_light) == 64, "luz_light layout");
     static_assert(sizeof(luz_model) == 128, "luz_model layout");
     static_assert(sizeof(luz_vertex) == 48, "luz_vertex layout");
-    if (light_count > f->lights_cap || !f->d_lights) {
-        uint32_t cap = 0, cap2 = 0;
-        if ((s = grow(ctx, (void**)&f->d_lights, cap, std::max(light_count, 1u), sizeof(luz_light))) != LUZ_OK) return s;
-        if ((s = grow(ctx, (void**)&f->d_light_slot, cap2, cap, 4)) != LUZ_OK) return s;
-        f->lights_cap = cap;
+    if ((s = reserve_upload(ctx, f, light_count, shadow_slots, model_count)) != LUZ_OK) return s;
+    LUZ_CUDA(ctx, cudaEventSynchronize(f->upload_done));   // the last upload has left the pinned block
+    char* h = (char*)f->h_upload;
+    auto host = [&](const void* d) { return h + ((const char*)d - (const char*)f->d_upload); };
+    memcpy(host(f->d_scene), scene, sizeof(luz_scene));
+    uint32_t* light_slot = (uint32_t*)host(f->d_light_slot);
+    uint32_t* slot_table = (uint32_t*)host(f->d_slot_table);
+    uint32_t next = 0;
+    for (uint32_t l = 0; l < light_count; ++l) {
+        light_slot[l] = next;
+        for (uint32_t k = 0, n = samples(l); k < n; ++k) slot_table[next++] = l | (k << 16);
     }
-    if (model_count > f->models_cap || !f->d_models) {
-        uint32_t cap = 0, cap2 = 0;
-        if ((s = grow(ctx, (void**)&f->d_models, cap, std::max(model_count, 1u), sizeof(luz_model))) != LUZ_OK) return s;
-        if ((s = grow(ctx, (void**)&f->d_model_skip, cap2, cap, 1)) != LUZ_OK) return s;
-        f->models_cap = cap;
-    }
-    if (!f->d_slot_table) LUZ_CUDA(ctx, cudaMalloc(&f->d_slot_table, (size_t)LUZ_MAX_SHADOW_SLOTS * 4));
-    f->h_slot_table = slot_table;
-    std::vector<uint8_t> skip(std::max(model_count, 1u), 0);
+    if (light_count) memcpy(host(f->d_lights), lights, (size_t)light_count * sizeof(luz_light));
+    if (model_count) memcpy(host(f->d_models), models, (size_t)model_count * sizeof(luz_model));
+    uint8_t* skip = (uint8_t*)host(f->d_model_skip);
     int32_t max_map = -1;
     for (uint32_t m = 0; m < model_count; ++m) {
         const luz_model& md = models[m];
@@ -574,20 +616,9 @@ static luz_status frame_upload_body(luz_ctx* ctx, luz_frame* f, const luz_scene*
     f->model_count = model_count;
     f->shadow_slots = shadow_slots;
     f->ao_samples = ao;
-    LUZ_CUDA(ctx, cudaMemcpyAsync(f->d_scene, scene, sizeof(luz_scene), cudaMemcpyHostToDevice, st));
-    if (light_count) {
-        LUZ_CUDA(ctx, cudaMemcpyAsync(f->d_lights, lights, (size_t)light_count * sizeof(luz_light), cudaMemcpyHostToDevice, st));
-        LUZ_CUDA(ctx, cudaMemcpyAsync(f->d_light_slot, light_slot.data(), (size_t)light_count * 4, cudaMemcpyHostToDevice, st));
-    }
-    if (shadow_slots)
-        LUZ_CUDA(ctx, cudaMemcpyAsync(f->d_slot_table, slot_table.data(), (size_t)shadow_slots * 4, cudaMemcpyHostToDevice, st));
-    if (model_count) {
-        LUZ_CUDA(ctx, cudaMemcpyAsync(f->d_models, models, (size_t)model_count * sizeof(luz_model), cudaMemcpyHostToDevice, st));
-        LUZ_CUDA(ctx, cudaMemcpyAsync(f->d_model_skip, skip.data(), model_count, cudaMemcpyHostToDevice, st));
-    }
-    // Pageable sources: the copies above are staged before returning; the vectors
-    // may go out of scope once the stream has consumed them.
-    LUZ_CUDA(ctx, cudaStreamSynchronize(st));
+    const size_t bytes = (size_t)((char*)f->d_model_skip + model_count - (char*)f->d_upload);
+    LUZ_CUDA(ctx, cudaMemcpyAsync(f->d_upload, h, bytes, cudaMemcpyHostToDevice, ctx->stream));
+    LUZ_CUDA(ctx, cudaEventRecord(f->upload_done, ctx->stream));
     return LUZ_OK;
 }
 

@@ -226,13 +226,15 @@ struct luz_frame {
     uint32_t h_lit_count = 0;
     // scene constants
     luz_scene h_scene{};
+    void* d_upload = nullptr;          // one block holding the following regions (reserve_upload)
+    void* h_upload = nullptr;          // its pinned copy
+    cudaEvent_t upload_done = nullptr; // h_upload may be rewritten after this
     luz_scene* d_scene = nullptr;
     luz_light* d_lights = nullptr;
-    uint32_t lights_cap = 0, light_count = 0;
+    uint32_t lights_cap = 0, light_count = 0, slots_cap = 0;
     luz_model* d_models = nullptr;
     uint32_t models_cap = 0, model_count = 0;
     uint32_t* d_slot_table = nullptr;  // per shadow slot: light | sample << 16
-    std::vector<uint32_t> h_slot_table;
     uint32_t* d_light_slot = nullptr;  // per light: first shadow slot
     uint8_t* d_model_skip = nullptr;   // per model: 1 = discarded by the alpha test, 2 = tested per hit
     int32_t max_map_index = -1;        // largest texture index of the uploaded ModelBlocks
