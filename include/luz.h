@@ -211,7 +211,7 @@ luz_status luz_ctx_device_status(luz_ctx* ctx, uint32_t* bits);
 /* Number of kernels this context has launched so far. */
 uint64_t luz_ctx_launch_count(const luz_ctx* ctx);
 /* Debug knob, off by default (no counterpart in the reference): the traversal steps a
- * shadow / AO ray may take before the visibility kernel ends it (counted as not
+ * traversed shadow / AO ray may take before the visibility kernel ends it (counted as not
  * occluded, AO: a miss) and raises LUZ_DEV_TRAVERSAL_CAP; 0 restores the library's cap
  * (2^22 steps). For testing that a cap which runs out ends the kernel with a status
  * instead of a hang. */
@@ -333,7 +333,7 @@ luz_status luz_blas_download_wide(luz_ctx* ctx, const luz_blas* blas, void* node
  * a TLAS build reads each BLAS root's box and bounding sphere from it), 4-wide nodes
  * (every traversal), triangles / instance records, other (sort keys,
  * order, shading copies of the vertex and index buffers; for a TLAS also the shading
- * and input records, near lists, leaf indices and build scratch).
+ * and input records and build scratch).
  * The counterpart of the reference's vkGetAccelerationStructureBuildSizesKHR query
  * (source/Graphics/VulkanWrapper.cpp:692-698, 809-812). */
 typedef struct luz_memory {
@@ -412,15 +412,15 @@ luz_status luz_frame_read_shadow_map(luz_ctx* ctx, luz_frame* frame, uint32_t li
  * map is alpha-tested per hit (opaque.frag's discard below 0.5), so the ray goes on
  * to the surface behind. Each 8x8 tile traces only the TLAS leaves its corner-ray
  * cone keeps (lists built per call from the TLAS's last build); the planes are those
- * of a full traversal bit for bit. Also records each pixel's hit instance for the
- * visibility pass's short-ray starts. */
+ * of a full traversal bit for bit. */
 luz_status luz_gbuffer_primary(luz_ctx* ctx, luz_frame* frame, const luz_tlas* tlas);
 /* Shadow (light.frag:86-109,137-146) and AO (light.frag:111-135) any-hit rays of
  * every lit pixel; writes the visibility bit planes (shadow: 1 = occluded, AO: 1 =
- * miss). Rays start below the TLAS root where that cannot change a bit: an AO ray
- * that stays near its primary-hit instance at that instance's leaf (per-call near
- * lists), a shadow ray at the leaves its 32-ray group's capsule reaches (per-call
- * beam lists). By default a shadow sample keeps bit 0 without a ray when the light pass's
+ * miss). Rays are traced one by one only where a group bound leaves them open, which
+ * never changes a bit: the shadow rays of 32 neighbouring pixels to one light are all
+ * unoccluded when the shaft around them reaches no node of any BLAS, an AO ray is a miss
+ * above the horizon of its 32 pixels; the other rays start at the instances, and the
+ * parts of their BLASes, that their group reaches. By default a shadow sample keeps bit 0 without a ray when the light pass's
  * term of its light cannot depend on the shadow factor (light.frag:209-226 adds
  * ((kD * albedo / pi + spec) * radiance) * max(dot(N, L), 0) with radiance =
  * ((color * intensity) * attenuation) * (1 - shadow)): (a) max(dot(N, L), 0) is 0 or
@@ -436,9 +436,10 @@ luz_status luz_trace_visibility(luz_ctx* ctx, luz_frame* frame, const luz_tlas* 
  * per-ray hit results. */
 luz_status luz_frame_set_shadow_cull(luz_frame* frame, int32_t enable);
 /* The same trace with per-ray work counters (a separate kernel build, for
- * roofline accounting): out[0] rays traversed, out[1] TLAS node visits, out[2] BLAS
- * node visits, out[3] triangle tests, out[4] instance leaves reached (entered or
- * rejected by the bounding-sphere test). Rays with nothing to
+ * roofline accounting): out[0] rays (resolved by a group bound or traversed), and of the
+ * traversed ones out[1] TLAS node visits, out[2] BLAS node visits, out[3] triangle tests,
+ * out[4] instance leaves reached (entered or rejected by the bounding-sphere test). Rays
+ * with nothing to
  * trace are not counted: a shadow ray left out by the cull above, a ray with a
  * non-finite origin or direction or tMin > tMax (AO: recorded as a miss). */
 luz_status luz_trace_visibility_stats(luz_ctx* ctx, luz_frame* frame, const luz_tlas* tlas,

@@ -416,9 +416,9 @@ static luz_status launch_frame(luz_ctx* ctx, luz_batch* b, bool stats) {
     A.scenes = (uint32_t)b->frames.size();
     A.clear_items = b->clear_items;
     A.prologue_items = A.scenes + b->clear_items + b->tile_items;
-    A.C = make_vis_common(ctx, &ctl->rays);
+    A.C = make_vis_common(ctx, batch_tuning(ctx), &ctl->rays);
     A.stats = stats ? b->d_stats : nullptr;
-    const uint32_t grid = (uint32_t)ctx->sm_count * vis_tuning(ctx).ctas_per_sm;
+    const uint32_t grid = (uint32_t)ctx->sm_count * batch_tuning(ctx).ctas_per_sm;
     prof_begin(ctx, LUZ_KERNEL_BATCH_FRAME);
     if (stats) batch_frame_kernel<true><<<grid, kVisThreads, kFrameSmem, st>>>(A);
     else batch_frame_kernel<false><<<grid, kVisThreads, kFrameSmem, st>>>(A);
@@ -631,7 +631,7 @@ luz_status luz_batch_autotune(luz_ctx* ctx, luz_batch* b, uint32_t reps, luz_vis
     LUZ_CUDA(ctx, cudaEventCreate(&e0));
     LUZ_CUDA(ctx, cudaEventCreate(&e1));
     const uint32_t refills[] = {8, 16, 32}, steps[] = {16, 32, 64}, ctas[] = {2, 3, 4};
-    const uint32_t base_smem = vis_tuning(ctx).smem_nodes;
+    const uint32_t base_smem = batch_tuning(ctx).smem_nodes;
     VisTuning best{0, 0, 0, 0, 0};
     float best_t = 3.0e38f;
     for (uint32_t rf : refills)

@@ -85,12 +85,12 @@ luz_status ensure_scratch(luz_ctx* ctx, size_t bytes) {
 
 static void free_frame_buffers(luz_frame* f) {
     void* ptrs[] = {f->albedo, f->normal, f->material, f->emission, f->depth, f->light,
-                    f->primary_hit, f->hit_instance, f->gb_coarse, f->gb_fine, f->shadow_bits, f->ao_bits, f->ao, f->ao_denoised, f->signal,
+                    f->primary_hit, f->gb_coarse, f->gb_fine, f->shadow_bits, f->ao_bits, f->ao, f->ao_denoised, f->signal,
                     f->unshadowed, f->denoised, f->surf, f->surf_mat,
                     f->features, f->lin_depth, f->taa, f->taa_next, f->compose, f->hist, f->hist_state,
-                    f->block_counts, f->lit_count, f->dn_list, f->dn_count, f->d_upload, f->work_counter, f->d_textures,
-                    f->d_texels, f->d_shadow_lights, f->d_shadow_maps, f->rays_a, f->rays_b, f->rays_c, f->beams,
-                    f->beam_lists};
+                    f->block_counts, f->lit_count, f->dn_list, f->dn_count, f->d_upload, f->d_textures,
+                    f->d_texels, f->d_shadow_lights, f->d_shadow_maps, f->rays_a, f->rays_b, f->rays_c,
+                    f->patches, f->start_lists, f->cuts, f->active, f->vis_counters};
     for (void* p : ptrs)
         if (p) cudaFree(p);
     if (f->h_upload) cudaFreeHost(f->h_upload);
@@ -109,7 +109,7 @@ static luz_status reserve_upload(luz_ctx* ctx, luz_frame* f, uint32_t lights, ui
     auto region = [&](size_t n) { const size_t at = bytes; bytes += (n + 255) & ~(size_t)255; return at; };
     const size_t scene = region(sizeof(luz_scene)), light = region((size_t)nl * sizeof(luz_light)),
                  first = region((size_t)nl * 4), slot = region((size_t)ns * 4),
-                 model = region((size_t)nm * sizeof(luz_model)), skip = region(nm);
+                 vlight = region((size_t)ns * 4), model = region((size_t)nm * sizeof(luz_model)), skip = region(nm);
     // the old block stays in place until the new one is there
     if (!f->upload_done) LUZ_CUDA(ctx, cudaEventCreateWithFlags(&f->upload_done, cudaEventDisableTiming));
     LUZ_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
@@ -131,6 +131,7 @@ static luz_status reserve_upload(luz_ctx* ctx, luz_frame* f, uint32_t lights, ui
     f->d_lights = (luz_light*)(d + light);
     f->d_light_slot = (uint32_t*)(d + first);
     f->d_slot_table = (uint32_t*)(d + slot);
+    f->d_vlights = (uint32_t*)(d + vlight);
     f->d_models = (luz_model*)(d + model);
     f->d_model_skip = (uint8_t*)(d + skip);
     return LUZ_OK;
@@ -443,8 +444,6 @@ void luz_tlas_destroy(luz_tlas* t) {
     if (t->h_input) cudaFreeHost(t->h_input);
     if (t->morton) cudaFree(t->morton);
     if (t->order) cudaFree(t->order);
-    if (t->near) cudaFree(t->near);
-    if (t->leaf_of) cudaFree(t->leaf_of);
     if (t->tmp) cudaFree(t->tmp);
     if (t->input_copied) cudaEventDestroy(t->input_copied);
     delete t;
@@ -476,10 +475,9 @@ luz_status luz_tlas_memory(const luz_tlas* t, luz_memory* out) {
     out->nodes = m * 64;
     out->wide_nodes = m * 128;
     out->leaves = cap * sizeof(DevInstance);
-    // level table; per instance: shading record, input record, Morton code and order,
-    // near list (4 x uint4) and leaf index; build scratch
-    out->other = 66 * 4 + cap * (sizeof(DevShadeInstance) + sizeof(DevInstanceInput) + 8 + 4 * sizeof(uint4) + 4) +
-                 t->tmp_bytes;
+    // level table; per instance: shading record, input record, Morton code and order;
+    // build scratch
+    out->other = 66 * 4 + cap * (sizeof(DevShadeInstance) + sizeof(DevInstanceInput) + 8) + t->tmp_bytes;
     return LUZ_OK;
 }
 
@@ -507,7 +505,6 @@ luz_status luz_frame_create(luz_ctx* ctx, uint32_t width, uint32_t height, luz_f
     A((void**)&f->depth, P * 4);
     A((void**)&f->light, P * 16);
     A((void**)&f->primary_hit, P * 8);
-    A((void**)&f->hit_instance, P * 4);
     A((void**)&f->gb_coarse, (size_t)((width + 63) / 64) * ((height + 63) / 64) * 256 * 4);
     A((void**)&f->gb_fine, (size_t)((width + 7) / 8) * ((height + 7) / 8) * 16 * 4);
     A((void**)&f->ao, P * 4);
@@ -528,7 +525,6 @@ luz_status luz_frame_create(luz_ctx* ctx, uint32_t width, uint32_t height, luz_f
     A((void**)&f->surf_mat, P * 16);
     A((void**)&f->block_counts, (size_t)chunks * 4);
     A((void**)&f->lit_count, 4);
-    A((void**)&f->work_counter, 8);
     if (e != cudaSuccess) {
         free_frame_buffers(f);
         delete f;
@@ -594,11 +590,20 @@ static luz_status frame_upload_body(luz_ctx* ctx, luz_frame* f, const luz_scene*
     memcpy(host(f->d_scene), scene, sizeof(luz_scene));
     uint32_t* light_slot = (uint32_t*)host(f->d_light_slot);
     uint32_t* slot_table = (uint32_t*)host(f->d_slot_table);
-    uint32_t next = 0;
+    uint32_t* vlights = (uint32_t*)host(f->d_vlights);
+    uint32_t next = 0, vlight_count = 0, most = 1;
     for (uint32_t l = 0; l < light_count; ++l) {
         light_slot[l] = next;
         for (uint32_t k = 0, n = samples(l); k < n; ++k) slot_table[next++] = l | (k << 16);
+        // virtual lights: the samples of one light, in groups of up to four that share a shaft
+        for (uint32_t k = light_slot[l]; k < next; k += 4) {
+            const uint32_t n = std::min(next - k, 4u);
+            vlights[vlight_count++] = k | (n << 16);
+            most = std::max(most, n);
+        }
     }
+    f->vlight_count = vlight_count;
+    f->vlight_shift = most > 2 ? 2 : most - 1;
     if (light_count) memcpy(host(f->d_lights), lights, (size_t)light_count * sizeof(luz_light));
     if (model_count) memcpy(host(f->d_models), models, (size_t)model_count * sizeof(luz_model));
     uint8_t* skip = (uint8_t*)host(f->d_model_skip);

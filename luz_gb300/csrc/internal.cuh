@@ -33,10 +33,10 @@ constexpr int kStackSize = 128;
 //   f6 child[4] (int bits: >= 0 a 4-wide node, < 0 a leaf ~index, kEmptyChild), f7 0.
 constexpr int kNode4F4 = 8;
 
-// Items (rays) per visibility chunk: the ray generation pass writes one chunk of
-// 32-B ray records (4 GiB at most; a 1080p frame with 57 rays per pixel fits one
-// chunk even when every pixel is lit), the traversal kernel consumes it.
-constexpr uint32_t kRayChunk = 1u << 27;
+// Rays per visibility chunk (shadow, AO): ray generation writes the 48-B records of one
+// chunk at most, the traversal kernel consumes them. A 1080p frame of 41 lights and 16 AO
+// samples fits one chunk even when every pixel is lit and no ray is resolved early.
+constexpr uint32_t kRayChunk = 1u << 27, kAoChunk = 1u << 26;
 
 // One TLAS leaf, in sorted (leaf) order. 96 B, 16-B aligned for vector loads.
 // sphere: the BLAS's bounding sphere in object space, (centre, radius): the root box
@@ -125,7 +125,7 @@ struct luz_ctx {
     void* h_pinned = nullptr;
     size_t pinned_bytes = 0;
     int sm_count = 0;
-    int raygen_blocks = 0;                      // resident ray-generation blocks per SM (0: not queried)
+    int raygen_blocks = 0, cull_blocks = 0;   // resident blocks per SM (0: not queried)
     bool registered = false;                    // counted among the process's live contexts
     luz::VisTuning vis_tuning{0, 0, 0, 0, 0};   // set == 0: library defaults
     uint32_t debug_step_cap = 0;                // traversal steps per ray, 0 = the library's cap
@@ -168,8 +168,6 @@ struct luz_tlas {
     luz::DevInstanceInput* h_input = nullptr;     // pinned staging
     uint32_t* morton = nullptr;
     uint32_t* order = nullptr;
-    uint4* near = nullptr;               // per instance (input order): near list of short rays
-    uint32_t* leaf_of = nullptr;         // per instance (input order): its TLAS leaf
     uint32_t node_count = 0;
     cudaEvent_t input_copied = nullptr;           // h_input may be rewritten after this
     // build temporaries
@@ -188,7 +186,6 @@ struct luz_frame {
     float* depth = nullptr;         // F32
     float4* light = nullptr;        // RGBA32F
     uint2* primary_hit = nullptr;
-    uint32_t* hit_instance = nullptr;    // input index of the primary hit's instance (~0 = miss)
     uint32_t* gb_coarse = nullptr;       // G-buffer candidate leaves per 64x64 tile (count + 255)
     uint32_t* gb_fine = nullptr;         // and per 8x8 tile (count + 15)
     // visibility
@@ -241,15 +238,22 @@ struct luz_frame {
     luz::DevTexture* d_textures = nullptr;
     void* d_texels = nullptr;
     uint32_t texture_count = 0;
-    unsigned long long* work_counter = nullptr;
-    // generated shadow / AO rays of one chunk (structure of arrays, rays_cap each):
-    // (origin, tMax) and (direction, pixel); tMax = -inf marks an item with no ray
+    // virtual lights: up to four samples of one light each (first slot | samples << 16),
+    // and log2 of the most samples one of them has
+    uint32_t* d_vlights = nullptr;
+    uint32_t vlight_count = 0, vlight_shift = 0;
+    // of one chunk (shafts.cuh): patch bounds, start lists per (virtual light, patch) and
+    // per AO patch, the lists' cuts, the shadow groups to trace, and the ray records
+    // (RayOut, structure of arrays)
+    void* patches = nullptr;
+    uint32_t* start_lists = nullptr;
+    float4* cuts = nullptr;
+    uint4* active = nullptr;
     float4* rays_a = nullptr;
     float4* rays_b = nullptr;
-    uint32_t* rays_c = nullptr;          // own instance of a ray that starts at its near list
-    float4* beams = nullptr;             // per group of 32 items: origin ball, end-point ball
-    uint32_t* beam_lists = nullptr;      // per group of 32 items: count + up to 31 TLAS leaves
-    uint32_t rays_cap = 0;
+    uint4* rays_c = nullptr;
+    void* vis_counters = nullptr;         // VisCounters per chunk
+    uint32_t lists_cap = 0, pairs_cap = 0, records_cap = 0, chunks_cap = 0;
 };
 
 // ---------------------------------------------------------------- error plumbing

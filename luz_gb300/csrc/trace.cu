@@ -222,7 +222,6 @@ __global__ void __launch_bounds__(kGbTile * kGbTile, kGbMinBlocks) gbuffer_kerne
         G.emission[pix] = 0u;
         G.depth[pix] = 1.0f;
         G.primary_hit[pix] = make_uint2(0xFFFFFFFFu, 0xFFFFFFFFu);
-        G.hit_instance[pix] = 0xFFFFFFFFu;
         return;
     }
 
@@ -312,23 +311,26 @@ __global__ void __launch_bounds__(kGbTile * kGbTile, kGbMinBlocks) gbuffer_kerne
     G.emission[pix] = pack_unorm8(em[0], em[1], em[2], em[3]);
     G.depth[pix] = depth;
     G.primary_hit[pix] = make_uint2(h.custom, h.prim);
-    G.hit_instance[pix] = h.inst_input;
 }
 
 // ---------------------------------------------------------------- lit-pixel compaction
-// A pixel is lit when length(N) != 0 (light.frag:178). The list follows a tiled
-// order of the image — kLitTile x kLitTile pixel tiles in row order, pixels in row
-// order inside a tile — so the 32 rays a warp takes at once (32 neighbouring items of
-// one light) start from a compact patch of pixels rather than a 32-pixel row.
-// Chunks of 1024 positions of that order.
+// A pixel is lit when length(N) != 0 (light.frag:178). The list follows a tiled order
+// of the image, so that what takes consecutive entries works on a compact patch of
+// pixels: blocks of 32x32 pixels in row order (one block of the kernels each), their 4x4
+// tiles in Morton order, pixels in row order inside a tile. 32 entries are 8x4 pixels
+// (a patch of ray generation), 256 are 16x16.
 constexpr int kChunk = 1024;
-constexpr uint32_t kLitTile = 4;   // measured at 1080p: 4x4 3.85 ms, 8x8 3.88, 16x16 3.94, rows 4.24
+constexpr uint32_t kLitTile = 4, kLitBlock = 32;
+static_assert(kLitBlock * kLitBlock == kChunk, "a block of pixels per block of threads");
 
 // Pixel at position o of the tiled order, or ~0u past the image.
 __device__ __forceinline__ uint32_t tiled_pixel(uint32_t o, uint32_t width, uint32_t height) {
-    const uint32_t tiles_x = (width + kLitTile - 1) / kLitTile;
-    const uint32_t tile = o / (kLitTile * kLitTile), w = o % (kLitTile * kLitTile);
-    const uint32_t x = (tile % tiles_x) * kLitTile + w % kLitTile, y = (tile / tiles_x) * kLitTile + w / kLitTile;
+    const uint32_t blocks_x = (width + kLitBlock - 1) / kLitBlock;
+    const uint32_t block = o / kChunk, tile = (o / (kLitTile * kLitTile)) & 63u, w = o % (kLitTile * kLitTile);
+    const uint32_t tx = (tile & 1u) | ((tile >> 1) & 2u) | ((tile >> 2) & 4u);
+    const uint32_t ty = ((tile >> 1) & 1u) | ((tile >> 2) & 2u) | ((tile >> 3) & 4u);
+    const uint32_t x = (block % blocks_x) * kLitBlock + tx * kLitTile + w % kLitTile;
+    const uint32_t y = (block / blocks_x) * kLitBlock + ty * kLitTile + w / kLitTile;
     return (x < width && y < height) ? y * width + x : ~0u;
 }
 
@@ -461,7 +463,6 @@ luz_status make_gbuf_params(luz_ctx* ctx, luz_frame* f, const luz_tlas* t, GbufP
     G.emission = f->emission;
     G.depth = f->depth;
     G.primary_hit = f->primary_hit;
-    G.hit_instance = f->hit_instance;
     G.status = ctx->d_status;
     G.textures = f->d_textures;
     G.texture_count = f->texture_count;
@@ -497,9 +498,7 @@ luz_status launch_gbuffer(luz_ctx* ctx, luz_frame* f, const luz_tlas* t) {
 // Compaction of the lit pixels (length(N) != 0) of the normal plane into the
 // (fragPos, pixel), (N, x | y << 16) list that ray generation and the light pass read.
 uint32_t lit_chunks(uint32_t width, uint32_t height) {
-    const uint64_t positions = (uint64_t)((width + kLitTile - 1) / kLitTile) * ((height + kLitTile - 1) / kLitTile) *
-                               kLitTile * kLitTile;
-    return (uint32_t)((positions + kChunk - 1) / kChunk);
+    return ((width + kLitBlock - 1) / kLitBlock) * ((height + kLitBlock - 1) / kLitBlock);
 }
 
 luz_status launch_lit_compaction(luz_ctx* ctx, luz_frame* f) {

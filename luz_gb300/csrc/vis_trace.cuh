@@ -19,6 +19,7 @@ constexpr int kVisThreads = 256;
 constexpr int kSmemStack = 16;                      // shared-memory stack entries per lane
 constexpr int kLocalStack = kStackSize - kSmemStack;
 constexpr uint32_t kRayStepCap = 1u << 22;
+constexpr uint32_t kMinCharge = 8;                  // a cap below this many steps ends every ray at once
 
 // Ray state that traversal touches only when it enters or leaves a BLAS, tests a
 // triangle or finishes lives in shared memory, one 32-bit field per row of
@@ -36,10 +37,22 @@ enum ColdField : int {
     kWiX, kWiY, kWiZ,             // world inverse direction and origin offsets, restored on
     kWnX, kWnY, kWnZ,             // the way out of a BLAS
     kWfX, kWfY, kWfZ,
+    kList, kCut,                  // entries (below): the ray's start list, the cut of the entered BLAS
     kColdFields
 };
 constexpr size_t kColdBytes = (size_t)kColdFields * kVisThreads * 4;
 constexpr size_t kStackBytes = (size_t)kVisThreads * kSmemStack * 4;
+
+// Entries of a start list (visibility_kernel): a stacked TLAS leaf ~(kEntryFlag | k) is
+// leaf k of the ray's list, entered at its cut, a 4-wide node outside the BLAS whose
+// children are nodes and triangles of it; kCutNode is that node's index on the way in.
+constexpr uint32_t kEntryFlag = 0x40000000u;   // leaf indices stay below 2^24
+constexpr int kCutNode = 0x7FFFFFFF;
+struct Entries {
+    const uint32_t* lists;       // words per list: kEntryWords
+    const float4* cuts;
+};
+constexpr uint32_t kEntryWords = 64, kEntryCuts = 32;   // words 1..31 leaves, 32..62 cuts (index + 1, 0 none)
 
 // Hot per-lane state (registers).
 struct LaneRay {
@@ -140,6 +153,37 @@ __device__ __forceinline__ bool gen_ray(const SceneVis& S, const VisCommon& C, u
     return ok;
 }
 
+// What the AO samples of a pixel share: its coordinates and the blue-noise texel's values.
+struct AoPixel {
+    uint32_t x, y;
+    float r, g;
+};
+__device__ __forceinline__ AoPixel ao_pixel(const VisCommon& C, int sampler, uint32_t px, uint32_t py) {
+    AoPixel q{px, py, 0.f, 0.f};
+    if (sampler != LUZ_SAMPLER_STRATIFIED) {
+        const uint32_t w = __ldg(reinterpret_cast<const uint32_t*>(C.blue_noise) + (py % C.bn_size) * C.bn_size + px % C.bn_size);
+        q.r = (float)(w & 0xFFu) / 255.0f;
+        q.g = (float)((w >> 8) & 0xFFu) / 255.0f;
+    }
+    return q;
+}
+
+// AO sample s of a pixel: gen_ray's steps. False when there is no ray (a miss).
+__device__ __forceinline__ bool ao_gen(const SceneVis& S, const AoPixel& q, uint32_t s, V3 p, V3 N, V3 cam, V3& wo,
+                                       V3& wd) {
+    float rx, ry;
+    if (S.sampler == LUZ_SAMPLER_STRATIFIED) {
+        stratified_rg(q.x, q.y, (int)s, S.frame, 0u, &rx, &ry);
+    } else {
+        const float offs = kGoldenRatio * (float)(128 * (int)s + S.frame % 128);   // blue_noise_rg
+        rx = fract_(q.r + offs);
+        ry = fract_(q.g + offs);
+    }
+    ao_ray(p, N, cam, rx, ry, wo, wd);
+    return S.instance_count > 0 && finite3(wo) && finite3(wd) && S.ao_min <= S.ao_max &&
+           !(wd.x == 0.0f && wd.y == 0.0f && wd.z == 0.0f);
+}
+
 // Starts a lane on a generated ray: cold state in shared memory, hot state in
 // registers, traversal at the TLAS root.
 __device__ __forceinline__ void start_ray(LaneRay& r, const Cold& c, const SceneVis& S, V3 wo, V3 wd, float tmin,
@@ -205,12 +249,12 @@ __device__ __forceinline__ float4 node_load(const float4* p) {
 // ray (kRayStepCap unless a debug cap is set) is charged `steps` per call, so a ray
 // ends after at most step_cap + steps; a ray that reaches it ends unoccluded (shadow)
 // or as a miss (AO) and raises LUZ_DEV_TRAVERSAL_CAP.
-template <bool kStats, bool kStaged>
+template <bool kStats, bool kStaged, bool kEntries = false>
 __device__ __forceinline__ void run_steps(LaneRay& r, const Cold& c, bool& active, const float4* smem_tlas,
                                           uint32_t staged, const float4* tlas, const DevInstance* insts,
                                           uint32_t* s_stack, int* lstack, uint32_t steps, uint32_t step_cap,
-                                          uint32_t& err, TraceCounters& cnt) {
-    if (active && (r.budget += steps) > step_cap) {
+                                          uint32_t& err, TraceCounters& cnt, const Entries& en = Entries{}) {
+    if (active && (r.budget += steps) + (steps < kMinCharge ? kMinCharge - steps : 0u) > step_cap) {
         err |= LUZ_DEV_TRAVERSAL_CAP;
         finish_ray(c, active, false);
     }
@@ -223,6 +267,7 @@ __device__ __forceinline__ void run_steps(LaneRay& r, const Cold& c, bool& activ
             if (kStats) { if (r.in_blas) cnt.blas_nodes++; else cnt.tlas_nodes++; }
             const float4* np = kStaged ? (r.in_blas ? r.nb : ((uint32_t)r.node < staged ? smem_tlas : tlas)) : r.nb;
             np += (size_t)r.node * kNode4F4;
+            if (kEntries && r.node == kCutNode) np = en.cuts + (size_t)__float_as_uint(c[kCut]) * kNode4F4;
             const int sx = r.signs & 1, sy = (r.signs >> 1) & 1, sz = r.signs >> 2;
             const float4 nx = node_load<kStaged>(np + sx), fx = node_load<kStaged>(np + (sx ^ 1)),
                          ny = node_load<kStaged>(np + 2 + sy), fy = node_load<kStaged>(np + 3 - sy),
@@ -268,7 +313,18 @@ __device__ __forceinline__ void run_steps(LaneRay& r, const Cold& c, bool& activ
             // Instance leaf: entered unless its mask or BLAS is empty or the ray
             // segment provably misses the BLAS's bounding sphere.
             if (kStats) cnt.instances++;
-            const DevInstance* I = insts + (~r.node);
+            uint32_t leaf = (uint32_t)~r.node;
+            int first = 0;
+            if (kEntries && (leaf & kEntryFlag)) {
+                const uint32_t* e = en.lists + (size_t)__float_as_uint(c[kList]) * kEntryWords + (leaf & (kEntryCuts - 1u));
+                leaf = __ldg(e);
+                const uint32_t cut = __ldg(e + kEntryCuts - 1);
+                if (cut) {
+                    first = kCutNode;
+                    c[kCut] = __uint_as_float(cut - 1u);
+                }
+            }
+            const DevInstance* I = insts + leaf;
             const float4* wp = reinterpret_cast<const float4*>(I->w2o);
             uint4 meta = __ldg(reinterpret_cast<const uint4*>(&I->custom_index));
             float4 q0 = __ldg(wp), q1 = __ldg(wp + 1), q2 = __ldg(wp + 2), sph = __ldg(&I->sphere);
@@ -293,7 +349,7 @@ __device__ __forceinline__ void run_steps(LaneRay& r, const Cold& c, bool& activ
                 else { err |= LUZ_DEV_STACK_OVERFLOW; finished = true; }
                 ++r.sp;
                 r.in_blas = true;
-                r.node = 0;
+                r.node = first;
                 if (!finished) continue;
             }
         } else {

@@ -2,12 +2,17 @@
 // of a frame (light.frag:86-135) and writes the hit/miss bit planes; and its batched
 // form, one launch over the rays of many scenes.
 //
-// Work items are (slot, lit pixel) pairs, slot-major, so neighbouring items share a
-// light and lie in neighbouring pixels. Each lane holds one ray as an explicit
-// traversal state. After every few traversal steps the warp counts its idle lanes
-// with a ballot; when enough are idle, one lane takes that many items with a single
-// atomic and the idle lanes pick theirs by rank (popc of the lower lanes' ballot
-// bits), then generate their rays while the others keep traversing.
+// A frame's rays are first resolved in groups: shafts.cuh culls whole (light, patch)
+// groups of shadow rays, aocull.cuh AO rays above their patch's horizon. What is left is
+// generated on full warps, tested against the boxes its group's list starts at, and
+// written as compact records. The traversal kernel keeps one ray per lane as an explicit
+// state; after every few steps a warp counts its idle lanes with a ballot and, when enough
+// are idle, one lane takes that many records with a single atomic and the idle lanes pick
+// theirs by rank. 1080p two-level frame (64 x 81,920 triangles, 1024 instances, 41 lights,
+// 16 AO rays; 18.4 M rays to trace): ray generation and lists 0.59 -> 0.83 ms, traversal
+// 2.27 -> 1.03 ms (BLAS node visits 121 M -> 40 M, TLAS 7.8 M -> 1.6 M) against tracing
+// every ray from the leaves its 32 neighbours' capsule reaches; 4K, 4096 instances, 145
+// lights, 64 AO rays: 18.5 + 94.2 ms -> 27 + 50 ms.
 //
 // Traversal runs over 4-wide nodes (the even-depth collapse of the binary LBVH):
 // one step tests four child boxes, with the near and far planes picked per ray by
@@ -18,368 +23,97 @@
 // (world origin and direction, output bit, watertight shear) sits in shared memory,
 // which keeps the kernel at 64 registers and 4 CTAs per SM without spills.
 #include <algorithm>
-#include <cmath>
 #include <cstring>
 
+#include "aocull.cuh"
+#include "shafts.cuh"
 #include "vis_trace.cuh"
 
 namespace luz {
 
-// ---------------------------------------------------------------- near lists
-// A ray whose whole segment stays within `reach` of its own instance's box can only
-// hit instances whose boxes come within `reach` of that box: for such a ray the
-// traversal starts at its own TLAS leaf with the leaves of those of them whose boxes
-// its segment overlaps on its stack, in place of the TLAS root. Short rays (AO rays of
-// radius aoMax) then skip the TLAS levels above their own instance. Per instance
-// (input order) the record holds (leaf, count, near[0..1]), (near[2..5]), (box lo,
-// near[6]), (box hi, near[7]), near[] as input indices; count = ~0 when there are more
-// than kNearMax such instances or the box is empty or not finite. The result is that
-// of the full traversal: a hit at q on instance j needs box_j within
-// |q - o| + dist(o, box_i) of box_i and the segment to overlap box_j, and entering an
-// instance whose leaf box the full traversal would cull finds no hit either (boxes
-// are conservative).
-constexpr uint32_t kNearMax = 8;
-// Shadow-ray beams: groups of kBeamGroup consecutive items (lanes of a warp in ray
-// generation), lists of up to kBeamMax TLAS leaves.
-#ifndef LUZ_BEAM_SHIFT
-#define LUZ_BEAM_SHIFT 5
-#endif
-constexpr uint32_t kBeamShift = LUZ_BEAM_SHIFT;
-constexpr uint32_t kBeamGroup = 1u << kBeamShift;
-constexpr uint32_t kBeamMax = 31;             // list room: count + 31 leaves (128 B per group)
-constexpr uint32_t kBeamWords = kBeamMax + 1;
-// Leaves a list may hold before its group falls back to the TLAS root: 15 up to 2048
-// instances, 31 above. The traversal kernel is built for each cap (its start loop
-// reads that many): on the 1080p two-level frame the longer lists cost 0.5 % of the
-// traversal and 3 % of the list kernel, on the 4096-instance scene they take the TLAS
-// visits per traversed ray from 3.1 to 0.9.
-constexpr uint32_t kBeamCapSmall = 15, kBeamCapLarge = 31;
-inline uint32_t beam_cap(uint32_t instances) { return instances > 2048 ? kBeamCapLarge : kBeamCapSmall; }
-#ifndef LUZ_NEAR_REACH
-#define LUZ_NEAR_REACH 1.5f
-#endif
-constexpr uint32_t kNearFlag = 0x80000000u;   // rays_b.w: the ray starts at its near list
-constexpr uint32_t kNearLeafBits = 24;        // rays_c: own leaf | overlapped near[] bits << 24
-constexpr uint32_t kNearMaxInstances = 16384; // pairs tested per call: 2.7e8 at most
-
-__device__ __forceinline__ bool box_ok(float4 lo, float4 hi) {
-    return lo.x <= hi.x && lo.y <= hi.y && lo.z <= hi.z;   // false for empty or NaN boxes
-}
-__device__ __forceinline__ float box_mag(float4 lo, float4 hi) {
-    return fmaxf(fmaxf(fmaxf(fabsf(lo.x), fabsf(lo.y)), fmaxf(fabsf(lo.z), fabsf(hi.x))),
-                 fmaxf(fabsf(hi.y), fabsf(hi.z)));
-}
-
-// One block per instance i: the instances (other than i, with valid boxes) whose box
-// distance to box_i is at most reach, grown by 2^-10 relative and 2^-18 of the boxes'
-// coordinate magnitude (the rounding of the distances here and in near_start), in
-// index order.
-__global__ void __launch_bounds__(256) near_list_kernel(const float4* __restrict__ inst_box,
-                                                        const uint32_t* __restrict__ leaf_of, uint32_t n,
-                                                        float reach, uint4* __restrict__ near) {
-    __shared__ uint32_t s_warp[8];
-    __shared__ uint32_t s_list[kNearMax];
-    const uint32_t i = blockIdx.x, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const float4 lo = inst_box[2 * i], hi = inst_box[2 * i + 1];
-    const bool valid = box_ok(lo, hi);
-    const float mi = box_mag(lo, hi);
-    uint32_t total = 0;
-    for (uint32_t base = 0; valid && base < n; base += blockDim.x) {
-        const uint32_t j = base + tid;
-        bool nb = false;
-        if (j < n && j != i) {
-            const float4 lj = inst_box[2 * j], hj = inst_box[2 * j + 1];
-            if (box_ok(lj, hj)) {
-                const float dx = fmaxf(fmaxf(lj.x - hi.x, lo.x - hj.x), 0.0f);
-                const float dy = fmaxf(fmaxf(lj.y - hi.y, lo.y - hj.y), 0.0f);
-                const float dz = fmaxf(fmaxf(lj.z - hi.z, lo.z - hj.z), 0.0f);
-                const float d2 = dx * dx + dy * dy + dz * dz;
-                const float lim = reach * (1.0f + 0x1p-10f) + 0x1p-18f * (mi + box_mag(lj, hj));
-                nb = d2 <= lim * lim;
+// Ray generation of the shadow rays: warps take up to kRaygenTake consecutive active groups
+// (shafts.cuh) at a time, fewer when there are not enough for two rounds of the grid; lane
+// = pixel of the group's patch, over the samples of its virtual light. Separated from
+// traversal so the long arithmetic of light.frag's sampling and the tests against the
+// group's list, the same leaves for all lanes, run on full warps. A ray that enters none
+// of the leaves is unoccluded and leaves no record: bound by issue (0.28 ms for the 5.2 M
+// samples that the shafts of a 1080p frame leave; the traversal that found the same on
+// partly filled warps took 0.28 ms longer).
+constexpr uint32_t kRaygenTake = 4;
+__global__ void __launch_bounds__(256, 3) shadow_raygen_kernel(SceneVis S, VisCommon C, Entries E,
+                                                               const uint4* __restrict__ active,
+                                                               const uint32_t* __restrict__ active_count,
+                                                               uint32_t* tickets, RayOut R) {
+    __shared__ float s_ray[8][kStageWords][kStageRays];
+    const uint32_t full = 0xFFFFFFFFu;
+    const uint32_t lit = *S.lit_count, lane = threadIdx.x & 31, n = *active_count;
+    RayStage stage{s_ray[threadIdx.x >> 5], 0u};
+    const uint32_t take = max(min(n / (2u * gridDim.x * (blockDim.x >> 5)), kRaygenTake), 1u);
+    for (;;) {
+        uint32_t g0 = 0;
+        if (lane == 0) g0 = atomicAdd(tickets, take);
+        g0 = __shfl_sync(full, g0, 0);
+        if (g0 >= n) break;
+        for (uint32_t g = g0; g < min(g0 + take, n); ++g) {
+            const uint4 a = __ldg(active + g);
+            const uint32_t first = a.y & 0xFFFFu, samples = a.y >> 16, j = a.z * kPatch + lane;
+            const uint32_t* list = E.lists + (size_t)a.x * kEntryWords;
+            const uint32_t cnt = __ldg(list);
+            for (uint32_t s = 0; s < samples; ++s) {
+                V3 wo{0.f, 0.f, 0.f}, wd{0.f, 0.f, 1.f};
+                float tmin = 0.f, tmax = 0.f;
+                uint32_t* out;
+                bool record_hit = true;
+                uint32_t pix = 0;
+                const bool ok = j < lit && gen_ray(S, C, first + s, j, wo, wd, tmin, tmax, out, record_hit, pix);
+                uint32_t mask = cnt == kListAll ? kFromRoot : 0u;
+                if (cnt != kListAll && __any_sync(full, ok)) {
+                    LaneRay r;
+                    r.tmin = tmin;
+                    r.tmax = tmax;
+                    r.idir = safe_inv(wd);
+                    set_origin(r, wo);
+                    near_planes(r);
+                    for (uint32_t k = 0; k < cnt; ++k) {
+                        const uint32_t leaf = __ldg(list + 1 + k), cut = __ldg(list + kEntryCuts + k);
+                        if (ok && leaf_overlaps(r, S.leaf_box, leaf) &&
+                            leaf_enters(S.instances + leaf, cut ? E.cuts + (size_t)(cut - 1u) * kNode4F4 : nullptr, wo, wd,
+                                        tmin, tmax))
+                            mask |= 1u << k;
+                    }
+                }
+                stage_rays(stage, R, lane, ok && mask != 0u, wo, tmax, wd, pix, a.x, first + s, mask);
             }
         }
-        const uint32_t bal = __ballot_sync(0xFFFFFFFFu, nb);
-        if (lane == 0) s_warp[warp] = __popc(bal);
-        __syncthreads();
-        uint32_t off = total, sum = 0;
-        for (uint32_t w = 0; w < blockDim.x / 32; ++w) {
-            if (w < warp) off += s_warp[w];
-            sum += s_warp[w];
-        }
-        const uint32_t pos = off + __popc(bal & ((1u << lane) - 1u));
-        if (nb && pos < kNearMax) s_list[pos] = j;
-        total += sum;
-        __syncthreads();
     }
-    if (tid == 0) {
-        const uint32_t cnt = valid && total <= kNearMax ? total : 0xFFFFFFFFu;
-        uint32_t l[kNearMax];
-#pragma unroll
-        for (uint32_t k = 0; k < kNearMax; ++k) l[k] = k < cnt ? s_list[k] : 0u;
-        near[4 * i] = make_uint4(leaf_of[i], cnt, l[0], l[1]);
-        near[4 * i + 1] = make_uint4(l[2], l[3], l[4], l[5]);
-        near[4 * i + 2] = make_uint4(__float_as_uint(lo.x), __float_as_uint(lo.y), __float_as_uint(lo.z), l[6]);
-        near[4 * i + 3] = make_uint4(__float_as_uint(hi.x), __float_as_uint(hi.y), __float_as_uint(hi.z), l[7]);
-    }
+    if (stage.n) stage_flush(stage, R, lane);
 }
 
-// Whether the segment o + t d, t in [tmin, tmax], may overlap the box: the slab
-// interval with the near / far distances widened by 2^-12 relative (their rounding;
-// the inverse direction is that of safe_inv, finite).
-__device__ __forceinline__ bool segment_overlaps(V3 o, V3 id, float tmin, float tmax, float4 lo, float4 hi) {
-    const float x0 = (lo.x - o.x) * id.x, x1 = (hi.x - o.x) * id.x;
-    const float y0 = (lo.y - o.y) * id.y, y1 = (hi.y - o.y) * id.y;
-    const float z0 = (lo.z - o.z) * id.z, z1 = (hi.z - o.z) * id.z;
-    const float tn = fmaxf(fmaxf(fminf(x0, x1), fminf(y0, y1)), fmaxf(fminf(z0, z1), tmin));
-    const float tf = fminf(fminf(fmaxf(x0, x1), fmaxf(y0, y1)), fminf(fmaxf(z0, z1), tmax));
-    return tn * (1.0f - 0x1p-12f) <= tf + fabsf(tf) * 0x1p-12f;
-}
-
-// The start of a ray of pixel pix at its near list, or ~0: the own instance's TLAS
-// leaf | the bits of the near instances whose boxes the segment may overlap << 24.
-// The segment's length plus the origin's distance to the box of the pixel's
-// primary-hit instance, grown by 2^-10 relative and 2^-18 of the coordinates'
-// magnitude, must stay within S.near_reach.
-__device__ __forceinline__ uint32_t near_start(const SceneVis& S, V3 o, V3 d, float tmin, float tmax, uint32_t pix) {
-    const float len = tmax * sqrtf(d.x * d.x + d.y * d.y + d.z * d.z);
-    if (!(len <= S.near_reach)) return ~0u;
-    const uint32_t inst = __ldg(S.hit_instance + pix);
-    if (inst >= S.instance_count) return ~0u;
-    const uint4* rec = S.near + 4 * (size_t)inst;
-    const uint4 u0 = __ldg(rec);
-    if (u0.y > kNearMax) return ~0u;
-    const uint4 u2 = __ldg(rec + 2), u3 = __ldg(rec + 3);
-    const float4 lo = make_float4(__uint_as_float(u2.x), __uint_as_float(u2.y), __uint_as_float(u2.z), 0.f),
-                 hi = make_float4(__uint_as_float(u3.x), __uint_as_float(u3.y), __uint_as_float(u3.z), 0.f);
-    if (!box_ok(lo, hi)) return ~0u;
-    const float ex = fmaxf(fmaxf(lo.x - o.x, o.x - hi.x), 0.0f);
-    const float ey = fmaxf(fmaxf(lo.y - o.y, o.y - hi.y), 0.0f);
-    const float ez = fmaxf(fmaxf(lo.z - o.z, o.z - hi.z), 0.0f);
-    const float m = fmaxf(box_mag(lo, hi), fmaxf(fmaxf(fabsf(o.x), fabsf(o.y)), fabsf(o.z)));
-    const float r = (sqrtf(ex * ex + ey * ey + ez * ez) + len) * (1.0f + 0x1p-10f) + 0x1p-18f * m;
-    if (!(r <= S.near_reach)) return ~0u;
-    uint32_t bits = 0;
-    if (u0.y > 0) {
-        const uint4 u1 = __ldg(rec + 1);
-        const uint32_t l[kNearMax] = {u0.z, u0.w, u1.x, u1.y, u1.z, u1.w, u2.w, u3.w};
-        const V3 id = safe_inv(d);
-#pragma unroll
-        for (uint32_t k = 0; k < kNearMax; ++k) {
-            if (k >= u0.y) break;
-            const uint4* nr = S.near + 4 * (size_t)l[k];
-            const uint4 a = __ldg(nr + 2), b = __ldg(nr + 3);
-            const float4 nlo = make_float4(__uint_as_float(a.x), __uint_as_float(a.y), __uint_as_float(a.z), 0.f),
-                         nhi = make_float4(__uint_as_float(b.x), __uint_as_float(b.y), __uint_as_float(b.z), 0.f);
-            if (segment_overlaps(o, id, tmin, tmax, nlo, nhi)) bits |= 1u << k;
-        }
-    }
-    return u0.x | (bits << kNearLeafBits);
-}
-
-// Ray generation pass of one chunk: items [k0, k0 + chunk) of the frame's
-// (slot, lit pixel) list, slot-major, one record per item in structure-of-arrays
-// form: rays_a = (origin, tMax), rays_b = (direction, pixel). An item with no ray
-// gets tMax = -inf (its AO miss is recorded here) and no rays_b entry. Separated from traversal so the
-// long arithmetic of light.frag's sampling runs on full warps, not on the few idle
-// lanes of a traversing warp. Also resets the traversal's work counter.
-__global__ void __launch_bounds__(256, 5) raygen_kernel(SceneVis S, VisCommon C, unsigned long long k0,
-                                                     unsigned long long chunk, float4* __restrict__ rays_a,
-                                                     float4* __restrict__ rays_b, uint32_t* __restrict__ rays_c,
-                                                     float4* __restrict__ beams) {
-    if (blockIdx.x == 0 && threadIdx.x == 0) *C.work_counter = 0ull;
+// The rays of a frame that have something to trace (the counting trace's figure: shafts
+// and horizons resolve most of them without a record).
+__global__ void __launch_bounds__(256) count_rays_kernel(SceneVis S, VisCommon C, unsigned long long* stats) {
     const uint32_t lit = *S.lit_count;
     const unsigned long long total = (unsigned long long)lit * (S.shadow_slots + S.ao_samples);
-    if (k0 >= total) return;
-    const unsigned long long end = min(total, k0 + chunk);
-    const uint32_t stride = gridDim.x * blockDim.x, lane = threadIdx.x & 31;
-    const unsigned long long shadow_items = (unsigned long long)lit * S.shadow_slots;
-    const float ninf = __int_as_float(0xff800000);
-    // (slot, j) of the thread's first item by one division, then stepped by the stride.
-    // The loop runs while any lane of the warp has an item (the beam reductions below
-    // take the whole warp): a warp's 32 items are consecutive and 32-aligned.
-    unsigned long long item = k0 + blockIdx.x * blockDim.x + threadIdx.x;
-    uint32_t slot = (uint32_t)(item / lit), j = (uint32_t)(item - (unsigned long long)slot * lit);
-    const uint32_t step_slot = stride / lit, step_j = stride - step_slot * lit;
-    for (; item - lane < end; item += stride) {
-        const bool live = item < end;
-        V3 wo{0.f, 0.f, 0.f}, wd{0.f, 0.f, 0.f};
-        float tmin = 0.f, tmax = 0.f;
+    uint32_t n = 0;
+    for (unsigned long long i = blockIdx.x * (unsigned long long)blockDim.x + threadIdx.x; i < total;
+         i += (unsigned long long)gridDim.x * blockDim.x) {
+        V3 wo, wd;
+        float tmin, tmax;
         uint32_t* out;
-        bool record_hit = false;
+        bool record_hit;
         uint32_t pix;
-        const bool ok = live && gen_ray(S, C, slot, j, wo, wd, tmin, tmax, out, record_hit, pix);
-        if (live) rays_a[item - k0] = make_float4(wo.x, wo.y, wo.z, ok ? tmax : ninf);
-        if (ok) {   // read only for rays
-            uint32_t tag = pix;
-            if (S.near_reach > 0.0f && !record_hit) {   // AO rays (shadow rays have their beams)
-                const uint32_t start = near_start(S, wo, wd, tmin, tmax, pix);
-                if (start != ~0u) {
-                    tag |= kNearFlag;
-                    rays_c[item - k0] = start;
-                }
-            }
-            rays_b[item - k0] = make_float4(wd.x, wd.y, wd.z, __uint_as_float(tag));
-        }
-        if (beams && item - lane < shadow_items) {
-            // Beam of a group of kBeamGroup items (lanes): balls around the origins and
-            // around the end points of its traced shadow rays, centred on the first such ray.
-            const bool sh = ok && record_hit;
-            const uint32_t first = lane & ~(kBeamGroup - 1u);
-            const uint32_t m = (__ballot_sync(0xFFFFFFFFu, sh) >> first) & (0xFFFFFFFFu >> (32 - kBeamGroup));
-            const unsigned long long g = (item - k0) >> kBeamShift;
-            if (m == 0u) {
-                if (lane == first) beams[2 * g] = make_float4(0.f, 0.f, 0.f, -1.0f);   // no traced shadow ray
-            }
-            {
-                const int src = (int)first + (m ? __ffs(m) - 1 : 0);
-                const V3 e = V3{wo.x + wd.x * tmax, wo.y + wd.y * tmax, wo.z + wd.z * tmax};
-                const V3 co = V3{__shfl_sync(0xFFFFFFFFu, wo.x, src), __shfl_sync(0xFFFFFFFFu, wo.y, src),
-                                 __shfl_sync(0xFFFFFFFFu, wo.z, src)};
-                const V3 ce = V3{__shfl_sync(0xFFFFFFFFu, e.x, src), __shfl_sync(0xFFFFFFFFu, e.y, src),
-                                 __shfl_sync(0xFFFFFFFFu, e.z, src)};
-                float ro = sh ? length(wo - co) : 0.0f, re = sh ? length(e - ce) : 0.0f;
-                uint32_t bad = sh && !(finite3(e) && ro <= 3.0e38f && re <= 3.0e38f) ? 1u : 0u;
-#pragma unroll
-                for (int o = kBeamGroup / 2; o >= 1; o >>= 1) {
-                    ro = fmaxf(ro, __shfl_xor_sync(0xFFFFFFFFu, ro, o));
-                    re = fmaxf(re, __shfl_xor_sync(0xFFFFFFFFu, re, o));
-                    bad |= __shfl_xor_sync(0xFFFFFFFFu, bad, o);
-                }
-                if (lane == first && m != 0u) {   // r_o = +inf: an end point not finite
-                    beams[2 * g] = make_float4(co.x, co.y, co.z, bad ? __int_as_float(0x7f800000) : ro);
-                    beams[2 * g + 1] = make_float4(ce.x, ce.y, ce.z, re);
-                }
-            }
-        }
-        slot += step_slot;
-        j += step_j;
-        if (j >= lit) { j -= lit; ++slot; }
+        const uint32_t slot = (uint32_t)(i / lit);
+        n += gen_ray(S, C, slot, (uint32_t)(i - (unsigned long long)slot * lit), wo, wd, tmin, tmax, out, record_hit, pix);
     }
+    n = __reduce_add_sync(0xFFFFFFFFu, n);
+    if ((threadIdx.x & 31) == 0) atomicAdd(stats, (unsigned long long)n);
 }
 
-// ---------------------------------------------------------------- beam lists
-// The traced shadow rays of a group of kBeamGroup consecutive items (one light sample,
-// neighbouring lit pixels in tile order) start in a ball B_o around their origins and
-// end in a ball B_e around their end points, so each lies in the convex hull of the
-// two balls, itself inside the capsule of radius max(r_o, r_e) around the segment
-// between the centres. A leaf whose box, grown by that radius, the segment misses
-// cannot be hit by any ray of the group: the group's rays traverse only the leaves the
-// capsule reaches (nearest first), or the TLAS from its root when there are more than
-// S.beam_cap of them. The radius is grown by 2^-10 relative and 2^-16 of the centres'
-// magnitude, above the rounding of the centres, radii, end points and hit points.
-constexpr uint32_t kBeamAll = 0xFFFFFFFFu;    // count: traverse from the TLAS root
-constexpr int kBeamStack = 48;                 // overflow: the list falls back to the TLAS root
-
-__global__ void __launch_bounds__(256) beam_list_kernel(SceneVis S, unsigned long long k0, unsigned long long chunk,
-                                                        const float4* __restrict__ beams, uint32_t* __restrict__ lists) {
-    const uint32_t lit = *S.lit_count;
-    const unsigned long long shadow_items = (unsigned long long)lit * S.shadow_slots;
-    if (k0 >= shadow_items) return;
-    const unsigned long long n = min(chunk, shadow_items - k0);
-    const unsigned long long g = (unsigned long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (g >= (n + kBeamGroup - 1) / kBeamGroup) return;
-    uint32_t* list = lists + kBeamWords * g;
-    const float4 bo = beams[2 * g], be = beams[2 * g + 1];
-    if (bo.w < 0.0f) return;   // no traced shadow ray in the group: the list is never read
-    const V3 o = V3{bo.x, bo.y, bo.z}, d = V3{be.x - bo.x, be.y - bo.y, be.z - bo.z};
-    const float r0 = fmaxf(bo.w, be.w);
-    const float mag = ((fabsf(bo.x) + fabsf(bo.y)) + (fabsf(bo.z) + fabsf(be.x))) + (fabsf(be.y) + fabsf(be.z));
-    const float r = r0 * (1.0f + 0x1p-10f) + 0x1p-16f * (mag + r0);
-    if (!(r <= 3.0e38f) || !finite3(o) || !finite3(d)) {
-        list[0] = kBeamAll;
-        return;
-    }
-    const V3 id = safe_inv(d);
-    uint32_t out[kBeamMax];
-    uint32_t cnt = 0;
-    int stack[kBeamStack];
-    int sp = 0, node = 0;
-    bool done = false;
-    for (uint32_t iter = 0; iter < kTraversalCap; ++iter) {
-        const float4* np = S.tlas_nodes + (size_t)node * kNode4F4;
-        const float4 lx = __ldg(np), hx = __ldg(np + 1), ly = __ldg(np + 2), hy = __ldg(np + 3), lz = __ldg(np + 4),
-                     hz = __ldg(np + 5), cf = __ldg(np + 6);
-        const float L[3][4] = {{lx.x, lx.y, lx.z, lx.w}, {ly.x, ly.y, ly.z, ly.w}, {lz.x, lz.y, lz.z, lz.w}};
-        const float H[3][4] = {{hx.x, hx.y, hx.z, hx.w}, {hy.x, hy.y, hy.z, hy.w}, {hz.x, hz.y, hz.z, hz.w}};
-        const int ch[4] = {__float_as_int(cf.x), __float_as_int(cf.y), __float_as_int(cf.z), __float_as_int(cf.w)};
-        float tk[4];
-        bool hk[4];
-#pragma unroll
-        for (int k = 0; k < 4; ++k) {
-            const float ax0 = (L[0][k] - r - o.x) * id.x, ax1 = (H[0][k] + r - o.x) * id.x;
-            const float ay0 = (L[1][k] - r - o.y) * id.y, ay1 = (H[1][k] + r - o.y) * id.y;
-            const float az0 = (L[2][k] - r - o.z) * id.z, az1 = (H[2][k] + r - o.z) * id.z;
-            const float tn = fmaxf(fmaxf(fminf(ax0, ax1), fminf(ay0, ay1)), fmaxf(fminf(az0, az1), 0.0f));
-            const float tf = fminf(fminf(fmaxf(ax0, ax1), fmaxf(ay0, ay1)), fminf(fmaxf(az0, az1), 1.0f));
-            hk[k] = ch[k] != kEmptyChild && tn <= tf + fabsf(tf) * 0x1p-12f;
-            tk[k] = tn;
-        }
-        // Hit children by entry distance (misses last): leaves appended nearest first,
-        // internal nodes pushed farthest first (the nearest is visited next).
-        int ck[4];
-#pragma unroll
-        for (int k = 0; k < 4; ++k) {
-            ck[k] = hk[k] ? ch[k] : kEmptyChild;
-            if (!hk[k]) tk[k] = __int_as_float(0x7f800000);
-        }
-#define LUZ_BX(a, b)                                                                          \
-        if (tk[b] < tk[a]) {                                                                  \
-            const float t_ = tk[a]; tk[a] = tk[b]; tk[b] = t_;                               \
-            const int c_ = ck[a]; ck[a] = ck[b]; ck[b] = c_;                                  \
-        }
-        LUZ_BX(0, 1) LUZ_BX(2, 3) LUZ_BX(0, 2) LUZ_BX(1, 3) LUZ_BX(1, 2)
-#undef LUZ_BX
-        bool overflow = false;
-#pragma unroll
-        for (int q = 0; q < 4; ++q) {
-            if (ck[q] < 0 && ck[q] != kEmptyChild) {
-                if (cnt < kBeamMax) out[cnt] = (uint32_t)~ck[q];
-                ++cnt;
-            }
-        }
-#pragma unroll
-        for (int q = 3; q >= 0; --q) {
-            if (ck[q] >= 0) {
-                if (sp < kBeamStack) stack[sp++] = ck[q];
-                else overflow = true;
-            }
-        }
-        if (overflow || cnt > S.beam_cap) {
-            list[0] = kBeamAll;
-            return;
-        }
-        if (sp == 0) {
-            done = true;
-            break;
-        }
-        node = stack[--sp];
-    }
-    if (!done) {   // the step cap ran out
-        list[0] = kBeamAll;
-        return;
-    }
-    list[0] = cnt;
-    for (uint32_t k = 0; k < cnt; ++k) list[1 + k] = out[k];
-}
-
-// The slab test of a TLAS leaf's box for the lane's (world-space) ray, as a 4-wide
-// node applies it to the slot holding that leaf.
-__device__ __forceinline__ bool leaf_overlaps(const LaneRay& r, const float4* __restrict__ leaf_box, uint32_t leaf) {
-    const float4 lo = __ldg(leaf_box + 2 * (size_t)leaf), hi = __ldg(leaf_box + 2 * (size_t)leaf + 1);
-    const bool sx = r.signs & 1, sy = (r.signs >> 1) & 1, sz = (r.signs >> 2) & 1;
-    float tn;
-    return slab_ordered(sx ? hi.x : lo.x, sx ? lo.x : hi.x, sy ? hi.y : lo.y, sy ? lo.y : hi.y, sz ? hi.z : lo.z,
-                        sz ? lo.z : hi.z, r, tn);
-}
-
-// Traversal of one chunk of generated rays (one scene; the TLAS top may be staged
-// in shared memory). Shared memory: staged TLAS nodes, then the stacks, then the
-// cold ray state.
-template <bool kStats, bool kStaged, uint32_t kCap>
+// Traversal of one chunk's ray records (one scene; the TLAS top may be staged in shared
+// memory). Shared memory: staged TLAS nodes, then the stacks, then the cold ray state.
+template <bool kStats, bool kStaged>
 __global__ void __launch_bounds__(kVisThreads, LUZ_VIS_MIN_BLOCKS)
-visibility_kernel(SceneVis S, VisCommon C, unsigned long long k0, unsigned long long chunk,
-                  const float4* __restrict__ rays_a, const float4* __restrict__ rays_b,
-                  const uint32_t* __restrict__ rays_c, unsigned long long* stats) {
+visibility_kernel(SceneVis S, VisCommon C, Entries E, RayOut R, unsigned long long* stats) {
     extern __shared__ float4 smem[];
     const uint32_t staged = min(S.tlas_node_count, C.smem_nodes);
     for (uint32_t i = threadIdx.x; i < staged * kNode4F4; i += blockDim.x) smem[i] = __ldg(S.tlas_nodes + i);
@@ -390,13 +124,11 @@ visibility_kernel(SceneVis S, VisCommon C, unsigned long long k0, unsigned long 
     int lstack[kLocalStack];
     __syncthreads();
     const uint32_t full = 0xFFFFFFFFu, lt_mask = (1u << lane) - 1u;
-    const uint32_t lit = *S.lit_count;
-    const unsigned long long total = (unsigned long long)lit * (S.shadow_slots + S.ao_samples);
-    const unsigned long long n = total > k0 ? min(chunk, total - k0) : 0ull;   // items of this chunk
-    uint32_t err = 0, rays = 0;
+    const uint32_t n = *R.count;
+    uint32_t err = 0;
     TraceCounters cnt{0, 0, 0, 0};
     LaneRay r{};
-    bool active = false, exhausted = false;
+    bool active = false, exhausted = n == 0;
     for (;;) {
         uint32_t idle = __ballot_sync(full, !active);
         if (!exhausted && __popc(idle) >= (int)C.refill) {
@@ -405,95 +137,39 @@ visibility_kernel(SceneVis S, VisCommon C, unsigned long long k0, unsigned long 
             if (lane == leader) base = atomicAdd(C.work_counter, (unsigned long long)__popc(idle));
             base = __shfl_sync(full, base, leader);
             if (base + __popc(idle) >= n) exhausted = true;
-            // Slot of the warp's first item, by one division in the leader; the
-            // lanes step from it (their items follow in rank order).
-            uint32_t slot0 = 0, j0 = 0;
-            if (lane == leader && base < n) {
-                const unsigned long long g = k0 + base;
-                slot0 = (uint32_t)(g / lit);
-                j0 = (uint32_t)(g - (unsigned long long)slot0 * lit);
-            }
-            slot0 = __shfl_sync(full, slot0, leader);
-            j0 = __shfl_sync(full, j0, leader);
-            if (!active) {
-                const uint32_t rank = __popc(idle & lt_mask);
-                const unsigned long long local = base + rank;
-                if (local < n) {
-                    uint32_t slot = slot0, j = j0 + rank;
-                    while (j >= lit) { j -= lit; ++slot; }
-                    const float4 a = __ldg(rays_a + local);
-                    const bool record_hit = slot < S.shadow_slots;
-                    const float tmin = record_hit ? 0.001f : S.ao_min;
-                    if (tmin <= a.w) {
-                        const float4 b = __ldg(rays_b + local);
-                        if (kStats) ++rays;
-                        const uint32_t tag = __float_as_uint(b.w), pix = tag & ~kNearFlag;
-                        uint32_t* out = record_hit ? S.shadow_bits + (size_t)slot * S.words + (pix >> 5)
-                                                   : S.ao_bits + (size_t)(slot - S.shadow_slots) * S.words + (pix >> 5);
-                        start_ray(r, c, S, V3{a.x, a.y, a.z}, V3{b.x, b.y, b.z}, tmin, a.w, out, record_hit, pix);
-                        bool go = true;
-                        if (record_hit && S.beam_lists) {
-                            // A shadow ray starts at its group's beam list unless that ran over.
-                            const uint4* bl = reinterpret_cast<const uint4*>(S.beam_lists + kBeamWords * (local >> kBeamShift));
-                            const uint4 u0 = __ldg(bl);
-                            if (u0.x != kBeamAll) {
-                                // The list's leaves whose boxes this ray's slab test keeps
-                                // (the test the TLAS node holding the leaf would apply),
-                                // the nearest first: it starts at the nearest, the others
-                                // stacked; with none it ends unoccluded.
-                                int sp = 0, cur = 0;
-#pragma unroll
-                                for (int q = (int)(kCap + 1) / 4 - 1; q >= 0; --q) {
-                                    if (4u * (uint32_t)q > u0.x) continue;
-                                    const uint4 u = q == 0 ? u0 : __ldg(bl + q);
-                                    const uint32_t l[4] = {u.x, u.y, u.z, u.w};
-#pragma unroll
-                                    for (int k = 3; k >= 0; --k) {
-                                        const uint32_t w = 4u * (uint32_t)q + (uint32_t)k;
-                                        if (w >= 1 && w <= u0.x && leaf_overlaps(r, S.leaf_box, l[k])) {
-                                            if (cur) {   // past the shared part (kCap 31): local
-                                                if (kCap < kSmemStack || sp < kSmemStack) s_stack[sp * 32] = (uint32_t)cur;
-                                                else lstack[sp - kSmemStack] = cur;
-                                                ++sp;
-                                            }
-                                            cur = ~(int)l[k];
-                                        }
-                                    }
-                                }
-                                go = cur != 0;
-                                r.node = cur;
-                                r.sp = sp;
-                            }
-                        }
-                        if (tag & kNearFlag) {
-                            // Start at the own instance's leaf, the overlapped near
-                            // instances' leaves stacked.
-                            const uint32_t start = __ldg(rays_c + local), leaf = start & ((1u << kNearLeafBits) - 1u);
-                            r.node = ~(int)leaf;
-                            if (start >> kNearLeafBits) {
-                                const uint4* rec = S.near + 4 * (size_t)__ldg(S.order + leaf);
-                                const uint4 u0 = __ldg(rec), u1 = __ldg(rec + 1);
-                                const uint32_t l[kNearMax] = {u0.z, u0.w, u1.x, u1.y, u1.z, u1.w,
-                                                              __ldg(rec + 2).w, __ldg(rec + 3).w};
-                                int sp = 0;
-#pragma unroll
-                                for (uint32_t k = 0; k < kNearMax; ++k)
-                                    if ((start >> (kNearLeafBits + k)) & 1u) s_stack[(sp++) * 32] = ~__ldg(S.leaf_of + l[k]);
-                                r.sp = sp;
-                            }
-                        }
-                        active = go;
+            const unsigned long long k = base + __popc(idle & lt_mask);
+            if (!active && k < n) {
+                const float4 a = __ldg(R.a + k), b = __ldg(R.b + k);
+                const uint4 q = __ldg(R.c + k);
+                const bool sh = q.y < S.shadow_slots;
+                const uint32_t pix = __float_as_uint(b.w);
+                start_ray(r, c, S, V3{a.x, a.y, a.z}, V3{b.x, b.y, b.z}, sh ? 0.001f : S.ao_min, a.w,
+                          (sh ? S.shadow_bits + (size_t)q.y * S.words : S.ao_bits + (size_t)(q.y - S.shadow_slots) * S.words) +
+                              (pix >> 5),
+                          sh, pix);
+                active = true;
+                if (q.z != kFromRoot) {
+                    // The leaves its tests left, the nearest first: it starts at the nearest,
+                    // the others stacked.
+                    c[kList] = __uint_as_float(q.x);
+                    r.node = ~(int)(kEntryFlag | (uint32_t)__ffs(q.z));
+                    for (uint32_t m = q.z & (q.z - 1u); m;) {
+                        const uint32_t top = 31u - __clz(m);
+                        m ^= 1u << top;
+                        const int e = ~(int)(kEntryFlag | (top + 1u));
+                        if (r.sp < kSmemStack) s_stack[r.sp * 32] = (uint32_t)e;
+                        else lstack[r.sp - kSmemStack] = e;
+                        ++r.sp;
                     }
                 }
             }
         }
         if (exhausted && __ballot_sync(full, active) == 0) break;
-        run_steps<kStats, kStaged>(r, c, active, smem, staged, S.tlas_nodes, S.instances, s_stack, lstack, C.steps,
-                                   C.step_cap, err,
-                                   cnt);
+        run_steps<kStats, kStaged, true>(r, c, active, smem, staged, S.tlas_nodes, S.instances, s_stack, lstack,
+                                         C.steps, C.step_cap, err, cnt, E);
     }
     if (err) atomicOr(C.status, err);
-    if (kStats) flush_stats(stats, rays, cnt);
+    if (kStats) flush_stats(stats, 0u, cnt);
 }
 
 // Many scenes in one launch: item g belongs to the scene s with
@@ -561,14 +237,15 @@ __global__ void batch_offsets_kernel(const SceneVis* scenes, uint32_t n, unsigne
 }
 
 // ---------------------------------------------------------------- host side
-// Defaults: the best shape of a sweep on the 1080p two-level scene (smem nodes
-// {0,128} x refill {2,4,8,16,24} x steps {8,16,32} x CTAs/SM {3,4}, kernel compiled
-// for 4 CTAs/SM; steps 16 until the near and beam lists made the rays shorter, then
-// refill {16,24,32} x steps {8,16,24}: 8 steps, 2.28 vs 2.33 ms). Staging the TLAS top
-// in shared memory did not pay: L1 holds it.
-static const VisTuning g_tuning{0, 24, 8, 4, 1};
+// Default launch shapes. Batches generate their rays in the traversal: 24 idle lanes to a
+// refill, 8 steps between checks. A single scene's records hold only rays that enter a BLAS,
+// which are short: a check every 2 steps and a refill at 20 idle lanes (1080p two-level frame,
+// refill {4..28} x steps {2,4,8,16}: 0.98 ms against 1.03 at 24 / 8, 4K scene 49.9 against
+// 52.3). Staging the TLAS top in shared memory does not pay: L1 holds it.
+static const VisTuning g_tuning{0, 20, 2, 4, 1}, g_batch_tuning{0, 24, 8, 4, 1};
 
 const VisTuning& vis_tuning(const luz_ctx* ctx) { return ctx->vis_tuning.set ? ctx->vis_tuning : g_tuning; }
+const VisTuning& batch_tuning(const luz_ctx* ctx) { return ctx->vis_tuning.set ? ctx->vis_tuning : g_batch_tuning; }
 
 SceneVis make_scene_vis(const luz_frame* f, const luz_tlas* t, int frame_index) {
     SceneVis S;
@@ -594,19 +271,11 @@ SceneVis make_scene_vis(const luz_frame* f, const luz_tlas* t, int frame_index) 
     S.shadow_bits = f->shadow_bits;
     S.ao_bits = f->ao_bits;
     S.cull = f->shadow_cull ? 1 : 0;
-    S.near = t->near;
-    S.order = t->order;
-    S.leaf_of = t->leaf_of;
-    S.hit_instance = f->hit_instance;
-    S.near_reach = 0.0f;
-    S.beam_lists = nullptr;
     S.leaf_box = nullptr;
-    S.beam_cap = 0;
     return S;
 }
 
-VisCommon make_vis_common(luz_ctx* ctx, unsigned long long* work_counter) {
-    const VisTuning& tu = vis_tuning(ctx);
+VisCommon make_vis_common(luz_ctx* ctx, const VisTuning& tu, unsigned long long* work_counter) {
     VisCommon C;
     C.blue_noise = ctx->d_blue_noise;
     C.bn_size = ctx->blue_noise_size;
@@ -629,17 +298,50 @@ luz_status clear_visibility(luz_ctx* ctx, luz_frame* f) {
 }
 
 
-// The traversal of one chunk, built for the scene's beam-list cap.
-template <bool kStats, uint32_t kCap>
-static void launch_traversal(bool staged, uint32_t grid, size_t smem, cudaStream_t st, const SceneVis& S,
-                             const VisCommon& C, unsigned long long k0, unsigned long long chunk, const luz_frame* f,
-                             unsigned long long* d_stats) {
-    if (staged)
-        visibility_kernel<kStats, true, kCap><<<grid, 256, smem, st>>>(S, C, k0, chunk, f->rays_a, f->rays_b,
-                                                                       f->rays_c, d_stats);
-    else
-        visibility_kernel<kStats, false, kCap><<<grid, 256, smem, st>>>(S, C, k0, chunk, f->rays_a, f->rays_b,
-                                                                        f->rays_c, d_stats);
+// Sizes of a frame's traces: every pixel lit and no ray resolved before the traversal.
+struct VisSizes {
+    uint32_t patches, supers;
+    uint32_t pairs, ao_patches;      // per chunk
+    uint32_t records;                // per chunk
+    uint32_t chunks;
+};
+
+static luz_status ensure_vis_buffers(luz_ctx* ctx, luz_frame* f, const VisSizes& z) {
+    if (f->patches && z.pairs + z.ao_patches <= f->lists_cap && z.pairs <= f->pairs_cap &&
+        z.records <= f->records_cap && z.chunks <= f->chunks_cap)
+        return LUZ_OK;
+    LUZ_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
+    auto again = [&](auto*& p, size_t bytes) -> cudaError_t {
+        cudaFree(p);
+        p = nullptr;
+        return bytes ? cudaMalloc(&p, bytes) : cudaSuccess;
+    };
+    if (!f->patches)   // the patches, then their blocks
+        LUZ_CUDA(ctx, cudaMalloc(&f->patches, ((size_t)z.patches + z.supers) * sizeof(PatchRec)));
+    if (z.pairs + z.ao_patches > f->lists_cap) {
+        f->lists_cap = 0;
+        LUZ_CUDA(ctx, again(f->start_lists, ((size_t)z.pairs + z.ao_patches) * kEntryWords * 4));
+        f->lists_cap = z.pairs + z.ao_patches;
+    }
+    if (z.pairs > f->pairs_cap) {
+        f->pairs_cap = 0;
+        LUZ_CUDA(ctx, again(f->cuts, (size_t)z.pairs * kCutsPerPair * kNode4F4 * sizeof(float4)));
+        LUZ_CUDA(ctx, again(f->active, (size_t)z.pairs * sizeof(uint4)));
+        f->pairs_cap = z.pairs;
+    }
+    if (z.records > f->records_cap) {
+        f->records_cap = 0;
+        LUZ_CUDA(ctx, again(f->rays_a, (size_t)z.records * sizeof(float4)));
+        LUZ_CUDA(ctx, again(f->rays_b, (size_t)z.records * sizeof(float4)));
+        LUZ_CUDA(ctx, again(f->rays_c, (size_t)z.records * sizeof(uint4)));
+        f->records_cap = z.records;
+    }
+    if (z.chunks > f->chunks_cap) {
+        f->chunks_cap = 0;
+        LUZ_CUDA(ctx, again(f->vis_counters, (size_t)z.chunks * sizeof(VisCounters)));
+        f->chunks_cap = z.chunks;
+    }
+    return LUZ_OK;
 }
 
 luz_status launch_visibility(luz_ctx* ctx, luz_frame* f, const luz_tlas* t, int frame_index,
@@ -650,96 +352,100 @@ luz_status launch_visibility(luz_ctx* ctx, luz_frame* f, const luz_tlas* t, int 
     if (f->shadow_slots + f->ao_samples == 0) return LUZ_OK;
     cudaStream_t st = ctx->stream;
     SceneVis S = make_scene_vis(f, t, frame_index);
-    VisCommon C = make_vis_common(ctx, f->work_counter);
     const VisTuning& tu = vis_tuning(ctx);
+    VisCommon C = make_vis_common(ctx, tu, nullptr);
     uint32_t staged = std::min<uint32_t>(S.tlas_node_count, tu.smem_nodes);
     size_t smem = (size_t)staged * kNode4F4 * 16 + kStackBytes + kColdBytes;
     static DeviceSetup setup;   // the traversal kernels' shared-memory limit
     s = device_setup(setup, setup_generation(), smem, [&]() -> luz_status {
-        const void* fns[8] = {(const void*)visibility_kernel<false, false, kBeamCapSmall>,
-                              (const void*)visibility_kernel<true, false, kBeamCapSmall>,
-                              (const void*)visibility_kernel<false, true, kBeamCapSmall>,
-                              (const void*)visibility_kernel<true, true, kBeamCapSmall>,
-                              (const void*)visibility_kernel<false, false, kBeamCapLarge>,
-                              (const void*)visibility_kernel<true, false, kBeamCapLarge>,
-                              (const void*)visibility_kernel<false, true, kBeamCapLarge>,
-                              (const void*)visibility_kernel<true, true, kBeamCapLarge>};
+        const void* fns[4] = {(const void*)visibility_kernel<false, false>, (const void*)visibility_kernel<true, false>,
+                              (const void*)visibility_kernel<false, true>, (const void*)visibility_kernel<true, true>};
         for (const void* fn : fns)
             LUZ_CUDA(ctx, cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
         return LUZ_OK;
     });
     if (s != LUZ_OK) return s;
     uint32_t grid = (uint32_t)ctx->sm_count * tu.ctas_per_sm;
+    // Chunks over the largest possible counts; what lies past the frame's actual counts
+    // returns at once on the device. Without instances no shadow ray has anything to hit.
+    VisSizes z{};
+    z.patches = (f->pixels + kPatch - 1) / kPatch;
+    z.supers = (z.patches + kSuper - 1) / kSuper;
+    const uint32_t shift = f->vlight_shift;
+    const unsigned long long max_pairs = t->count > 0 ? (unsigned long long)z.supers * kSuper * f->vlight_count : 0ull;
+    z.pairs = (uint32_t)std::min<unsigned long long>(max_pairs, (kRayChunk / kPatch) >> shift);
+    if (f->ao_samples) z.ao_patches = std::min(z.patches, std::max(kAoChunk / (kPatch * f->ao_samples), 1u));
+    z.records = ((z.pairs * kPatch) << shift) + z.ao_patches * kPatch * f->ao_samples;
+    const uint32_t shadow_chunks = z.pairs ? (uint32_t)((max_pairs + z.pairs - 1) / z.pairs) : 0u;
+    const uint32_t ao_chunks = z.ao_patches ? (z.patches + z.ao_patches - 1) / z.ao_patches : 0u;
+    z.chunks = std::max(shadow_chunks, ao_chunks);
     if (d_stats) LUZ_CUDA(ctx, cudaMemsetAsync(d_stats, 0, 5 * sizeof(unsigned long long), st));
-    // Chunks of at most rays_cap items over the largest possible ray count (every
-    // pixel lit); a chunk past the frame's actual count returns at once on the device.
-    const unsigned long long max_items = (unsigned long long)f->pixels * (f->shadow_slots + f->ao_samples);
-    const uint32_t need = (uint32_t)std::min<unsigned long long>(max_items, kRayChunk);
-    if (need > f->rays_cap) {   // first trace of this frame shape: allocate the ray records
-        LUZ_CUDA(ctx, cudaStreamSynchronize(st));
-        cudaFree(f->rays_a);
-        cudaFree(f->rays_b);
-        cudaFree(f->rays_c);
-        cudaFree(f->beams);
-        cudaFree(f->beam_lists);
-        f->rays_a = f->rays_b = nullptr;
-        f->rays_c = f->beam_lists = nullptr;
-        f->beams = nullptr;
-        f->rays_cap = 0;
-        const size_t groups = ((size_t)need + kBeamGroup - 1) / kBeamGroup;
-        LUZ_CUDA(ctx, cudaMalloc(&f->rays_a, (size_t)need * sizeof(float4)));
-        LUZ_CUDA(ctx, cudaMalloc(&f->rays_b, (size_t)need * sizeof(float4)));
-        LUZ_CUDA(ctx, cudaMalloc(&f->rays_c, (size_t)need * sizeof(uint32_t)));
-        LUZ_CUDA(ctx, cudaMalloc(&f->beams, groups * 2 * sizeof(float4)));
-        LUZ_CUDA(ctx, cudaMalloc(&f->beam_lists, groups * kBeamWords * sizeof(uint32_t)));
-        f->rays_cap = need;
+    if (z.chunks == 0) return LUZ_OK;
+    if ((s = ensure_vis_buffers(ctx, f, z)) != LUZ_OK) return s;
+    VisCounters* counters = (VisCounters*)f->vis_counters;
+    if (!shadow_chunks) LUZ_CUDA(ctx, cudaMemsetAsync(counters, 0, (size_t)z.chunks * sizeof(VisCounters), st));
+    if (t->count) S.leaf_box = tlas_leaf_boxes(t);
+    const uint32_t cap = list_cap(t->count);
+    if (ctx->raygen_blocks == 0) {   // resident blocks per SM: the persistent grids are one wave
+        int a = 0, b = 0;
+        LUZ_CUDA(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&a, cull_kernel<true, false>, kCullThreads, 0));
+        LUZ_CUDA(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, shadow_raygen_kernel, 256, 0));
+        ctx->cull_blocks = std::max(a, 1);
+        ctx->raygen_blocks = std::max(b, 1);
     }
-    const unsigned long long chunk = std::min<unsigned long long>(max_items, f->rays_cap);
-    // Near lists of this TLAS for the AO rays that stay within LUZ_NEAR_REACH AO radii
-    // of their own instance's box. The list kernel tests every pair of instances, so
-    // larger TLASes (above kNearMaxInstances) start their AO rays at the root.
-    const float reach = LUZ_NEAR_REACH * f->h_scene.ao_max;
-    if (t->count > 0 && t->count <= kNearMaxInstances && reach > 0.0f && std::isfinite(reach)) {
-        near_list_kernel<<<t->count, 256, 0, st>>>(tlas_instance_boxes(t), t->leaf_of, t->count, reach, t->near);
-        LUZ_LAUNCHED(ctx, "near_list_kernel");
-        S.near_reach = reach;
+    const uint32_t sms = (uint32_t)ctx->sm_count;
+    const Entries entries{f->start_lists, f->cuts};
+    prof_begin(ctx, LUZ_KERNEL_RAYGEN);
+    PatchRec* patches = (PatchRec*)f->patches;
+    if (shadow_chunks) {
+        patch_kernel<<<std::min(z.supers, sms * 8), kSuper * 32, 0, st>>>(S, patches, patches + z.patches, counters,
+                                                                          z.chunks);
+        LUZ_LAUNCHED(ctx, "patch_kernel");
     }
-    const bool beam = t->count > 0 && f->shadow_slots > 0;
-    if (beam) {
-        S.beam_lists = f->beam_lists;
-        S.leaf_box = tlas_leaf_boxes(t);
+    if (d_stats) {
+        count_rays_kernel<<<sms * 4, 256, 0, st>>>(S, C, d_stats);
+        LUZ_LAUNCHED(ctx, "count_rays_kernel");
     }
-    S.beam_cap = beam_cap(t->count);
-    if (ctx->raygen_blocks == 0) {   // resident 256-thread blocks per SM: the grid is one wave
-        int blocks = 0;
-        LUZ_CUDA(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks, raygen_kernel, 256, 0));
-        ctx->raygen_blocks = std::max(blocks, 1);
-    }
-    const int raygen_blocks = ctx->raygen_blocks;
-    for (unsigned long long k0 = 0; k0 < max_items; k0 += chunk) {
-        prof_begin(ctx, LUZ_KERNEL_RAYGEN);
-        raygen_kernel<<<(uint32_t)(ctx->sm_count * raygen_blocks), 256, 0, st>>>(S, C, k0, chunk, f->rays_a,
-                                                                                  f->rays_b, f->rays_c,
-                                                                                  beam ? f->beams : nullptr);
-        LUZ_LAUNCHED(ctx, "raygen_kernel");
-        if (beam) {   // timed with ray generation
-            const unsigned long long groups = (chunk + kBeamGroup - 1) / kBeamGroup;
-            beam_list_kernel<<<(uint32_t)((groups + 255) / 256), 256, 0, st>>>(S, k0, chunk, f->beams, f->beam_lists);
-            LUZ_LAUNCHED(ctx, "beam_list_kernel");
+    for (uint32_t k = 0; k < z.chunks; ++k) {
+        if (k) prof_begin(ctx, LUZ_KERNEL_RAYGEN);
+        VisCounters* n = counters + k;
+        C.work_counter = &n->traversed;
+        const RayOut R{f->rays_a, f->rays_b, f->rays_c, &n->records};
+        const bool shadow = k < shadow_chunks, ao = k < ao_chunks;
+        const ShaftOut A{patches, patches + z.patches, f->d_vlights, f->vlight_count, (unsigned long long)k * z.pairs,
+                         shadow ? z.pairs : 0u, cap, f->start_lists, f->cuts, f->active, &n->groups};
+        const AoOut O{k * z.ao_patches, ao ? std::min(z.ao_patches, z.patches - k * z.ao_patches) : 0u, cap,
+                      f->ao_samples < kAoMinSamples ? 0u : std::min(kAoStepsPerSample * f->ao_samples, kAoSteps),
+                      f->start_lists + (size_t)z.pairs * kEntryWords, z.pairs, R};
+        const uint32_t shaft_work = A.cap / kSuper, max_grid = sms * ctx->cull_blocks;
+        auto cull_grid = [&](uint32_t warps) { return std::min((warps + kCullWarps - 1) / kCullWarps, max_grid); };
+        if (shadow && ao && f->pixels <= kCullTogether) {
+            cull_kernel<true, true><<<cull_grid(shaft_work + O.patches), kCullThreads, 0, st>>>(S, C, A, O, n->cull_tickets);
+            LUZ_LAUNCHED(ctx, "cull_kernel");
+        } else {
+            if (shadow) {
+                cull_kernel<false, true><<<cull_grid(shaft_work), kCullThreads, 0, st>>>(S, C, A, O, n->cull_tickets);
+                LUZ_LAUNCHED(ctx, "cull_kernel<shadow>");
+            }
+            if (ao) {
+                cull_kernel<true, false><<<cull_grid(O.patches), kCullThreads, 0, st>>>(S, C, A, O, n->cull_tickets + 1);
+                LUZ_LAUNCHED(ctx, "cull_kernel<ao>");
+            }
+        }
+        if (shadow) {
+            shadow_raygen_kernel<<<std::min((z.pairs + 7) / 8, sms * ctx->raygen_blocks), 256, 0, st>>>(
+                S, C, entries, f->active, &n->groups, &n->raygen_tickets, R);
+            LUZ_LAUNCHED(ctx, "shadow_raygen_kernel");
         }
         prof_end(ctx);
         if (d_stats) {
-            if (S.beam_cap == kBeamCapLarge)
-                launch_traversal<true, kBeamCapLarge>(staged, grid, smem, st, S, C, k0, chunk, f, d_stats);
-            else
-                launch_traversal<true, kBeamCapSmall>(staged, grid, smem, st, S, C, k0, chunk, f, d_stats);
+            if (staged) visibility_kernel<true, true><<<grid, 256, smem, st>>>(S, C, entries, R, d_stats);
+            else visibility_kernel<true, false><<<grid, 256, smem, st>>>(S, C, entries, R, d_stats);
             LUZ_LAUNCHED(ctx, "visibility_kernel<stats>");
         } else {
             prof_begin(ctx, LUZ_KERNEL_TRAVERSAL);
-            if (S.beam_cap == kBeamCapLarge)
-                launch_traversal<false, kBeamCapLarge>(staged, grid, smem, st, S, C, k0, chunk, f, nullptr);
-            else
-                launch_traversal<false, kBeamCapSmall>(staged, grid, smem, st, S, C, k0, chunk, f, nullptr);
+            if (staged) visibility_kernel<false, true><<<grid, 256, smem, st>>>(S, C, entries, R, nullptr);
+            else visibility_kernel<false, false><<<grid, 256, smem, st>>>(S, C, entries, R, nullptr);
             prof_end(ctx);
             LUZ_LAUNCHED(ctx, "visibility_kernel");
         }
@@ -754,8 +460,8 @@ luz_status launch_visibility_batch(luz_ctx* ctx, const SceneVis* d_scenes, uint3
     batch_offsets_kernel<<<1, 32, 0, st>>>(d_scenes, n, d_offsets);
     LUZ_LAUNCHED(ctx, "batch_offsets_kernel");
     LUZ_CUDA(ctx, cudaMemsetAsync(work_counter, 0, 8, st));
-    VisCommon C = make_vis_common(ctx, work_counter);
-    const VisTuning& tu = vis_tuning(ctx);
+    const VisTuning& tu = batch_tuning(ctx);
+    VisCommon C = make_vis_common(ctx, tu, work_counter);
     size_t smem = kStackBytes + kColdBytes;
     uint32_t grid = (uint32_t)ctx->sm_count * tu.ctas_per_sm;
     if (d_stats) {

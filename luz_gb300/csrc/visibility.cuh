@@ -22,17 +22,7 @@ struct SceneVis {
     uint32_t width, words;
     uint32_t* shadow_bits;
     uint32_t* ao_bits;
-    // Short rays (near lists, visibility_kernel only; near_reach = 0 disables them)
-    const uint4* near;
-    const uint32_t* order;      // TLAS leaf -> instance input index
-    const uint32_t* leaf_of;    // instance input index -> TLAS leaf
-    const uint32_t* hit_instance;
-    float near_reach;
-    // Shadow-ray beam lists (visibility_kernel only; null disables them): per group of
-    // 32 items, count + 7 TLAS leaves
-    const uint32_t* beam_lists;
-    const float4* leaf_box;      // TLAS leaf boxes (lo, hi), leaf order
-    uint32_t beam_cap;           // leaves a beam list may hold before it falls back
+    const float4* leaf_box;      // TLAS leaf boxes (lo, hi), leaf order (visibility_kernel only)
 };
 
 struct VisCommon {
@@ -44,14 +34,14 @@ struct VisCommon {
     uint32_t step_cap;        // traversal steps per ray before it is ended (LUZ_DEV_TRAVERSAL_CAP)
 };
 
-// The context's visibility launch shape (the library defaults until one is set).
+// The context's visibility launch shape (the library defaults until one is set), of a
+// single scene's traces and of batches.
 const VisTuning& vis_tuning(const luz_ctx* ctx);
+const VisTuning& batch_tuning(const luz_ctx* ctx);
 // Launch-independent inputs of the visibility kernels (blue noise, status word, shape).
-VisCommon make_vis_common(luz_ctx* ctx, unsigned long long* work_counter);
+VisCommon make_vis_common(luz_ctx* ctx, const VisTuning& tu, unsigned long long* work_counter);
 SceneVis make_scene_vis(const luz_frame* f, const luz_tlas* t, int frame_index);
-// World boxes of the last TLAS build's instances (input order, lo / hi float4 pairs)
-// and its leaf boxes (leaf order).
-const float4* tlas_instance_boxes(const luz_tlas* t);
+// Boxes of the last TLAS build's leaves (leaf order, lo / hi float4 pairs).
 const float4* tlas_leaf_boxes(const luz_tlas* t);
 luz_status clear_visibility(luz_ctx* ctx, luz_frame* f);
 luz_status launch_visibility_batch(luz_ctx* ctx, const SceneVis* d_scenes, uint32_t n,
