@@ -36,10 +36,7 @@ constexpr int pW1 = 0;
 constexpr int pW2 = pW1 + 64 * sW1;
 constexpr int pW3 = pW2 + 64 * sW;
 constexpr int pW4 = pW3 + 64 * sW;
-constexpr int pW2T = pW4 + 56 * sW;     // transposed copies for the backward pass: [in][out]
-constexpr int pW3T = pW2T + 64 * sW;
-constexpr int pW4T = pW3T + 64 * sW;
-constexpr int pEnd = pW4T + 64 * sW;
+constexpr int pEnd = pW4 + 56 * sW;
 constexpr int kBias = 64 + 64 + 64 + 56;   // b1 | b2 | b3 | b4 (padded)
 
 __device__ __forceinline__ uint32_t pack2(float lo, float hi) {
@@ -63,7 +60,7 @@ struct FeatParams {
     float4* denoised4; // if set: the same for the filtered plane
     float4* signal;    // read at lit pixels (written by the split pass), zeroed at background pixels
     float4* unshadowed;
-    uint32_t* list;    // if set: lit pixels appended (x | y << 16), row-major within a block
+    uint32_t* list;    // if set: lit pixels appended (x | y << 16), a 16x16 block at a time
     uint32_t* list_count;
 };
 
@@ -74,12 +71,14 @@ __constant__ float c_lin_lut[256];   // pow(i/255, 2.2)
 __global__ void __launch_bounds__(256) features_kernel(FeatParams F) {
     __shared__ uint32_t s_warp[8];
     __shared__ uint32_t s_base;
-    const uint32_t pix = blockIdx.x * blockDim.x + threadIdx.x;
-    const uint32_t x = pix % F.width, y = pix / F.width;
-    const bool inside = pix < F.width * F.height;
+    // a block is 16x16 pixels: the list's entries, and so the denoiser's tiles, are compact
+    const uint32_t blocks_x = (F.width + 15) / 16;
+    const uint32_t x = (blockIdx.x % blocks_x) * 16 + (threadIdx.x & 15), y = (blockIdx.x / blocks_x) * 16 + (threadIdx.x >> 4);
+    const uint32_t pix = y * F.width + x;
+    const bool inside = x < F.width && y < F.height;
     float4 n = inside ? F.normal[pix] : make_float4(0.f, 0.f, 0.f, 0.f);
     const bool lit = inside && !(length(V3{n.x, n.y, n.z}) == 0.0f);
-    if (F.list) {   // block-aggregated append, in pixel order within the block
+    if (F.list) {   // block-aggregated append, in row order within the block
         const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
         const uint32_t mask = __ballot_sync(0xFFFFFFFFu, lit);
         if (lane == 0) s_warp[warp] = __popc(mask);
@@ -127,7 +126,49 @@ __global__ void __launch_bounds__(256) features_kernel(FeatParams F) {
 struct ImageGeom {
     uint32_t width, height, pixels;   // one image
     uint32_t images;
+    uint32_t tiles_x, tiles;          // 16x8-pixel tiles per row and image; tiles_x 0: runs of 128 pixels
 };
+
+// The 128-pixel tiles of the network kernels: 16x8 pixels, whose 7x7 windows overlap in
+// 22x14 pixels (10 KB of S and U, against 30 KB for a run of a row: the difference between
+// staying in L1 and not beside the operands), unless the images' edges would waste more
+// than an eighth of the tiles' pixels.
+// (Inference leaves out tiles of background: 2 x 720p, a third background, 252 -> 200 us.)
+static ImageGeom image_geom(uint32_t width, uint32_t height, uint32_t images) {
+    ImageGeom g{width, height, width * height, images, (width + 15) / 16, 0};
+    g.tiles = g.tiles_x * ((height + 7) / 8);
+    if ((uint64_t)g.tiles * 128 * 8 > (uint64_t)g.pixels * 9) {
+        g.tiles_x = 0;
+        g.tiles = 0;
+    }
+    return g;
+}
+static uint32_t tile_count(const ImageGeom& g) {
+    return g.tiles_x ? g.tiles * g.images : (uint32_t)(((uint64_t)g.pixels * g.images + 127) / 128);
+}
+
+// Pixel `row` of tile `tile`: its image, place and index over all images; false past an edge.
+__device__ __forceinline__ bool tile_pixel(const ImageGeom& G, uint32_t tile, uint32_t row, uint32_t& img, int& x, int& y,
+                                           uint32_t& gp) {
+    if (G.tiles_x) {
+        img = tile / G.tiles;
+        const uint32_t t = tile - img * G.tiles, ty = t / G.tiles_x;
+        x = (int)((t - ty * G.tiles_x) * 16u + (row & 15u));
+        y = (int)(ty * 8u + (row >> 4));
+        const bool in = img < G.images && x < (int)G.width && y < (int)G.height;
+        if (!in) { img = 0; x = 0; y = 0; }
+        gp = img * G.pixels + (uint32_t)y * G.width + (uint32_t)x;
+        return in;
+    }
+    gp = tile * 128u + row;
+    const bool in = gp < G.pixels * G.images;
+    if (!in) gp = 0;
+    img = gp / G.pixels;
+    const uint32_t local = gp - img * G.pixels;
+    x = (int)(local % G.width);
+    y = (int)(local / G.width);
+    return in;
+}
 
 // Depth of a neighbour relative to the centre, (d_q - d_p) / d_p clamped to [-1, 1],
 // from the centre's reciprocal.
@@ -139,16 +180,6 @@ __device__ __forceinline__ float relative_depth(float dq, float dc, float inv_dc
 // neighbour receives direct light in that channel: the pixel's own U is 0 then too).
 __device__ __forceinline__ float filtered_ratio(float ws, float wu) {
     return wu > 0.0f ? fminf(fmaxf(ws / wu, 0.0f), 1.0f) : 1.0f;
-}
-
-// Tap k of the 7x7 filter around pixel (x, y) of image img (image-clamped); zeros when
-// !ok or k >= 49.
-__device__ __forceinline__ float4 signal_tap(const float4* __restrict__ sig, const ImageGeom& G, bool ok,
-                                             uint32_t img, int x, int y, int k) {
-    if (!ok || k >= 49) return make_float4(0.f, 0.f, 0.f, 0.f);
-    const int qx = min(max(x + k % 7 - 3, 0), (int)G.width - 1);
-    const int qy = min(max(y + k / 7 - 3, 0), (int)G.height - 1);
-    return __ldg(sig + img * G.pixels + (uint32_t)qy * G.width + (uint32_t)qx);
 }
 
 // ---------------------------------------------------------------- inference
@@ -166,6 +197,7 @@ struct InferParams {
     // only the listed pixels are written
     const uint32_t* list;
     const uint32_t* list_count;
+    uint32_t tiles;          // without a list: tiles of the images
 };
 
 // ---------------------------------------------------------------- inference on tcgen05
@@ -247,6 +279,14 @@ __device__ __forceinline__ void group_sync(uint32_t group) {
     asm volatile("bar.sync %0, 128;" :: "r"(group + 1u) : "memory");
 }
 
+// Whether any thread of the warpgroup has p set (a barrier of the group as well).
+__device__ __forceinline__ bool group_any(uint32_t group, bool p) {
+    uint32_t r;
+    asm volatile("{\n\t.reg .pred q, s;\n\tsetp.ne.b32 q, %2, 0;\n\tbarrier.red.or.pred s, %1, 128, q;\n\t"
+                 "selp.u32 %0, 1, 0, s;\n\t}\n" : "=r"(r) : "r"(group + 1u), "r"(p ? 1u : 0u) : "memory");
+    return r != 0u;
+}
+
 // Issues a layer from the group's first thread after the group's shared-memory writes
 // and accumulator reads, commits it to the group's mbarrier, and every thread waits
 // (bounded) for the products. A thread whose wait runs out raises the status and waits
@@ -317,11 +357,49 @@ __device__ __forceinline__ float exp2_approx(float x) {
     return r;
 }
 
+// Index of tap k of the 7x7 window around (x, y). kInterior: every tap is inside the image
+// (rows addressed directly); otherwise clamped.
+template <bool kInterior>
+struct TapAt {
+    uint32_t rows[7];
+    int qx[7];
+    __device__ __forceinline__ TapAt(uint32_t base, int x, int y, const ImageGeom& G) {
+#pragma unroll
+        for (int d = 0; d < 7; ++d) {
+            if (kInterior) {
+                rows[d] = base + (uint32_t)(y + d - 3) * G.width + (uint32_t)(x - 3);
+            } else {
+                rows[d] = base + (uint32_t)min(max(y + d - 3, 0), (int)G.height - 1) * G.width;
+                qx[d] = min(max(x + d - 3, 0), (int)G.width - 1);
+            }
+        }
+    }
+    __device__ __forceinline__ uint32_t operator()(int k) const {
+        return rows[k / 7] + (uint32_t)(kInterior ? k % 7 : qx[k % 7]);
+    }
+};
+
+// The largest of this thread's 49 logits (accumulator + bias).
+__device__ __forceinline__ float logit_max(uint32_t tmem_lane, const float2* b4, float b48) {
+    float m = -3.0e38f;
+#pragma unroll
+    for (int c0 = 0; c0 < 48; c0 += 16) {
+        float v[16];
+        tc_load16(tmem_lane + (uint32_t)c0, v);
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+            const float2 z = add2(make_float2(v[2 * j], v[2 * j + 1]), b4[c0 / 2 + j]);
+            m = fmaxf(m, fmaxf(z.x, z.y));
+        }
+    }
+    float v[16];
+    tc_load16(tmem_lane + 48u, v);
+    return fmaxf(m, v[0] + b48);
+}
+
 // Second pass of the softmax and the 7x7 filter: with w_k = 2^((z_k - m) * log2 e),
 // z_k = logit + bias, sums of w_k x the shadowed light S_k (r, g, b) and AO_k (acc),
 // of w_k x the unshadowed light U_k (accu, r, g, b) and of w_k (the return value).
-// kInterior: every tap of the thread's pixel is inside the image (rows addressed
-// directly); otherwise clamped.
 template <bool kInterior>
 __device__ __forceinline__ float signal_filter(uint32_t tmem_lane, const float2* b4, float b48, float m,
                                                const float4* __restrict__ sig, const float4* __restrict__ uns,
@@ -331,18 +409,7 @@ __device__ __forceinline__ float signal_filter(uint32_t tmem_lane, const float2*
     const float2 l2e = make_float2(kLog2e, kLog2e);
     const float nm = -m * kLog2e;
     const float2 nm2 = make_float2(nm, nm);
-    uint32_t rows[7];
-    int qx[7];
-#pragma unroll
-    for (int d = 0; d < 7; ++d) {
-        if (kInterior) {
-            rows[d] = base + (uint32_t)(y + d - 3) * G.width + (uint32_t)(x - 3);
-        } else {
-            rows[d] = base + (uint32_t)min(max(y + d - 3, 0), (int)G.height - 1) * G.width;
-            qx[d] = min(max(x + d - 3, 0), (int)G.width - 1);
-        }
-    }
-    auto at = [&](int k) -> uint32_t { return rows[k / 7] + (uint32_t)(kInterior ? k % 7 : qx[k % 7]); };
+    const TapAt<kInterior> at(base, x, y, G);
     float2 s = make_float2(0.f, 0.f);
     float2 a_xy = make_float2(0.f, 0.f), a_zw = make_float2(0.f, 0.f), u_xy = make_float2(0.f, 0.f);
     float u_z = 0.f;
@@ -420,15 +487,15 @@ __global__ void __launch_bounds__(kTcThreads, kTcBlocksPerSm) denoise_infer_tc_k
     const uint32_t a_addr = smem_u32(a);
     uint32_t phase = 0;
     bool failed = false;
-    const uint32_t total = P.list ? *P.list_count : P.G.pixels * P.G.images;
-    const uint32_t tiles = (total + 127) / 128;
+    const uint32_t total = P.list ? *P.list_count : 0u;
+    const uint32_t tiles = P.list ? (total + 127) / 128 : P.tiles;
     const uint32_t stride = gridDim.x * kTcGroups;
     uint32_t tile = blockIdx.x * kTcGroups + group;
     uint32_t next_xy = (P.list && tile * 128 + row < total) ? P.list[tile * 128 + row] : 0u;
     for (; tile < tiles; tile += stride) {
         // features of pixel `row`: 9 taps of 8 channels (relative depth in channel 5), then 8 zeros
         const uint32_t item = tile * 128 + row;
-        const bool has = item < total;
+        bool has = item < total;
         uint32_t img = 0, gp = 0;
         int x = 0, y = 0;
         if (P.list) {
@@ -437,12 +504,8 @@ __global__ void __launch_bounds__(kTcThreads, kTcBlocksPerSm) denoise_infer_tc_k
             gp = (uint32_t)y * P.G.width + (uint32_t)x;
             const uint32_t nitem = item + stride * 128;   // this thread's entry of the next tile
             next_xy = nitem < total ? P.list[nitem] : 0u;
-        } else if (has) {
-            gp = item;
-            img = gp / P.G.pixels;
-            const uint32_t local = gp - img * P.G.pixels;
-            x = (int)(local % P.G.width);
-            y = (int)(local / P.G.width);
+        } else {
+            has = tile_pixel(P.G, tile, row, img, x, y, gp);
         }
         // the centre depth and the 9 taps are loaded without waiting on one another
         // (clamped, always in bounds); background centres get a zero row
@@ -457,6 +520,13 @@ __global__ void __launch_bounds__(kTcThreads, kTcBlocksPerSm) denoise_infer_tc_k
             td[tap] = has ? P.lin_depth[tq[tap]] : 0.0f;
         }
         const bool valid = dc > 0.0f;
+        if (!P.list && !group_any(group, valid)) {   // a tile of background: zeros
+            if (has) {
+                P.out[gp] = make_float4(0.f, 0.f, 0.f, 0.f);
+                if (P.out_ao) P.out_ao[gp] = 0.0f;
+            }
+            continue;
+        }
         const float inv_dc = valid ? 1.0f / dc : 0.0f;
 #pragma unroll
         for (int tap = 0; tap < 9; ++tap) {
@@ -476,22 +546,7 @@ __global__ void __launch_bounds__(kTcThreads, kTcBlocksPerSm) denoise_infer_tc_k
         tc_run_layer(group, tmem, a_addr, smem_u32(tsm + kTcW4), 4, bar, phase, failed, status);
         // softmax over the 49 logits and the 7x7 filter of the noisy AO
         const float2* b4 = reinterpret_cast<const float2*>(sbias + 192);
-        float m = -3.0e38f;
-#pragma unroll
-        for (int c0 = 0; c0 < 48; c0 += 16) {
-            float v[16];
-            tc_load16(tmem_lane + (uint32_t)c0, v);
-#pragma unroll
-            for (int j = 0; j < 8; ++j) {
-                const float2 z = add2(make_float2(v[2 * j], v[2 * j + 1]), b4[c0 / 2 + j]);
-                m = fmaxf(m, fmaxf(z.x, z.y));
-            }
-        }
-        {
-            float v[16];
-            tc_load16(tmem_lane + 48u, v);
-            m = fmaxf(m, v[0] + sbias[192 + 48]);
-        }
+        const float m = logit_max(tmem_lane, b4, sbias[192 + 48]);
         const uint32_t base = img * P.G.pixels;
         const bool interior = has && x >= 3 && y >= 3 && x + 3 < (int)P.G.width && y + 3 < (int)P.G.height;
         float4 acc;
@@ -530,72 +585,74 @@ struct TrainParams {
     float shadow_weight;       // loss weight of each shadow-ratio output (AO: 1)
     float* partial;            // [gridDim.x][kParams]
     float* partial_loss;       // [gridDim.x]
+    uint32_t tiles;            // of the images
 };
 
 // ---------------------------------------------------------------- training on tcgen05
-// Forward, backward and the weight gradients of a 128-pixel tile as tcgen05.mma
-// products (M = 128, BF16 operands in shared memory, FP32 accumulators in tensor
-// memory), one warpgroup per SM, thread p = pixel p of the tile:
-//   forward   D = A * W^T for the four layers (A = X, H1, H2, H3; as inference);
-//   backward  dH_l = dZ_{l+1} * W_{l+1} (B = the transposed weights W^T, K = outputs);
-//   gradients dW_l += dZ_l^T * [H_{l-1} | 1]^T over the tile's pixels (M = outputs,
-//             rows 64..127 of A zero; N = 80 with the bias column of ones; K = the 128
-//             pixels), accumulated in tensor memory over all tiles of the block.
-// Every operand sits in the K-major no-swizzle core-matrix layout of the inference
-// kernel; the activations and dZ are written twice by their threads: as a row of the
-// next product's A and as a column of the transposed copy (dW's A and B). One
-// partial per block in the FP32 parameter layout, summed in block order.
-constexpr int kTtW1 = 0;                            // [64 x 80] forward B
+// Forward, backward and the weight gradients as tcgen05.mma products (M = 128, BF16
+// operands in shared memory, FP32 accumulators in tensor memory). A block per SM holds two
+// warpgroups with a 128-pixel tile each, thread p = pixel p of its tile:
+//   forward   D = A * W^T for the four layers (A = X, H1, H2, H3, each kept for the way
+//             back); the groups run on their own, one waits for products while the other
+//             gathers, filters or runs an epilogue;
+//   backward  dH_l = dZ_{l+1} * W_{l+1};
+//   gradients dW_l^T += [H_{l-1} | 1]^T * dZ_l over the pixels of both tiles, issued by one
+//             thread in a fixed order (so the sums are deterministic), accumulated in tensor
+//             memory over all tiles of the block. The products overlap the next epilogue.
+// Every matrix is stored once, pixel (or output) rows by columns in 8x8 core matrices: a
+// K-major operand where the product sums over its columns, an MN-major one (the other
+// order of the same core matrices' strides) where it sums over its rows. dW^T's M = 128
+// rows run past the 72 or 80 columns of H or X into the memory that follows, inside the
+// block's allocation; those rows of the accumulator are never read.
+//
+// Bound by latency at two warps per scheduler: of 28,000 cycles a pair of tiles takes, the
+// eight products with their barriers are 16,000 and the two passes over the 49 taps (two
+// float4 each) 10,000. 1 M pixels: 1.31 -> 0.40 ms against one warpgroup per SM that also
+// wrote transposed copies of every matrix by 2-byte stores (207 KB of shared memory for
+// one tile).
+constexpr int kTtGroups = 2, kTtThreads = 128 * kTtGroups;
+constexpr int kTtXK = 10, kTtHK = 9;                // core-matrix columns of X and H: 72 + 8, 64 + 8
+constexpr int kTtX = 0;                             // [128 x 80] X, column 72 ones
+constexpr int kTtH = kTtX + 128 * kTtXK * 16;       // 3 x [128 x 72] H, column 64 ones
+constexpr int kTtHBytes = 128 * kTtHK * 16;
+constexpr int kTtDZ = kTtH + 3 * kTtHBytes;         // [128 x 64] dZ
+constexpr int kTtTile = kTtDZ + 128 * 64 * 2;       // one group's bytes
+constexpr int kTtW1 = kTtGroups * kTtTile;          // [64 x 80]
 constexpr int kTtW2 = kTtW1 + 64 * 80 * 2;          // [64 x 64]
 constexpr int kTtW3 = kTtW2 + 64 * 64 * 2;
 constexpr int kTtW4 = kTtW3 + 64 * 64 * 2;          // rows >= 49 zero
-constexpr int kTtW4T = kTtW4 + 64 * 64 * 2;         // [64 hidden x 64 outputs] backward B
-constexpr int kTtW3T = kTtW4T + 64 * 64 * 2;
-constexpr int kTtW2T = kTtW3T + 64 * 64 * 2;
-constexpr int kTtA = kTtW2T + 64 * 64 * 2;          // [128 x 80] X, then H1, H2, H3
-constexpr int kTtXT = kTtA + 128 * 80 * 2;          // [80 x 128] X^T, row 72 ones
-constexpr int kTtHT = kTtXT + 80 * 128 * 2;         // 3 x [80 x 128] H^T, row 64 ones
-constexpr int kTtDZ = kTtHT + 3 * 80 * 128 * 2;     // [128 x 64] dZ
-constexpr int kTtDZT = kTtDZ + 128 * 64 * 2;        // [128 x 128] dZ^T in rows 0..63
-constexpr int kTtBias = kTtDZT + 128 * 128 * 2;
-constexpr int kTtBar = kTtBias + kBias * 4;
-constexpr int kTtSmem = kTtBar + 32;
-static_assert(kTtSmem + 1024 <= 232448, "training tile must fit in shared memory");
-// tensor-memory columns: forward D, backward dH, dW1..dW4 (80 each)
-constexpr uint32_t kTtFwd = 0, kTtDH = 64, kTtDW1 = 128, kTtDW2 = 208, kTtDW3 = 288, kTtDW4 = 368;
-constexpr uint32_t kTtAlloc = 512;
+constexpr int kTtBias = kTtW4 + 64 * 64 * 2;
+constexpr int kTtBar = kTtBias + kBias * 4;         // one mbarrier per group, one for dW
+constexpr int kTtSmem = kTtBar + 48;
+static_assert(kTtSmem + 1024 <= 232448, "training tiles must fit in shared memory");
+static_assert(kTtX + (16 - kTtXK) * 128 <= kTtH && (16 - kTtHK) * 128 <= 128 * 64 * 2, "M = 128 reads stay inside a tile");
+// tensor-memory columns: forward D and backward dH of the groups, dW1..dW4 (64 each)
+constexpr uint32_t kTtDW = 64 * kTtGroups, kTtAlloc = 512;
+static_assert(kTtDW + 4 * 64 <= kTtAlloc, "tensor-memory columns");
 
-__host__ __device__ constexpr uint32_t tc_idesc(uint32_t n) {
-    return (1u << 4) | (1u << 7) | (1u << 10) | ((n >> 3) << 17) | ((128u >> 4) << 24);
+// Instruction descriptor of kind::f16: FP32 accumulator, BF16 A and B, M = 128, N = 64;
+// an operand is MN-major where its flag is set.
+__host__ __device__ constexpr uint32_t tc_idesc(bool a_mn, bool b_mn) {
+    return kTcIdesc | (a_mn ? 1u << 15 : 0u) | (b_mn ? 1u << 16 : 0u);
 }
-
-// D[tmem] (+)= A[128 x 16 ksteps] * B[N x 16 ksteps]^T; a / b: shared addresses,
-// ka / kb: their core-matrix columns (K / 8).
-__device__ __forceinline__ void tc_mma(uint32_t tmem, uint32_t a, uint32_t ka, uint32_t b, uint32_t kb, int ksteps,
-                                       uint32_t idesc, bool accumulate) {
-    for (int s = 0; s < ksteps; ++s) {
-        const uint64_t da = umma_desc(a + (uint32_t)s * 256u, 128u, ka * 128u);
-        const uint64_t db = umma_desc(b + (uint32_t)s * 256u, 128u, kb * 128u);
-        asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-                     "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}\n"
-                     :: "r"(tmem), "l"(da), "l"(db), "r"(idesc), "r"((s > 0 || accumulate) ? 1u : 0u));
-    }
+// Descriptor of the 16 k's from k-step s on of an operand with kblocks core-matrix
+// columns: K-major, a step is two core matrices of a row; MN-major, two rows of them.
+__device__ __forceinline__ uint64_t k_major(uint32_t addr, uint32_t kblocks, int s) {
+    return umma_desc(addr + (uint32_t)s * 256u, 128u, kblocks * 128u);
 }
-
-// Makes the block's shared-memory writes and tensor-memory reads visible to the
-// products that thread 0 issues next.
-__device__ __forceinline__ void tt_before_issue() {
-    asm volatile("fence.proxy.async.shared::cta;");
-    asm volatile("tcgen05.fence::before_thread_sync;");
-    __syncthreads();
-    asm volatile("tcgen05.fence::after_thread_sync;");
+__device__ __forceinline__ uint64_t mn_major(uint32_t addr, uint32_t kblocks, int s) {
+    return umma_desc(addr + (uint32_t)s * 2u * kblocks * 128u, kblocks * 128u, 128u);
 }
-
-// Commits the issued products to the mbarrier and waits for them (bounded; see
-// tc_run_layer).
-__device__ __forceinline__ void tt_commit_wait(uint32_t bar, uint32_t& phase, bool& failed, uint32_t* status) {
-    if (threadIdx.x == 0)
-        asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" :: "r"(bar));
+__device__ __forceinline__ void tc_mma1(uint32_t tmem, uint64_t da, uint64_t db, uint32_t idesc, bool accumulate) {
+    asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
+                 "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}\n"
+                 :: "r"(tmem), "l"(da), "l"(db), "r"(idesc), "r"(accumulate ? 1u : 0u));
+}
+__device__ __forceinline__ void tc_commit(uint32_t bar) {
+    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" :: "r"(bar));
+}
+// Waits for a phase (bounded; see tc_run_layer).
+__device__ __forceinline__ void tt_wait(uint32_t bar, uint32_t& phase, bool& failed, uint32_t* status) {
     if (!failed && !tc_wait(bar, phase)) {
         atomicOr(status, (uint32_t)LUZ_DEV_MMA_WAIT);
         failed = true;
@@ -604,21 +661,11 @@ __device__ __forceinline__ void tt_commit_wait(uint32_t bar, uint32_t& phase, bo
     asm volatile("tcgen05.fence::after_thread_sync;");
 }
 
-// Element (r, k) of a core-matrix tile with kblocks core columns, as a 2-byte offset.
-__device__ __forceinline__ uint32_t elem_offset(uint32_t r, uint32_t k, uint32_t kblocks) {
-    return core_offset(r, k >> 3, kblocks) + (k & 7u) * 2u;
-}
-
-__device__ __forceinline__ void st_bf16(unsigned char* base, uint32_t off, float v) {
-    *reinterpret_cast<__nv_bfloat16*>(base + off) = __float2bfloat16(v);
-}
-
 // Forward epilogue of layers 1-3: bias + ReLU + BF16 of this thread's 64 accumulator
-// columns into row `row` of A (the next layer's input) and column `row` of the
-// transposed copy ht; bit j of mask = (h_j > 0).
-__device__ __forceinline__ void tt_relu_out(uint32_t tl, const float* sb, unsigned char* a, unsigned char* ht,
-                                            uint32_t row, uint64_t& mask) {
-    mask = 0;
+// columns into row `row` of H; bit j of mask = (h_j > 0).
+__device__ __forceinline__ void tt_relu_out(uint32_t tl, const float* sb, unsigned char* h, uint32_t row, uint64_t& mask) {
+    const float2* b2 = reinterpret_cast<const float2*>(sb);
+    uint32_t m[2] = {0u, 0u};
 #pragma unroll
     for (int c0 = 0; c0 < 64; c0 += 16) {
         float v[16];
@@ -626,86 +673,88 @@ __device__ __forceinline__ void tt_relu_out(uint32_t tl, const float* sb, unsign
         uint32_t w[8];
 #pragma unroll
         for (int j = 0; j < 8; ++j) {
-            const float lo = fmaxf(v[2 * j] + sb[c0 + 2 * j], 0.0f), hi = fmaxf(v[2 * j + 1] + sb[c0 + 2 * j + 1], 0.0f);
-            w[j] = pack2(lo, hi);
-            const __nv_bfloat162 q = *reinterpret_cast<const __nv_bfloat162*>(&w[j]);
-            *reinterpret_cast<__nv_bfloat16*>(ht + elem_offset((uint32_t)(c0 + 2 * j), row, 16)) = q.x;
-            *reinterpret_cast<__nv_bfloat16*>(ht + elem_offset((uint32_t)(c0 + 2 * j + 1), row, 16)) = q.y;
-            mask |= (uint64_t)(__bfloat162float(q.x) > 0.0f) << (c0 + 2 * j);
-            mask |= (uint64_t)(__bfloat162float(q.y) > 0.0f) << (c0 + 2 * j + 1);
+            w[j] = bias_relu_bf16x2(v[2 * j], v[2 * j + 1], b2[c0 / 2 + j]);
+            // h >= 0: positive where a bit other than the sign is set
+            m[c0 / 32] |= ((w[j] & 0x7FFFu) ? 1u : 0u) << ((c0 & 31) + 2 * j);
+            m[c0 / 32] |= ((w[j] & 0x7FFF0000u) ? 1u : 0u) << ((c0 & 31) + 2 * j + 1);
         }
-        *reinterpret_cast<uint4*>(a + core_offset(row, (uint32_t)c0 / 8u, 8u)) = make_uint4(w[0], w[1], w[2], w[3]);
-        *reinterpret_cast<uint4*>(a + core_offset(row, (uint32_t)c0 / 8u + 1u, 8u)) = make_uint4(w[4], w[5], w[6], w[7]);
+        *reinterpret_cast<uint4*>(h + core_offset(row, (uint32_t)c0 / 8u, kTtHK)) = make_uint4(w[0], w[1], w[2], w[3]);
+        *reinterpret_cast<uint4*>(h + core_offset(row, (uint32_t)c0 / 8u + 1u, kTtHK)) = make_uint4(w[4], w[5], w[6], w[7]);
     }
+    mask = (uint64_t)m[0] | ((uint64_t)m[1] << 32);
 }
 
-// Backward epilogue of layers 3-1: dZ = dH * ReLU'(h) of this thread's 64 columns into
-// row `row` of dZ (when dz != null) and column `row` of dZ^T.
-__device__ __forceinline__ void tt_dz_out(uint32_t tl, uint64_t mask, unsigned char* dz, unsigned char* dzt,
-                                          uint32_t row) {
+// Backward pass of the softmax and the filter: dL/dz_k = w_k (g_k - gw) with the weights
+// w_k = 2^((z_k - m) * log2 e) * inv again from the logits, g_k = dL/dw_k = dy.w AO_k +
+// sum over c of (dq_c S_kc - dr_c U_kc) and gw = sum(w g), as row `row` of dZ.
+template <bool kInterior>
+__device__ __forceinline__ void signal_backward(uint32_t tmem_lane, const float2* b4, float b48, float m, float inv,
+                                                const float4* __restrict__ sig, const float4* __restrict__ uns,
+                                                uint32_t base, int x, int y, const ImageGeom& G, float dyw, float3 dq,
+                                                float3 dr, float gw, unsigned char* dz, uint32_t row) {
+    constexpr float kLog2e = 1.4426950408889634f;
+    const float nm = -m * kLog2e;
+    const TapAt<kInterior> at(base, x, y, G);
+    const float2 q_xy = make_float2(dq.x, dq.y), q_zw = make_float2(dq.z, dyw), r_xy = make_float2(-dr.x, -dr.y);
+    auto tap = [&](int k, float z) {
+        const uint32_t q = at(k);
+        const float4 s4 = __ldg(sig + q), u4 = __ldg(uns + q);
+        float2 g = fma2(q_xy, make_float2(s4.x, s4.y), make_float2(-gw, 0.0f));
+        g = fma2(q_zw, make_float2(s4.z, s4.w), g);
+        g = fma2(r_xy, make_float2(u4.x, u4.y), g);
+        return (exp2_approx(fmaf(z, kLog2e, nm)) * inv) * fmaf(-dr.z, u4.z, g.x + g.y);
+    };
 #pragma unroll
-    for (int c0 = 0; c0 < 64; c0 += 16) {
+    for (int c0 = 0; c0 < 48; c0 += 16) {
         float v[16];
-        tc_load16(tl + (uint32_t)c0, v);
+        tc_load16(tmem_lane + (uint32_t)c0, v);
         uint32_t w[8];
 #pragma unroll
         for (int j = 0; j < 8; ++j) {
-            const float lo = ((mask >> (c0 + 2 * j)) & 1u) ? v[2 * j] : 0.0f;
-            const float hi = ((mask >> (c0 + 2 * j + 1)) & 1u) ? v[2 * j + 1] : 0.0f;
+            const float2 z = add2(make_float2(v[2 * j], v[2 * j + 1]), b4[c0 / 2 + j]);
+            const float lo = tap(c0 + 2 * j, z.x), hi = tap(c0 + 2 * j + 1, z.y);
             w[j] = pack2(lo, hi);
-            const __nv_bfloat162 q = *reinterpret_cast<const __nv_bfloat162*>(&w[j]);
-            *reinterpret_cast<__nv_bfloat16*>(dzt + elem_offset((uint32_t)(c0 + 2 * j), row, 16)) = q.x;
-            *reinterpret_cast<__nv_bfloat16*>(dzt + elem_offset((uint32_t)(c0 + 2 * j + 1), row, 16)) = q.y;
         }
-        if (dz) {
-            *reinterpret_cast<uint4*>(dz + core_offset(row, (uint32_t)c0 / 8u, 8u)) = make_uint4(w[0], w[1], w[2], w[3]);
-            *reinterpret_cast<uint4*>(dz + core_offset(row, (uint32_t)c0 / 8u + 1u, 8u)) =
-                make_uint4(w[4], w[5], w[6], w[7]);
-        }
+        *reinterpret_cast<uint4*>(dz + core_offset(row, (uint32_t)c0 / 8u, 8u)) = make_uint4(w[0], w[1], w[2], w[3]);
+        *reinterpret_cast<uint4*>(dz + core_offset(row, (uint32_t)c0 / 8u + 1u, 8u)) = make_uint4(w[4], w[5], w[6], w[7]);
     }
+    float v[16];
+    tc_load16(tmem_lane + 48u, v);
+    *reinterpret_cast<uint4*>(dz + core_offset(row, 6u, 8u)) = make_uint4(pack2(tap(48, v[0] + b48), 0.0f), 0u, 0u, 0u);
+    *reinterpret_cast<uint4*>(dz + core_offset(row, 7u, 8u)) = make_uint4(0u, 0u, 0u, 0u);
 }
 
-__global__ void __launch_bounds__(128, 1) denoise_train_tc_kernel(TrainParams P, uint32_t* status) {
+__global__ void __launch_bounds__(kTtThreads, 1) denoise_train_tc_kernel(TrainParams P, uint32_t* status) {
     extern __shared__ __align__(1024) unsigned char tsm[];
     float* sbias = reinterpret_cast<float*>(tsm + kTtBias);
-    uint32_t* tslot = reinterpret_cast<uint32_t*>(tsm + kTtBar + 8);
-    const uint32_t tid = threadIdx.x, warp = tid >> 5, row = tid;
-    const uint32_t bar = smem_u32(tsm + kTtBar);
-    // weights into the core-matrix layout: forward (n-major W) and backward (W^T)
-    for (uint32_t e = tid; e < 64 * 10; e += 128) {
+    uint32_t* tslot = reinterpret_cast<uint32_t*>(tsm + kTtBar + 24);
+    __shared__ float s_loss[kTtThreads / 32];
+    const uint32_t tid = threadIdx.x, warp = tid >> 5, group = tid >> 7, row = tid & 127u;
+    const uint32_t bar = smem_u32(tsm + kTtBar + 8 * group), bar_w = smem_u32(tsm + kTtBar + 16);
+    unsigned char* tile_mem = tsm + group * kTtTile;
+    unsigned char* xs = tile_mem + kTtX;
+    unsigned char* hs[3] = {tile_mem + kTtH, tile_mem + kTtH + kTtHBytes, tile_mem + kTtH + 2 * kTtHBytes};
+    unsigned char* dz = tile_mem + kTtDZ;
+    for (uint32_t e = tid; e < 64 * 10; e += kTtThreads) {
         const uint32_t n = e / 10, kb = e % 10;
         *reinterpret_cast<uint4*>(tsm + kTtW1 + core_offset(n, kb, 10)) =
             *reinterpret_cast<const uint4*>(P.wpack + pW1 + n * sW1 + kb * 8);
     }
-    for (uint32_t e = tid; e < 64 * 8; e += 128) {
-        const uint32_t n = e / 8, kb = e % 8;
-        const uint32_t o = core_offset(n, kb, 8);
+    for (uint32_t e = tid; e < 64 * 8; e += kTtThreads) {
+        const uint32_t n = e / 8, kb = e % 8, o = core_offset(n, kb, 8);
         *reinterpret_cast<uint4*>(tsm + kTtW2 + o) = *reinterpret_cast<const uint4*>(P.wpack + pW2 + n * sW + kb * 8);
         *reinterpret_cast<uint4*>(tsm + kTtW3 + o) = *reinterpret_cast<const uint4*>(P.wpack + pW3 + n * sW + kb * 8);
         *reinterpret_cast<uint4*>(tsm + kTtW4 + o) =
             n < 56 ? *reinterpret_cast<const uint4*>(P.wpack + pW4 + n * sW + kb * 8) : make_uint4(0, 0, 0, 0);
-        *reinterpret_cast<uint4*>(tsm + kTtW4T + o) = *reinterpret_cast<const uint4*>(P.wpack + pW4T + n * sW + kb * 8);
-        *reinterpret_cast<uint4*>(tsm + kTtW3T + o) = *reinterpret_cast<const uint4*>(P.wpack + pW3T + n * sW + kb * 8);
-        *reinterpret_cast<uint4*>(tsm + kTtW2T + o) = *reinterpret_cast<const uint4*>(P.wpack + pW2T + n * sW + kb * 8);
     }
-    for (uint32_t i = tid; i < (uint32_t)kBias; i += 128) sbias[i] = P.bias[i];
-    // constant parts: zero dZ^T (rows 64..127 stay zero, rows 49..63 of the last layer
-    // too) and the ones / zero rows of the transposed activations
-    for (uint32_t i = tid; i < 128 * 128 * 2 / 16; i += 128)
-        reinterpret_cast<uint4*>(tsm + kTtDZT)[i] = make_uint4(0, 0, 0, 0);
-    for (uint32_t i = tid; i < 128 * 64 * 2 / 16; i += 128)
-        reinterpret_cast<uint4*>(tsm + kTtDZ)[i] = make_uint4(0, 0, 0, 0);
-    {
-        const __nv_bfloat16 one = __float2bfloat16(1.0f), zero = __float2bfloat16(0.0f);
-        for (uint32_t k = 72; k < 80; ++k)
-            *reinterpret_cast<__nv_bfloat16*>(tsm + kTtXT + elem_offset(k, row, 16)) = k == 72 ? one : zero;
-        for (int l = 0; l < 3; ++l)
-            for (uint32_t k = 64; k < 80; ++k)
-                *reinterpret_cast<__nv_bfloat16*>(tsm + kTtHT + l * 80 * 128 * 2 + elem_offset(k, row, 16)) =
-                    k == 64 ? one : zero;
-    }
+    for (uint32_t i = tid; i < (uint32_t)kBias; i += kTtThreads) sbias[i] = P.bias[i];
+    // the columns of ones (the bias inputs of dW) with zeros after them
+    const uint4 one = make_uint4(0x00003F80u, 0u, 0u, 0u);
+    *reinterpret_cast<uint4*>(xs + core_offset(row, 9, kTtXK)) = one;
+    for (int l = 0; l < 3; ++l) *reinterpret_cast<uint4*>(hs[l] + core_offset(row, 8, kTtHK)) = one;
     if (tid == 0) {
-        asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" :: "r"(bar));
+        for (int k = 0; k < 3; ++k)
+            asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" :: "r"(smem_u32(tsm + kTtBar + 8 * k)));
         asm volatile("fence.mbarrier_init.release.cluster;");
     }
     if (warp == 0) {
@@ -716,113 +765,72 @@ __global__ void __launch_bounds__(128, 1) denoise_train_tc_kernel(TrainParams P,
     asm volatile("tcgen05.fence::before_thread_sync;");
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;");
-    const uint32_t tmem = *tslot;
-    const uint32_t lane_off = ((warp & 3u) * 32u) << 16;
-    unsigned char* a = tsm + kTtA;
-    unsigned char* xt = tsm + kTtXT;
-    unsigned char* ht[3] = {tsm + kTtHT, tsm + kTtHT + 80 * 128 * 2, tsm + kTtHT + 2 * 80 * 128 * 2};
-    unsigned char* dz = tsm + kTtDZ;
-    unsigned char* dzt = tsm + kTtDZT;
-    const uint32_t a_addr = smem_u32(a), dz_addr = smem_u32(dz), dzt_addr = smem_u32(dzt);
-    const uint32_t xt_addr = smem_u32(xt);
-    const uint32_t ht_addr[3] = {smem_u32(ht[0]), smem_u32(ht[1]), smem_u32(ht[2])};
-    const uint32_t wf[4] = {smem_u32(tsm + kTtW1), smem_u32(tsm + kTtW2), smem_u32(tsm + kTtW3), smem_u32(tsm + kTtW4)};
-    const uint32_t wt[3] = {smem_u32(tsm + kTtW2T), smem_u32(tsm + kTtW3T), smem_u32(tsm + kTtW4T)};
-    const uint32_t dw_col[4] = {kTtDW1, kTtDW2, kTtDW3, kTtDW4};
-    uint32_t phase = 0;
+    const uint32_t tmem = *tslot, lane_off = ((warp & 3u) * 32u) << 16;
+    const uint32_t tg = tmem + 64u * group, tl = tg + lane_off;   // this group's columns, this warp's lanes
+    const uint32_t w_addr[4] = {smem_u32(tsm + kTtW1), smem_u32(tsm + kTtW2), smem_u32(tsm + kTtW3), smem_u32(tsm + kTtW4)};
+    uint32_t phase = 0, phase_w = 0;
     bool failed = false, accumulated = false;
     float loss = 0.f;
-    const uint32_t total = P.G.pixels * P.G.images;
-    const uint32_t tiles = (total + 127) / 128;
-    for (uint32_t tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
-        // ---- features of pixel `row` (9 taps of 8 channels, relative depth in channel 5)
-        const uint32_t gp = tile * 128 + row;
-        const bool has = gp < total;
-        uint32_t img = 0;
-        int x = 0, y = 0;
-        if (has) {
-            img = gp / P.G.pixels;
-            const uint32_t local = gp - img * P.G.pixels;
-            x = (int)(local % P.G.width);
-            y = (int)(local / P.G.width);
-        }
+    const uint32_t pairs = (P.tiles + kTtGroups - 1) / kTtGroups;
+    for (uint32_t pair = blockIdx.x; pair < pairs; pair += gridDim.x) {
+        // ---- features of pixel `row`: 9 taps of 8 channels, relative depth in channel 5
+        uint32_t img, gp;
+        int x, y;
+        const uint32_t tile = pair * kTtGroups + group;
+        const bool has = tile_pixel(P.G, tile, row, img, x, y, gp) && tile < P.tiles;
         const float dc = has ? P.lin_depth[gp] : 0.0f;
         const bool valid = dc > 0.0f;
         const float inv_dc = valid ? 1.0f / dc : 0.0f;
+        const float4 tgt = valid ? P.target[gp] : make_float4(0.f, 0.f, 0.f, 0.f);
+        uint4 fv[9];
+        float td[9];
 #pragma unroll
-        for (int tap = 0; tap < 9; ++tap) {
-            const int qx = min(max(x + tap % 3 - 1, 0), (int)P.G.width - 1);
-            const int qy = min(max(y + tap / 3 - 1, 0), (int)P.G.height - 1);
+        for (int k = 0; k < 9; ++k) {
+            const int qx = min(max(x + k % 3 - 1, 0), (int)P.G.width - 1), qy = min(max(y + k / 3 - 1, 0), (int)P.G.height - 1);
             const uint32_t q = img * P.G.pixels + (uint32_t)qy * P.G.width + (uint32_t)qx;
-            uint4 v = make_uint4(0, 0, 0, 0);
-            if (valid) {
-                v = P.feat[q];
-                const float dq = P.lin_depth[q];
-                const float rel = dq > 0.0f ? relative_depth(dq, dc, inv_dc) : 0.0f;
-                v.z = (v.z & 0xFFFFu) | (pack2(0.0f, rel) & 0xFFFF0000u);
-            }
-            *reinterpret_cast<uint4*>(a + core_offset(row, (uint32_t)tap, 10)) = v;
-            const uint32_t w4[4] = {v.x, v.y, v.z, v.w};
-#pragma unroll
-            for (int c = 0; c < 4; ++c) {
-                *reinterpret_cast<uint16_t*>(xt + elem_offset((uint32_t)(tap * 8 + 2 * c), row, 16)) =
-                    (uint16_t)(w4[c] & 0xFFFFu);
-                *reinterpret_cast<uint16_t*>(xt + elem_offset((uint32_t)(tap * 8 + 2 * c + 1), row, 16)) =
-                    (uint16_t)(w4[c] >> 16);
-            }
+            fv[k] = valid ? P.feat[q] : make_uint4(0, 0, 0, 0);
+            td[k] = valid ? P.lin_depth[q] : 0.0f;
         }
-        *reinterpret_cast<uint4*>(a + core_offset(row, 9, 10)) = make_uint4(0, 0, 0, 0);
+        if (accumulated) tt_wait(bar_w, phase_w, failed, status);   // dW1 of the last tiles has read X and dZ
+#pragma unroll
+        for (int k = 0; k < 9; ++k) {
+            uint4 v = fv[k];
+            const float rel = td[k] > 0.0f ? relative_depth(td[k], dc, inv_dc) : 0.0f;
+            v.z = (v.z & 0xFFFFu) | (pack2(0.0f, rel) & 0xFFFF0000u);
+            *reinterpret_cast<uint4*>(xs + core_offset(row, (uint32_t)k, kTtXK)) = v;
+        }
         // ---- forward
         uint64_t mask[3];
-        const uint32_t tl = tmem + lane_off;
 #pragma unroll
         for (int l = 0; l < 4; ++l) {
-            tt_before_issue();
-            if (tid == 0) tc_mma(tmem + kTtFwd, a_addr, l == 0 ? 10u : 8u, wf[l], l == 0 ? 10u : 8u, l == 0 ? 5 : 4,
-                                 tc_idesc(64), false);
-            tt_commit_wait(bar, phase, failed, status);
-            if (l < 3) tt_relu_out(tl + kTtFwd, sbias + 64 * l, a, ht[l], row, mask[l]);
+            asm volatile("fence.proxy.async.shared::cta;");
+            asm volatile("tcgen05.fence::before_thread_sync;");
+            group_sync(group);
+            asm volatile("tcgen05.fence::after_thread_sync;");
+            if (row == 0) {
+                const uint32_t a = smem_u32(l == 0 ? xs : hs[l - 1]), ak = l == 0 ? kTtXK : kTtHK, wk = l == 0 ? 10u : 8u;
+#pragma unroll
+                for (int s = 0; s < (l == 0 ? 5 : 4); ++s)
+                    tc_mma1(tg, k_major(a, ak, s), k_major(w_addr[l], wk, s), tc_idesc(false, false), s > 0);
+                tc_commit(bar);
+            }
+            tt_wait(bar, phase, failed, status);
+            if (l < 3) tt_relu_out(tl, sbias + 64 * l, hs[l], row, mask[l]);
         }
-        // ---- softmax, filter, loss and dL/dz of the last layer (this thread's pixel)
-        const float* b4 = sbias + 192;
-        float z[49];
-#pragma unroll
-        for (int c0 = 0; c0 < 64; c0 += 16) {
-            float v[16];
-            tc_load16(tl + kTtFwd + (uint32_t)c0, v);
-#pragma unroll
-            for (int j = 0; j < 16; ++j)
-                if (c0 + j < 49) z[c0 + j] = v[j] + b4[c0 + j];
-        }
-        float m = -3.0e38f;
-#pragma unroll
-        for (int k = 0; k < 49; ++k) m = fmaxf(m, z[k]);
-        float sum = 0.f;
-#pragma unroll
-        for (int k = 0; k < 49; ++k) {
-            z[k] = __expf(z[k] - m);
-            sum += z[k];
-        }
-        const float inv = 1.0f / sum;
-        float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
-        float3 au = make_float3(0.f, 0.f, 0.f);
-#pragma unroll
-        for (int k = 0; k < 49; ++k) {
-            z[k] *= inv;   // the normalised weight w_k
-            const float4 sv = signal_tap(P.sig, P.G, has, img, x, y, k);
-            const float4 uv = signal_tap(P.uns, P.G, has, img, x, y, k);
-            acc.x += z[k] * sv.x;
-            acc.y += z[k] * sv.y;
-            acc.z += z[k] * sv.z;
-            acc.w += z[k] * sv.w;
-            au.x += z[k] * uv.x;
-            au.y += z[k] * uv.y;
-            au.z += z[k] * uv.z;
-        }
+        // ---- softmax and filter
+        const float2* b4 = reinterpret_cast<const float2*>(sbias + 192);
+        const float b48 = sbias[192 + 48], m = logit_max(tl, b4, b48);
+        const uint32_t base = img * P.G.pixels;
+        const bool interior = __all_sync(0xFFFFFFFFu, has && x >= 3 && y >= 3 && x + 3 < (int)P.G.width && y + 3 < (int)P.G.height);
+        float4 acc;
+        float3 au;
+        const float inv = 1.0f / (interior ? signal_filter<true>(tl, b4, b48, m, P.sig, P.uns, base, x, y, P.G, acc, au)
+                                           : signal_filter<false>(tl, b4, b48, m, P.sig, P.uns, base, x, y, P.G, acc, au));
+        acc = make_float4(acc.x * inv, acc.y * inv, acc.z * inv, acc.w * inv);
+        au = make_float3(au.x * inv, au.y * inv, au.z * inv);
         const float4 yv = make_float4(filtered_ratio(acc.x, au.x), filtered_ratio(acc.y, au.y),
                                       filtered_ratio(acc.z, au.z), acc.w);
-        const float4 tg = valid ? P.target[gp] : make_float4(0.f, 0.f, 0.f, 0.f);
-        const float4 err = valid ? make_float4(yv.x - tg.x, yv.y - tg.y, yv.z - tg.z, yv.w - tg.w)
+        const float4 err = valid ? make_float4(yv.x - tgt.x, yv.y - tgt.y, yv.z - tgt.z, yv.w - tgt.w)
                                  : make_float4(0.f, 0.f, 0.f, 0.f);
         const float4 cw = (P.weight && valid) ? P.weight[gp]
                                               : make_float4(P.shadow_weight, P.shadow_weight, P.shadow_weight, 1.0f);
@@ -833,73 +841,102 @@ __global__ void __launch_bounds__(128, 1) denoise_train_tc_kernel(TrainParams P,
         const float3 dq = make_float3(au.x > 0.f ? dy.x / au.x : 0.f, au.y > 0.f ? dy.y / au.y : 0.f,
                                       au.z > 0.f ? dy.z / au.z : 0.f);
         const float3 dr = make_float3(dq.x * yv.x, dq.y * yv.y, dq.z * yv.z);
-        float g[49];
-        float sdot = 0.f;
+        // sum(w g), g_k = dL/dw_k, from the sums of the filter
+        const float gw = dy.w * acc.w + (dq.x * acc.x - dr.x * au.x) + (dq.y * acc.y - dr.y * au.y) +
+                         (dq.z * acc.z - dr.z * au.z);
+        if (interior) signal_backward<true>(tl, b4, b48, m, inv, P.sig, P.uns, base, x, y, P.G, dy.w, dq, dr, gw, dz, row);
+        else signal_backward<false>(tl, b4, b48, m, inv, P.sig, P.uns, base, x, y, P.G, dy.w, dq, dr, gw, dz, row);
+        if (!has) {   // past the batch: whatever the clamped taps held counts for nothing
 #pragma unroll
-        for (int k = 0; k < 49; ++k) {
-            const float4 sv = signal_tap(P.sig, P.G, has, img, x, y, k);
-            const float4 uv = signal_tap(P.uns, P.G, has, img, x, y, k);
-            g[k] = dy.w * sv.w + (dq.x * sv.x - dr.x * uv.x) + (dq.y * sv.y - dr.y * uv.y) + (dq.z * sv.z - dr.z * uv.z);
-            sdot += z[k] * g[k];
+            for (uint32_t c = 0; c < 8; ++c)
+                *reinterpret_cast<uint4*>(dz + core_offset(row, c, 8u)) = make_uint4(0u, 0u, 0u, 0u);
         }
-#pragma unroll
-        for (int k = 0; k < 64; k += 2) {
-            const float lo = k < 49 ? z[k] * (g[k] - sdot) : 0.0f;
-            const float hi = k + 1 < 49 ? z[k + 1] * (g[k + 1] - sdot) : 0.0f;
-            const uint32_t w = pack2(lo, hi);
-            *reinterpret_cast<uint32_t*>(dz + elem_offset(row, (uint32_t)k, 8)) = w;
-            const __nv_bfloat162 q = *reinterpret_cast<const __nv_bfloat162*>(&w);
-            if (k < 49) *reinterpret_cast<__nv_bfloat16*>(dzt + elem_offset((uint32_t)k, row, 16)) = q.x;
-            if (k + 1 < 49) *reinterpret_cast<__nv_bfloat16*>(dzt + elem_offset((uint32_t)k + 1, row, 16)) = q.y;
-        }
-        // ---- backward: dW_l += dZ_l^T [H_{l-1} | 1]^T and dH_{l-1} = dZ_l W_l, l = 4..2;
-        // dW_1 += dZ_1^T [X | 1]^T
+        // ---- backward: dH_{l-1} = dZ_l W_l and dW_l^T += [H_{l-1} | 1]^T dZ_l, l = 4..2;
+        // dW_1^T += [X | 1]^T dZ_1
 #pragma unroll
         for (int l = 3; l >= 0; --l) {
-            tt_before_issue();
+            asm volatile("fence.proxy.async.shared::cta;");
+            asm volatile("tcgen05.fence::before_thread_sync;");
+            __syncthreads();
+            asm volatile("tcgen05.fence::after_thread_sync;");
             if (tid == 0) {
-                tc_mma(tmem + dw_col[l], dzt_addr, 16u, l == 0 ? xt_addr : ht_addr[l - 1], 16u, 8, tc_idesc(80),
-                       accumulated);
-                if (l > 0) tc_mma(tmem + kTtDH, dz_addr, 8u, wt[l - 1], 8u, 4, tc_idesc(64), false);
+                const uint32_t tile0 = smem_u32(tsm);
+                if (l > 0) {
+                    for (uint32_t t = 0; t < kTtGroups; ++t) {
+#pragma unroll
+                        for (int s = 0; s < 4; ++s)
+                            tc_mma1(tmem + 64u * t, k_major(tile0 + t * kTtTile + kTtDZ, 8, s), mn_major(w_addr[l], 8, s),
+                                    tc_idesc(false, true), s > 0);
+                        tc_commit(smem_u32(tsm + kTtBar + 8 * t));
+                    }
+                }
+                const uint32_t h = l == 0 ? kTtX : kTtH + (uint32_t)(l - 1) * kTtHBytes, hk = l == 0 ? kTtXK : kTtHK;
+                for (uint32_t t = 0; t < kTtGroups; ++t)
+#pragma unroll
+                    for (int s = 0; s < 8; ++s)
+                        tc_mma1(tmem + kTtDW + 64u * (uint32_t)l, mn_major(tile0 + t * kTtTile + h, hk, s),
+                                mn_major(tile0 + t * kTtTile + kTtDZ, 8, s), tc_idesc(true, true),
+                                accumulated || t > 0 || s > 0);
+                tc_commit(bar_w);
             }
-            tt_commit_wait(bar, phase, failed, status);
-            if (l > 0) tt_dz_out(tl + kTtDH, mask[l - 1], l > 1 ? dz : nullptr, dzt, row);
+            if (l > 0) {
+                tt_wait(bar, phase, failed, status);
+                uint32_t w[32];   // dZ_{l-1} = dH * ReLU'(h)
+#pragma unroll
+                for (int c0 = 0; c0 < 64; c0 += 16) {
+                    float v[16];
+                    tc_load16(tl + (uint32_t)c0, v);
+#pragma unroll
+                    for (int j = 0; j < 8; ++j)
+                        w[c0 / 2 + j] = pack2(((mask[l - 1] >> (c0 + 2 * j)) & 1u) ? v[2 * j] : 0.0f,
+                                              ((mask[l - 1] >> (c0 + 2 * j + 1)) & 1u) ? v[2 * j + 1] : 0.0f);
+                }
+                tt_wait(bar_w, phase_w, failed, status);   // dW_l has read dZ
+#pragma unroll
+                for (int c = 0; c < 8; ++c)
+                    *reinterpret_cast<uint4*>(dz + core_offset(row, (uint32_t)c, 8u)) =
+                        make_uint4(w[4 * c], w[4 * c + 1], w[4 * c + 2], w[4 * c + 3]);
+            }
         }
         accumulated = true;
     }
-    // ---- this block's partial gradient: lanes 0..63 of the dW columns (rows = outputs)
+    if (accumulated) tt_wait(bar_w, phase_w, failed, status);
+    if (failed) {   // products still in flight before the columns are read and freed
+        tc_wait(bar, phase ^ 1u);
+        tc_wait(bar_w, phase_w ^ 1u);
+    }
+    // ---- this block's partial gradient: lane = input (the ones column: the bias), column =
+    // output; the groups take two layers each
     float* out = P.partial + (size_t)blockIdx.x * kParams;
-    const uint32_t tl = tmem + lane_off;
 #pragma unroll
-    for (int l = 0; l < 4; ++l) {
+    for (int i = 0; i < 2; ++i) {
+        const int l = (int)group * 2 + i;
         const int nin = l == 0 ? 72 : 64, nout = l == 3 ? 49 : 64;
         const int ow = l == 0 ? oW1 : (l == 1 ? oW2 : (l == 2 ? oW3 : oW4));
         const int ob = l == 0 ? ob1 : (l == 1 ? ob2 : (l == 2 ? ob3 : ob4));
-        for (int c0 = 0; c0 < 80; c0 += 16) {
+        for (int c0 = 0; c0 < 64; c0 += 16) {
             float v[16];
-            tc_load16(tl + dw_col[l] + (uint32_t)c0, v);
-            if ((int)row < nout && accumulated) {
+            tc_load16(tmem + kTtDW + 64u * (uint32_t)l + lane_off + (uint32_t)c0, v);
 #pragma unroll
-                for (int j = 0; j < 16; ++j) {
-                    const int c = c0 + j;
-                    if (c < nin) out[ow + (int)row * nin + c] = v[j];
-                    else if (c == nin) out[ob + (int)row] = v[j];
-                }
+            for (int j = 0; j < 16; ++j) {
+                const int n = c0 + j;
+                const float g = accumulated ? v[j] : 0.0f;
+                if (n < nout && (int)row < nin) out[ow + n * nin + (int)row] = g;
+                else if (n < nout && (int)row == nin) out[ob + n] = g;
             }
         }
     }
     // loss of the block
-    loss += __shfl_xor_sync(0xFFFFFFFFu, loss, 1);
-    loss += __shfl_xor_sync(0xFFFFFFFFu, loss, 2);
-    loss += __shfl_xor_sync(0xFFFFFFFFu, loss, 4);
-    loss += __shfl_xor_sync(0xFFFFFFFFu, loss, 8);
-    loss += __shfl_xor_sync(0xFFFFFFFFu, loss, 16);
-    __shared__ float s_loss[4];
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) loss += __shfl_xor_sync(0xFFFFFFFFu, loss, o);
     if ((tid & 31) == 0) s_loss[warp] = loss;
-    if (failed) tc_wait(bar, phase ^ 1u);
     asm volatile("tcgen05.fence::before_thread_sync;");
     __syncthreads();
-    if (tid == 0) P.partial_loss[blockIdx.x] = s_loss[0] + s_loss[1] + s_loss[2] + s_loss[3];
+    if (tid == 0) {
+        float t = 0.f;
+        for (int w = 0; w < kTtThreads / 32; ++w) t += s_loss[w];
+        P.partial_loss[blockIdx.x] = t;
+    }
     if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" :: "r"(tmem), "r"(kTtAlloc));
 }
 
@@ -932,7 +969,7 @@ __global__ void adam_kernel(float* w, float* m, float* v, const float* grad, flo
     w[i] -= lr * (mi / bc1) / (sqrtf(vi / bc2) + eps);
 }
 
-// FP32 master → packed BF16 weights (n-major + transposed copies) and padded biases.
+// FP32 master → packed BF16 weights (n-major) and padded biases.
 __global__ void pack_kernel(const float* w, __nv_bfloat16* pk, float* bias) {
     int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i < pEnd) {
@@ -940,10 +977,7 @@ __global__ void pack_kernel(const float* w, __nv_bfloat16* pk, float* bias) {
         if (i < pW2) { int n = i / sW1, k = i % sW1; v = k < 72 ? w[oW1 + n * 72 + k] : 0.f; }
         else if (i < pW3) { int j = i - pW2, n = j / sW, k = j % sW; v = k < 64 ? w[oW2 + n * 64 + k] : 0.f; }
         else if (i < pW4) { int j = i - pW3, n = j / sW, k = j % sW; v = k < 64 ? w[oW3 + n * 64 + k] : 0.f; }
-        else if (i < pW2T) { int j = i - pW4, n = j / sW, k = j % sW; v = (k < 64 && n < 49) ? w[oW4 + n * 64 + k] : 0.f; }
-        else if (i < pW3T) { int j = i - pW2T, n = j / sW, k = j % sW; v = k < 64 ? w[oW2 + k * 64 + n] : 0.f; }
-        else if (i < pW4T) { int j = i - pW3T, n = j / sW, k = j % sW; v = k < 64 ? w[oW3 + k * 64 + n] : 0.f; }
-        else { int j = i - pW4T, n = j / sW, k = j % sW; v = k < 49 ? w[oW4 + k * 64 + n] : 0.f; }
+        else { int j = i - pW4, n = j / sW, k = j % sW; v = (k < 64 && n < 49) ? w[oW4 + n * 64 + k] : 0.f; }
         pk[i] = __float2bfloat16(v);
     }
     if (i < kBias) {
@@ -1024,13 +1058,13 @@ static luz_status run_infer(luz_ctx* ctx, luz_denoiser* d, const luz_denoise_bat
     P.lin_depth = b->lin_depth;
     P.sig = (const float4*)b->noisy;
     P.uns = (const float4*)b->unshadowed;
-    P.G = ImageGeom{b->width, b->height, b->width * b->height, b->images};
+    P.G = image_geom(b->width, b->height, b->images);
+    P.tiles = tile_count(P.G);
     P.out = out;
     P.out_ao = out_ao;
     P.list = list;
     P.list_count = list_count;
-    uint32_t tiles = (P.G.pixels * P.G.images + 127) / 128;
-    uint32_t grid = std::min<uint32_t>((tiles + kTcGroups - 1) / kTcGroups, (uint32_t)ctx->sm_count * kTcBlocksPerSm);
+    uint32_t grid = std::min<uint32_t>((P.tiles + kTcGroups - 1) / kTcGroups, (uint32_t)ctx->sm_count * kTcBlocksPerSm);
     prof_begin(ctx, LUZ_KERNEL_DENOISE);
     denoise_infer_tc_kernel<<<grid, kTcThreads, kTcSmem, ctx->stream>>>(P, ctx->d_status);
     prof_end(ctx);
@@ -1049,12 +1083,12 @@ static luz_status run_gradient(luz_ctx* ctx, luz_denoiser* d, const luz_denoise_
     P.uns = (const float4*)b->unshadowed;
     P.target = (const float4*)b->target;
     P.weight = (const float4*)b->weight;
-    P.G = ImageGeom{b->width, b->height, b->width * b->height, b->images};
+    P.G = image_geom(b->width, b->height, b->images);
+    P.tiles = tile_count(P.G);
     P.grad_scale = 2.0f / (float)((double)P.G.pixels * P.G.images);
     P.shadow_weight = d->shadow_weight;
     P.partial = d->partial;
     P.partial_loss = d->partial_loss;
-    LUZ_CUDA(ctx, cudaMemsetAsync(d->partial, 0, (size_t)d->ctas * kParams * 4, ctx->stream));
     static DeviceSetup setup;
     luz_status st = device_setup(setup, setup_generation(), kTtSmem, [&]() -> luz_status {
         LUZ_CUDA(ctx, cudaFuncSetAttribute(denoise_train_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -1063,7 +1097,7 @@ static luz_status run_gradient(luz_ctx* ctx, luz_denoiser* d, const luz_denoise_
     });
     if (st != LUZ_OK) return st;
     prof_begin(ctx, LUZ_KERNEL_DENOISE_TRAIN);
-    denoise_train_tc_kernel<<<d->ctas, 128, kTtSmem, ctx->stream>>>(P, ctx->d_status);
+    denoise_train_tc_kernel<<<d->ctas, kTtThreads, kTtSmem, ctx->stream>>>(P, ctx->d_status);
     prof_end(ctx);
     LUZ_LAUNCHED(ctx, "denoise_train_tc_kernel");
     reduce_partials_kernel<<<(kParams + 255) / 256, 256, 0, ctx->stream>>>(d->partial, d->ctas, d->grad,
@@ -1213,7 +1247,7 @@ static luz_status launch_features(luz_ctx* ctx, luz_frame* f, bool for_denoise) 
     F.list_count = f->dn_count;
     if (for_denoise) LUZ_CUDA(ctx, cudaMemsetAsync(f->dn_count, 0, 4, ctx->stream));
     prof_begin(ctx, LUZ_KERNEL_FEATURES);
-    features_kernel<<<(f->pixels + 255) / 256, 256, 0, ctx->stream>>>(F);
+    features_kernel<<<((f->width + 15) / 16) * ((f->height + 15) / 16), 256, 0, ctx->stream>>>(F);
     prof_end(ctx);
     LUZ_LAUNCHED(ctx, "denoise_features_kernel");
     return LUZ_OK;
