@@ -591,25 +591,35 @@ __global__ void bvh4_emit_kernel(const SegDesc* segs, const uint32_t* seg_node_o
 }
 
 
-__global__ void __launch_bounds__(1024) tlas_bvh4_kernel(const float4* nodes, uint32_t m, const uint32_t* levels,
-                                                         float4* nodes4) {
-    tlas_bvh4_block(nodes, m, levels, nodes4);
-}
-
 // ---------------------------------------------------------------- TLAS
 
+// Ordered keys of a box centre's bounds (an empty range where there is none), reduced over
+// the warp and merged by its first lane.
+__device__ __forceinline__ void merge_bounds(bool have, V3 c, uint32_t* bounds) {
+    uint32_t k[6] = {0xFFFFFFFFu, 0xFFFFFFFFu, 0xFFFFFFFFu, 0u, 0u, 0u};
+    if (have) {
+        k[0] = k[3] = float_to_ordered(c.x);
+        k[1] = k[4] = float_to_ordered(c.y);
+        k[2] = k[5] = float_to_ordered(c.z);
+    }
+#pragma unroll
+    for (int a = 0; a < 6; ++a)
+        k[a] = a < 3 ? __reduce_min_sync(0xFFFFFFFFu, k[a]) : __reduce_max_sync(0xFFFFFFFFu, k[a]);
+    if ((threadIdx.x & 31) == 0) {
+#pragma unroll
+        for (int a = 0; a < 3; ++a) atomicMin(bounds + a, k[a]);
+#pragma unroll
+        for (int a = 3; a < 6; ++a) atomicMax(bounds + a, k[a]);
+    }
+}
+
+// seg_bounds: NULL where the next kernel takes the bounds from the boxes.
 __global__ void tlas_instance_kernel(const DevInstanceInput* in, uint32_t n, float4* inst_box,
                                      DevShadeInstance* shade, uint32_t* seg_bounds) {
-    uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
+    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     V3 c;
-    if (!tlas_instance_one(in, i, inst_box, shade, c)) return;
-    atomicMin(seg_bounds + 0, float_to_ordered(c.x));
-    atomicMin(seg_bounds + 1, float_to_ordered(c.y));
-    atomicMin(seg_bounds + 2, float_to_ordered(c.z));
-    atomicMax(seg_bounds + 3, float_to_ordered(c.x));
-    atomicMax(seg_bounds + 4, float_to_ordered(c.y));
-    atomicMax(seg_bounds + 5, float_to_ordered(c.z));
+    const bool have = i < n && tlas_instance_one(in, i, inst_box, shade, c);
+    if (seg_bounds) merge_bounds(have, c, seg_bounds);
 }
 
 __global__ void tlas_setup_kernel(uint32_t* bounds, SegDesc* seg, SegDesc value, uint32_t* zero) {
@@ -641,19 +651,344 @@ __global__ void tlas_emit_kernel(const DevInstanceInput* in, const float4* inst_
     tlas_emit_one(in, inst_box, j, keys[j], vals[j], inst_out, leaf_box, morton_out, order_out);
 }
 
-
-
-__global__ void __launch_bounds__(1024)
-bfs_relayout_kernel(const float4* src, float4* dst, uint32_t m, uint32_t* queue,
-                    uint32_t* newidx, uint32_t* levels) {
-    bfs_relayout_block(src, dst, m, queue, newidx, levels);
+__global__ void tlas_record_kernel(const DevInstanceInput* in, const uint32_t* order, uint32_t n, DevInstance* inst_out) {
+    uint32_t j = blockIdx.x * blockDim.x + threadIdx.x;
+    if (j < n) tlas_emit_record(in, j, order[j], inst_out);
 }
 
-// The TLAS build of tlas_build_block as one CTA of 1024 threads.
+constexpr uint32_t kTlasLevels = 64;   // above the depth of 30-bit codes split by index
+
+// Breadth-first relayout and 4-wide collapse of a tree too large for tlas_fused_kernel. A
+// node's place is its level's start plus its rank among the level's node indices: one pass
+// of the radix sort over (depth, node), stable and with the depth as its digit, gives the
+// order, and the digits' offsets are the level table. Every step takes the whole chip
+// (8000 instances: relayout and collapse by one block, level by level, 119 us; these kernels
+// and their sort pass 27).
+__global__ void tlas_depth_kernel(const uint32_t* node_parent, uint32_t m, unsigned long long* keys, uint32_t* vals) {
+    const uint32_t q = blockIdx.x * blockDim.x + threadIdx.x;
+    if (q >= m) return;
+    uint32_t d = 0, p = node_parent[q];
+    while (p != 0xFFFFFFFFu && d + 1 < kTlasLevels) {
+        ++d;
+        p = node_parent[p >> 1];
+    }
+    keys[q] = d;
+    vals[q] = q;
+}
+
+// Level table {L, start_0, ..., start_L}, and the inverse of the order.
+__global__ void tlas_newidx_kernel(const uint32_t* order, uint32_t m, const uint32_t* offsets, uint32_t* newidx,
+                                   uint32_t* levels) {
+    const uint32_t b = blockIdx.x * blockDim.x + threadIdx.x;
+    if (b < m) newidx[order[b]] = b;
+    if (b < kTlasLevels && offsets[b] < m) {
+        levels[1 + b] = offsets[b];
+        if (offsets[b + 1] == m) {
+            levels[0] = b + 1;
+            levels[2 + b] = m;
+        }
+    }
+}
+
+__global__ void __launch_bounds__(128) tlas_relayout_kernel(const float4* __restrict__ src,
+                                                            const unsigned long long* __restrict__ depth,
+                                                            const uint32_t* __restrict__ order,
+                                                            const uint32_t* __restrict__ newidx, uint32_t m,
+                                                            const uint32_t* __restrict__ levels, float4* dst, float4* nodes4) {
+    __shared__ uint32_t s_start[kTlasLevels + 1], s_even[kTlasLevels];
+    const uint32_t L = levels[0];
+    if (threadIdx.x <= L) s_start[threadIdx.x] = levels[1 + threadIdx.x];
+    __syncthreads();
+    if (threadIdx.x < L) {
+        uint32_t acc = 0;
+        for (uint32_t l = 0; l < threadIdx.x; l += 2) acc += s_start[l + 1] - s_start[l];
+        s_even[threadIdx.x] = acc;   // 4-wide nodes before this level
+    }
+    __syncthreads();
+    const uint32_t b = blockIdx.x * blockDim.x + threadIdx.x;
+    if (b >= m) return;
+    const uint32_t d = (uint32_t)depth[b];
+    const float4* s = src + (size_t)order[b] * kNodeF4;
+    const float4 n0 = s[0], n1 = s[1], n2 = s[2], n3 = s[3];
+    const int c[2] = {__float_as_int(n3.x), __float_as_int(n3.y)};
+    float4* o = dst + (size_t)b * kNodeF4;
+    o[0] = n0;
+    o[1] = n1;
+    o[2] = n2;
+    o[3] = make_float4(__int_as_float(c[0] < 0 ? c[0] : (int)newidx[c[0]]),
+                       __int_as_float(c[1] < 0 ? c[1] : (int)newidx[c[1]]), 0.f, 0.f);
+    if (d & 1u) return;
+    Slot4 s4;
+    s4.k = 0;
+    for (int side = 0; side < 2; ++side) {
+        if (c[side] < 0) {
+            slot4_put(s4, s, side, c[side]);
+            continue;
+        }
+        const float4* k = src + (size_t)c[side] * kNodeF4;
+        const float4 k3 = k[3];
+        const int g[2] = {__float_as_int(k3.x), __float_as_int(k3.y)};
+        for (int t = 0; t < 2; ++t)
+            slot4_put(s4, k, t, g[t] < 0 ? g[t] : (int)(s_even[d + 2] + newidx[g[t]] - s_start[d + 2]));
+    }
+    slot4_store(s4, nodes4 + (size_t)(s_even[d] + b - s_start[d]) * kNode4F4);
+}
+
+// Shared memory of tlas_fused_kernel for n instances: sort keys (their space holds the
+// arrival flags later), the nodes' own boxes, children, parents, breadth-first ranks and
+// depths. 43 bytes an instance: 172 KB at kFusedTlasMax.
+struct TlasShared {
+    uint32_t keys;       // power of two, at least a warp
+    uint32_t nodes;
+    size_t box, child, parent, leaf_parent, rank, depth, bytes;
+};
+__host__ __device__ inline TlasShared tlas_shared(uint32_t n) {
+    TlasShared s;
+    s.keys = 32;
+    while (s.keys < n) s.keys <<= 1;
+    s.nodes = n > 2 ? n - 1 : 1;
+    s.box = (size_t)s.keys * 8;
+    s.child = s.box + (size_t)s.nodes * 24;
+    s.parent = s.child + (size_t)s.nodes * 4;
+    s.leaf_parent = s.parent + (size_t)s.nodes * 2;
+    s.rank = s.leaf_parent + (size_t)n * 2;
+    s.depth = s.rank + (size_t)s.nodes * 2;
+    s.bytes = s.depth + s.nodes;
+    return s;
+}
+constexpr uint32_t kTlasOneBlock = 768;
+
+// The whole TLAS build of up to kFusedTlasMax instances as one block: the same results as
+// the kernels of the larger builds, bit for bit. Bound by latency: a few dozen steps that
+// each wait for the one before, so the tree lives in shared memory and only records that
+// outlive the build go to device memory. Three things keep the steps few: the sort network's
+// distances below a warp run in registers (34 barriers for 4096 keys instead of 78); a
+// node's place in breadth-first order is its level's start plus its rank among the level's
+// node indices (the ranges of a level are disjoint and a node's index lies in its own), one
+// stable counting sort by depth in place of a pass per level; and a node's box is kept
+// once, as its own box, so that the refit, the relayout and the 4-wide collapse read
+// shared memory. 65 instances: 36 -> 15 us; 201: 52 -> 19; 1024: 85 -> 42
+// (three kernels); 4096: 264 -> 153 (the same build with the tree in device memory, a pass
+// per level).
+//
+// kTreeOnly: the instance boxes are there, and the records are written from the order
+// by a kernel after this one; both take the whole chip, where one block is bound by its own
+// loads and inverses. Three kernels from kTlasOneBlock on: 500 instances 28.8 us and two
+// gaps of 2.5 against 29.0, 700 36.6 and the gaps against 38.4, 1024 42.3 against 50.4.
+template <bool kTreeOnly>
 __global__ void __launch_bounds__(1024) tlas_fused_kernel(TlasBuildArgs A, uint32_t* dev_status) {
-    __shared__ unsigned long long s_keys[kFusedTlasMax];
-    __shared__ uint32_t s_bounds[6];
-    tlas_build_block<TlasBuildArgs>(A, s_keys, s_bounds, dev_status);
+    extern __shared__ unsigned long long s_keys[];
+    __shared__ uint32_t s_bounds[6], s_total[kTlasLevels], s_start[kTlasLevels + 1], s_even[kTlasLevels + 1];
+    __shared__ uint16_t s_count[32][kTlasLevels];
+    const uint32_t full = 0xFFFFFFFFu, tid = threadIdx.x, nt = blockDim.x, lane = tid & 31, warp = tid >> 5;
+    const uint32_t n = A.n;
+    const TlasShared L = tlas_shared(n);
+    const uint32_t P = L.keys, m = L.nodes;
+    char* base = reinterpret_cast<char*>(s_keys);
+    float* s_box = reinterpret_cast<float*>(base + L.box);   // [6][m]
+    short2* s_child = reinterpret_cast<short2*>(base + L.child);
+    uint16_t* s_parent = reinterpret_cast<uint16_t*>(base + L.parent);
+    uint16_t* s_leaf_parent = reinterpret_cast<uint16_t*>(base + L.leaf_parent);
+    uint16_t* s_rank = reinterpret_cast<uint16_t*>(base + L.rank);
+    uint8_t* s_depth = reinterpret_cast<uint8_t*>(base + L.depth);
+    uint32_t* s_flag = reinterpret_cast<uint32_t*>(s_keys);
+
+    if (tid < 6) s_bounds[tid] = tid < 3 ? 0xFFFFFFFFu : 0u;
+    for (uint32_t q = tid; q < m; q += nt) s_parent[q] = 0xFFFFu;
+    for (uint32_t g = tid; g < n; g += nt) s_leaf_parent[g] = 0xFFFFu;
+    __syncthreads();
+    // instance boxes and the bounds of their centres
+    for (uint32_t i = tid; i < P; i += nt) {
+        V3 c;
+        bool have = false;
+        if (i < n) {
+            if (kTreeOnly) {
+                const float4 l = A.inst_box[2 * i], h = A.inst_box[2 * i + 1];
+                c = V3{(l.x + h.x) * 0.5f + 0.0f, (l.y + h.y) * 0.5f + 0.0f, (l.z + h.z) * 0.5f + 0.0f};
+                have = finite3(c);
+            } else {
+                have = tlas_instance_one(A.in, i, A.inst_box, A.shade, c);
+            }
+        }
+        merge_bounds(have, c, s_bounds);
+    }
+    __syncthreads();
+    // (Morton code, index) sorted: the stable order of the radix sort. Steps of 32 keys and
+    // more exchange through shared memory, shorter ones between the lanes of a warp.
+    {
+        V3 cmin, ext;
+        decode_bounds(s_bounds, cmin, ext);
+        for (uint32_t i = tid; i < P; i += nt) {
+            unsigned long long v = ~0ull;
+            if (i < n) {
+                const float4 l = A.inst_box[2 * i], h = A.inst_box[2 * i + 1];
+                const unsigned long long code = morton30(V3{l.x, l.y, l.z}, V3{h.x, h.y, h.z}, cmin, ext);
+                v = (code << 32) | i;
+            }
+#pragma unroll
+            for (uint32_t k = 2; k <= 32; k <<= 1)
+#pragma unroll
+                for (uint32_t j = k >> 1; j > 0; j >>= 1) {
+                    const unsigned long long o = __shfl_xor_sync(full, v, j);
+                    v = ((i & j) == 0) == ((i & k) == 0) ? min(v, o) : max(v, o);
+                }
+            s_keys[i] = v;
+        }
+    }
+    __syncthreads();
+    for (uint32_t k = 64; k <= P; k <<= 1) {
+        for (uint32_t j = k >> 1; j >= 32; j >>= 1) {
+            for (uint32_t t = tid; t < P / 2; t += nt) {
+                const uint32_t i = 2 * t - (t & (j - 1));
+                const unsigned long long a = s_keys[i], b = s_keys[i + j];
+                if ((a > b) == ((i & k) == 0)) { s_keys[i] = b; s_keys[i + j] = a; }
+            }
+            __syncthreads();
+        }
+        for (uint32_t i = tid; i < P; i += nt) {
+            unsigned long long v = s_keys[i];
+#pragma unroll
+            for (uint32_t j = 16; j > 0; j >>= 1) {
+                const unsigned long long o = __shfl_xor_sync(full, v, j);
+                v = ((i & j) == 0) == ((i & k) == 0) ? min(v, o) : max(v, o);
+            }
+            s_keys[i] = v;
+        }
+        __syncthreads();
+    }
+    // leaves, and the hierarchy
+    for (uint32_t j = tid; j < n; j += nt) {
+        const uint32_t i = (uint32_t)s_keys[j];
+        tlas_emit_leaf(A.inst_box, j, s_keys[j] >> 32, i, A.leaf_box, A.morton_out, A.order_out);
+        if (!kTreeOnly) tlas_emit_record(A.in, j, i, A.inst_out);
+    }
+    if (n == 1) {
+        if (tid == 0) {
+            const float inf = __int_as_float(0x7f800000);
+            const float4 lo = A.leaf_box[0], hi = A.leaf_box[1];
+            A.nodes_out[0] = make_float4(lo.x, hi.x, lo.y, hi.y);
+            A.nodes_out[1] = make_float4(inf, -inf, inf, -inf);
+            A.nodes_out[2] = make_float4(lo.z, hi.z, inf, -inf);
+            A.nodes_out[3] = make_float4(__int_as_float(~0), __int_as_float(kEmptyChild), 0.f, 0.f);
+            Slot4 s4;
+            s4.k = 0;
+            slot4_put(s4, lo, hi, ~0);
+            slot4_store(s4, A.nodes4);
+            A.levels[0] = 1u;
+            A.levels[1] = 0u;
+            A.levels[2] = 1u;
+        }
+        return;
+    }
+    for (uint32_t i = tid; i < m; i += nt) {
+        int lo, hi, gamma;
+        if (!karras_range([](int j) { return (uint32_t)(s_keys[j] >> 32); }, (int)n, (int)i, lo, hi, gamma, dev_status))
+            continue;
+        const int c0 = lo == gamma ? ~gamma : gamma, c1 = hi == gamma + 1 ? ~(gamma + 1) : gamma + 1;
+        (c0 < 0 ? s_leaf_parent : s_parent)[gamma] = (uint16_t)(i << 1);
+        (c1 < 0 ? s_leaf_parent : s_parent)[gamma + 1] = (uint16_t)((i << 1) | 1u);
+        s_child[i] = make_short2((short)c0, (short)c1);
+    }
+    __syncthreads();
+    // breadth-first ranks: a stable counting sort of the node indices by depth
+    for (uint32_t q = tid; q < m; q += nt) {
+        uint32_t d = 0, p = s_parent[q];
+        while (p != 0xFFFFu && d + 1 < kTlasLevels) {
+            ++d;
+            p = s_parent[p >> 1];
+        }
+        s_depth[q] = (uint8_t)d;
+        s_flag[q] = 0u;   // the keys have been read
+    }
+    for (uint32_t l = tid; l < kTlasLevels; l += nt) s_total[l] = 0u;
+    for (uint32_t b = 0; b < m; b += nt) {
+        for (uint32_t k = tid; k < (nt >> 5) * kTlasLevels; k += nt) (&s_count[0][0])[k] = 0u;
+        __syncthreads();
+        const uint32_t q = b + tid, d = q < m ? s_depth[q] : kTlasLevels;
+        const uint32_t peers = __match_any_sync(full, d), before = __popc(peers & ((1u << lane) - 1u));
+        if (q < m && before == 0) s_count[warp][d] = (uint16_t)__popc(peers);
+        __syncthreads();
+        for (uint32_t l = tid; l < kTlasLevels; l += nt) {
+            uint32_t run = s_total[l];
+            for (uint32_t w = 0; w < nt >> 5; ++w) {
+                const uint32_t t = s_count[w][l];
+                s_count[w][l] = (uint16_t)run;
+                run += t;
+            }
+            s_total[l] = run;
+        }
+        __syncthreads();
+        if (q < m) s_rank[q] = (uint16_t)(s_count[warp][d] + before);
+        __syncthreads();
+    }
+    if (tid == 0) {
+        uint32_t at = 0, even = 0, l = 0;
+        for (; l < kTlasLevels && s_total[l]; ++l) {
+            s_start[l] = at;
+            s_even[l] = even;
+            A.levels[1 + l] = at;
+            at += s_total[l];
+            if (!(l & 1u)) even += s_total[l];
+        }
+        A.levels[0] = l;
+        A.levels[1 + l] = at;
+    }
+    __syncthreads();
+    // refit: the second child to arrive at a node completes it
+    auto box_of = [&](int c, float4& lo, float4& hi) {
+        if (c < 0) {
+            lo = A.leaf_box[2 * ~c];
+            hi = A.leaf_box[2 * ~c + 1];
+        } else {
+            lo = make_float4(s_box[c], s_box[m + c], s_box[2 * m + c], 0.f);
+            hi = make_float4(s_box[3 * m + c], s_box[4 * m + c], s_box[5 * m + c], 0.f);
+        }
+    };
+    for (uint32_t g = tid; g < n; g += nt) {
+        float4 lo = A.leaf_box[2 * g], hi = A.leaf_box[2 * g + 1];
+        uint32_t p = s_leaf_parent[g];
+        while (p != 0xFFFFu) {   // at most the tree's depth
+            const uint32_t i = p >> 1;
+            __threadfence_block();
+            if (atomicAdd(s_flag + i, 1u) != 1u) break;
+            __threadfence_block();
+            const short2 c = s_child[i];
+            float4 lo0 = lo, hi0 = hi, lo1 = lo, hi1 = hi;
+            if (p & 1u) box_of(c.x, lo0, hi0);
+            else box_of(c.y, lo1, hi1);
+            lo = make_float4(fmin_(lo0.x, lo1.x), fmin_(lo0.y, lo1.y), fmin_(lo0.z, lo1.z), 0.f);
+            hi = make_float4(fmax_(hi0.x, hi1.x), fmax_(hi0.y, hi1.y), fmax_(hi0.z, hi1.z), 0.f);
+            s_box[i] = lo.x; s_box[m + i] = lo.y; s_box[2 * m + i] = lo.z;
+            s_box[3 * m + i] = hi.x; s_box[4 * m + i] = hi.y; s_box[5 * m + i] = hi.z;
+            float4* node = A.nodes_out + (size_t)(s_start[s_depth[i]] + s_rank[i]) * kNodeF4;
+            const int c0 = c.x < 0 ? c.x : (int)(s_start[s_depth[c.x]] + s_rank[c.x]);
+            const int c1 = c.y < 0 ? c.y : (int)(s_start[s_depth[c.y]] + s_rank[c.y]);
+            node[0] = make_float4(lo0.x, hi0.x, lo0.y, hi0.y);
+            node[1] = make_float4(lo1.x, hi1.x, lo1.y, hi1.y);
+            node[2] = make_float4(lo0.z, hi0.z, lo1.z, hi1.z);
+            node[3] = make_float4(__int_as_float(c0), __int_as_float(c1), 0.f, 0.f);
+            p = s_parent[i];
+        }
+    }
+    __syncthreads();
+    // 4-wide nodes: the even levels, a slot per grandchild (or child, where that is a leaf)
+    for (uint32_t i = tid; i < m; i += nt) {
+        const uint32_t d = s_depth[i];
+        if (d & 1u) continue;
+        Slot4 s4;
+        s4.k = 0;
+        auto put = [&](int c) {
+            float4 lo, hi;
+            box_of(c, lo, hi);
+            slot4_put(s4, lo, hi, c < 0 ? c : (int)(s_even[s_depth[c]] + s_rank[c]));
+        };
+        const short2 c = s_child[i];
+        if (c.x < 0) put(c.x);
+        else { const short2 k = s_child[c.x]; put(k.x); put(k.y); }
+        if (c.y < 0) put(c.y);
+        else { const short2 k = s_child[c.y]; put(k.x); put(k.y); }
+        slot4_store(s4, A.nodes4 + (size_t)(s_even[d] + s_rank[i]) * kNode4F4);
+    }
 }
 
 // ---------------------------------------------------------------- host drivers
@@ -1042,16 +1377,33 @@ luz_status launch_tlas_build(luz_ctx* ctx, luz_tlas* t) {
     uint32_t* leaf_parent = A.leaf_parent;
     uint32_t* flags = A.flags;
     float4* karras_nodes = A.karras_nodes;
-    uint32_t* queue = A.queue;
     uint32_t* newidx = A.newidx;
     SegDesc* d_seg = ts.d_seg;
     uint32_t* d_zero = ts.d_zero;
 
     if (n <= kFusedTlasMax) {
+        static DeviceSetup setup;   // the kernel's shared-memory limit
+        luz_status s = device_setup(setup, setup_generation(), 1, [&]() -> luz_status {
+            for (const void* fn : {(const void*)tlas_fused_kernel<false>, (const void*)tlas_fused_kernel<true>})
+                LUZ_CUDA(ctx, cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                   (int)tlas_shared(kFusedTlasMax).bytes));
+            return LUZ_OK;
+        });
+        if (s != LUZ_OK) return s;
+        const uint32_t threads = std::min(std::max((n + 31u) & ~31u, 64u), 1024u);
         prof_begin(ctx, LUZ_KERNEL_TLAS_BUILD);
-        tlas_fused_kernel<<<1, 1024, 0, st>>>(A, ctx->d_status);
+        if (n <= kTlasOneBlock) {
+            tlas_fused_kernel<false><<<1, threads, tlas_shared(n).bytes, st>>>(A, ctx->d_status);
+            LUZ_LAUNCHED(ctx, "tlas_fused_kernel");
+        } else {
+            tlas_instance_kernel<<<cdiv(n, 64), 64, 0, st>>>(A.in, n, A.inst_box, A.shade, nullptr);
+            LUZ_LAUNCHED(ctx, "tlas_instance_kernel");
+            tlas_fused_kernel<true><<<1, threads, tlas_shared(n).bytes, st>>>(A, ctx->d_status);
+            LUZ_LAUNCHED(ctx, "tlas_fused_kernel<tree>");
+            tlas_record_kernel<<<cdiv(n, 64), 64, 0, st>>>(A.in, A.order_out, n, A.inst_out);
+            LUZ_LAUNCHED(ctx, "tlas_record_kernel");
+        }
         prof_end(ctx);
-        LUZ_LAUNCHED(ctx, "tlas_fused_kernel");
         return LUZ_OK;
     }
     SegDesc sd{};
@@ -1085,10 +1437,14 @@ luz_status launch_tlas_build(luz_ctx* ctx, luz_tlas* t) {
     refit_kernel<<<cdiv(n, 128), 128, 0, st>>>(d_seg, d_zero, 1, n, leaf_box, node_parent,
                                                leaf_parent, flags);
     LUZ_LAUNCHED(ctx, "refit_kernel");
-    bfs_relayout_kernel<<<1, 1024, 0, st>>>(karras_nodes, t->nodes, m, queue, newidx, t->levels);
-    LUZ_LAUNCHED(ctx, "bfs_relayout_kernel");
-    tlas_bvh4_kernel<<<1, 1024, 0, st>>>(t->nodes, m, t->levels, t->nodes4);
-    LUZ_LAUNCHED(ctx, "tlas_bvh4_kernel");
+    tlas_depth_kernel<<<cdiv(m, 128), 128, 0, st>>>(node_parent, m, sb.keys[0], sb.vals[0]);
+    LUZ_LAUNCHED(ctx, "tlas_depth_kernel");
+    if ((s = run_sort(ctx, sb, m, 1, res)) != LUZ_OK) return s;
+    tlas_newidx_kernel<<<cdiv(m, 128), 128, 0, st>>>(sb.vals[res], m, sb.offsets, newidx, t->levels);
+    LUZ_LAUNCHED(ctx, "tlas_newidx_kernel");
+    tlas_relayout_kernel<<<cdiv(m, 128), 128, 0, st>>>(karras_nodes, sb.keys[res], sb.vals[res], newidx, m, t->levels,
+                                                       t->nodes, t->nodes4);
+    LUZ_LAUNCHED(ctx, "tlas_relayout_kernel");
     return LUZ_OK;
 }
 

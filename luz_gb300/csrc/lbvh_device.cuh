@@ -23,11 +23,42 @@ __device__ __forceinline__ void decode_bounds(const uint32_t* b, V3& cmin, V3& e
     ext = cmax - cmin;
 }
 
-__device__ __forceinline__ int kdelta(const unsigned long long* keys, int n, int i, int j) {
+// key(j): the 30-bit Morton code at sorted position j.
+template <typename Key>
+__device__ __forceinline__ int kdelta(const Key& key, int n, int i, int j) {
     if (j < 0 || j >= n) return -1;
-    uint32_t ki = (uint32_t)keys[i] & 0x3FFFFFFFu, kj = (uint32_t)keys[j] & 0x3FFFFFFFu;
+    const uint32_t ki = key(i), kj = key(j);
     if (ki != kj) return __clz(ki ^ kj);
     return 32 + __clz((uint32_t)i ^ (uint32_t)j);
+}
+
+// Leaf range [lo, hi] of internal node i of n >= 2 keys and the last leaf of its left
+// child (gamma). False when the keys are not sorted (status word raised).
+template <typename Key>
+__device__ __forceinline__ bool karras_range(const Key& key, int n, int i, int& lo, int& hi, int& gamma,
+                                             uint32_t* dev_status) {
+    int d = (kdelta(key, n, i, i + 1) - kdelta(key, n, i, i - 1)) >= 0 ? 1 : -1;
+    int dmin = kdelta(key, n, i, i - d);
+    int lmax = 2;
+    int guard = 0;
+    while (kdelta(key, n, i, i + lmax * d) > dmin) {
+        lmax <<= 1;
+        if (++guard > 40) { atomicOr(dev_status, (uint32_t)LUZ_DEV_KARRAS_RANGE); return false; }
+    }
+    int l = 0;
+    for (int t = lmax >> 1; t >= 1; t >>= 1)
+        if (kdelta(key, n, i, i + (l + t) * d) > dmin) l += t;
+    int j = i + l * d;
+    int dnode = kdelta(key, n, i, j);
+    int split = 0, step = l;
+    do {
+        step = (step + 1) >> 1;
+        if (kdelta(key, n, i, i + (split + step) * d) > dnode) split += step;
+    } while (step > 1);
+    gamma = i + split * d + min(d, 0);
+    lo = min(i, j);
+    hi = max(i, j);
+    return true;
 }
 
 __device__ __forceinline__ void write_inverted_slot(float4* node, int slot) {
@@ -60,26 +91,8 @@ __device__ __forceinline__ void karras_node(const SegDesc& sd, int i, const unsi
         return;
     }
     const unsigned long long* k = keys + sd.prim_off;
-    int d = (kdelta(k, n, i, i + 1) - kdelta(k, n, i, i - 1)) >= 0 ? 1 : -1;
-    int dmin = kdelta(k, n, i, i - d);
-    int lmax = 2;
-    int guard = 0;
-    while (kdelta(k, n, i, i + lmax * d) > dmin) {
-        lmax <<= 1;
-        if (++guard > 40) { atomicOr(dev_status, (uint32_t)LUZ_DEV_KARRAS_RANGE); return; }
-    }
-    int l = 0;
-    for (int t = lmax >> 1; t >= 1; t >>= 1)
-        if (kdelta(k, n, i, i + (l + t) * d) > dmin) l += t;
-    int j = i + l * d;
-    int dnode = kdelta(k, n, i, j);
-    int split = 0, step = l;
-    do {
-        step = (step + 1) >> 1;
-        if (kdelta(k, n, i, i + (split + step) * d) > dnode) split += step;
-    } while (step > 1);
-    int gamma = i + split * d + min(d, 0);
-    int lo = min(i, j), hi = max(i, j);
+    int lo, hi, gamma;
+    if (!karras_range([k](int j) { return (uint32_t)k[j] & 0x3FFFFFFFu; }, n, i, lo, hi, gamma, dev_status)) return;
     if (sd.node_range) sd.node_range[i] = make_uint2((uint32_t)lo, (uint32_t)hi);
     int c0, c1;
     if (lo == gamma) { c0 = ~gamma; leaf_parent[sd.prim_off + gamma] = ((uint32_t)i << 1) | 0u; }
@@ -160,6 +173,14 @@ __device__ __forceinline__ void slot4_put(Slot4& s, const float4* n2, int side, 
     s.lx[s.k] = a.x; s.hx[s.k] = a.y; s.ly[s.k] = a.z; s.hy[s.k] = a.w;
     s.lz[s.k] = side ? z.z : z.x;
     s.hz[s.k] = side ? z.w : z.y;
+    s.ch[s.k] = child;
+    ++s.k;
+}
+
+__device__ __forceinline__ void slot4_put(Slot4& s, float4 lo, float4 hi, int child) {
+    s.lx[s.k] = lo.x; s.hx[s.k] = hi.x; s.ly[s.k] = lo.y; s.hy[s.k] = hi.y;
+    s.lz[s.k] = lo.z;
+    s.hz[s.k] = hi.z;
     s.ch[s.k] = child;
     ++s.k;
 }
@@ -277,12 +298,18 @@ __device__ __forceinline__ bool tlas_instance_one(const DevInstanceInput* in, ui
     return finite3(c);
 }
 
-// Leaf j of the sorted order: instance record, leaf box, sorted Morton key and order.
-__device__ __forceinline__ void tlas_emit_one(const DevInstanceInput* in, const float4* inst_box, uint32_t j,
-                                              unsigned long long key, uint32_t i, DevInstance* inst_out,
-                                              float4* leaf_box, uint32_t* morton_out, uint32_t* order_out) {
+// Leaf j of the sorted order, instance i: sorted Morton key and order, and leaf box.
+__device__ __forceinline__ void tlas_emit_leaf(const float4* inst_box, uint32_t j, unsigned long long key, uint32_t i,
+                                               float4* leaf_box, uint32_t* morton_out, uint32_t* order_out) {
     morton_out[j] = (uint32_t)key & 0x3FFFFFFFu;
     order_out[j] = i;
+    leaf_box[2 * j] = inst_box[2 * i];
+    leaf_box[2 * j + 1] = inst_box[2 * i + 1];
+}
+
+// Its instance record.
+__device__ __forceinline__ void tlas_emit_record(const DevInstanceInput* in, uint32_t j, uint32_t i,
+                                                 DevInstance* inst_out) {
     const DevInstanceInput ii = in[i];
     DevInstance d;
     affine_inverse(ii.o2w, d.w2o);
@@ -300,8 +327,13 @@ __device__ __forceinline__ void tlas_emit_one(const DevInstanceInput* in, const 
     d.input_index = i;
     d.blas_prims = ii.blas_prims;
     inst_out[j] = d;
-    leaf_box[2 * j] = inst_box[2 * i];
-    leaf_box[2 * j + 1] = inst_box[2 * i + 1];
+}
+
+__device__ __forceinline__ void tlas_emit_one(const DevInstanceInput* in, const float4* inst_box, uint32_t j,
+                                              unsigned long long key, uint32_t i, DevInstance* inst_out,
+                                              float4* leaf_box, uint32_t* morton_out, uint32_t* order_out) {
+    tlas_emit_leaf(inst_box, j, key, i, leaf_box, morton_out, order_out);
+    tlas_emit_record(in, j, i, inst_out);
 }
 
 // Breadth-first relayout of one tree by one block (any multiple of 32 threads up to
