@@ -186,8 +186,7 @@ struct luz_frame {
     float* depth = nullptr;         // F32
     float4* light = nullptr;        // RGBA32F
     uint2* primary_hit = nullptr;
-    uint32_t* gb_coarse = nullptr;       // G-buffer candidate leaves per 64x64 tile (count + 255)
-    uint32_t* gb_fine = nullptr;         // and per 8x8 tile (count + 15)
+    uint32_t* gb_fine = nullptr;         // G-buffer candidate leaves per 8x8 tile (count + 15)
     // visibility
     uint32_t* shadow_bits = nullptr;
     uint32_t* ao_bits = nullptr;
