@@ -325,6 +325,7 @@ union CullShared {
 template <bool kAo, bool kShaft>
 __global__ void __launch_bounds__(kCullThreads, kAo ? (kShaft ? 4 : 6) : 5)
 cull_kernel(SceneVis S, VisCommon C, ShaftOut A, AoOut O, uint32_t* tickets) {
+    chain_wait();
     __shared__ CullShared s_mem[kCullWarps];
     const uint32_t full = 0xFFFFFFFFu, lane = threadIdx.x & 31;
     CullShared& sm = s_mem[threadIdx.x >> 5];

@@ -65,6 +65,7 @@ void* g_scratch_ptr[kMaxDevices] = {};
 // Writes the segment descriptor and resets the header from kernel parameters, so no
 // host memory is copied.
 __global__ void noalloc_setup_kernel(Header* h, SegDesc seg) {
+    chain_wait();
     if (threadIdx.x == 0) {
         h->status = 0;
         h->zero = 0;
@@ -78,6 +79,7 @@ __global__ void noalloc_setup_kernel(Header* h, SegDesc seg) {
 __global__ void noalloc_indices_kernel(const uint32_t* __restrict__ in, uint32_t count,
                                        uint32_t vertex_count, uint32_t* __restrict__ out,
                                        uint32_t* status) {
+    chain_wait();
     uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= count) return;
     uint32_t v = in[i];
@@ -168,43 +170,42 @@ extern "C" luz_status luz_blas_build_noalloc(const luz_vertex* d_vertices, uint3
     const uint32_t tiles = n > 0 ? cdiv(n, kSortTile) : 1;
 
     // The array keeps the previous call's contents: reset everything read before written.
-    noalloc_setup_kernel<<<1, 32, 0, st>>>(h, seg);
+    chain(noalloc_setup_kernel, 1, 32, 0, st, h, seg);
     NOALLOC_LAUNCHED();
     NOALLOC_CUDA(cudaMemsetAsync(node_parent, 0xFF, (size_t)m * 4, st));
     NOALLOC_CUDA(cudaMemsetAsync(leaf_parent, 0xFF, (size_t)(n ? n : 1) * 4, st));
     NOALLOC_CUDA(cudaMemsetAsync(flags, 0, (size_t)m * 4, st));
     if (n > 0) {
-        noalloc_indices_kernel<<<cdiv(index_count, 256), 256, 0, st>>>(d_indices, index_count, vertex_count,
+        chain(noalloc_indices_kernel, cdiv(index_count, 256), 256, 0, st, d_indices, index_count, vertex_count,
                                                                         idx, status);
         NOALLOC_LAUNCHED();
-        blas_bounds_kernel<<<cdiv(n, 256 * kBoundsIters), 256, 0, st>>>(d_seg, zero, 1, n, bounds);
+        chain(blas_bounds_kernel, cdiv(n, 256 * kBoundsIters), 256, 0, st, d_seg, zero, 1, n, bounds);
         NOALLOC_LAUNCHED();
-        blas_morton_kernel<<<cdiv(n, 256), 256, 0, st>>>(d_seg, zero, 1, n, bounds, keys[0], vals[0]);
+        chain(blas_morton_kernel, cdiv(n, 256), 256, 0, st, d_seg, zero, 1, n, bounds, keys[0], vals[0]);
         NOALLOC_LAUNCHED();
         NOALLOC_CUDA(cudaMemsetAsync(hist, 0, (size_t)kPasses * kRadix * 4, st));
         NOALLOC_CUDA(cudaMemsetAsync(tile_status, 0, (size_t)kPasses * tiles * kRadix * 4, st));
         NOALLOC_CUDA(cudaMemsetAsync(tile_counter, 0, (size_t)kPasses * 4, st));
-        sort_histogram_kernel<<<std::max(1u, std::min(cdiv(n, 4096), 256u)), 256, 0, st>>>(keys[0], n, kPasses, hist);
+        chain(sort_histogram_kernel, std::max(1u, std::min(cdiv(n, 4096), 256u)), 256, 0, st, keys[0], n, kPasses, hist);
         NOALLOC_LAUNCHED();
-        sort_scan_kernel<<<kPasses, 256, 0, st>>>(hist, offsets);
+        chain(sort_scan_kernel, kPasses, 256, 0, st, hist, offsets);
         NOALLOC_LAUNCHED();
         for (int p = 0; p < kPasses; ++p) {
             int cur = p & 1;
-            onesweep_pass_kernel<<<tiles, kSortThreads, 0, st>>>(
-                keys[cur], vals[cur], keys[cur ^ 1], vals[cur ^ 1], n, 8 * p, offsets + p * kRadix,
+            chain(onesweep_pass_kernel, tiles, kSortThreads, 0, st, keys[cur], vals[cur], keys[cur ^ 1], vals[cur ^ 1], n, 8 * p, offsets + p * kRadix,
                 tile_status + (size_t)p * tiles * kRadix, tile_counter + p, status);
             NOALLOC_LAUNCHED();
         }
     }
     // kPasses is even: the sorted keys are back in keys[0].
-    karras_kernel<<<cdiv(m, 256), 256, 0, st>>>(d_seg, zero, 1, m, keys[0], node_parent, leaf_parent, status);
+    chain(karras_kernel, cdiv(m, 256), 256, 0, st, d_seg, zero, 1, m, keys[0], node_parent, leaf_parent, status);
     NOALLOC_LAUNCHED();
     if (n > 0) {
-        blas_emit_kernel<<<cdiv(n, 256), 256, 0, st>>>(d_seg, zero, 1, n, keys[0], vals[0], leaf_box);
+        chain(blas_emit_kernel, cdiv(n, 256), 256, 0, st, d_seg, zero, 1, n, keys[0], vals[0], leaf_box);
         NOALLOC_LAUNCHED();
-        refit_kernel<<<cdiv(n, 256), 256, 0, st>>>(d_seg, zero, 1, n, leaf_box, node_parent, leaf_parent, flags);
+        chain(refit_kernel, cdiv(n, 256), 256, 0, st, d_seg, zero, 1, n, leaf_box, node_parent, leaf_parent, flags);
         NOALLOC_LAUNCHED();
-        blas_radius_kernel<<<cdiv(n, 256), 256, 0, st>>>(d_seg, zero, 1, n);
+        chain(blas_radius_kernel, cdiv(n, 256), 256, 0, st, d_seg, zero, 1, n);
         NOALLOC_LAUNCHED();
     }
     // Synchronous, like the reference's per-mesh build (GPUScene.cpp:132-137): read

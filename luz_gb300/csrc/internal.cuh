@@ -302,6 +302,32 @@ luz_status guarded(luz_ctx* ctx, F&& body) noexcept {
         if (e_ != cudaSuccess) return luz::cuda_error(ctx, e_, #call); \
     } while (0)
 
+namespace luz {
+// Launches a kernel whose launch work overlaps the end of the one before it in the stream:
+// its blocks are scheduled when that one's last block has finished, and the kernel begins
+// with chain_wait, which waits until everything before it in the stream is complete and
+// visible. Every thread calls it before it touches memory, so that the end of a kernel
+// implies the end of all before it. A copy, a memset or a kernel launched the ordinary way
+// orders as ever. The gap between two short kernels: 2.5 us -> 1. (Letting the next kernel's
+// blocks in from the start of the one before gained nothing more on small frames and cost
+// 3 % on large ones: the traversal's blocks arrive before the shared memory is theirs.)
+template <typename... Params, typename... Args>
+inline void chain(void (*kernel)(Params...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, Args&&... args) {
+    cudaLaunchAttribute attr{};
+    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t config{};
+    config.gridDim = grid;
+    config.blockDim = block;
+    config.dynamicSmemBytes = smem;
+    config.stream = stream;
+    config.attrs = &attr;
+    config.numAttrs = 1;
+    (void)cudaLaunchKernelEx(&config, kernel, static_cast<Params>(args)...);   // an error stays for LUZ_LAUNCHED
+}
+__device__ __forceinline__ void chain_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+}  // namespace luz
+
 #define LUZ_LAUNCHED(ctx, name)                                  \
     do {                                                         \
         (ctx)->launches++;                                       \

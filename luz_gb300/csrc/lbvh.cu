@@ -61,6 +61,7 @@ __device__ __forceinline__ float leaf_pad(float lo, float hi) {
 // depend on the order, so the result is the one of any reduction order.
 __global__ void __launch_bounds__(256) blas_bounds_kernel(const SegDesc* segs, const uint32_t* seg_prim_off,
                                                           int nseg, uint32_t total, uint32_t* seg_bounds) {
+    chain_wait();
     const uint32_t full = 0xFFFFFFFFu;
     const bool leader = (threadIdx.x & 31) == 0;
     int acc_s = -1;
@@ -119,6 +120,7 @@ __global__ void __launch_bounds__(256) blas_bounds_kernel(const SegDesc* segs, c
 __global__ void blas_morton_kernel(const SegDesc* segs, const uint32_t* seg_prim_off, int nseg,
                                    uint32_t total, const uint32_t* seg_bounds,
                                    unsigned long long* keys, uint32_t* vals) {
+    chain_wait();
     uint32_t g = blockIdx.x * blockDim.x + threadIdx.x;
     if (g >= total) return;
     int s = find_seg(seg_prim_off, nseg, g);
@@ -137,6 +139,7 @@ __global__ void blas_morton_kernel(const SegDesc* segs, const uint32_t* seg_prim
 // ---------------------------------------------------------------- onesweep radix sort
 __global__ void sort_histogram_kernel(const unsigned long long* keys, uint32_t n, int passes,
                                       uint32_t* hist) {
+    chain_wait();
     __shared__ uint32_t s_hist[kMaxPasses][kRadix];
     for (int i = threadIdx.x; i < kMaxPasses * kRadix; i += blockDim.x) (&s_hist[0][0])[i] = 0;
     __syncthreads();
@@ -174,6 +177,7 @@ __device__ __forceinline__ uint32_t block_excl_scan_256(uint32_t v, uint32_t* s_
 }
 
 __global__ void sort_scan_kernel(const uint32_t* hist, uint32_t* offsets) {
+    chain_wait();
     __shared__ uint32_t s_tmp[8];
     int p = blockIdx.x;
     uint32_t v = hist[p * kRadix + threadIdx.x];
@@ -194,6 +198,7 @@ onesweep_pass_kernel(const unsigned long long* __restrict__ kin, const uint32_t*
                      unsigned long long* __restrict__ kout, uint32_t* __restrict__ vout, uint32_t n,
                      int shift, const uint32_t* __restrict__ pass_offsets, uint32_t* tile_status,
                      uint32_t* tile_counter, uint32_t* dev_status) {
+    chain_wait();
     __shared__ uint32_t s_tile;
     __shared__ uint32_t s_warp_hist[kSortWarps][kRadix];
     __shared__ uint32_t s_digit_excl[kRadix];
@@ -300,6 +305,7 @@ onesweep_pass_kernel(const unsigned long long* __restrict__ kin, const uint32_t*
 __global__ void karras_kernel(const SegDesc* segs, const uint32_t* seg_node_off, int nseg,
                               uint32_t total_nodes, const unsigned long long* keys,
                               uint32_t* node_parent, uint32_t* leaf_parent, uint32_t* dev_status) {
+    chain_wait();
     uint32_t q = blockIdx.x * blockDim.x + threadIdx.x;
     if (q >= total_nodes) return;
     int s = find_seg(seg_node_off, nseg, q);
@@ -313,6 +319,7 @@ __global__ void karras_kernel(const SegDesc* segs, const uint32_t* seg_node_off,
 __global__ void blas_emit_kernel(const SegDesc* segs, const uint32_t* seg_prim_off, int nseg,
                                  uint32_t total, const unsigned long long* keys,
                                  const uint32_t* vals, float4* leaf_box) {
+    chain_wait();
     uint32_t g = blockIdx.x * blockDim.x + threadIdx.x;
     if (g >= total) return;
     int s = find_seg(seg_prim_off, nseg, g);
@@ -339,6 +346,7 @@ __global__ void blas_emit_kernel(const SegDesc* segs, const uint32_t* seg_prim_o
 __global__ void refit_kernel(const SegDesc* segs, const uint32_t* seg_prim_off, int nseg,
                              uint32_t total, const float4* leaf_box, const uint32_t* node_parent,
                              const uint32_t* leaf_parent, uint32_t* flags) {
+    chain_wait();
     uint32_t g = blockIdx.x * blockDim.x + threadIdx.x;
     if (g >= total) return;
     int s = find_seg(seg_prim_off, nseg, g);
@@ -359,6 +367,7 @@ __global__ void __launch_bounds__(kRefitLeaves)
 refit_local_kernel(const SegDesc* segs, const uint32_t* seg_prim_off, int nseg, uint32_t total,
                    const float4* leaf_box, const uint32_t* node_parent, const uint32_t* leaf_parent,
                    uint32_t* flags) {
+    chain_wait();
     __shared__ float s_box[kRefitLeaves][2][6];   // per local node: child slot 0 / 1 (lo xyz, hi xyz)
     __shared__ uint32_t s_flag[kRefitLeaves];
     __shared__ uint32_t s_parent[kRefitLeaves];   // parent and leaf range of node (g - prim_off)
@@ -444,6 +453,7 @@ refit_local_kernel(const SegDesc* segs, const uint32_t* seg_prim_off, int nseg, 
 // build intersects each instance's transformed root box with the transformed sphere.
 __global__ void blas_radius_kernel(const SegDesc* segs, const uint32_t* seg_prim_off, int nseg,
                                    uint32_t total) {
+    chain_wait();
     uint32_t g = blockIdx.x * blockDim.x + threadIdx.x;
     bool in = g < total;
     int s = in ? find_seg(seg_prim_off, nseg, g) : -1;
@@ -481,6 +491,7 @@ __global__ void blas_radius_kernel(const SegDesc* segs, const uint32_t* seg_prim
 // flags[q] = 1 when internal node q lies at even depth in its segment's tree.
 __global__ void even_depth_kernel(const SegDesc* segs, const uint32_t* seg_node_off, int nseg, uint32_t total_nodes,
                                   const uint32_t* node_parent, uint32_t* flags) {
+    chain_wait();
     uint32_t q = blockIdx.x * blockDim.x + threadIdx.x;
     if (q >= total_nodes) return;
     int s = find_seg(seg_node_off, nseg, q);
@@ -495,6 +506,7 @@ __global__ void even_depth_kernel(const SegDesc* segs, const uint32_t* seg_node_
 
 // Chunked exclusive scan of u32 (chunks of 1024 = 256 threads x 4).
 __global__ void __launch_bounds__(256) chunk_sum_kernel(const uint32_t* in, uint32_t n, uint32_t* sums) {
+    chain_wait();
     __shared__ uint32_t s_tmp[8];
     uint32_t base = blockIdx.x * 1024 + threadIdx.x * 4, c = 0;
     for (int k = 0; k < 4; ++k) c += base + k < n ? in[base + k] : 0u;
@@ -509,6 +521,7 @@ __global__ void __launch_bounds__(256) chunk_sum_kernel(const uint32_t* in, uint
 }
 
 __global__ void __launch_bounds__(1024) chunk_scan_kernel(uint32_t* sums, uint32_t chunks) {
+    chain_wait();
     __shared__ uint32_t s_warp[32];
     __shared__ uint32_t s_carry;
     int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -538,6 +551,7 @@ __global__ void __launch_bounds__(1024) chunk_scan_kernel(uint32_t* sums, uint32
 
 __global__ void __launch_bounds__(256) chunk_apply_kernel(const uint32_t* in, uint32_t n, const uint32_t* offs,
                                                           uint32_t* out) {
+    chain_wait();
     __shared__ uint32_t s_tmp[8];
     uint32_t base = blockIdx.x * 1024 + threadIdx.x * 4;
     uint32_t v[4], c = 0;
@@ -565,6 +579,7 @@ __global__ void __launch_bounds__(256) chunk_apply_kernel(const uint32_t* in, ui
 // idx4[q]: exclusive prefix of the even-depth flags over all segments' nodes.
 __global__ void bvh4_emit_kernel(const SegDesc* segs, const uint32_t* seg_node_off, int nseg, uint32_t total_nodes,
                                  const uint32_t* flags, const uint32_t* idx4) {
+    chain_wait();
     uint32_t q = blockIdx.x * blockDim.x + threadIdx.x;
     if (q >= total_nodes || !flags[q]) return;
     int s = find_seg(seg_node_off, nseg, q);
@@ -616,6 +631,7 @@ __device__ __forceinline__ void merge_bounds(bool have, V3 c, uint32_t* bounds) 
 // seg_bounds: NULL where the next kernel takes the bounds from the boxes.
 __global__ void tlas_instance_kernel(const DevInstanceInput* in, uint32_t n, float4* inst_box,
                                      DevShadeInstance* shade, uint32_t* seg_bounds) {
+    chain_wait();
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     V3 c;
     const bool have = i < n && tlas_instance_one(in, i, inst_box, shade, c);
@@ -623,6 +639,7 @@ __global__ void tlas_instance_kernel(const DevInstanceInput* in, uint32_t n, flo
 }
 
 __global__ void tlas_setup_kernel(uint32_t* bounds, SegDesc* seg, SegDesc value, uint32_t* zero) {
+    chain_wait();
     if (threadIdx.x < 6) bounds[threadIdx.x] = threadIdx.x < 3 ? 0xFFFFFFFFu : 0u;
     if (threadIdx.x == 0) {
         *seg = value;
@@ -632,6 +649,7 @@ __global__ void tlas_setup_kernel(uint32_t* bounds, SegDesc* seg, SegDesc value,
 
 __global__ void tlas_morton_kernel(const float4* inst_box, uint32_t n, const uint32_t* seg_bounds,
                                    unsigned long long* keys, uint32_t* vals) {
+    chain_wait();
     uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     float4 l = inst_box[2 * i], h = inst_box[2 * i + 1];
@@ -646,12 +664,14 @@ __global__ void tlas_emit_kernel(const DevInstanceInput* in, const float4* inst_
                                  const unsigned long long* keys, const uint32_t* vals,
                                  DevInstance* inst_out, float4* leaf_box, uint32_t* morton_out,
                                  uint32_t* order_out) {
+    chain_wait();
     uint32_t j = blockIdx.x * blockDim.x + threadIdx.x;
     if (j >= n) return;
     tlas_emit_one(in, inst_box, j, keys[j], vals[j], inst_out, leaf_box, morton_out, order_out);
 }
 
 __global__ void tlas_record_kernel(const DevInstanceInput* in, const uint32_t* order, uint32_t n, DevInstance* inst_out) {
+    chain_wait();
     uint32_t j = blockIdx.x * blockDim.x + threadIdx.x;
     if (j < n) tlas_emit_record(in, j, order[j], inst_out);
 }
@@ -665,6 +685,7 @@ constexpr uint32_t kTlasLevels = 64;   // above the depth of 30-bit codes split 
 // (8000 instances: relayout and collapse by one block, level by level, 119 us; these kernels
 // and their sort pass 27).
 __global__ void tlas_depth_kernel(const uint32_t* node_parent, uint32_t m, unsigned long long* keys, uint32_t* vals) {
+    chain_wait();
     const uint32_t q = blockIdx.x * blockDim.x + threadIdx.x;
     if (q >= m) return;
     uint32_t d = 0, p = node_parent[q];
@@ -679,6 +700,7 @@ __global__ void tlas_depth_kernel(const uint32_t* node_parent, uint32_t m, unsig
 // Level table {L, start_0, ..., start_L}, and the inverse of the order.
 __global__ void tlas_newidx_kernel(const uint32_t* order, uint32_t m, const uint32_t* offsets, uint32_t* newidx,
                                    uint32_t* levels) {
+    chain_wait();
     const uint32_t b = blockIdx.x * blockDim.x + threadIdx.x;
     if (b < m) newidx[order[b]] = b;
     if (b < kTlasLevels && offsets[b] < m) {
@@ -695,6 +717,7 @@ __global__ void __launch_bounds__(128) tlas_relayout_kernel(const float4* __rest
                                                             const uint32_t* __restrict__ order,
                                                             const uint32_t* __restrict__ newidx, uint32_t m,
                                                             const uint32_t* __restrict__ levels, float4* dst, float4* nodes4) {
+    chain_wait();
     __shared__ uint32_t s_start[kTlasLevels + 1], s_even[kTlasLevels];
     const uint32_t L = levels[0];
     if (threadIdx.x <= L) s_start[threadIdx.x] = levels[1 + threadIdx.x];
@@ -777,6 +800,7 @@ constexpr uint32_t kTlasOneBlock = 768;
 // gaps of 2.5 against 29.0, 700 36.6 and the gaps against 38.4, 1024 42.3 against 50.4.
 template <bool kTreeOnly>
 __global__ void __launch_bounds__(1024) tlas_fused_kernel(TlasBuildArgs A, uint32_t* dev_status) {
+    chain_wait();
     extern __shared__ unsigned long long s_keys[];
     __shared__ uint32_t s_bounds[6], s_total[kTlasLevels], s_start[kTlasLevels + 1], s_even[kTlasLevels + 1];
     __shared__ uint16_t s_count[32][kTlasLevels];
@@ -1041,14 +1065,13 @@ static luz_status run_sort(luz_ctx* ctx, SortBuffers& sb, uint32_t n, int passes
     LUZ_CUDA(ctx, cudaMemsetAsync(sb.tile_status, 0, (size_t)passes * sb.tiles * 256 * 4, st));
     LUZ_CUDA(ctx, cudaMemsetAsync(sb.tile_counter, 0, (size_t)passes * 4, st));
     uint32_t hblocks = std::min<uint32_t>(std::max(1u, cdiv(n, 256 * 16)), (uint32_t)ctx->sm_count * 4);
-    sort_histogram_kernel<<<hblocks, 256, 0, st>>>(sb.keys[0], n, passes, sb.hist);
+    chain(sort_histogram_kernel, hblocks, 256, 0, st, sb.keys[0], n, passes, sb.hist);
     LUZ_LAUNCHED(ctx, "sort_histogram_kernel");
-    sort_scan_kernel<<<passes, 256, 0, st>>>(sb.hist, sb.offsets);
+    chain(sort_scan_kernel, passes, 256, 0, st, sb.hist, sb.offsets);
     LUZ_LAUNCHED(ctx, "sort_scan_kernel");
     int cur = 0;
     for (int p = 0; p < passes; ++p) {
-        onesweep_pass_kernel<<<sb.tiles, kSortThreads, 0, st>>>(
-            sb.keys[cur], sb.vals[cur], sb.keys[cur ^ 1], sb.vals[cur ^ 1], n, 8 * p,
+        chain(onesweep_pass_kernel, sb.tiles, kSortThreads, 0, st, sb.keys[cur], sb.vals[cur], sb.keys[cur ^ 1], sb.vals[cur ^ 1], n, 8 * p,
             sb.offsets + p * 256, sb.tile_status + (size_t)p * sb.tiles * 256, sb.tile_counter + p,
             ctx->d_status);
         LUZ_LAUNCHED(ctx, "onesweep_pass_kernel");
@@ -1180,9 +1203,9 @@ luz_status build_blas_batch(luz_ctx* ctx, uint32_t count, const luz_blas_desc* d
     LUZ_CUDA(ctx, cudaMemsetAsync(d_leaf_parent, 0xFF, (size_t)std::max(N, 1u) * 4, st));
     LUZ_CUDA(ctx, cudaMemsetAsync(d_flags, 0, (size_t)M * 4, st));
     if (N > 0) {
-        blas_bounds_kernel<<<cdiv(N, 256 * kBoundsIters), 256, 0, st>>>(d_segs, d_prim_off, count, N, d_bounds);
+        chain(blas_bounds_kernel, cdiv(N, 256 * kBoundsIters), 256, 0, st, d_segs, d_prim_off, count, N, d_bounds);
         LUZ_LAUNCHED(ctx, "blas_bounds_kernel");
-        blas_morton_kernel<<<cdiv(N, 256), 256, 0, st>>>(d_segs, d_prim_off, count, N, d_bounds,
+        chain(blas_morton_kernel, cdiv(N, 256), 256, 0, st, d_segs, d_prim_off, count, N, d_bounds,
                                                          sb.keys[0], sb.vals[0]);
         LUZ_LAUNCHED(ctx, "blas_morton_kernel");
     }
@@ -1193,33 +1216,33 @@ luz_status build_blas_batch(luz_ctx* ctx, uint32_t count, const luz_blas_desc* d
     }
     // Every segment has at least one node; segments with 0 or 1 primitive get their
     // single node (empty / one leaf) here without reading keys.
-    karras_kernel<<<cdiv(M, 256), 256, 0, st>>>(d_segs, d_node_off, count, M, sb.keys[res],
+    chain(karras_kernel, cdiv(M, 256), 256, 0, st, d_segs, d_node_off, count, M, sb.keys[res],
                                                 d_node_parent, d_leaf_parent, ctx->d_status);
     LUZ_LAUNCHED(ctx, "karras_kernel");
     if (N > 0) {
-        blas_emit_kernel<<<cdiv(N, 256), 256, 0, st>>>(d_segs, d_prim_off, count, N, sb.keys[res],
+        chain(blas_emit_kernel, cdiv(N, 256), 256, 0, st, d_segs, d_prim_off, count, N, sb.keys[res],
                                                        sb.vals[res], d_leaf_box);
         LUZ_LAUNCHED(ctx, "blas_emit_kernel");
-        refit_local_kernel<<<cdiv(N, kRefitLeaves), kRefitLeaves, 0, st>>>(d_segs, d_prim_off, count, N,
+        chain(refit_local_kernel, cdiv(N, kRefitLeaves), kRefitLeaves, 0, st, d_segs, d_prim_off, count, N,
                                                                            d_leaf_box, d_node_parent, d_leaf_parent,
                                                                            d_flags);
         LUZ_LAUNCHED(ctx, "refit_local_kernel");
-        blas_radius_kernel<<<cdiv(N, 256), 256, 0, st>>>(d_segs, d_prim_off, count, N);
+        chain(blas_radius_kernel, cdiv(N, 256), 256, 0, st, d_segs, d_prim_off, count, N);
         LUZ_LAUNCHED(ctx, "blas_radius_kernel");
     }
     // 4-wide collapse of every segment's tree (the traversal structure of the
     // shadow/AO rays; the binary tree stays the parity-checked structure).
     {
         uint32_t chunks = cdiv(M, 1024);
-        even_depth_kernel<<<cdiv(M, 256), 256, 0, st>>>(d_segs, d_node_off, count, M, d_node_parent, d_even);
+        chain(even_depth_kernel, cdiv(M, 256), 256, 0, st, d_segs, d_node_off, count, M, d_node_parent, d_even);
         LUZ_LAUNCHED(ctx, "even_depth_kernel");
-        chunk_sum_kernel<<<chunks, 256, 0, st>>>(d_even, M, d_sums);
+        chain(chunk_sum_kernel, chunks, 256, 0, st, d_even, M, d_sums);
         LUZ_LAUNCHED(ctx, "chunk_sum_kernel");
-        chunk_scan_kernel<<<1, 1024, 0, st>>>(d_sums, chunks);
+        chain(chunk_scan_kernel, 1, 1024, 0, st, d_sums, chunks);
         LUZ_LAUNCHED(ctx, "chunk_scan_kernel");
-        chunk_apply_kernel<<<chunks, 256, 0, st>>>(d_even, M, d_sums, d_idx4);
+        chain(chunk_apply_kernel, chunks, 256, 0, st, d_even, M, d_sums, d_idx4);
         LUZ_LAUNCHED(ctx, "chunk_apply_kernel");
-        bvh4_emit_kernel<<<cdiv(M, 256), 256, 0, st>>>(d_segs, d_node_off, count, M, d_even, d_idx4);
+        chain(bvh4_emit_kernel, cdiv(M, 256), 256, 0, st, d_segs, d_node_off, count, M, d_even, d_idx4);
         LUZ_LAUNCHED(ctx, "bvh4_emit_kernel");
     }
     LUZ_CUDA(ctx, cudaEventRecord(ctx->build_ev[1], st));
@@ -1393,14 +1416,14 @@ luz_status launch_tlas_build(luz_ctx* ctx, luz_tlas* t) {
         const uint32_t threads = std::min(std::max((n + 31u) & ~31u, 64u), 1024u);
         prof_begin(ctx, LUZ_KERNEL_TLAS_BUILD);
         if (n <= kTlasOneBlock) {
-            tlas_fused_kernel<false><<<1, threads, tlas_shared(n).bytes, st>>>(A, ctx->d_status);
+            chain(tlas_fused_kernel<false>, 1, threads, tlas_shared(n).bytes, st, A, ctx->d_status);
             LUZ_LAUNCHED(ctx, "tlas_fused_kernel");
         } else {
-            tlas_instance_kernel<<<cdiv(n, 64), 64, 0, st>>>(A.in, n, A.inst_box, A.shade, nullptr);
+            chain(tlas_instance_kernel, cdiv(n, 64), 64, 0, st, A.in, n, A.inst_box, A.shade, nullptr);
             LUZ_LAUNCHED(ctx, "tlas_instance_kernel");
-            tlas_fused_kernel<true><<<1, threads, tlas_shared(n).bytes, st>>>(A, ctx->d_status);
+            chain(tlas_fused_kernel<true>, 1, threads, tlas_shared(n).bytes, st, A, ctx->d_status);
             LUZ_LAUNCHED(ctx, "tlas_fused_kernel<tree>");
-            tlas_record_kernel<<<cdiv(n, 64), 64, 0, st>>>(A.in, A.order_out, n, A.inst_out);
+            chain(tlas_record_kernel, cdiv(n, 64), 64, 0, st, A.in, A.order_out, n, A.inst_out);
             LUZ_LAUNCHED(ctx, "tlas_record_kernel");
         }
         prof_end(ctx);
@@ -1414,35 +1437,35 @@ luz_status launch_tlas_build(luz_ctx* ctx, luz_tlas* t) {
     // Bounds initialiser, segment descriptor and zero offset are written by a kernel from
     // its parameters: a copy from host memory would, inside a CUDA graph, re-read a
     // host address that no longer holds them.
-    tlas_setup_kernel<<<1, 32, 0, st>>>(bounds, d_seg, sd, d_zero);
+    chain(tlas_setup_kernel, 1, 32, 0, st, bounds, d_seg, sd, d_zero);
     LUZ_LAUNCHED(ctx, "tlas_setup_kernel");
     LUZ_CUDA(ctx, cudaMemsetAsync(node_parent, 0xFF, (size_t)m * 4, st));
     LUZ_CUDA(ctx, cudaMemsetAsync(leaf_parent, 0xFF, (size_t)n * 4, st));
     LUZ_CUDA(ctx, cudaMemsetAsync(flags, 0, (size_t)m * 4, st));
 
-    tlas_instance_kernel<<<cdiv(n, 128), 128, 0, st>>>(t->d_input, n, inst_box, t->shade, bounds);
+    chain(tlas_instance_kernel, cdiv(n, 128), 128, 0, st, t->d_input, n, inst_box, t->shade, bounds);
     LUZ_LAUNCHED(ctx, "tlas_instance_kernel");
-    tlas_morton_kernel<<<cdiv(n, 128), 128, 0, st>>>(inst_box, n, bounds, sb.keys[0], sb.vals[0]);
+    chain(tlas_morton_kernel, cdiv(n, 128), 128, 0, st, inst_box, n, bounds, sb.keys[0], sb.vals[0]);
     LUZ_LAUNCHED(ctx, "tlas_morton_kernel");
     int res = 0;
     luz_status s = run_sort(ctx, sb, n, 4, res);
     if (s != LUZ_OK) return s;
-    karras_kernel<<<cdiv(m, 128), 128, 0, st>>>(d_seg, d_zero, 1, m, sb.keys[res], node_parent,
+    chain(karras_kernel, cdiv(m, 128), 128, 0, st, d_seg, d_zero, 1, m, sb.keys[res], node_parent,
                                                 leaf_parent, ctx->d_status);
     LUZ_LAUNCHED(ctx, "karras_kernel");
-    tlas_emit_kernel<<<cdiv(n, 128), 128, 0, st>>>(t->d_input, inst_box, n, sb.keys[res],
+    chain(tlas_emit_kernel, cdiv(n, 128), 128, 0, st, t->d_input, inst_box, n, sb.keys[res],
                                                    sb.vals[res], t->instances, leaf_box,
                                                    t->morton, t->order);
     LUZ_LAUNCHED(ctx, "tlas_emit_kernel");
-    refit_kernel<<<cdiv(n, 128), 128, 0, st>>>(d_seg, d_zero, 1, n, leaf_box, node_parent,
+    chain(refit_kernel, cdiv(n, 128), 128, 0, st, d_seg, d_zero, 1, n, leaf_box, node_parent,
                                                leaf_parent, flags);
     LUZ_LAUNCHED(ctx, "refit_kernel");
-    tlas_depth_kernel<<<cdiv(m, 128), 128, 0, st>>>(node_parent, m, sb.keys[0], sb.vals[0]);
+    chain(tlas_depth_kernel, cdiv(m, 128), 128, 0, st, node_parent, m, sb.keys[0], sb.vals[0]);
     LUZ_LAUNCHED(ctx, "tlas_depth_kernel");
     if ((s = run_sort(ctx, sb, m, 1, res)) != LUZ_OK) return s;
-    tlas_newidx_kernel<<<cdiv(m, 128), 128, 0, st>>>(sb.vals[res], m, sb.offsets, newidx, t->levels);
+    chain(tlas_newidx_kernel, cdiv(m, 128), 128, 0, st, sb.vals[res], m, sb.offsets, newidx, t->levels);
     LUZ_LAUNCHED(ctx, "tlas_newidx_kernel");
-    tlas_relayout_kernel<<<cdiv(m, 128), 128, 0, st>>>(karras_nodes, sb.keys[res], sb.vals[res], newidx, m, t->levels,
+    chain(tlas_relayout_kernel, cdiv(m, 128), 128, 0, st, karras_nodes, sb.keys[res], sb.vals[res], newidx, m, t->levels,
                                                        t->nodes, t->nodes4);
     LUZ_LAUNCHED(ctx, "tlas_relayout_kernel");
     return LUZ_OK;

@@ -11,6 +11,7 @@ namespace luz {
 
 template <int kMode>
 __global__ void __launch_bounds__(256) light_pass_kernel(LightParams P) {
+    chain_wait();
     extern __shared__ luz_light s_lights[];
     const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
     const uint32_t lit = *P.lit_count;
@@ -26,6 +27,7 @@ __global__ void __launch_bounds__(256) light_pass_kernel(LightParams P) {
 __global__ void __launch_bounds__(256) ao_resolve_kernel(const float4* normal, const uint32_t* ao_bits,
                                                          uint32_t words, uint32_t samples,
                                                          uint32_t pixels, float* ao) {
+    chain_wait();
     uint32_t pix = blockIdx.x * blockDim.x + threadIdx.x;
     if (pix >= pixels) return;
     float4 nn = normal[pix];
@@ -89,7 +91,7 @@ luz_status launch_light_pass(luz_ctx* ctx, luz_frame* f, int mode) {
     }
     uint32_t blocks = (f->pixels + 255) / 256;
     prof_begin(ctx, LUZ_KERNEL_LIGHT_PASS);
-    kernels[mode]<<<blocks, 256, smem, ctx->stream>>>(P);
+    chain(kernels[mode], blocks, 256, smem, ctx->stream, P);
     prof_end(ctx);
     LUZ_LAUNCHED(ctx, "light_pass_kernel");
     return LUZ_OK;
@@ -97,7 +99,7 @@ luz_status launch_light_pass(luz_ctx* ctx, luz_frame* f, int mode) {
 
 luz_status launch_ao_resolve(luz_ctx* ctx, luz_frame* f) {
     uint32_t blocks = (f->pixels + 255) / 256;
-    ao_resolve_kernel<<<blocks, 256, 0, ctx->stream>>>(f->normal, f->ao_bits, f->words,
+    chain(ao_resolve_kernel, blocks, 256, 0, ctx->stream, f->normal, f->ao_bits, f->words,
                                                       f->ao_samples, f->pixels, f->ao);
     LUZ_LAUNCHED(ctx, "ao_resolve_kernel");
     return LUZ_OK;

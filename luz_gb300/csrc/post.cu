@@ -166,6 +166,7 @@ __device__ __forceinline__ float4 clip_aabb(float mnx, float mny, float mnz, flo
 }
 
 __global__ void __launch_bounds__(256) taa_kernel(TaaParams P) {
+    chain_wait();
     __shared__ float4 s_light[kTaaSpan * kTaaSpan];
     __shared__ float s_depth[kTaaSpan * kTaaSpan];
     const int ox = (int)(blockIdx.x * kTaaTile) - 2, oy = (int)(blockIdx.y * kTaaTile) - 2;
@@ -272,7 +273,7 @@ luz_status launch_taa(luz_ctx* ctx, luz_frame* f, int reconstruct) {
     memcpy(P.prev_jitter, s.prev_jitter, 8);
     dim3 grid((f->width + kTaaTile - 1) / kTaaTile, (f->height + kTaaTile - 1) / kTaaTile);
     prof_begin(ctx, LUZ_KERNEL_TAA);
-    taa_kernel<<<grid, 256, 0, ctx->stream>>>(P);
+    chain(taa_kernel, grid, 256, 0, ctx->stream, P);
     prof_end(ctx);
     LUZ_LAUNCHED(ctx, "taa_kernel");
     std::swap(f->taa, f->taa_next);   // the output is the next frame's history
@@ -296,6 +297,7 @@ __device__ __forceinline__ uint32_t histogram_bin(float r, float g, float b) {
 
 __global__ void __launch_bounds__(256) histogram_kernel(const float4* __restrict__ img, uint32_t n,
                                                         uint32_t* __restrict__ bins) {
+    chain_wait();
     __shared__ uint32_t s_bins[256];
     s_bins[threadIdx.x] = 0u;
     __syncthreads();
@@ -311,6 +313,7 @@ __global__ void __launch_bounds__(256) histogram_kernel(const float4* __restrict
 // (floats); state[0] holds the adapted luminance across frames.
 __global__ void __launch_bounds__(256) histogram_average_kernel(const uint32_t* __restrict__ bins, uint32_t n,
                                                                 float delta_time, float* state, uint32_t* out) {
+    chain_wait();
     __shared__ float s[256];
     const uint32_t i = threadIdx.x;
     const float count = (float)bins[i];
@@ -374,6 +377,7 @@ __device__ __forceinline__ uint32_t unorm8c(float x) {
 }
 
 __global__ void __launch_bounds__(256) compose_kernel(ComposeParams P) {
+    chain_wait();
     uint32_t x = blockIdx.x * 16 + (threadIdx.x & 15), y = blockIdx.y * 16 + (threadIdx.x >> 4);
     if (x >= P.w || y >= P.h) return;
     float tu = ((float)x + 0.5f) / (float)P.w, tv = ((float)y + 0.5f) / (float)P.h;
@@ -425,9 +429,9 @@ extern "C" luz_status luz_luminance_histogram(luz_ctx* ctx, luz_frame* f, int32_
     cudaStream_t st = ctx->stream;
     LUZ_CUDA(ctx, cudaMemsetAsync(f->hist, 0, 256 * 4, st));
     uint32_t blocks = std::min<uint32_t>((f->pixels + 255) / 256, (uint32_t)ctx->sm_count * 8);
-    histogram_kernel<<<blocks, 256, 0, st>>>(img, f->pixels, f->hist);
+    chain(histogram_kernel, blocks, 256, 0, st, img, f->pixels, f->hist);
     LUZ_LAUNCHED(ctx, "histogram_kernel");
-    histogram_average_kernel<<<1, 256, 0, st>>>(f->hist, f->pixels, delta_time, f->hist_state, f->hist + 256);
+    chain(histogram_average_kernel, 1, 256, 0, st, f->hist, f->pixels, delta_time, f->hist_state, f->hist + 256);
     LUZ_LAUNCHED(ctx, "histogram_average_kernel");
     static_assert(sizeof(luz_histogram) == 260 * 4, "luz_histogram layout");
     LUZ_CUDA(ctx, cudaMemcpyAsync(out, f->hist + 256, sizeof(luz_histogram), cudaMemcpyDeviceToHost, st));
@@ -450,7 +454,7 @@ extern "C" luz_status luz_compose(luz_ctx* ctx, luz_frame* f, int32_t source, in
     P.h = f->height;
     P.image_type = image_type;
     dim3 grid((f->width + 15) / 16, (f->height + 15) / 16);
-    compose_kernel<<<grid, 256, 0, ctx->stream>>>(P);
+    chain(compose_kernel, grid, 256, 0, ctx->stream, P);
     LUZ_LAUNCHED(ctx, "compose_kernel");
     return LUZ_OK;
 }

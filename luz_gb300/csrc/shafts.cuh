@@ -174,6 +174,14 @@ __device__ __forceinline__ float warp_sum(float v) {
     return v;
 }
 
+// p[0, n) = 0 by the whole grid (p 16-B aligned).
+__device__ __forceinline__ void clear_words(uint32_t* p, size_t n) {
+    const size_t t = blockIdx.x * (size_t)blockDim.x + threadIdx.x, step = gridDim.x * (size_t)blockDim.x;
+    uint4* p4 = reinterpret_cast<uint4*>(p);
+    for (size_t i = t; i < n / 4; i += step) p4[i] = make_uint4(0u, 0u, 0u, 0u);
+    if (t < n % 4) p[n - 1 - t] = 0u;
+}
+
 // One block per block of patches, one warp per patch: the patches' bounds, then the
 // block's (the unions of the boxes; the mean normal with its least dot product over the
 // patches' origin and offset boxes). fminf / fmaxf leave out a NaN pixel, which has no
@@ -181,9 +189,13 @@ __device__ __forceinline__ float warp_sum(float v) {
 __global__ void __launch_bounds__(kSuper * 32) patch_kernel(SceneVis S, PatchRec* __restrict__ patches,
                                                            PatchRec* __restrict__ supers,
                                                            VisCounters* __restrict__ counters, uint32_t chunks) {
+    chain_wait();
     __shared__ float s_rec[kSuper][32];
-    if (blockIdx.x == 0)   // for the chunks' launches that follow
+    // for the chunks' launches that follow: zero counters and hit/miss planes
+    if (blockIdx.x == 0)
         for (uint32_t k = threadIdx.x; k < chunks; k += blockDim.x) counters[k] = VisCounters{};
+    clear_words(S.shadow_bits, (size_t)S.shadow_slots * S.words);
+    clear_words(S.ao_bits, (size_t)S.ao_samples * S.words);
     const uint32_t lit = *S.lit_count, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const uint32_t count = (lit + kPatch - 1) / kPatch;
     const V3 cam = V3{S.cam[0], S.cam[1], S.cam[2]};

@@ -117,6 +117,7 @@ __device__ __forceinline__ void cone_margins(const V3 (&n)[5], float (&w)[5]) {
 // Clears the coarse tile's counts of lit pixels for the G-buffer kernel.
 __global__ void __launch_bounds__(kGbListThreads) gb_lists_kernel(GbufParams G, const float4* __restrict__ leaf_box, uint32_t n,
                                                        uint32_t* __restrict__ fine, uint32_t* __restrict__ lit_counts) {
+    chain_wait();
     constexpr uint32_t per = kGbCoarse / kGbTile, tiles = per * per, warps = kGbListThreads / 32;
     static_assert(tiles * 4 <= kGbListThreads, "four lanes per cone");
     __shared__ float4 s_box[2 * kGbCoarseMax];
@@ -256,6 +257,7 @@ __global__ void __launch_bounds__(kGbListThreads) gb_lists_kernel(GbufParams G, 
 __global__ void __launch_bounds__(kGbTile * kGbTile, kGbMinBlocks) gbuffer_kernel(GbufParams G,
                                                                                    const uint32_t* __restrict__ lists,
                                                                                    uint32_t* lit_counts) {
+    chain_wait();
     uint32_t tiles_x = (G.width + kGbTile - 1) / kGbTile;
     uint32_t tx = blockIdx.x % tiles_x, ty = blockIdx.x / tiles_x;
     uint32_t x = tx * kGbTile + (threadIdx.x % kGbTile), y = ty * kGbTile + (threadIdx.x / kGbTile);
@@ -408,6 +410,7 @@ __device__ __forceinline__ bool pixel_lit(const float4* normal, uint32_t pix) {
 // The counts where the planes did not come from gbuffer_kernel.
 __global__ void __launch_bounds__(256) lit_count_kernel(const float4* normal, uint32_t width, uint32_t height,
                                                         uint32_t* chunk_counts) {
+    chain_wait();
     __shared__ uint32_t s_tmp[8];
     uint32_t base = blockIdx.x * kChunk + threadIdx.x * 4;
     uint32_t c = 0;
@@ -424,6 +427,7 @@ __global__ void __launch_bounds__(256) lit_count_kernel(const float4* normal, ui
 
 __global__ void __launch_bounds__(1024) lit_scan_kernel(uint32_t* chunk_counts, uint32_t chunks,
                                                         uint32_t* total) {
+    chain_wait();
     __shared__ uint32_t s_warp[32];
     __shared__ uint32_t s_carry;
     int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -474,6 +478,7 @@ __global__ void __launch_bounds__(256) lit_write_kernel(const float4* __restrict
                                                         const float* inverse_proj,
                                                         const float* inverse_view, const float* ambient,
                                                         float4* surf, uint4* surf_mat, float4* light, uint32_t* lit_count) {
+    chain_wait();
     constexpr uint32_t kPer = kChunk / 256;
     __shared__ uint32_t s_lit[kPer * 8], s_sum[8];
     __shared__ float s_ip[16], s_iv[16];
@@ -590,13 +595,13 @@ luz_status launch_gbuffer(luz_ctx* ctx, luz_frame* f, const luz_tlas* t) {
     const uint32_t coarse = ((f->width + kGbCoarse - 1) / kGbCoarse) * ((f->height + kGbCoarse - 1) / kGbCoarse);
     prof_begin(ctx, LUZ_KERNEL_GBUFFER);
     if (t->count > 0 && t->count <= kGbListMaxInstances) {
-        gb_lists_kernel<<<coarse, kGbListThreads, 0, ctx->stream>>>(G, tlas_leaf_boxes(t), t->count, f->gb_fine, f->block_counts);
+        chain(gb_lists_kernel, coarse, kGbListThreads, 0, ctx->stream, G, tlas_leaf_boxes(t), t->count, f->gb_fine, f->block_counts);
         LUZ_LAUNCHED(ctx, "gb_lists_kernel");
     } else {   // every tile through the TLAS (count word kGbListAll), or none of them
         LUZ_CUDA(ctx, cudaMemsetAsync(f->gb_fine, t->count ? 0xFF : 0, (size_t)tiles * (kGbFineMax + 1) * 4, ctx->stream));
         LUZ_CUDA(ctx, cudaMemsetAsync(f->block_counts, 0, (size_t)lit_chunks(f->width, f->height) * 4, ctx->stream));
     }
-    gbuffer_kernel<<<tiles, kGbTile * kGbTile, 0, ctx->stream>>>(G, f->gb_fine, f->block_counts);
+    chain(gbuffer_kernel, tiles, kGbTile * kGbTile, 0, ctx->stream, G, f->gb_fine, f->block_counts);
     prof_end(ctx);
     LUZ_LAUNCHED(ctx, "gbuffer_kernel");
     return launch_lit_compaction(ctx, f, true);
@@ -608,16 +613,16 @@ luz_status launch_gbuffer(luz_ctx* ctx, luz_frame* f, const luz_tlas* t) {
 luz_status launch_lit_compaction(luz_ctx* ctx, luz_frame* f, bool counted) {
     const uint32_t chunks = lit_chunks(f->width, f->height);
     if (!counted) {
-        lit_count_kernel<<<chunks, 256, 0, ctx->stream>>>(f->normal, f->width, f->height, f->block_counts);
+        chain(lit_count_kernel, chunks, 256, 0, ctx->stream, f->normal, f->width, f->height, f->block_counts);
         LUZ_LAUNCHED(ctx, "lit_count_kernel");
     }
     const bool sum = chunks <= kLitSumChunks;
     if (!sum) {
-        lit_scan_kernel<<<1, 1024, 0, ctx->stream>>>(f->block_counts, chunks, f->lit_count);
+        chain(lit_scan_kernel, 1, 1024, 0, ctx->stream, f->block_counts, chunks, f->lit_count);
         LUZ_LAUNCHED(ctx, "lit_scan_kernel");
     }
     auto* write = sum ? lit_write_kernel<true> : lit_write_kernel<false>;
-    write<<<chunks, 256, 0, ctx->stream>>>(f->normal, f->depth, f->albedo, f->material, f->emission, f->width, f->height,
+    chain(write, chunks, 256, 0, ctx->stream, f->normal, f->depth, f->albedo, f->material, f->emission, f->width, f->height,
                                            f->block_counts,
                                            (const float*)((const char*)f->d_scene + offsetof(luz_scene, inverse_proj)),
                                            (const float*)((const char*)f->d_scene + offsetof(luz_scene, inverse_view)),

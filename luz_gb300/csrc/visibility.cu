@@ -44,6 +44,7 @@ __global__ void __launch_bounds__(256, 3) shadow_raygen_kernel(SceneVis S, VisCo
                                                                const uint4* __restrict__ active,
                                                                const uint32_t* __restrict__ active_count,
                                                                uint32_t* tickets, RayOut R) {
+    chain_wait();
     __shared__ float s_ray[8][kStageWords][kStageRays];
     const uint32_t full = 0xFFFFFFFFu;
     const uint32_t lit = *S.lit_count, lane = threadIdx.x & 31, n = *active_count;
@@ -92,6 +93,7 @@ __global__ void __launch_bounds__(256, 3) shadow_raygen_kernel(SceneVis S, VisCo
 // The rays of a frame that have something to trace (the counting trace's figure: shafts
 // and horizons resolve most of them without a record).
 __global__ void __launch_bounds__(256) count_rays_kernel(SceneVis S, VisCommon C, unsigned long long* stats) {
+    chain_wait();
     const uint32_t lit = *S.lit_count;
     const unsigned long long total = (unsigned long long)lit * (S.shadow_slots + S.ao_samples);
     uint32_t n = 0;
@@ -114,6 +116,7 @@ __global__ void __launch_bounds__(256) count_rays_kernel(SceneVis S, VisCommon C
 template <bool kStats, bool kStaged>
 __global__ void __launch_bounds__(kVisThreads, LUZ_VIS_MIN_BLOCKS)
 visibility_kernel(SceneVis S, VisCommon C, Entries E, RayOut R, unsigned long long* stats) {
+    chain_wait();
     extern __shared__ float4 smem[];
     const uint32_t staged = min(S.tlas_node_count, C.smem_nodes);
     for (uint32_t i = threadIdx.x; i < staged * kNode4F4; i += blockDim.x) smem[i] = __ldg(S.tlas_nodes + i);
@@ -346,9 +349,8 @@ static luz_status ensure_vis_buffers(luz_ctx* ctx, luz_frame* f, const VisSizes&
 
 luz_status launch_visibility(luz_ctx* ctx, luz_frame* f, const luz_tlas* t, int frame_index,
                              unsigned long long* d_stats) {
-    luz_status s = clear_visibility(ctx, f);
+    luz_status s = ensure_lit_list(ctx, f);
     if (s != LUZ_OK) return s;
-    if ((s = ensure_lit_list(ctx, f)) != LUZ_OK) return s;
     if (f->shadow_slots + f->ao_samples == 0) return LUZ_OK;
     cudaStream_t st = ctx->stream;
     SceneVis S = make_scene_vis(f, t, frame_index);
@@ -380,6 +382,7 @@ luz_status launch_visibility(luz_ctx* ctx, luz_frame* f, const luz_tlas* t, int 
     const uint32_t ao_chunks = z.ao_patches ? (z.patches + z.ao_patches - 1) / z.ao_patches : 0u;
     z.chunks = std::max(shadow_chunks, ao_chunks);
     if (d_stats) LUZ_CUDA(ctx, cudaMemsetAsync(d_stats, 0, 5 * sizeof(unsigned long long), st));
+    if (!shadow_chunks && (s = clear_visibility(ctx, f)) != LUZ_OK) return s;   // else by patch_kernel
     if (z.chunks == 0) return LUZ_OK;
     if ((s = ensure_vis_buffers(ctx, f, z)) != LUZ_OK) return s;
     VisCounters* counters = (VisCounters*)f->vis_counters;
@@ -398,12 +401,12 @@ luz_status launch_visibility(luz_ctx* ctx, luz_frame* f, const luz_tlas* t, int 
     prof_begin(ctx, LUZ_KERNEL_RAYGEN);
     PatchRec* patches = (PatchRec*)f->patches;
     if (shadow_chunks) {
-        patch_kernel<<<std::min(z.supers, sms * 8), kSuper * 32, 0, st>>>(S, patches, patches + z.patches, counters,
+        chain(patch_kernel, std::min(z.supers, sms * 8), kSuper * 32, 0, st, S, patches, patches + z.patches, counters,
                                                                           z.chunks);
         LUZ_LAUNCHED(ctx, "patch_kernel");
     }
     if (d_stats) {
-        count_rays_kernel<<<sms * 4, 256, 0, st>>>(S, C, d_stats);
+        chain(count_rays_kernel, sms * 4, 256, 0, st, S, C, d_stats);
         LUZ_LAUNCHED(ctx, "count_rays_kernel");
     }
     for (uint32_t k = 0; k < z.chunks; ++k) {
@@ -420,32 +423,31 @@ luz_status launch_visibility(luz_ctx* ctx, luz_frame* f, const luz_tlas* t, int 
         const uint32_t shaft_work = A.cap / kSuper, max_grid = sms * ctx->cull_blocks;
         auto cull_grid = [&](uint32_t warps) { return std::min((warps + kCullWarps - 1) / kCullWarps, max_grid); };
         if (shadow && ao && f->pixels <= kCullTogether) {
-            cull_kernel<true, true><<<cull_grid(shaft_work + O.patches), kCullThreads, 0, st>>>(S, C, A, O, n->cull_tickets);
+            chain(cull_kernel<true, true>, cull_grid(shaft_work + O.patches), kCullThreads, 0, st, S, C, A, O, n->cull_tickets);
             LUZ_LAUNCHED(ctx, "cull_kernel");
         } else {
             if (shadow) {
-                cull_kernel<false, true><<<cull_grid(shaft_work), kCullThreads, 0, st>>>(S, C, A, O, n->cull_tickets);
+                chain(cull_kernel<false, true>, cull_grid(shaft_work), kCullThreads, 0, st, S, C, A, O, n->cull_tickets);
                 LUZ_LAUNCHED(ctx, "cull_kernel<shadow>");
             }
             if (ao) {
-                cull_kernel<true, false><<<cull_grid(O.patches), kCullThreads, 0, st>>>(S, C, A, O, n->cull_tickets + 1);
+                chain(cull_kernel<true, false>, cull_grid(O.patches), kCullThreads, 0, st, S, C, A, O, n->cull_tickets + 1);
                 LUZ_LAUNCHED(ctx, "cull_kernel<ao>");
             }
         }
         if (shadow) {
-            shadow_raygen_kernel<<<std::min((z.pairs + 7) / 8, sms * ctx->raygen_blocks), 256, 0, st>>>(
-                S, C, entries, f->active, &n->groups, &n->raygen_tickets, R);
+            chain(shadow_raygen_kernel, std::min((z.pairs + 7) / 8, sms * ctx->raygen_blocks), 256, 0, st, S, C, entries, f->active, &n->groups, &n->raygen_tickets, R);
             LUZ_LAUNCHED(ctx, "shadow_raygen_kernel");
         }
         prof_end(ctx);
         if (d_stats) {
-            if (staged) visibility_kernel<true, true><<<grid, 256, smem, st>>>(S, C, entries, R, d_stats);
-            else visibility_kernel<true, false><<<grid, 256, smem, st>>>(S, C, entries, R, d_stats);
+            if (staged) chain(visibility_kernel<true, true>, grid, 256, smem, st, S, C, entries, R, d_stats);
+            else chain(visibility_kernel<true, false>, grid, 256, smem, st, S, C, entries, R, d_stats);
             LUZ_LAUNCHED(ctx, "visibility_kernel<stats>");
         } else {
             prof_begin(ctx, LUZ_KERNEL_TRAVERSAL);
-            if (staged) visibility_kernel<false, true><<<grid, 256, smem, st>>>(S, C, entries, R, nullptr);
-            else visibility_kernel<false, false><<<grid, 256, smem, st>>>(S, C, entries, R, nullptr);
+            if (staged) chain(visibility_kernel<false, true>, grid, 256, smem, st, S, C, entries, R, nullptr);
+            else chain(visibility_kernel<false, false>, grid, 256, smem, st, S, C, entries, R, nullptr);
             prof_end(ctx);
             LUZ_LAUNCHED(ctx, "visibility_kernel");
         }
