@@ -509,7 +509,11 @@ void* luz_frame_plane_device_ptr(luz_frame* frame, int32_t plane);
 
 /* ------------------------------------------------------------------ batches
  * Many independent scenes of uneven size as one unit (no counterpart in the
- * reference, which renders one scene per frame). A render runs, by default, ONE
+ * reference, which renders one scene per frame). A render takes one of two forms. Scenes
+ * of 200,000 pixels and more on average, or up to two scenes of any size, run in lanes:
+ * every pass of a scene as the launches of a single frame, the scenes spread over up to
+ * eight streams that fork from the context's and join it again; a lane's buffers are those
+ * of a single frame's trace, for its largest scene. Many small scenes run as ONE
  * persistent launch (the frame kernel) over every scene: the per-frame TLAS builds,
  * the clearing of the hit/miss planes, the G-buffer passes with their lit-pixel lists,
  * the shadow/AO traversal of all scenes' rays from one work counter, and the light
@@ -517,9 +521,8 @@ void* luz_frame_plane_device_ptr(luz_frame* frame, int32_t plane);
  * before them, each wait bounded (LUZ_DEV_BATCH_QUEUE when one gives up). The meshes'
  * BLASes are built before, once, by luz_blas_build_batch (the reference builds them
  * once at load, GPUScene.cpp:108-138). The frame kernel takes scenes of up to 4096
- * instances and 688 lights; a batch with a larger scene renders staged (every TLAS
- * build, G-buffer and light pass its own launch around one visibility launch over all
- * scenes), which luz_batch_set_fused(ctx, b, 0) also selects. Both forms give the same
+ * instances and 688 lights; a batch with a larger scene always runs in lanes, which
+ * luz_batch_set_fused(ctx, b, 0) also selects. Both forms give the same
  * planes bit for bit. Scene constants and instances are uploaded / packed once at
  * creation (the arrays may be freed after luz_batch_create); luz_batch_capture records
  * a render as one CUDA graph that luz_batch_replay launches; luz_batch_autotune picks
@@ -542,17 +545,18 @@ uint32_t luz_batch_count(const luz_batch* b);
 /* The frame of scene i (planes readable with luz_frame_read). */
 luz_frame* luz_batch_frame(luz_batch* b, uint32_t i);
 luz_status luz_batch_render(luz_ctx* ctx, luz_batch* b, int32_t frame_index);
-/* A render with the counting visibility kernel: out[0..4] as luz_trace_visibility_stats. */
+/* A render that traces every ray from its TLAS root and counts: out[0..4] as
+ * luz_trace_visibility_stats, the same in either form. */
 luz_status luz_batch_stats(luz_ctx* ctx, luz_batch* b, int32_t frame_index, uint64_t out[5]);
 /* Records one render (on the context's explicit stream) into a CUDA graph. */
 luz_status luz_batch_capture(luz_ctx* ctx, luz_batch* b, int32_t frame_index);
 luz_status luz_batch_replay(luz_ctx* ctx, luz_batch* b);
 luz_status luz_batch_autotune(luz_ctx* ctx, luz_batch* b, uint32_t reps, luz_vis_tuning* chosen,
                               float* best_ms);
-/* on = 1: renders run the frame kernel (LUZ_ERR_LIMIT when a scene does not fit it);
- * on = 0: staged launches. Drops a captured graph. */
+/* on = 1: renders run the frame kernel where it is the faster form (LUZ_ERR_LIMIT when a
+ * scene does not fit it); on = 0: lanes. Drops a captured graph. */
 luz_status luz_batch_set_fused(luz_ctx* ctx, luz_batch* b, int32_t on);
-/* 1 when the batch renders with the frame kernel. */
+/* 1 unless the batch was set, or is left by its scenes, to lanes alone. */
 int32_t luz_batch_fused(const luz_batch* b);
 
 /* ------------------------------------------------------------------ denoiser

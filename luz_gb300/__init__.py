@@ -582,10 +582,10 @@ class _BorrowedFrame(Frame):
 
 class Batch:
     """Many scenes rendered as one unit (luz_batch_*): one batched BLAS build over the
-    meshes of every scene at creation, then per render ONE persistent launch (the frame
-    kernel: every TLAS build, G-buffer, the traversal of all scenes' rays and every
-    light pass), or the staged launches (set_fused(False)); optionally as one CUDA
-    graph."""
+    meshes of every scene at creation, then per render every scene's passes spread over
+    a few streams (lanes), or, for many small scenes unless set_fused(False), ONE
+    persistent launch (the frame kernel: every TLAS build, G-buffer, the traversal of all
+    scenes' rays and every light pass); optionally as one CUDA graph."""
 
     def __init__(self, ctx: "Context", scenes: list[HostScene]):
         self.ctx, self.scenes = ctx, scenes
@@ -638,7 +638,7 @@ class Batch:
 
     @property
     def fused(self) -> bool:
-        """True when renders run the frame kernel."""
+        """True where the frame kernel may run (it does where it is the faster form)."""
         return bool(lib.luz_batch_fused(self._h))
 
     def set_fused(self, on: bool) -> None:

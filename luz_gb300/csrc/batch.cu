@@ -1,13 +1,13 @@
-// batch.cu — many independent scenes of uneven size rendered as one unit. The frame
-// kernel (batch_frame_kernel) runs a whole frame of every scene in ONE persistent
-// launch: the per-frame TLAS builds, the clearing of the hit/miss planes, the G-buffer
-// tiles with their lit-pixel compaction, the shadow/AO traversal of all scenes' rays and
-// the light passes, ordered by tickets from a few counters and per-scene flags, every
-// wait bounded. Recordable as one CUDA graph (a memset of the counters and the kernel)
-// and replayed with a single launch; a launch-shape autotuner. The staged form (every
-// TLAS build, G-buffer and light pass its own launch around one visibility launch)
-// remains for scenes the frame kernel does not take. (No counterpart in the reference,
-// which renders one scene per frame.)
+// batch.cu — many independent scenes of uneven size rendered as one unit, in one of two
+// forms. Lanes: each scene's passes as the launches of a single frame, the scenes spread
+// over a few streams that fork from the context's and join it again. The frame kernel
+// (batch_frame_kernel), for many small scenes, runs a whole frame of every scene in ONE
+// persistent launch: the per-frame TLAS builds, the clearing of the hit/miss planes, the
+// G-buffer tiles with their lit-pixel compaction, the shadow/AO traversal of all scenes'
+// rays and the light passes, ordered by tickets from a few counters and per-scene flags,
+// every wait bounded. Either is recordable as one CUDA graph and replayed with a single
+// launch; a launch-shape autotuner. (No counterpart in the reference, which renders one
+// scene per frame.)
 #include <algorithm>
 #include <cstddef>
 #include <cstring>
@@ -20,7 +20,7 @@
 
 namespace luz {
 luz_status pack_tlas_input(luz_ctx* ctx, luz_tlas* t, const luz_instance* inst, uint32_t n);
-luz_status launch_tlas_build(luz_ctx* ctx, luz_tlas* t);
+luz_status launch_tlas_kernels(luz_ctx* ctx, luz_tlas* t);
 luz_status launch_gbuffer(luz_ctx* ctx, luz_frame* f, const luz_tlas* t);
 luz_status launch_light_pass(luz_ctx* ctx, luz_frame* f, int mode);
 luz_status make_gbuf_params(luz_ctx* ctx, luz_frame* f, const luz_tlas* t, GbufParams& G);
@@ -362,6 +362,13 @@ __global__ void __launch_bounds__(kVisThreads, LUZ_VIS_MIN_BLOCKS) batch_frame_k
 }  // namespace luz
 
 struct luz_batch {
+    // A stream of its own for some of the scenes (the first lane's is the context's), their
+    // traces' buffers, and the event that joins it.
+    struct Lane {
+        cudaStream_t stream = nullptr;
+        cudaEvent_t joined = nullptr;
+        luz::VisScratch scratch;
+    };
     luz_ctx* ctx = nullptr;
     std::vector<luz_tlas*> tlas;
     std::vector<luz_frame*> frames;
@@ -375,7 +382,7 @@ struct luz_batch {
     int frame_index = 0;
     // frame kernel
     bool fusable = false;            // every scene fits the frame kernel
-    bool fused = false;              // renders run the frame kernel
+    bool fused = false;              // renders run the frame kernel where it is the faster form
     luz::FrameScene* d_fs = nullptr;
     uint32_t* d_tile_off = nullptr;
     luz::ClearItem* d_clears = nullptr;
@@ -383,6 +390,11 @@ struct luz_batch {
     size_t ctl_bytes = 0;
     uint32_t* d_light_off = nullptr;
     uint32_t clear_items = 0, tile_items = 0;
+    // lanes
+    std::vector<Lane> lanes;
+    std::vector<uint32_t> order, lane_of;   // scenes in launch order; the lane of each scene
+    cudaEvent_t fork = nullptr;
+    bool small = false;              // the frame kernel is the faster form
 };
 
 namespace luz {
@@ -428,17 +440,122 @@ static luz_status launch_frame(luz_ctx* ctx, luz_batch* b, bool stats) {
     return LUZ_OK;
 }
 
+// The frame kernel starts every ray at its TLAS root and traces the G-buffer without tile
+// lists, but is one launch: it stays the faster form for many small scenes. kLanes = 8 is the
+// number of streams that the device takes work from at once. Renders, us, frame kernel and
+// lanes: 12 scenes of 256x256 196 / 235, 64 510 / 981, 12 of 512x512 376 / 360, 40 793 / 729,
+// 12 of 1280x720 813 / 553; few scenes are faster in lanes at any size, a lane each: 2 of
+// 64x64 325 / 193, 2 of 256x256 94 / 81.
+constexpr uint64_t kLanePixels = 200000;    // mean pixels of a scene from which on the lanes are taken
+constexpr uint32_t kLaneScenes = 2;         // and scenes up to which they always are
+constexpr uint32_t kLanes = 8;
+
+static bool runs_frame_kernel(const luz_batch* b) { return b->fused && b->small; }
+
+static void drop_graph(luz_batch* b) {
+    if (b->exec) cudaGraphExecDestroy(b->exec);
+    if (b->graph) cudaGraphDestroy(b->graph);
+    b->exec = nullptr;
+    b->graph = nullptr;
+}
+
+static void drop_lanes(luz_batch* b) {
+    for (auto& lane : b->lanes) {
+        lane.scratch.release();
+        if (lane.joined) cudaEventDestroy(lane.joined);
+        if (lane.stream) cudaStreamDestroy(lane.stream);
+    }
+    b->lanes.clear();
+    if (b->fork) cudaEventDestroy(b->fork);
+    b->fork = nullptr;
+}
+
+// `count` lanes and the scenes' assignment to them: largest first, each to the least loaded.
+static luz_status make_lanes(luz_ctx* ctx, luz_batch* b, uint32_t count) {
+    const uint32_t n = (uint32_t)b->frames.size();
+    LUZ_CUDA(ctx, cudaEventCreateWithFlags(&b->fork, cudaEventDisableTiming));
+    b->lanes.resize(count);
+    for (size_t k = 1; k < count; ++k) {
+        LUZ_CUDA(ctx, cudaStreamCreateWithFlags(&b->lanes[k].stream, cudaStreamNonBlocking));
+        LUZ_CUDA(ctx, cudaEventCreateWithFlags(&b->lanes[k].joined, cudaEventDisableTiming));
+    }
+    std::vector<uint64_t> work(n), load(count, 0);
+    b->order.resize(n);
+    b->lane_of.resize(n);
+    for (uint32_t i = 0; i < n; ++i) {
+        b->order[i] = i;
+        work[i] = (uint64_t)b->frames[i]->pixels * (1u + b->frames[i]->shadow_slots + b->frames[i]->ao_samples);
+    }
+    std::stable_sort(b->order.begin(), b->order.end(), [&](uint32_t x, uint32_t y) { return work[x] > work[y]; });
+    for (uint32_t i : b->order) {
+        const size_t k = std::min_element(load.begin(), load.end()) - load.begin();
+        b->lane_of[i] = (uint32_t)k;
+        load[k] += work[i];
+    }
+    return LUZ_OK;
+}
+
+// The lanes and their traces' buffers, in fewer lanes where the memory for more is not
+// there; nothing to do when they are.
+static luz_status reserve_lanes(luz_ctx* ctx, luz_batch* b) {
+    const uint32_t n = (uint32_t)b->frames.size();
+    uint32_t count = b->lanes.empty() ? std::min(kLanes, n) : (uint32_t)b->lanes.size();
+    for (;; count /= 2) {
+        luz_status s = b->lanes.empty() ? make_lanes(ctx, b, count) : LUZ_OK;
+        for (uint32_t i = 0; s == LUZ_OK && i < n; ++i) {
+            VisScratch& v = b->lanes[b->lane_of[i]].scratch;
+            const VisScratch before = v;
+            s = reserve_visibility(ctx, b->frames[i], b->tlas[i], v);
+            if (memcmp(&before, &v, sizeof v)) drop_graph(b);   // it holds the buffers' addresses
+        }
+        if (s == LUZ_OK) return s;
+        cudaGetLastError();
+        LUZ_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
+        drop_lanes(b);
+        if (s != LUZ_ERR_OOM || count <= 1) return s;
+    }
+}
+
+// Every scene's passes as launches of their own, the scenes spread over the lanes: the small
+// scenes' short kernels and every kernel's last blocks run beside those of other lanes.
+static luz_status launch_lanes(luz_ctx* ctx, luz_batch* b, int frame_index) {
+    luz_status s = reserve_lanes(ctx, b);
+    if (s != LUZ_OK) return s;
+    const cudaStream_t own = ctx->stream;
+    const size_t lanes = b->lanes.size();
+    LUZ_CUDA(ctx, cudaEventRecord(b->fork, own));
+    for (size_t k = 1; k < lanes; ++k) LUZ_CUDA(ctx, cudaStreamWaitEvent(b->lanes[k].stream, b->fork, 0));
+    for (uint32_t i : b->order) {
+        luz_batch::Lane& lane = b->lanes[b->lane_of[i]];
+        luz_frame* f = b->frames[i];
+        if (b->lane_of[i]) ctx->stream = lane.stream;
+        s = launch_tlas_kernels(ctx, b->tlas[i]);
+        if (s == LUZ_OK) s = launch_gbuffer(ctx, f, b->tlas[i]);
+        if (s == LUZ_OK) s = launch_visibility(ctx, f, b->tlas[i], frame_index, nullptr, lane.scratch);
+        if (s == LUZ_OK) s = launch_light_pass(ctx, f, 0);
+        ctx->stream = own;
+        if (s != LUZ_OK) break;
+    }
+    for (size_t k = 1; k < lanes; ++k) {   // also after an error: the lanes end in the context's stream
+        LUZ_CUDA(ctx, cudaEventRecord(b->lanes[k].joined, b->lanes[k].stream));
+        LUZ_CUDA(ctx, cudaStreamWaitEvent(own, b->lanes[k].joined, 0));
+    }
+    return s;
+}
+
+// stats: every ray traced from its TLAS root by a counting launch, in either form.
 static luz_status batch_record(luz_ctx* ctx, luz_batch* b, int frame_index, bool stats) {
     luz_status s = set_frame_index(ctx, b, frame_index);
     if (s != LUZ_OK) return s;
-    if (b->fused) return launch_frame(ctx, b, stats);
+    if (runs_frame_kernel(b)) return launch_frame(ctx, b, stats);
+    if (!stats) return launch_lanes(ctx, b, frame_index);
     for (size_t i = 0; i < b->frames.size(); ++i) {
-        if ((s = launch_tlas_build(ctx, b->tlas[i])) != LUZ_OK) return s;
+        if ((s = launch_tlas_kernels(ctx, b->tlas[i])) != LUZ_OK) return s;
         if ((s = launch_gbuffer(ctx, b->frames[i], b->tlas[i])) != LUZ_OK) return s;
         if ((s = clear_visibility(ctx, b->frames[i])) != LUZ_OK) return s;
     }
-    if ((s = launch_visibility_batch(ctx, b->d_scenes, (uint32_t)b->frames.size(), b->d_offsets, b->d_work,
-                                     stats ? b->d_stats : nullptr)) != LUZ_OK)
+    if ((s = launch_visibility_count(ctx, b->d_scenes, (uint32_t)b->frames.size(), b->d_offsets, b->d_work, b->d_stats)) !=
+        LUZ_OK)
         return s;
     for (auto* f : b->frames)
         if ((s = launch_light_pass(ctx, f, 0)) != LUZ_OK) return s;
@@ -494,13 +611,6 @@ static luz_status setup_frame_kernel(luz_ctx* ctx, luz_batch* b) {
     return LUZ_OK;
 }
 
-static void drop_graph(luz_batch* b) {
-    if (b->exec) cudaGraphExecDestroy(b->exec);
-    if (b->graph) cudaGraphDestroy(b->graph);
-    b->exec = nullptr;
-    b->graph = nullptr;
-}
-
 }  // namespace luz
 
 using namespace luz;
@@ -541,6 +651,13 @@ static luz_status batch_create_body(luz_ctx* ctx, uint32_t count, const luz_batc
     if (e != cudaSuccess) return fail(cuda_error(ctx, e, "batch allocation"));
     luz_status fs = setup_frame_kernel(ctx, b);
     if (fs != LUZ_OK) return fail(fs);
+    uint64_t pixels = 0;
+    for (auto* f : b->frames) pixels += f->pixels;
+    b->small = count > kLaneScenes && pixels < kLanePixels * count;
+    if (!runs_frame_kernel(b) && (fs = reserve_lanes(ctx, b)) != LUZ_OK) {
+        if (fs != LUZ_ERR_OOM || !b->fusable) return fail(fs);
+        b->small = true;   // no memory for the lanes' traces: the frame kernel needs none
+    }
     *out = b;
     return LUZ_OK;
 }
@@ -553,6 +670,7 @@ void luz_batch_destroy(luz_batch* b) {
     if (!b) return;
     cudaDeviceSynchronize();
     drop_graph(b);
+    drop_lanes(b);
     for (auto* f : b->frames) luz_frame_destroy(f);
     for (auto* t : b->tlas) luz_tlas_destroy(t);
     void* p[] = {b->d_scenes, b->d_offsets, b->d_work, b->d_stats, b->d_fs, b->d_tile_off, b->d_clears, b->d_ctl,
@@ -589,6 +707,10 @@ luz_status luz_batch_capture(luz_ctx* ctx, luz_batch* b, int32_t frame_index) {
         return set_error(ctx, LUZ_ERR_INVALID, "capture needs an explicit stream");
     LUZ_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
     drop_graph(b);
+    if (!runs_frame_kernel(b)) {   // no allocation while recording
+        luz_status s = reserve_lanes(ctx, b);
+        if (s != LUZ_OK) return s;
+    }
     // The frame index is written before capture: the records are then constant.
     if (frame_index != b->frame_index) {
         for (auto& s : b->h_scenes) s.frame = frame_index;
@@ -618,8 +740,7 @@ luz_status luz_batch_replay(luz_ctx* ctx, luz_batch* b) {
     return LUZ_OK;
 }
 
-// Times the visibility launch of the batch (with the frame kernel: the whole frame
-// launch) for each candidate shape and keeps the fastest (median of `reps` launches). Candidates: refill {8,16,32} x steps
+// Times a render of the batch for each candidate shape of the traversal and keeps the fastest (median of `reps` launches). Candidates: refill {8,16,32} x steps
 // {16,32,64} x CTAs per SM {2,3,4}. Drops a captured graph (its shape is stale).
 luz_status luz_batch_autotune(luz_ctx* ctx, luz_batch* b, uint32_t reps, luz_vis_tuning* chosen, float* best_ms) {
     if (!ctx || !b) return LUZ_ERR_INVALID;
@@ -640,15 +761,8 @@ luz_status luz_batch_autotune(luz_ctx* ctx, luz_batch* b, uint32_t reps, luz_vis
                 ctx->vis_tuning = VisTuning{0, rf, sp, ct, 1};
                 std::vector<float> ts;
                 for (uint32_t r = 0; r <= reps; ++r) {
-                    if (!b->fused)
-                        for (auto* f : b->frames)
-                            if ((s = clear_visibility(ctx, f)) != LUZ_OK) return s;
                     cudaEventRecord(e0, ctx->stream);
-                    if (b->fused)
-                        s = launch_frame(ctx, b, false);
-                    else
-                        s = launch_visibility_batch(ctx, b->d_scenes, (uint32_t)b->frames.size(), b->d_offsets,
-                                                    b->d_work, nullptr);
+                    s = runs_frame_kernel(b) ? launch_frame(ctx, b, false) : launch_lanes(ctx, b, b->frame_index);
                     if (s != LUZ_OK) return s;
                     cudaEventRecord(e1, ctx->stream);
                     LUZ_CUDA(ctx, cudaEventSynchronize(e1));
@@ -678,7 +792,7 @@ luz_status luz_batch_set_fused(luz_ctx* ctx, luz_batch* b, int32_t on) {
         return set_error(ctx, LUZ_ERR_LIMIT, "a scene of the batch does not fit the frame kernel");
     if ((on != 0) != b->fused) drop_graph(b);
     b->fused = on != 0;
-    return LUZ_OK;
+    return runs_frame_kernel(b) ? LUZ_OK : reserve_lanes(ctx, b);
 }
 
 int32_t luz_batch_fused(const luz_batch* b) { return b && b->fused ? 1 : 0; }

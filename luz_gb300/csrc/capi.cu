@@ -16,7 +16,7 @@ luz_status tlas_alloc(luz_ctx* ctx, luz_tlas* t);
 luz_status build_tlas(luz_ctx* ctx, luz_tlas* t, const luz_instance* inst, uint32_t n);
 luz_status launch_gbuffer(luz_ctx* ctx, luz_frame* f, const luz_tlas* t);
 luz_status launch_visibility(luz_ctx* ctx, luz_frame* f, const luz_tlas* t, int frame_index,
-                             unsigned long long* d_stats);
+                             unsigned long long* d_stats, VisScratch& scratch);
 luz_status frame_lit_count(luz_ctx* ctx, luz_frame* f, uint32_t* count);
 luz_status launch_light_pass(luz_ctx* ctx, luz_frame* f, int mode);
 uint32_t lit_chunks(uint32_t width, uint32_t height);
@@ -89,10 +89,10 @@ static void free_frame_buffers(luz_frame* f) {
                     f->unshadowed, f->denoised, f->surf, f->surf_mat,
                     f->features, f->lin_depth, f->taa, f->taa_next, f->compose, f->hist, f->hist_state,
                     f->block_counts, f->lit_count, f->dn_list, f->dn_count, f->d_upload, f->d_textures,
-                    f->d_texels, f->d_shadow_lights, f->d_shadow_maps, f->rays_a, f->rays_b, f->rays_c,
-                    f->patches, f->start_lists, f->cuts, f->active, f->vis_counters};
+                    f->d_texels, f->d_shadow_lights, f->d_shadow_maps};
     for (void* p : ptrs)
         if (p) cudaFree(p);
+    f->vis.release();
     if (f->h_upload) cudaFreeHost(f->h_upload);
     if (f->upload_done) cudaEventDestroy(f->upload_done);
 }
@@ -672,7 +672,7 @@ luz_status luz_gbuffer_primary(luz_ctx* ctx, luz_frame* f, const luz_tlas* t) {
 
 luz_status luz_trace_visibility(luz_ctx* ctx, luz_frame* f, const luz_tlas* t, int32_t frame_index) {
     if (!ctx || !f || !t) return LUZ_ERR_INVALID;
-    return launch_visibility(ctx, f, t, frame_index, nullptr);
+    return launch_visibility(ctx, f, t, frame_index, nullptr, f->vis);
 }
 
 luz_status luz_frame_set_shadow_cull(luz_frame* f, int32_t enable) {
@@ -689,7 +689,7 @@ luz_status luz_trace_visibility_stats(luz_ctx* ctx, luz_frame* f, const luz_tlas
     luz_status s = LUZ_OK;
     cudaError_t z = cudaMemsetAsync(d, 0, 5 * sizeof(unsigned long long), ctx->stream);   // zero when nothing is traced
     if (z != cudaSuccess) s = cuda_error(ctx, z, "stats clear");
-    if (s == LUZ_OK) s = launch_visibility(ctx, f, t, frame_index, d);
+    if (s == LUZ_OK) s = launch_visibility(ctx, f, t, frame_index, d, f->vis);
     if (s == LUZ_OK) {
         cudaError_t e = cudaMemcpyAsync(out, d, 5 * sizeof(unsigned long long), cudaMemcpyDeviceToHost, ctx->stream);
         if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
@@ -723,7 +723,7 @@ luz_status luz_render_frame(luz_ctx* ctx, luz_frame* f, luz_tlas* t, const luz_i
     luz_status s;
     if ((s = luz_tlas_build(ctx, t, instances, instance_count)) != LUZ_OK) return s;
     if ((s = launch_gbuffer(ctx, f, t)) != LUZ_OK) return s;
-    if ((s = launch_visibility(ctx, f, t, frame_index, nullptr)) != LUZ_OK) return s;
+    if ((s = launch_visibility(ctx, f, t, frame_index, nullptr, f->vis)) != LUZ_OK) return s;
     return launch_light_pass(ctx, f, 0);
 }
 

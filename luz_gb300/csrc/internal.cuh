@@ -175,6 +175,30 @@ struct luz_tlas {
     size_t tmp_bytes = 0;
 };
 
+namespace luz {
+// Buffers of one trace, grown on demand: of a chunk (shafts.cuh) the patch bounds, start
+// lists per (virtual light, patch) and per AO patch, the lists' cuts, the shadow groups to
+// trace and the ray records (RayOut, structure of arrays), and the chunks' counters. A
+// frame has its own; traces that run one after the other can share one.
+struct VisScratch {
+    void* patches = nullptr;
+    uint32_t* start_lists = nullptr;
+    float4* cuts = nullptr;
+    uint4* active = nullptr;
+    float4* rays_a = nullptr;
+    float4* rays_b = nullptr;
+    uint4* rays_c = nullptr;
+    void* counters = nullptr;             // VisCounters per chunk
+    uint32_t patches_cap = 0, lists_cap = 0, pairs_cap = 0, records_cap = 0, chunks_cap = 0;
+    void release() {
+        for (void* p : {patches, (void*)start_lists, (void*)cuts, (void*)active, (void*)rays_a, (void*)rays_b,
+                        (void*)rays_c, counters})
+            if (p) cudaFree(p);
+        *this = VisScratch{};
+    }
+};
+}  // namespace luz
+
 struct luz_frame {
     luz_ctx* ctx = nullptr;
     uint32_t width = 0, height = 0, pixels = 0, words = 0;  // words per bit plane
@@ -241,18 +265,7 @@ struct luz_frame {
     // and log2 of the most samples one of them has
     uint32_t* d_vlights = nullptr;
     uint32_t vlight_count = 0, vlight_shift = 0;
-    // of one chunk (shafts.cuh): patch bounds, start lists per (virtual light, patch) and
-    // per AO patch, the lists' cuts, the shadow groups to trace, and the ray records
-    // (RayOut, structure of arrays)
-    void* patches = nullptr;
-    uint32_t* start_lists = nullptr;
-    float4* cuts = nullptr;
-    uint4* active = nullptr;
-    float4* rays_a = nullptr;
-    float4* rays_b = nullptr;
-    uint4* rays_c = nullptr;
-    void* vis_counters = nullptr;         // VisCounters per chunk
-    uint32_t lists_cap = 0, pairs_cap = 0, records_cap = 0, chunks_cap = 0;
+    luz::VisScratch vis;
 };
 
 // ---------------------------------------------------------------- error plumbing

@@ -1288,6 +1288,7 @@ static size_t tlas_tmp_bytes(uint32_t cap) {
 }
 
 luz_status launch_tlas_build(luz_ctx* ctx, luz_tlas* t);
+luz_status launch_tlas_kernels(luz_ctx* ctx, luz_tlas* t);
 
 luz_status tlas_alloc(luz_ctx* ctx, luz_tlas* t) {
     uint32_t cap = std::max(t->max_instances, 1u);
@@ -1384,11 +1385,17 @@ const float4* tlas_leaf_boxes(const luz_tlas* t) { return carve_tlas(const_cast<
 // Device part of a TLAS build from the packed staging buffer: one host-to-device copy
 // from pinned memory and the LBVH kernels; no host synchronisation (graph-capturable).
 luz_status launch_tlas_build(luz_ctx* ctx, luz_tlas* t) {
+    if (t->count)
+        LUZ_CUDA(ctx, cudaMemcpyAsync(t->d_input, t->h_input, (size_t)t->count * sizeof(DevInstanceInput),
+                                      cudaMemcpyHostToDevice, ctx->stream));
+    return launch_tlas_kernels(ctx, t);
+}
+
+// The kernels alone, over the instances on the device.
+luz_status launch_tlas_kernels(luz_ctx* ctx, luz_tlas* t) {
     cudaStream_t st = ctx->stream;
     const uint32_t n = t->count;
     if (n == 0) return LUZ_OK;
-    LUZ_CUDA(ctx, cudaMemcpyAsync(t->d_input, t->h_input, (size_t)n * sizeof(DevInstanceInput),
-                                  cudaMemcpyHostToDevice, st));
     const uint32_t m = std::max(n, 2u) - 1;
     TlasScratch ts = carve_tlas(t);
     const TlasBuildArgs& A = ts.a;

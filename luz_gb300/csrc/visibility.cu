@@ -175,11 +175,11 @@ visibility_kernel(SceneVis S, VisCommon C, Entries E, RayOut R, unsigned long lo
     if (kStats) flush_stats(stats, 0u, cnt);
 }
 
-// Many scenes in one launch: item g belongs to the scene s with
-// offsets[s] <= g < offsets[s+1]; each lane carries its scene's TLAS and outputs.
-template <bool kStats>
+// The rays of many scenes traced from their TLAS roots in one counting launch: item g
+// belongs to the scene s with offsets[s] <= g < offsets[s+1]; each lane carries its scene's
+// TLAS and outputs.
 __global__ void __launch_bounds__(kVisThreads, LUZ_VIS_MIN_BLOCKS)
-visibility_batch_kernel(const SceneVis* __restrict__ scenes, uint32_t n, const unsigned long long* __restrict__ offsets,
+visibility_count_kernel(const SceneVis* __restrict__ scenes, uint32_t n, const unsigned long long* __restrict__ offsets,
                         VisCommon C, unsigned long long* stats) {
     extern __shared__ float4 smem[];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -215,16 +215,16 @@ visibility_batch_kernel(const SceneVis* __restrict__ scenes, uint32_t n, const u
                     uint32_t slot = (uint32_t)(local / lit);
                     uint32_t j = (uint32_t)(local - (unsigned long long)slot * lit);
                     active = setup_ray(r, c, S, C, slot, j);
-                    if (kStats && active) ++rays;
+                    if (active) ++rays;
                 }
             }
         }
         if (exhausted && __ballot_sync(full, active) == 0) break;
-        run_steps<kStats, false>(r, c, active, nullptr, 0u, r.tlas, r.insts, s_stack, lstack, C.steps, C.step_cap, err,
+        run_steps<true, false>(r, c, active, nullptr, 0u, r.tlas, r.insts, s_stack, lstack, C.steps, C.step_cap, err,
                                  cnt);
     }
     if (err) atomicOr(C.status, err);
-    if (kStats) flush_stats(stats, rays, cnt);
+    flush_stats(stats, rays, cnt);
 }
 
 // offsets[s] = rays of scenes 0..s-1 (lit pixels x samples), read after the
@@ -306,49 +306,75 @@ struct VisSizes {
     uint32_t patches, supers;
     uint32_t pairs, ao_patches;      // per chunk
     uint32_t records;                // per chunk
-    uint32_t chunks;
+    uint32_t shadow_chunks, ao_chunks, chunks;
 };
 
-static luz_status ensure_vis_buffers(luz_ctx* ctx, luz_frame* f, const VisSizes& z) {
-    if (f->patches && z.pairs + z.ao_patches <= f->lists_cap && z.pairs <= f->pairs_cap &&
-        z.records <= f->records_cap && z.chunks <= f->chunks_cap)
+// Chunks over the largest possible counts; what lies past the frame's actual counts
+// returns at once on the device. Without instances no shadow ray has anything to hit.
+static VisSizes vis_sizes(const luz_frame* f, const luz_tlas* t) {
+    VisSizes z{};
+    z.patches = (f->pixels + kPatch - 1) / kPatch;
+    z.supers = (z.patches + kSuper - 1) / kSuper;
+    const uint32_t shift = f->vlight_shift;
+    const unsigned long long max_pairs = t->count > 0 ? (unsigned long long)z.supers * kSuper * f->vlight_count : 0ull;
+    z.pairs = (uint32_t)std::min<unsigned long long>(max_pairs, (kRayChunk / kPatch) >> shift);
+    if (f->ao_samples) z.ao_patches = std::min(z.patches, std::max(kAoChunk / (kPatch * f->ao_samples), 1u));
+    z.records = ((z.pairs * kPatch) << shift) + z.ao_patches * kPatch * f->ao_samples;
+    z.shadow_chunks = z.pairs ? (uint32_t)((max_pairs + z.pairs - 1) / z.pairs) : 0u;
+    z.ao_chunks = z.ao_patches ? (z.patches + z.ao_patches - 1) / z.ao_patches : 0u;
+    z.chunks = std::max(z.shadow_chunks, z.ao_chunks);
+    return z;
+}
+
+static luz_status ensure_vis_buffers(luz_ctx* ctx, VisScratch& v, const VisSizes& z) {
+    const uint32_t patches = z.patches + z.supers, lists = z.pairs + z.ao_patches;
+    if (patches <= v.patches_cap && lists <= v.lists_cap && z.pairs <= v.pairs_cap && z.records <= v.records_cap &&
+        z.chunks <= v.chunks_cap)
         return LUZ_OK;
     LUZ_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
     auto again = [&](auto*& p, size_t bytes) -> cudaError_t {
         cudaFree(p);
         p = nullptr;
-        return bytes ? cudaMalloc(&p, bytes) : cudaSuccess;
+        return bytes ? cudaMalloc((void**)&p, bytes) : cudaSuccess;
     };
-    if (!f->patches)   // the patches, then their blocks
-        LUZ_CUDA(ctx, cudaMalloc(&f->patches, ((size_t)z.patches + z.supers) * sizeof(PatchRec)));
-    if (z.pairs + z.ao_patches > f->lists_cap) {
-        f->lists_cap = 0;
-        LUZ_CUDA(ctx, again(f->start_lists, ((size_t)z.pairs + z.ao_patches) * kEntryWords * 4));
-        f->lists_cap = z.pairs + z.ao_patches;
+    if (patches > v.patches_cap) {   // the patches, then their blocks
+        v.patches_cap = 0;
+        LUZ_CUDA(ctx, again(v.patches, (size_t)patches * sizeof(PatchRec)));
+        v.patches_cap = patches;
     }
-    if (z.pairs > f->pairs_cap) {
-        f->pairs_cap = 0;
-        LUZ_CUDA(ctx, again(f->cuts, (size_t)z.pairs * kCutsPerPair * kNode4F4 * sizeof(float4)));
-        LUZ_CUDA(ctx, again(f->active, (size_t)z.pairs * sizeof(uint4)));
-        f->pairs_cap = z.pairs;
+    if (lists > v.lists_cap) {
+        v.lists_cap = 0;
+        LUZ_CUDA(ctx, again(v.start_lists, (size_t)lists * kEntryWords * 4));
+        v.lists_cap = lists;
     }
-    if (z.records > f->records_cap) {
-        f->records_cap = 0;
-        LUZ_CUDA(ctx, again(f->rays_a, (size_t)z.records * sizeof(float4)));
-        LUZ_CUDA(ctx, again(f->rays_b, (size_t)z.records * sizeof(float4)));
-        LUZ_CUDA(ctx, again(f->rays_c, (size_t)z.records * sizeof(uint4)));
-        f->records_cap = z.records;
+    if (z.pairs > v.pairs_cap) {
+        v.pairs_cap = 0;
+        LUZ_CUDA(ctx, again(v.cuts, (size_t)z.pairs * kCutsPerPair * kNode4F4 * sizeof(float4)));
+        LUZ_CUDA(ctx, again(v.active, (size_t)z.pairs * sizeof(uint4)));
+        v.pairs_cap = z.pairs;
     }
-    if (z.chunks > f->chunks_cap) {
-        f->chunks_cap = 0;
-        LUZ_CUDA(ctx, again(f->vis_counters, (size_t)z.chunks * sizeof(VisCounters)));
-        f->chunks_cap = z.chunks;
+    if (z.records > v.records_cap) {
+        v.records_cap = 0;
+        LUZ_CUDA(ctx, again(v.rays_a, (size_t)z.records * sizeof(float4)));
+        LUZ_CUDA(ctx, again(v.rays_b, (size_t)z.records * sizeof(float4)));
+        LUZ_CUDA(ctx, again(v.rays_c, (size_t)z.records * sizeof(uint4)));
+        v.records_cap = z.records;
+    }
+    if (z.chunks > v.chunks_cap) {
+        v.chunks_cap = 0;
+        LUZ_CUDA(ctx, again(v.counters, (size_t)z.chunks * sizeof(VisCounters)));
+        v.chunks_cap = z.chunks;
     }
     return LUZ_OK;
 }
 
+luz_status reserve_visibility(luz_ctx* ctx, const luz_frame* f, const luz_tlas* t, VisScratch& scratch) {
+    const VisSizes z = vis_sizes(f, t);
+    return z.chunks ? ensure_vis_buffers(ctx, scratch, z) : LUZ_OK;
+}
+
 luz_status launch_visibility(luz_ctx* ctx, luz_frame* f, const luz_tlas* t, int frame_index,
-                             unsigned long long* d_stats) {
+                             unsigned long long* d_stats, VisScratch& v) {
     luz_status s = ensure_lit_list(ctx, f);
     if (s != LUZ_OK) return s;
     if (f->shadow_slots + f->ao_samples == 0) return LUZ_OK;
@@ -368,24 +394,13 @@ luz_status launch_visibility(luz_ctx* ctx, luz_frame* f, const luz_tlas* t, int 
     });
     if (s != LUZ_OK) return s;
     uint32_t grid = (uint32_t)ctx->sm_count * tu.ctas_per_sm;
-    // Chunks over the largest possible counts; what lies past the frame's actual counts
-    // returns at once on the device. Without instances no shadow ray has anything to hit.
-    VisSizes z{};
-    z.patches = (f->pixels + kPatch - 1) / kPatch;
-    z.supers = (z.patches + kSuper - 1) / kSuper;
-    const uint32_t shift = f->vlight_shift;
-    const unsigned long long max_pairs = t->count > 0 ? (unsigned long long)z.supers * kSuper * f->vlight_count : 0ull;
-    z.pairs = (uint32_t)std::min<unsigned long long>(max_pairs, (kRayChunk / kPatch) >> shift);
-    if (f->ao_samples) z.ao_patches = std::min(z.patches, std::max(kAoChunk / (kPatch * f->ao_samples), 1u));
-    z.records = ((z.pairs * kPatch) << shift) + z.ao_patches * kPatch * f->ao_samples;
-    const uint32_t shadow_chunks = z.pairs ? (uint32_t)((max_pairs + z.pairs - 1) / z.pairs) : 0u;
-    const uint32_t ao_chunks = z.ao_patches ? (z.patches + z.ao_patches - 1) / z.ao_patches : 0u;
-    z.chunks = std::max(shadow_chunks, ao_chunks);
+    const VisSizes z = vis_sizes(f, t);
+    const uint32_t shadow_chunks = z.shadow_chunks, ao_chunks = z.ao_chunks;
     if (d_stats) LUZ_CUDA(ctx, cudaMemsetAsync(d_stats, 0, 5 * sizeof(unsigned long long), st));
     if (!shadow_chunks && (s = clear_visibility(ctx, f)) != LUZ_OK) return s;   // else by patch_kernel
     if (z.chunks == 0) return LUZ_OK;
-    if ((s = ensure_vis_buffers(ctx, f, z)) != LUZ_OK) return s;
-    VisCounters* counters = (VisCounters*)f->vis_counters;
+    if ((s = ensure_vis_buffers(ctx, v, z)) != LUZ_OK) return s;
+    VisCounters* counters = (VisCounters*)v.counters;
     if (!shadow_chunks) LUZ_CUDA(ctx, cudaMemsetAsync(counters, 0, (size_t)z.chunks * sizeof(VisCounters), st));
     if (t->count) S.leaf_box = tlas_leaf_boxes(t);
     const uint32_t cap = list_cap(t->count);
@@ -397,9 +412,9 @@ luz_status launch_visibility(luz_ctx* ctx, luz_frame* f, const luz_tlas* t, int 
         ctx->raygen_blocks = std::max(b, 1);
     }
     const uint32_t sms = (uint32_t)ctx->sm_count;
-    const Entries entries{f->start_lists, f->cuts};
+    const Entries entries{v.start_lists, v.cuts};
     prof_begin(ctx, LUZ_KERNEL_RAYGEN);
-    PatchRec* patches = (PatchRec*)f->patches;
+    PatchRec* patches = (PatchRec*)v.patches;
     if (shadow_chunks) {
         chain(patch_kernel, std::min(z.supers, sms * 8), kSuper * 32, 0, st, S, patches, patches + z.patches, counters,
                                                                           z.chunks);
@@ -413,13 +428,13 @@ luz_status launch_visibility(luz_ctx* ctx, luz_frame* f, const luz_tlas* t, int 
         if (k) prof_begin(ctx, LUZ_KERNEL_RAYGEN);
         VisCounters* n = counters + k;
         C.work_counter = &n->traversed;
-        const RayOut R{f->rays_a, f->rays_b, f->rays_c, &n->records};
+        const RayOut R{v.rays_a, v.rays_b, v.rays_c, &n->records};
         const bool shadow = k < shadow_chunks, ao = k < ao_chunks;
         const ShaftOut A{patches, patches + z.patches, f->d_vlights, f->vlight_count, (unsigned long long)k * z.pairs,
-                         shadow ? z.pairs : 0u, cap, f->start_lists, f->cuts, f->active, &n->groups};
+                         shadow ? z.pairs : 0u, cap, v.start_lists, v.cuts, v.active, &n->groups};
         const AoOut O{k * z.ao_patches, ao ? std::min(z.ao_patches, z.patches - k * z.ao_patches) : 0u, cap,
                       f->ao_samples < kAoMinSamples ? 0u : std::min(kAoStepsPerSample * f->ao_samples, kAoSteps),
-                      f->start_lists + (size_t)z.pairs * kEntryWords, z.pairs, R};
+                      v.start_lists + (size_t)z.pairs * kEntryWords, z.pairs, R};
         const uint32_t shaft_work = A.cap / kSuper, max_grid = sms * ctx->cull_blocks;
         auto cull_grid = [&](uint32_t warps) { return std::min((warps + kCullWarps - 1) / kCullWarps, max_grid); };
         if (shadow && ao && f->pixels <= kCullTogether) {
@@ -436,7 +451,7 @@ luz_status launch_visibility(luz_ctx* ctx, luz_frame* f, const luz_tlas* t, int 
             }
         }
         if (shadow) {
-            chain(shadow_raygen_kernel, std::min((z.pairs + 7) / 8, sms * ctx->raygen_blocks), 256, 0, st, S, C, entries, f->active, &n->groups, &n->raygen_tickets, R);
+            chain(shadow_raygen_kernel, std::min((z.pairs + 7) / 8, sms * ctx->raygen_blocks), 256, 0, st, S, C, entries, v.active, &n->groups, &n->raygen_tickets, R);
             LUZ_LAUNCHED(ctx, "shadow_raygen_kernel");
         }
         prof_end(ctx);
@@ -455,25 +470,18 @@ luz_status launch_visibility(luz_ctx* ctx, luz_frame* f, const luz_tlas* t, int 
     return LUZ_OK;
 }
 
-luz_status launch_visibility_batch(luz_ctx* ctx, const SceneVis* d_scenes, uint32_t n,
-                                   unsigned long long* d_offsets, unsigned long long* work_counter,
-                                   unsigned long long* d_stats) {
+luz_status launch_visibility_count(luz_ctx* ctx, const SceneVis* d_scenes, uint32_t n, unsigned long long* d_offsets,
+                                   unsigned long long* work_counter, unsigned long long* d_stats) {
     cudaStream_t st = ctx->stream;
     batch_offsets_kernel<<<1, 32, 0, st>>>(d_scenes, n, d_offsets);
     LUZ_LAUNCHED(ctx, "batch_offsets_kernel");
     LUZ_CUDA(ctx, cudaMemsetAsync(work_counter, 0, 8, st));
+    LUZ_CUDA(ctx, cudaMemsetAsync(d_stats, 0, 5 * sizeof(unsigned long long), st));
     const VisTuning& tu = batch_tuning(ctx);
     VisCommon C = make_vis_common(ctx, tu, work_counter);
-    size_t smem = kStackBytes + kColdBytes;
-    uint32_t grid = (uint32_t)ctx->sm_count * tu.ctas_per_sm;
-    if (d_stats) {
-        LUZ_CUDA(ctx, cudaMemsetAsync(d_stats, 0, 5 * sizeof(unsigned long long), st));
-        visibility_batch_kernel<true><<<grid, 256, smem, st>>>(d_scenes, n, d_offsets, C, d_stats);
-        LUZ_LAUNCHED(ctx, "visibility_batch_kernel<stats>");
-    } else {
-        visibility_batch_kernel<false><<<grid, 256, smem, st>>>(d_scenes, n, d_offsets, C, nullptr);
-        LUZ_LAUNCHED(ctx, "visibility_batch_kernel");
-    }
+    visibility_count_kernel<<<(uint32_t)ctx->sm_count * tu.ctas_per_sm, 256, kStackBytes + kColdBytes, st>>>(
+        d_scenes, n, d_offsets, C, d_stats);
+    LUZ_LAUNCHED(ctx, "visibility_count_kernel");
     return LUZ_OK;
 }
 

@@ -44,8 +44,11 @@ SceneVis make_scene_vis(const luz_frame* f, const luz_tlas* t, int frame_index);
 // Boxes of the last TLAS build's leaves (leaf order, lo / hi float4 pairs).
 const float4* tlas_leaf_boxes(const luz_tlas* t);
 luz_status clear_visibility(luz_ctx* ctx, luz_frame* f);
-luz_status launch_visibility_batch(luz_ctx* ctx, const SceneVis* d_scenes, uint32_t n,
-                                   unsigned long long* d_offsets, unsigned long long* work_counter,
-                                   unsigned long long* d_stats);
+// Allocates what the traces of frame f over t need from the scratch.
+luz_status reserve_visibility(luz_ctx* ctx, const luz_frame* f, const luz_tlas* t, VisScratch& scratch);
+luz_status launch_visibility(luz_ctx* ctx, luz_frame* f, const luz_tlas* t, int frame_index, unsigned long long* d_stats,
+                             VisScratch& scratch);
+luz_status launch_visibility_count(luz_ctx* ctx, const SceneVis* d_scenes, uint32_t n, unsigned long long* d_offsets,
+                                   unsigned long long* work_counter, unsigned long long* d_stats);
 
 }  // namespace luz
