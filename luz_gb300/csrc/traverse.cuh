@@ -77,11 +77,16 @@ __device__ __forceinline__ bool wt_test(const WtRay& r, V3 v0, V3 v1, V3 v2, flo
     return true;
 }
 
+// For the conservative box tests only: the fast reciprocal's 2 ulp are far inside their
+// margin of 2^-16 (exact divisions made ray generation 2 to 4 % slower); it holds below
+// 2^126.
 __device__ __forceinline__ V3 safe_inv(V3 d) {
     const float tiny = 1e-20f;
     float x = fabsf(d.x) > tiny ? d.x : copysignf(tiny, d.x);
     float y = fabsf(d.y) > tiny ? d.y : copysignf(tiny, d.y);
     float z = fabsf(d.z) > tiny ? d.z : copysignf(tiny, d.z);
+    if (fmaxf(fmaxf(fabsf(x), fabsf(y)), fabsf(z)) < 0x1p125f)
+        return V3{__fdividef(1.0f, x), __fdividef(1.0f, y), __fdividef(1.0f, z)};
     return V3{1.0f / x, 1.0f / y, 1.0f / z};
 }
 

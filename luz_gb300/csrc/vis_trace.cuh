@@ -243,6 +243,14 @@ __device__ __forceinline__ float4 node_load(const float4* p) {
     return __ldg(p);
 }
 
+// Lanes of a warp stand at three kinds of step, of which entering an instance and testing a
+// triangle cost several node steps each and concern few lanes at a time. They wait until
+// kWaitEntries or kWaitTris lanes are at one, or fewer than kWaitNodes are at a node (so
+// every wait ends). Traversal of a 1080p two-level frame 1.03 -> 0.975 ms, of 1021x573 over
+// 8000 instances 2.73 -> 2.49, of 720p over 201 cubes 0.347 -> 0.297, against every kind in
+// every step (4 / 4 / 8: 0.98, 2.53, 0.316; 16 / 16 / 6: 0.99, 2.56, 0.29).
+constexpr uint32_t kWaitEntries = 12, kWaitTris = 12, kWaitNodes = 6;
+
 // Up to `steps` traversal steps of one lane's ray; clears `active` when it ends.
 // tlas / insts: the scene's TLAS nodes and instances (kernel parameters in the
 // single-scene kernel, the lane's own scene in the batched one). The step cap of a
@@ -258,9 +266,16 @@ __device__ __forceinline__ void run_steps(LaneRay& r, const Cold& c, bool& activ
         err |= LUZ_DEV_TRAVERSAL_CAP;
         finish_ray(c, active, false);
     }
-    for (uint32_t s = 0; s < steps && active; ++s) {
-        bool finished = false, hit = false;
-        if (r.node >= 0) {
+    const uint32_t full = 0xFFFFFFFFu;
+    for (uint32_t s = 0; s < steps; ++s) {
+        const bool at_node = active && r.node >= 0, at_leaf = active && r.node < 0;
+        const uint32_t nodes = __popc(__ballot_sync(full, at_node));
+        const uint32_t entries = __popc(__ballot_sync(full, at_leaf && !r.in_blas));
+        const uint32_t tris = __popc(__ballot_sync(full, at_leaf && r.in_blas));
+        const bool do_entries = entries >= kWaitEntries || nodes < kWaitNodes;
+        const bool do_tris = tris >= kWaitTris || nodes < kWaitNodes;
+        bool finished = false, hit = false, pop = false;
+        if (at_node) {
             // 4-wide node: test the four child boxes, continue with the nearest hit
             // child and push the other hits. Empty slots hold inverted boxes, which
             // no ray overlaps.
@@ -307,9 +322,10 @@ __device__ __forceinline__ void run_steps(LaneRay& r, const Cold& c, bool& activ
                     }
                 }
                 r.node = bc;
-                if (!finished) continue;
+            } else {
+                pop = true;
             }
-        } else if (!r.in_blas) {
+        } else if (at_leaf && !r.in_blas && do_entries) {
             // Instance leaf: entered unless its mask or BLAS is empty or the ray
             // segment provably misses the BLAS's bounding sphere.
             if (kStats) cnt.instances++;
@@ -350,9 +366,10 @@ __device__ __forceinline__ void run_steps(LaneRay& r, const Cold& c, bool& activ
                 ++r.sp;
                 r.in_blas = true;
                 r.node = first;
-                if (!finished) continue;
+            } else {
+                pop = true;
             }
-        } else {
+        } else if (at_leaf && r.in_blas && do_tris) {
             if (kStats) cnt.tris++;
             const float4* bt = reinterpret_cast<const float4*>((unsigned long long)__float_as_uint(c[kBtLo]) |
                                                                ((unsigned long long)__float_as_uint(c[kBtHi]) << 32));
@@ -364,10 +381,12 @@ __device__ __forceinline__ void run_steps(LaneRay& r, const Cold& c, bool& activ
                 t >= r.tmin && t <= r.tmax) {
                 finished = true;
                 hit = true;
+            } else {
+                pop = true;
             }
         }
         // pop (at most one TLAS marker lies between two nodes)
-        while (!finished) {
+        while (pop && !finished) {
             if (r.sp == 0) { finished = true; break; }
             --r.sp;
             int v = r.sp < kSmemStack ? (int)s_stack[r.sp * 32] : lstack[r.sp - kSmemStack];

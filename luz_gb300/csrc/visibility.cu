@@ -10,9 +10,9 @@
 // are idle, one lane takes that many records with a single atomic and the idle lanes pick
 // theirs by rank. 1080p two-level frame (64 x 81,920 triangles, 1024 instances, 41 lights,
 // 16 AO rays; 18.4 M rays to trace): ray generation and lists 0.59 -> 0.83 ms, traversal
-// 2.27 -> 1.03 ms (BLAS node visits 121 M -> 40 M, TLAS 7.8 M -> 1.6 M) against tracing
+// 2.27 -> 0.97 ms (BLAS node visits 121 M -> 40 M, TLAS 7.8 M -> 1.6 M) against tracing
 // every ray from the leaves its 32 neighbours' capsule reaches; 4K, 4096 instances, 145
-// lights, 64 AO rays: 18.5 + 94.2 ms -> 27 + 50 ms.
+// lights, 64 AO rays: 18.5 + 94.2 ms -> 27 + 44 ms.
 //
 // Traversal runs over 4-wide nodes (the even-depth collapse of the binary LBVH):
 // one step tests four child boxes, with the near and far planes picked per ray by
@@ -240,12 +240,12 @@ __global__ void batch_offsets_kernel(const SceneVis* scenes, uint32_t n, unsigne
 }
 
 // ---------------------------------------------------------------- host side
-// Default launch shapes. Batches generate their rays in the traversal: 24 idle lanes to a
-// refill, 8 steps between checks. A single scene's records hold only rays that enter a BLAS,
-// which are short: a check every 2 steps and a refill at 20 idle lanes (1080p two-level frame,
-// refill {4..28} x steps {2,4,8,16}: 0.98 ms against 1.03 at 24 / 8, 4K scene 49.9 against
-// 52.3). Staging the TLAS top in shared memory does not pay: L1 holds it.
-static const VisTuning g_tuning{0, 20, 2, 4, 1}, g_batch_tuning{0, 24, 8, 4, 1};
+// Default launch shapes. Batches' frame kernels generate their rays in the traversal: 24 idle
+// lanes to a refill, 8 steps between checks. A single scene's records hold only rays that
+// enter a BLAS, which are short: a check every 4 steps and a refill at 16 idle lanes (refill
+// {4..28} x steps {2,4,8,16}: 1080p two-level frame 0.966 ms against 1.009 at 24 / 8, 4K
+// scene 43.8 against 46.0). Staging the TLAS top in shared memory does not pay: L1 holds it.
+static const VisTuning g_tuning{0, 16, 4, 4, 1}, g_batch_tuning{0, 24, 8, 4, 1};
 
 const VisTuning& vis_tuning(const luz_ctx* ctx) { return ctx->vis_tuning.set ? ctx->vis_tuning : g_tuning; }
 const VisTuning& batch_tuning(const luz_ctx* ctx) { return ctx->vis_tuning.set ? ctx->vis_tuning : g_batch_tuning; }
