@@ -32,7 +32,7 @@ constexpr uint32_t kFrameTile = 16;                   // G-buffer item: 16x16 pi
 constexpr uint32_t kClearWords = 16384;               // clear item: 64 KB of a hit/miss plane
 constexpr uint32_t kFrameWaitIters = 1u << 22;        // polls (128 ns apart) before a wait gives up
 constexpr size_t kFrameSmem = kStackBytes + kColdBytes;   // traversal stacks + cold ray state
-constexpr uint32_t kFrameMaxLights = (uint32_t)(kFrameSmem / sizeof(luz_light));
+constexpr uint32_t kFrameMaxLights = (uint32_t)(kFrameSmem / sizeof(LightRec));
 static_assert(kVisThreads == kFrameTile * kFrameTile, "a G-buffer item is one pixel per thread");
 static_assert(kFrameSmem >= kFusedTlasMax * sizeof(unsigned long long), "TLAS sort keys fit the shared memory");
 
@@ -206,8 +206,8 @@ __device__ __noinline__ void frame_tlas_item(const FrameScene& F, unsigned long 
 
 // Light-pass item: lit pixels [c * 256, c * 256 + 256) of scene F, lights staged in
 // shared memory.
-__device__ __noinline__ void frame_light_item(const FrameScene& F, uint32_t c, luz_light* s_lights) {
-    for (uint32_t i = threadIdx.x; i < F.lp.light_count; i += kVisThreads) s_lights[i] = F.lp.lights[i];
+__device__ __noinline__ void frame_light_item(const FrameScene& F, uint32_t c, LightRec* s_lights) {
+    for (uint32_t i = threadIdx.x; i < F.lp.light_count; i += kVisThreads) s_lights[i] = light_rec(F.lp.lights[i], F.lp.light_slot[i]);
     __syncthreads();
     const uint32_t t = c * kVisThreads + threadIdx.x;
     if (t < ld_acquire_u32(F.lit_count)) light_pass_pixel<kPlain, true>(F.lp, s_lights, t);
@@ -334,7 +334,7 @@ __global__ void __launch_bounds__(kVisThreads, LUZ_VIS_MIN_BLOCKS) batch_frame_k
 
     // ---- 3. light passes
     __syncthreads();
-    luz_light* s_lights = reinterpret_cast<luz_light*>(smem);
+    LightRec* s_lights = reinterpret_cast<LightRec*>(smem);
     bool resolved = false;
     for (;;) {
         if (tid == 0) {

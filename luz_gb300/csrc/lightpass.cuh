@@ -37,18 +37,39 @@ struct LightParams {
     const float* srgb_lut;       // pow(i / 255, 2.2), i = 0..255: the albedo decode of light.frag:172
 };
 
-// The Cook-Torrance terms of light.frag:17-45 (DistributionGGX, GeometrySchlickGGX,
-// GeometrySmith) are evaluated inline in light_pass_kernel, their quotients folded into
-// one division per light: D * G / (4 NdotV NdotL + 1e-4) =
-// a2 NdotV NdotL / (pi dd^2 gv gl (4 NdotV NdotL + 1e-4)).
 constexpr float kInvPi = 1.0f / kPi;
 
-// light.frag:47-49; pow(x, 5.0) evaluated as x^4 * x.
-__device__ __forceinline__ V3 fresnel_schlick(float cos_theta, V3 F0) {
-    float x = clamp01(1.0f - cos_theta);
-    float x2 = x * x;
-    float p5 = (x2 * x2) * x;
-    return F0 + (V3{1.0f, 1.0f, 1.0f} - F0) * p5;
+// A light as the loop over the lights reads it (64 B of shared memory, as luz_light):
+// what depends on the light alone is evaluated once per block.
+struct LightRec {
+    float pos[3];
+    int type;
+    float radiance[3];     // color * intensity
+    uint32_t first;        // first shadow slot
+    float axis[3];         // normalize(-direction)
+    float outer;
+    float cone;            // inner angle - outer angle
+    int samples;           // shadow samples (0: none)
+    uint32_t pad;
+    uint32_t plain;        // radiance finite and of ordinary size
+};
+static_assert(sizeof(LightRec) == sizeof(luz_light) && sizeof(LightRec) % 16 == 0, "vector loads");
+
+__device__ __forceinline__ LightRec light_rec(const luz_light& lt, uint32_t first) {
+    LightRec r;
+    const V3 c = V3{lt.color[0], lt.color[1], lt.color[2]} * lt.intensity;
+    const V3 axis = normalize(-V3{lt.direction[0], lt.direction[1], lt.direction[2]});
+    for (int k = 0; k < 3; ++k) r.pos[k] = lt.position[k];
+    r.type = lt.type;
+    r.radiance[0] = c.x; r.radiance[1] = c.y; r.radiance[2] = c.z;
+    r.first = first;
+    r.axis[0] = axis.x; r.axis[1] = axis.y; r.axis[2] = axis.z;
+    r.outer = lt.outer_angle;
+    r.cone = lt.inner_angle - lt.outer_angle;
+    r.samples = max(lt.num_shadow_samples, 0);
+    r.pad = 0u;
+    r.plain = fmaxf(fmaxf(fabsf(c.x), fabsf(c.y)), fabsf(c.z)) < 1e15f && finite3(c);
+    return r;
 }
 
 __device__ __forceinline__ float unorm8_to_float(uint32_t b) { return (float)b / 255.0f; }
@@ -70,12 +91,26 @@ __device__ __forceinline__ uint32_t bit_at(const uint32_t* __restrict__ planes, 
 // shadow ratio R and AO: ambient * AO + U * R + emission.
 enum : int { kPlain = 0, kDenoisedAo = 1, kSplit = 2, kCompose = 3 };
 
+// light.frag:47-49; pow(x, 5.0) evaluated as x^4 * x.
+__device__ __forceinline__ V3 fresnel_schlick(float cos_theta, V3 F0) {
+    float x = clamp01(1.0f - cos_theta);
+    float x2 = x * x;
+    float p5 = (x2 * x2) * x;
+    return F0 + (V3{1.0f, 1.0f, 1.0f} - F0) * p5;
+}
+
 // light.frag main (light.frag:171-235) for lit pixel t of the compacted list, in mode
-// kMode; lights: the frame's lights (a shared-memory copy or the device array).
+// kMode; lights: the frame's lights (in shared memory).
 // kCoherent: the G-buffer planes, the lit-pixel list and the hit/miss planes were
 // written earlier in the same launch (the batch frame kernel) and are read through L2.
+//
+// Bound by issue. What depends on a light alone is evaluated once per block, and a light
+// behind the surface or with every sample occluded, whose terms are zeros, is left out
+// where all of its factors are finite (a pixel's and a light's `plain` and a distance above
+// 1e-3). 1080p, 41 lights: 0.220 -> 0.128 ms; 1601x899, 24 lights of two samples:
+// 0.204 -> 0.157.
 template <int kMode, bool kCoherent = false>
-__device__ __forceinline__ void light_pass_pixel(const LightParams& P, const luz_light* lights, uint32_t t) {
+__device__ __forceinline__ void light_pass_pixel(const LightParams& P, const LightRec* lights, uint32_t t) {
     const V3 amb = V3{P.ambient[0], P.ambient[1], P.ambient[2]};
     // lit pixel t: fragPos is the G-buffer pass's DepthToWorld of this pixel
     // (light.frag:186), N its normal
@@ -107,48 +142,65 @@ __device__ __forceinline__ void light_pass_pixel(const LightParams& P, const luz
     const float NdotV = fmax_(dot(N, V), 0.0f);
     const float gv = NdotV * (1.0f - k) + k;                 // GeometrySchlickGGX(NdotV) denominator
     const V3 diffuse_albedo = albedo * ((1.0f - metallic) * kInvPi);
+    const bool plain = a2 >= 1e-5f && finite3(V) && dot(N, N) < 4.0f;
     // EvaluateShadow's origin (light.frag:138-139), used by the 2D shadow maps
     const V3 shadow_origin = p + N * fmax_(length(p - cam) * 0.01f, 0.05f);
+    const uint32_t* shadow_word = P.shadow_bits + (pix >> 5);
     for (uint32_t i = 0; i < (kMode == kCompose ? 0u : P.light_count); ++i) {
-        const luz_light& lt = lights[i];
-        const V3 L = light_vector(lt, p);                    // light.frag:194-198
-        const float attenuation = light_attenuation(lt, p, L);   // light.frag:199-208
-        // EvaluateShadow (light.frag:137-169): ray-traced factor = hits / samples.
-        float shadow = 1.0f;
+        const float4* rec = reinterpret_cast<const float4*>(lights + i);
+        const float4 ra = rec[0], rb = rec[1], rc = rec[2], rd = rec[3];
+        const int type = __float_as_int(ra.w);
+        const V3 axis = V3{rc.x, rc.y, rc.z};
+        // light.frag:194-208: light_vector and light_attenuation
+        V3 L = axis;
+        float attenuation = 1.0f, dist = 1.0f;
+        if (type != LUZ_LIGHT_DIRECTIONAL) {
+            const V3 to = V3{ra.x, ra.y, ra.z} - p;
+            dist = length(to);
+            L = to * (1.0f / dist);
+        }
+        const float NL = dot(N, L);
+        const bool zero = plain && __float_as_uint(rd.w) && dist > 1e-3f;   // all terms are finite
+        if (kMode != kSplit && zero && NL <= 0.0f) continue;
+        // EvaluateShadow (light.frag:137-169): ray-traced factor = hits / samples; lit = 1 - factor
+        float shadow = 1.0f, lit = 0.0f;
         if (P.shadow_type == LUZ_SHADOW_RAYTRACING) {
-            int ns = lt.num_shadow_samples;
-            if (ns <= 0) {
-                shadow = 0.0f;
-            } else {
-                uint32_t first = P.light_slot[i];
-                uint32_t hits = 0;
-                for (int s = 0; s < ns; ++s) hits += bit_at<kCoherent>(P.shadow_bits, first + s, P.words, pix);
-                shadow = (float)hits / (float)ns;
-                if constexpr (kMode == kSplit) {
-                    hits_all += hits;
-                    slots_all += (uint32_t)ns;
-                }
+            const int ns = __float_as_int(rd.y);
+            uint32_t hits = 0;
+            const uint32_t* word = shadow_word + (size_t)__float_as_uint(rb.w) * P.words;
+            for (int s = 0; s < ns; ++s, word += P.words)
+                hits += ((kCoherent ? __ldcg(word) : __ldg(word)) >> (pix & 31)) & 1u;
+            // 1 - hits / samples; the division only where some of the samples are occluded
+            lit = hits == 0 ? 1.0f : 0.0f;
+            if (hits != 0 && (int)hits != ns) lit = 1.0f - (float)hits / (float)ns;
+            if constexpr (kMode == kSplit) {
+                hits_all += hits;
+                slots_all += (uint32_t)ns;
             }
         } else if (P.shadow_type == LUZ_SHADOW_MAP && i < P.shadow_count && P.shadow_lights[i].faces) {
             shadow = shadow_map_factor(P.shadow_lights[i], p, shadow_origin);   // light.frag:147-164
+            lit = 1.0f - shadow;
         }
         if constexpr (kMode == kSplit) shadow_sum += shadow;
-        V3 color = V3{lt.color[0], lt.color[1], lt.color[2]};
-        V3 radiance = ((color * lt.intensity) * attenuation) * (1.0f - shadow);
-        V3 H = normalize(V + L);
+        if (zero && (kMode == kSplit ? NL <= 0.0f : lit == 0.0f)) continue;
+        if (type != LUZ_LIGHT_DIRECTIONAL) {
+            attenuation = 1.0f / (dist * dist);
+            if (type == LUZ_LIGHT_SPOT) attenuation *= clamp01((dot(L, axis) - rc.w) / rd.x);
+        }
+        const V3 unshadowed = V3{rb.x, rb.y, rb.z} * attenuation;
+        const V3 H = normalize(V + L);
         const float NdotH = fmax_(dot(N, H), 0.0f);
-        const float NdotL = fmax_(dot(N, L), 0.0f);
+        const float NdotL = fmax_(NL, 0.0f);
         const float dd = NdotH * NdotH * (a2 - 1.0f) + 1.0f;
         const float gl = NdotL * (1.0f - k) + k;
-        V3 F = fresnel_schlick(clamp01(dot(H, V)), F0);
+        const V3 F = fresnel_schlick(clamp01(dot(H, V)), F0);
         // D * G / (4 NdotV NdotL + 1e-4) with D = a2 / (pi dd^2) and
         // G = NdotV NdotL / (gv gl), as one quotient
         const float spec_scale = (a2 * (NdotV * NdotL)) /
                                  ((kPi * dd * dd) * (gv * gl) * ((4.0f * NdotV) * NdotL + 0.0001f));
-        V3 spec = F * spec_scale;
-        V3 diffuse = (V3{1.0f, 1.0f, 1.0f} - F) * diffuse_albedo;
-        Lo = Lo + (diffuse + spec) * radiance * NdotL;
-        if constexpr (kMode == kSplit) Lu = Lu + (diffuse + spec) * ((color * lt.intensity) * attenuation) * NdotL;
+        const V3 f = (V3{1.0f, 1.0f, 1.0f} - F) * diffuse_albedo + F * spec_scale;
+        Lo = Lo + f * (unshadowed * lit) * NdotL;
+        if constexpr (kMode == kSplit) Lu = Lu + f * unshadowed * NdotL;
     }
     float ao;
     if constexpr (kMode == kCompose) {
