@@ -21,7 +21,6 @@ namespace luz {
 namespace {
 
 constexpr uint32_t kMaxTris = LUZ_NOALLOC_MAX_TRIANGLES;
-constexpr uint32_t kMaxNodes = kMaxTris;                 // max(n-1, 1) <= n for n >= 1
 constexpr uint32_t kTiles = (kMaxTris + kSortTile - 1) / kSortTile;
 constexpr int kPasses = 4;                               // 30-bit Morton keys, one segment
 
@@ -38,11 +37,11 @@ constexpr size_t kOffHist = al(kOffVals1 + (size_t)4 * kMaxTris);
 constexpr size_t kOffOffsets = al(kOffHist + (size_t)kPasses * kRadix * 4);
 constexpr size_t kOffTileStatus = al(kOffOffsets + (size_t)kPasses * kRadix * 4);
 constexpr size_t kOffTileCounter = al(kOffTileStatus + (size_t)kPasses * kTiles * kRadix * 4);
-constexpr size_t kOffLeafBox = al(kOffTileCounter + (size_t)kPasses * 4);
-constexpr size_t kOffNodeParent = al(kOffLeafBox + (size_t)32 * kMaxTris);
-constexpr size_t kOffLeafParent = al(kOffNodeParent + (size_t)4 * kMaxNodes);
-constexpr size_t kOffFlags = al(kOffLeafParent + (size_t)4 * kMaxTris);
-constexpr size_t kScratchBytes = al(kOffFlags + (size_t)4 * kMaxNodes);
+constexpr size_t kOffEnds0 = al(kOffTileCounter + (size_t)kPasses * 4);
+constexpr size_t kOffEnds1 = al(kOffEnds0 + (size_t)8 * kMaxTris);
+constexpr size_t kOffFlags = al(kOffEnds1 + (size_t)8 * kMaxTris);
+// (24 bytes per triangle are room that keeps the array at its documented size)
+constexpr size_t kScratchBytes = al(kOffFlags + (size_t)28 * kMaxTris);
 static_assert(kScratchBytes == LUZ_NOALLOC_SCRATCH_BYTES, "scratch size in luz.h is out of date");
 
 // Header words at kOffHeader.
@@ -63,15 +62,23 @@ std::mutex g_mutex;
 void* g_scratch_ptr[kMaxDevices] = {};
 
 // Writes the segment descriptor and resets the header from kernel parameters, so no
-// host memory is copied.
-__global__ void noalloc_setup_kernel(Header* h, SegDesc seg) {
+// host memory is copied, and clears what the build counts in: the sort's words (from
+// `sort`) and the merges' flags.
+__global__ void __launch_bounds__(256) noalloc_setup_kernel(Header* h, SegDesc seg, uint32_t* hist, uint32_t hist_words,
+                                                            uint32_t* tiles, uint32_t tile_words, uint32_t* counters,
+                                                            uint32_t* flags, uint32_t n) {
     chain_wait();
-    if (threadIdx.x == 0) {
+    const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x, step = gridDim.x * blockDim.x;
+    if (t == 0) {
         h->status = 0;
         h->zero = 0;
         for (int k = 0; k < 6; ++k) h->bounds[k] = k < 3 ? 0xFFFFFFFFu : 0u;
         h->seg = seg;
     }
+    for (uint32_t i = t; i < hist_words; i += step) hist[i] = 0u;
+    for (uint32_t i = t; i < tile_words; i += step) tiles[i] = 0u;
+    for (uint32_t i = t; i < n; i += step) flags[i] = 0u;
+    if (t < (uint32_t)kPasses) counters[t] = 0u;
 }
 
 // Copies the caller's indices into scratch; an index outside the vertex buffer is
@@ -151,9 +158,8 @@ extern "C" luz_status luz_blas_build_noalloc(const luz_vertex* d_vertices, uint3
     uint32_t* offsets = (uint32_t*)(base + kOffOffsets);
     uint32_t* tile_status = (uint32_t*)(base + kOffTileStatus);
     uint32_t* tile_counter = (uint32_t*)(base + kOffTileCounter);
-    float4* leaf_box = (float4*)(base + kOffLeafBox);
-    uint32_t* node_parent = (uint32_t*)(base + kOffNodeParent);
-    uint32_t* leaf_parent = (uint32_t*)(base + kOffLeafParent);
+    uint2* ends0 = (uint2*)(base + kOffEnds0);
+    uint2* ends1 = (uint2*)(base + kOffEnds1);
     uint32_t* flags = (uint32_t*)(base + kOffFlags);
 
     SegDesc seg{};
@@ -166,46 +172,36 @@ extern "C" luz_status luz_blas_build_noalloc(const luz_vertex* d_vertices, uint3
     seg.tris = (float4*)d_tris;
     seg.morton = d_morton;
     seg.order = d_order;
-    const uint32_t m = n > 1 ? n - 1 : 1;
     const uint32_t tiles = n > 0 ? cdiv(n, kSortTile) : 1;
 
     // The array keeps the previous call's contents: reset everything read before written.
-    chain(noalloc_setup_kernel, 1, 32, 0, st, h, seg);
+    const uint32_t tile_words = kPasses * tiles * kRadix;
+    chain(noalloc_setup_kernel, std::min(cdiv(std::max(n, tile_words), 256), 304u), 256, 0, st, h, seg, hist,
+          (uint32_t)(kPasses * kRadix), tile_status, tile_words, tile_counter, flags, n);
     NOALLOC_LAUNCHED();
-    NOALLOC_CUDA(cudaMemsetAsync(node_parent, 0xFF, (size_t)m * 4, st));
-    NOALLOC_CUDA(cudaMemsetAsync(leaf_parent, 0xFF, (size_t)(n ? n : 1) * 4, st));
-    NOALLOC_CUDA(cudaMemsetAsync(flags, 0, (size_t)m * 4, st));
     if (n > 0) {
-        chain(noalloc_indices_kernel, cdiv(index_count, 256), 256, 0, st, d_indices, index_count, vertex_count,
-                                                                        idx, status);
+        chain(noalloc_indices_kernel, cdiv(index_count, 256), 256, 0, st, d_indices, index_count, vertex_count, idx, status);
         NOALLOC_LAUNCHED();
-        chain(blas_bounds_kernel, cdiv(n, 256 * kBoundsIters), 256, 0, st, d_seg, zero, 1, n, bounds);
+        const uint32_t rows = bounds_rows(n);
+        chain(blas_bounds_kernel, cdiv(n, 256 * rows), 256, 0, st, d_seg, zero, 1, n, rows, bounds);
         NOALLOC_LAUNCHED();
-        chain(blas_morton_kernel, cdiv(n, 256), 256, 0, st, d_seg, zero, 1, n, bounds, keys[0], vals[0]);
-        NOALLOC_LAUNCHED();
-        NOALLOC_CUDA(cudaMemsetAsync(hist, 0, (size_t)kPasses * kRadix * 4, st));
-        NOALLOC_CUDA(cudaMemsetAsync(tile_status, 0, (size_t)kPasses * tiles * kRadix * 4, st));
-        NOALLOC_CUDA(cudaMemsetAsync(tile_counter, 0, (size_t)kPasses * 4, st));
-        chain(sort_histogram_kernel, std::max(1u, std::min(cdiv(n, 4096), 256u)), 256, 0, st, keys[0], n, kPasses, hist);
-        NOALLOC_LAUNCHED();
-        chain(sort_scan_kernel, kPasses, 256, 0, st, hist, offsets);
+        chain(blas_morton_kernel, morton_blocks(n), 256, 0, st, d_seg, zero, 1, n, bounds, keys[0], vals[0], kPasses, hist);
         NOALLOC_LAUNCHED();
         for (int p = 0; p < kPasses; ++p) {
             int cur = p & 1;
-            chain(onesweep_pass_kernel, tiles, kSortThreads, 0, st, keys[cur], vals[cur], keys[cur ^ 1], vals[cur ^ 1], n, 8 * p, offsets + p * kRadix,
-                tile_status + (size_t)p * tiles * kRadix, tile_counter + p, status);
+            chain(onesweep_pass_kernel, tiles, kSortThreads, 0, st, keys[cur], vals[cur], keys[cur ^ 1], vals[cur ^ 1], n,
+                  8 * p, hist + p * kRadix, offsets + p * kRadix, tile_status + (size_t)p * tiles * kRadix, tile_counter + p,
+                  status);
             NOALLOC_LAUNCHED();
         }
-    }
-    // kPasses is even: the sorted keys are back in keys[0].
-    chain(karras_kernel, cdiv(m, 256), 256, 0, st, d_seg, zero, 1, m, keys[0], node_parent, leaf_parent, status);
-    NOALLOC_LAUNCHED();
-    if (n > 0) {
-        chain(blas_emit_kernel, cdiv(n, 256), 256, 0, st, d_seg, zero, 1, n, keys[0], vals[0], leaf_box);
-        NOALLOC_LAUNCHED();
-        chain(refit_kernel, cdiv(n, 256), 256, 0, st, d_seg, zero, 1, n, leaf_box, node_parent, leaf_parent, flags);
+        // kPasses is even: the sorted keys are back in keys[0].
+        const MergeArgs A{keys[0], nullptr, {ends0, ends1}, flags, status, n};
+        chain(blas_tree_kernel, merge_blocks(n), kMergeLeaves, 0, st, d_seg, zero, 1, vals[0], A);
         NOALLOC_LAUNCHED();
         chain(blas_radius_kernel, cdiv(n, 256), 256, 0, st, d_seg, zero, 1, n);
+        NOALLOC_LAUNCHED();
+    } else {
+        chain(empty_segments_kernel, 1, 32, 0, st, d_seg, 1, nullptr);
         NOALLOC_LAUNCHED();
     }
     // Synchronous, like the reference's per-mesh build (GPUScene.cpp:132-137): read

@@ -4,14 +4,13 @@
 // Pipeline (each step a kernel on the context stream):
 //   bounds   : centroid bounds per segment (order-preserving uint atomics, exact)
 //   morton   : 64-bit key = segment << 30 | morton30(centroid), value = primitive
-//   sort     : LSD radix sort, 8-bit digits, one upsweep histogram kernel for all
-//              passes + one "onesweep" kernel per pass (tile-local warp multi-split
+//   sort     : LSD radix sort, 8-bit digits, the histograms of all passes counted with
+//              the keys + one "onesweep" kernel per pass (tile-local warp multi-split
 //              ranking, decoupled look-back across tiles). Stable.
-//   karras   : T. Karras, "Maximizing Parallelism in the Construction of BVHs,
-//              Octrees, and k-d Trees", HPG 2012 — one thread per internal node,
+//   tree     : triangles / instances gathered into leaf order, padded leaf boxes, and the
+//              radix tree of T. Karras, "Maximizing Parallelism in the Construction of BVHs,
+//              Octrees, and k-d Trees", HPG 2012, built bottom-up with its boxes;
 //              duplicate codes split by index (delta = 32 + clz(i ^ j)).
-//   emit     : gather triangles / instances into leaf order, padded leaf boxes
-//   refit    : bottom-up, second arrival at a node (atomic flag) merges its children
 //   bfs      : (TLAS) breadth-first relayout so that the top of the tree is a prefix
 //              of the node array, staged into shared memory by the traversal.
 // Replaces the driver builds behind vkw::CmdBuildBLAS / vkw::CmdBuildTLAS
@@ -53,15 +52,20 @@ __device__ __forceinline__ float leaf_pad(float lo, float hi) {
 
 // ---------------------------------------------------------------- bounds + morton
 // seg_bounds: 6 ordered uints per segment (min xyz, max xyz); init min=~0, max=0.
-// A block walks kBoundsIters rows of 256 consecutive primitives. Per row, a warp whose
+// A block walks `rows` rows of 256 consecutive primitives. Per row, a warp whose
 // lanes all belong to one segment reduces its ordered centroid keys (redux.sync) and
 // lane 0 merges them into a running min/max of that segment, which goes to the global
-// words (six atomics) only when the segment changes or the block's range ends; a warp
-// that straddles a segment boundary issues per-lane atomics. Min and max do not
-// depend on the order, so the result is the one of any reduction order.
+// words (six atomics) only when the segment changes; a warp that straddles a segment
+// boundary issues per-lane atomics. At the end of the block's range the warps' running
+// values are merged first where they are of one segment. Min and max do not
+// depend on the order, so the result is the one of any reduction order. Bound by latency:
+// few rows where that still gives blocks for the chip (81,920 triangles: 13.7 us with 16
+// rows and six atomics per warp, 3.1 with one).
 __global__ void __launch_bounds__(256) blas_bounds_kernel(const SegDesc* segs, const uint32_t* seg_prim_off,
-                                                          int nseg, uint32_t total, uint32_t* seg_bounds) {
+                                                          int nseg, uint32_t total, uint32_t rows, uint32_t* seg_bounds) {
     chain_wait();
+    __shared__ int s_seg[8];
+    __shared__ uint32_t s_acc[8][6];
     const uint32_t full = 0xFFFFFFFFu;
     const bool leader = (threadIdx.x & 31) == 0;
     int acc_s = -1;
@@ -72,9 +76,9 @@ __global__ void __launch_bounds__(256) blas_bounds_kernel(const SegDesc* segs, c
         for (int a = 0; a < 3; ++a) if (acc[a] != 0xFFFFFFFFu) atomicMin(b + a, acc[a]);
         for (int a = 3; a < 6; ++a) if (acc[a] != 0u) atomicMax(b + a, acc[a]);
     };
-    const uint32_t base = blockIdx.x * (blockDim.x * kBoundsIters);
-    for (int it = 0; it < kBoundsIters; ++it) {
-        const uint32_t row = base + (uint32_t)it * blockDim.x;
+    const uint32_t base = blockIdx.x * (blockDim.x * rows);
+    for (uint32_t it = 0; it < rows; ++it) {
+        const uint32_t row = base + it * blockDim.x;
         if (row >= total) break;   // uniform across the block
         const uint32_t g = row + threadIdx.x;
         const bool in = g < total;
@@ -113,47 +117,72 @@ __global__ void __launch_bounds__(256) blas_bounds_kernel(const SegDesc* segs, c
             for (int a = 3; a < 6; ++a) atomicMax(b + a, k[a]);
         }
     }
-    if (leader) flush();
+    if (leader) {
+        const uint32_t w = threadIdx.x >> 5;
+        s_seg[w] = acc_s;
+        for (int a = 0; a < 6; ++a) s_acc[w][a] = acc[a];
+    }
+    __syncthreads();
+    bool same = true;   // of the warps that have a running value
+    for (int w = 0; w < 8; ++w) same = same && (s_seg[w] == s_seg[0] || s_seg[w] < 0);
+    if (!same) {
+        if (leader) flush();
+    } else if (threadIdx.x < 6 && s_seg[0] >= 0) {
+        uint32_t v = s_acc[0][threadIdx.x];
+        for (int w = 1; w < 8; ++w) v = threadIdx.x < 3 ? min(v, s_acc[w][threadIdx.x]) : max(v, s_acc[w][threadIdx.x]);
+        uint32_t* b = seg_bounds + 6 * s_seg[0] + threadIdx.x;
+        if (threadIdx.x < 3) { if (v != 0xFFFFFFFFu) atomicMin(b, v); }
+        else if (v != 0u) atomicMax(b, v);
+    }
 }
 
+// The sort's digit histograms: a block counts its keys in shared memory and adds what it
+// found. Used by the kernels that make the keys, so that they are not read again.
+struct BlockHist {
+    uint32_t (*h)[kRadix];
+    int passes;
+    __device__ __forceinline__ void clear() const {
+        for (int i = threadIdx.x; i < passes * kRadix; i += blockDim.x) (&h[0][0])[i] = 0u;
+        __syncthreads();
+    }
+    __device__ __forceinline__ void count(unsigned long long key) const {
+        for (int p = 0; p < passes; ++p) atomicAdd(&h[p][(key >> (8 * p)) & 0xFF], 1u);
+    }
+    __device__ __forceinline__ void add(uint32_t* hist) const {
+        __syncthreads();
+        for (int i = threadIdx.x; i < passes * kRadix; i += blockDim.x) {
+            const uint32_t v = (&h[0][0])[i];
+            if (v) atomicAdd(hist + i, v);
+        }
+    }
+};
 
-__global__ void blas_morton_kernel(const SegDesc* segs, const uint32_t* seg_prim_off, int nseg,
-                                   uint32_t total, const uint32_t* seg_bounds,
-                                   unsigned long long* keys, uint32_t* vals) {
+__global__ void __launch_bounds__(256) blas_morton_kernel(const SegDesc* segs, const uint32_t* seg_prim_off, int nseg,
+                                                          uint32_t total, const uint32_t* seg_bounds,
+                                                          unsigned long long* keys, uint32_t* vals, int passes,
+                                                          uint32_t* hist) {
     chain_wait();
-    uint32_t g = blockIdx.x * blockDim.x + threadIdx.x;
-    if (g >= total) return;
-    int s = find_seg(seg_prim_off, nseg, g);
-    const SegDesc sd = segs[s];
-    uint32_t p = g - sd.prim_off;
-    uint32_t i0 = sd.indices[3 * p], i1 = sd.indices[3 * p + 1], i2 = sd.indices[3 * p + 2];
-    V3 lo, hi;
-    tri_box(load_pos(sd.vertices, i0), load_pos(sd.vertices, i1), load_pos(sd.vertices, i2), lo, hi);
-    V3 cmin, ext;
-    decode_bounds(seg_bounds + 6 * s, cmin, ext);
-    uint32_t m = morton30(lo, hi, cmin, ext);
-    keys[g] = ((unsigned long long)s << 30) | m;
-    vals[g] = g;
+    __shared__ uint32_t s_hist[kMaxPasses][kRadix];
+    const BlockHist H{s_hist, passes};
+    H.clear();
+    for (uint32_t g = blockIdx.x * blockDim.x + threadIdx.x; g < total; g += gridDim.x * blockDim.x) {
+        int s = find_seg(seg_prim_off, nseg, g);
+        const SegDesc sd = segs[s];
+        uint32_t p = g - sd.prim_off;
+        uint32_t i0 = sd.indices[3 * p], i1 = sd.indices[3 * p + 1], i2 = sd.indices[3 * p + 2];
+        V3 lo, hi;
+        tri_box(load_pos(sd.vertices, i0), load_pos(sd.vertices, i1), load_pos(sd.vertices, i2), lo, hi);
+        V3 cmin, ext;
+        decode_bounds(seg_bounds + 6 * s, cmin, ext);
+        const unsigned long long key = ((unsigned long long)s << 30) | morton30(lo, hi, cmin, ext);
+        keys[g] = key;
+        vals[g] = g;
+        H.count(key);
+    }
+    H.add(hist);
 }
 
 // ---------------------------------------------------------------- onesweep radix sort
-__global__ void sort_histogram_kernel(const unsigned long long* keys, uint32_t n, int passes,
-                                      uint32_t* hist) {
-    chain_wait();
-    __shared__ uint32_t s_hist[kMaxPasses][kRadix];
-    for (int i = threadIdx.x; i < kMaxPasses * kRadix; i += blockDim.x) (&s_hist[0][0])[i] = 0;
-    __syncthreads();
-    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        unsigned long long k = keys[i];
-        for (int p = 0; p < passes; ++p) atomicAdd(&s_hist[p][(k >> (8 * p)) & 0xFF], 1u);
-    }
-    __syncthreads();
-    for (int i = threadIdx.x; i < passes * kRadix; i += blockDim.x) {
-        uint32_t v = (&s_hist[0][0])[i];
-        if (v) atomicAdd(hist + i, v);
-    }
-}
-
 // Block-wide exclusive scan of one value per thread (blockDim.x == 256).
 __device__ __forceinline__ uint32_t block_excl_scan_256(uint32_t v, uint32_t* s_tmp /*8*/,
                                                         uint32_t* total) {
@@ -176,14 +205,6 @@ __device__ __forceinline__ uint32_t block_excl_scan_256(uint32_t v, uint32_t* s_
     return wsum + x - v;
 }
 
-__global__ void sort_scan_kernel(const uint32_t* hist, uint32_t* offsets) {
-    chain_wait();
-    __shared__ uint32_t s_tmp[8];
-    int p = blockIdx.x;
-    uint32_t v = hist[p * kRadix + threadIdx.x];
-    offsets[p * kRadix + threadIdx.x] = block_excl_scan_256(v, s_tmp, nullptr);
-}
-
 __device__ __forceinline__ uint32_t ld_volatile_u32(const uint32_t* p) {
     uint32_t v;
     asm volatile("ld.volatile.global.u32 %0, [%1];" : "=r"(v) : "l"(p));
@@ -196,8 +217,8 @@ __device__ __forceinline__ void st_volatile_u32(uint32_t* p, uint32_t v) {
 __global__ void __launch_bounds__(kSortThreads)
 onesweep_pass_kernel(const unsigned long long* __restrict__ kin, const uint32_t* __restrict__ vin,
                      unsigned long long* __restrict__ kout, uint32_t* __restrict__ vout, uint32_t n,
-                     int shift, const uint32_t* __restrict__ pass_offsets, uint32_t* tile_status,
-                     uint32_t* tile_counter, uint32_t* dev_status) {
+                     int shift, const uint32_t* __restrict__ pass_hist, uint32_t* __restrict__ pass_offsets,
+                     uint32_t* tile_status, uint32_t* tile_counter, uint32_t* dev_status) {
     chain_wait();
     __shared__ uint32_t s_tile;
     __shared__ uint32_t s_warp_hist[kSortWarps][kRadix];
@@ -208,10 +229,13 @@ onesweep_pass_kernel(const unsigned long long* __restrict__ kin, const uint32_t*
     __shared__ uint32_t s_vals[kSortTile];
 
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    if (tid == 0) s_tile = atomicAdd(tile_counter, 1u);
+    // Tiles in the order the blocks start, so that a look-back waits only on blocks that run;
+    // a grid that fits the chip at a block per SM needs no order.
+    const bool ordered = gridDim.x > kSortResident;
+    if (ordered && tid == 0) s_tile = atomicAdd(tile_counter, 1u);
     for (int i = tid; i < kSortWarps * kRadix; i += kSortThreads) (&s_warp_hist[0][0])[i] = 0;
     __syncthreads();
-    const uint32_t tile = s_tile;
+    const uint32_t tile = ordered ? s_tile : blockIdx.x;
     const uint32_t base = tile * kSortTile;
 
     unsigned long long key[kSortItems];
@@ -249,26 +273,37 @@ onesweep_pass_kernel(const unsigned long long* __restrict__ kin, const uint32_t*
     uint32_t* my_status = tile_status + (size_t)tile * kRadix + tid;
     uint32_t global_base;
     if (tile == 0) {
-        global_base = pass_offsets[tid];
+        // the pass's digit offsets: the exclusive scan of its histogram
+        global_base = block_excl_scan_256(pass_hist[tid], s_tmp, nullptr);
+        pass_offsets[tid] = global_base;
         st_volatile_u32(my_status, kFlagPrefix | (global_base + tile_count));
     } else {
         st_volatile_u32(my_status, kFlagAggregate | tile_count);
         uint32_t excl = 0;
         int j = (int)tile - 1;
         uint32_t spins = 0;
-        while (j >= 0) {
-            uint32_t s = ld_volatile_u32(tile_status + (size_t)j * kRadix + tid);
-            uint32_t flag = s & ~kValueMask;
-            if (flag == 0) {
-                if (++spins > kLookbackSpinLimit) {
-                    atomicOr(dev_status, (uint32_t)LUZ_DEV_SORT_LOOKBACK_TIMEOUT);
-                    break;
-                }
-                continue;
+        bool done = false;
+        while (!done) {
+            // kLookback words of earlier tiles in flight at a time (tile 0 ends every look-back)
+            uint32_t w[kLookback];
+#pragma unroll
+            for (int k = 0; k < kLookback; ++k)
+                w[k] = j - k >= 0 ? ld_volatile_u32(tile_status + (size_t)(j - k) * kRadix + tid) : 0u;
+            int used = 0;
+#pragma unroll
+            for (int k = 0; k < kLookback; ++k) {
+                if (done || used != k) continue;
+                const uint32_t flag = w[k] & ~kValueMask;
+                if (flag == 0) continue;
+                excl += w[k] & kValueMask;
+                done = flag == kFlagPrefix;
+                ++used;
             }
-            excl += s & kValueMask;
-            if (flag == kFlagPrefix) break;
-            --j;
+            j -= used;
+            if (!done && used == 0 && ++spins > kLookbackSpinLimit) {
+                atomicOr(dev_status, (uint32_t)LUZ_DEV_SORT_LOOKBACK_TIMEOUT);
+                done = true;
+            }
         }
         global_base = excl;
         st_volatile_u32(my_status, kFlagPrefix | (excl + tile_count));
@@ -298,150 +333,263 @@ onesweep_pass_kernel(const unsigned long long* __restrict__ kin, const uint32_t*
     }
 }
 
-// ---------------------------------------------------------------- Karras hierarchy
+// ---------------------------------------------------------------- hierarchy + refit
+// The radix tree bottom-up, boxes and all, in one kernel (the scheme of C. Apetrei, "Fast and
+// Simple Agglomerative LBVH Construction", CGVC 2014): a thread per leaf climbs; a range
+// [l, r] of leaves merges with the neighbour it shares the longer prefix with, and the
+// second of the two to arrive goes on with the union. The tree is the one of T. Karras
+// (HPG 2012), and so is its numbering: a node that is a left child has the index of its
+// last leaf, a right child that of its first, the root 0.
+//
+// A block takes a span of consecutive leaves. Merges whose union lies inside them happen
+// in shared memory; whether one does follows from the prefix lengths between the block's
+// leaves alone: the union of a merge at prefix length d ends inside the block on either side
+// where that side has a shorter prefix. Other merges, and all above them, meet in device
+// memory: each side stores its node, then its far end with the prefix there, then counts
+// itself with an acquire-release atomic, and the second reads the sibling's box from its node. Bound by the
+// latency of those climbs. 81,920 triangles: 32 us against 51 (a search per node for its range and
+// split, leaves, and a refit through device memory: 11.9 + 4.4 + 34.6 us).
+// The leaves of a block: from the place with the shortest prefix in a window of kMergeStep
+// leaves around kMergeStep * block to that of the next block, 511 at most. The merges that
+// cross a block's ends are the ancestors of the nodes split there: a split high up in the
+// tree has few, one at a fixed distance as many as any node (81,920 triangles: 54 us with
+// blocks of 512 leaves).
+struct MergeSpan {
+    uint32_t first, count;
+};
 
+struct MergeShared {
+    float box[kMergeLeaves][2][6];    // per merge position: the two sides' boxes
+    uint32_t end[kMergeLeaves][2];
+    uint32_t flag[kMergeLeaves];
+    int8_t delta[kMergeLeaves + 1];   // prefix length between leaf b0 - 1 + k and the next (-1: none)
+    int8_t before[kMergeLeaves], after[kMergeLeaves];   // least delta of the pairs before / after a position's
+    int8_t warp_min[kMergeLeaves / 32];
+    uint32_t cut[kMergeLeaves / 32];
+};
 
-
-__global__ void karras_kernel(const SegDesc* segs, const uint32_t* seg_node_off, int nseg,
-                              uint32_t total_nodes, const unsigned long long* keys,
-                              uint32_t* node_parent, uint32_t* leaf_parent, uint32_t* dev_status) {
-    chain_wait();
-    uint32_t q = blockIdx.x * blockDim.x + threadIdx.x;
-    if (q >= total_nodes) return;
-    int s = find_seg(seg_node_off, nseg, q);
-    const SegDesc sd = segs[s];
-    karras_node(sd, (int)(q - sd.node_off), keys, node_parent, leaf_parent, dev_status);
+// Called by whole blocks of kMergeLeaves = 2 kMergeStep threads: half of them look at either end.
+__device__ __forceinline__ MergeSpan merge_span(MergeShared& S, const unsigned long long* keys, uint32_t total) {
+    const uint32_t tid = threadIdx.x, t = blockIdx.x + tid / kMergeStep, i = tid % kMergeStep;
+    const uint32_t at = t * kMergeStep + i - kMergeStep / 2;   // (t = 0 is the first leaf)
+    uint32_t key = 0xFFFFFFFFu;
+    if (t > 0 && at < total) {
+        const unsigned long long a = keys[at - 1], b = keys[at];
+        key = ((a == b ? 64u + __clz((at - 1) ^ at) : (uint32_t)__clzll((long long)(a ^ b))) << 16) | i;
+    }
+    key = __reduce_min_sync(0xFFFFFFFFu, key);
+    if ((tid & 31) == 0) S.cut[tid >> 5] = key;
+    __syncthreads();
+    uint32_t end[2];
+#pragma unroll
+    for (uint32_t h = 0; h < 2; ++h) {
+        uint32_t k = 0xFFFFFFFFu;
+#pragma unroll
+        for (uint32_t w = 0; w < kMergeStep / 32; ++w) k = min(k, S.cut[h * (kMergeStep / 32) + w]);
+        const uint32_t b = blockIdx.x + h;
+        end[h] = b == 0 ? 0u : (k == 0xFFFFFFFFu ? total : b * kMergeStep + (k & 0xFFFFu) - kMergeStep / 2);
+    }
+    return MergeSpan{end[0], end[1] - end[0]};
 }
 
-// ---------------------------------------------------------------- leaves + refit
-// BLAS: gather triangles into leaf order; padded leaf boxes; sorted morton/order into
-// the segment's own arrays.
-__global__ void blas_emit_kernel(const SegDesc* segs, const uint32_t* seg_prim_off, int nseg,
-                                 uint32_t total, const unsigned long long* keys,
-                                 const uint32_t* vals, float4* leaf_box) {
-    chain_wait();
-    uint32_t g = blockIdx.x * blockDim.x + threadIdx.x;
-    if (g >= total) return;
-    int s = find_seg(seg_prim_off, nseg, g);
-    const SegDesc sd = segs[s];
-    uint32_t j = g - sd.prim_off;
-    uint32_t prim = vals[g] - sd.prim_off;
-    sd.morton[j] = (uint32_t)keys[g] & 0x3FFFFFFFu;
-    sd.order[j] = prim;
-    uint32_t i0 = sd.indices[3 * prim], i1 = sd.indices[3 * prim + 1], i2 = sd.indices[3 * prim + 2];
-    V3 a = load_pos(sd.vertices, i0), b = load_pos(sd.vertices, i1), c = load_pos(sd.vertices, i2);
-    float4* t = sd.tris + (size_t)j * kTriF4;
-    t[0] = make_float4(a.x, a.y, a.z, __int_as_float((int)prim));
-    t[1] = make_float4(b.x, b.y, b.z, 0.f);
-    t[2] = make_float4(c.x, c.y, c.z, 0.f);
-    V3 lo, hi;
-    tri_box(a, b, c, lo, hi);
-    float px = leaf_pad(lo.x, hi.x), py = leaf_pad(lo.y, hi.y), pz = leaf_pad(lo.z, hi.z);
-    leaf_box[2 * g] = make_float4(lo.x - px, lo.y - py, lo.z - pz, 0.f);
-    leaf_box[2 * g + 1] = make_float4(hi.x + px, hi.y + py, hi.z + pz, 0.f);
+// Prefix length between leaf g and g + 1 of all segments' leaves (-1 across a segment's end).
+__device__ __forceinline__ int pair_delta(const SegDesc& sd, const unsigned long long* keys, uint32_t g) {
+    if (g < sd.prim_off || g - sd.prim_off + 1 >= sd.prim_count) return -1;   // (g may be prim_off - 1)
+    const uint32_t a = (uint32_t)keys[g] & 0x3FFFFFFFu, b = (uint32_t)keys[g + 1] & 0x3FFFFFFFu;
+    if (a != b) return __clz(a ^ b);
+    const uint32_t i = g - sd.prim_off;
+    return 32 + __clz(i ^ (i + 1));
 }
 
-
-
-__global__ void refit_kernel(const SegDesc* segs, const uint32_t* seg_prim_off, int nseg,
-                             uint32_t total, const float4* leaf_box, const uint32_t* node_parent,
-                             const uint32_t* leaf_parent, uint32_t* flags) {
-    chain_wait();
-    uint32_t g = blockIdx.x * blockDim.x + threadIdx.x;
-    if (g >= total) return;
-    int s = find_seg(seg_prim_off, nseg, g);
-    refit_leaf<false>(segs[s], g, leaf_box, node_parent, leaf_parent, flags);
-}
-
-// The refit with the nodes of a block's own leaves in shared memory. Block b takes the
-// kRefitLeaves consecutive leaves [b0, b0 + kRefitLeaves) of the sorted order. An
-// internal node whose leaf range (kept by the hierarchy pass) lies inside them has both
-// children inside as well, so its two child boxes, its arrival count, its parent and
-// its range live in shared memory at index (first leaf of its segment + node index -
-// b0): the node index lies in its own leaf range. The climbs through these nodes touch
-// shared memory only, and the block writes their slots to device memory at the end,
-// one node per thread. The first node whose range leaves the block (and so every node above
-// it) goes through refit_leaf's device-memory protocol. Same slots as refit_kernel, bit
-// for bit: every box is a min / max union.
-__global__ void __launch_bounds__(kRefitLeaves)
-refit_local_kernel(const SegDesc* segs, const uint32_t* seg_prim_off, int nseg, uint32_t total,
-                   const float4* leaf_box, const uint32_t* node_parent, const uint32_t* leaf_parent,
-                   uint32_t* flags) {
-    chain_wait();
-    __shared__ float s_box[kRefitLeaves][2][6];   // per local node: child slot 0 / 1 (lo xyz, hi xyz)
-    __shared__ uint32_t s_flag[kRefitLeaves];
-    __shared__ uint32_t s_parent[kRefitLeaves];   // parent and leaf range of node (g - prim_off)
-    __shared__ uint2 s_range[kRefitLeaves];
-    const uint32_t b0 = blockIdx.x * kRefitLeaves, g = b0 + threadIdx.x;
-    s_flag[threadIdx.x] = 0u;
-    int s = 0;
-    SegDesc sd{};
-    if (g < total) {
-        s = find_seg(seg_prim_off, nseg, g);
-        sd = segs[s];
-        // the node with the index of this leaf position (every leaf position of a segment
-        // but its last has one): loaded once, coalesced, for the climbs of the block
-        const uint32_t q = g - sd.prim_off;
-        if (q + 1 < sd.prim_count) {
-            s_parent[threadIdx.x] = node_parent[sd.node_off + q];
-            s_range[threadIdx.x] = sd.node_range[q];
+// The leaf of thread t is span.first + t (in: it is of the span), of segment sd with box
+// [lo, hi]; called by whole blocks of kMergeLeaves threads. leaf_box(j, lo, hi): the box of leaf j of the segment,
+// written before by the thread of that leaf.
+template <typename LeafBox>
+__device__ __forceinline__ void merge_block(MergeShared& S, const MergeArgs& A, MergeSpan span, const SegDesc& sd, bool in,
+                                            float4 lo, float4 hi, const LeafBox& leaf_box) {
+    const uint32_t full = 0xFFFFFFFFu, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const uint32_t b0 = span.first, g = b0 + tid;
+    S.flag[tid] = 0u;
+    const int dg = in ? pair_delta(sd, A.keys, g) : 127;   // past the span: no bound
+    S.delta[tid + 1] = (int8_t)dg;
+    if (tid == 0) S.delta[0] = (int8_t)(in && g > 0 ? pair_delta(sd, A.keys, g - 1) : -1);
+    // least deltas of the pairs after / before each position's pair, inside the block (the
+    // pair before its first leaf counts)
+    int up = dg, down = dg;   // inclusive within the warp
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const int u = __shfl_up_sync(full, up, o), v = __shfl_down_sync(full, down, o);
+        if (lane >= (uint32_t)o) up = min(up, u);
+        if (lane + o < 32) down = min(down, v);
+    }
+    if (lane == 31) S.warp_min[warp] = (int8_t)up;
+    __syncthreads();
+    {
+        int u = __shfl_up_sync(full, up, 1), v = __shfl_down_sync(full, down, 1);
+        if (lane == 0) u = 127;
+        if (lane == 31) v = 127;
+        u = min(u, (int)S.delta[0]);
+        for (uint32_t w = 0; w < kMergeLeaves / 32; ++w) {
+            if (w < warp) u = min(u, (int)S.warp_min[w]);
+            if (w > warp) v = min(v, (int)S.warp_min[w]);
         }
+        S.before[tid] = (int8_t)u;
+        S.after[tid] = (int8_t)v;
     }
     __syncthreads();
-    if (g < total) {
-        float4 lo = leaf_box[2 * g], hi = leaf_box[2 * g + 1];
-        uint32_t p = leaf_parent[g];
-        const uint32_t node_count = sd.prim_count > 1 ? sd.prim_count - 1 : 1;
-        bool global = sd.prim_count <= 1;   // a one-primitive segment's node has one child (one arrival)
-        for (uint32_t guard = 0; guard <= sd.prim_count + 1; ++guard) {
-            const uint32_t local = p >> 1;
-            if (p == 0xFFFFFFFFu || local >= node_count) break;
-            // the node index lies in its own leaf range: a node whose index is outside the
-            // block's positions spans other blocks' leaves (and so does every node above it)
-            const uint32_t k = sd.prim_off + local - b0;
-            if (!global) {
-                if (k >= (uint32_t)kRefitLeaves) {
-                    global = true;
-                } else {
-                    const uint2 range = s_range[k];
-                    global = sd.prim_off + range.x < b0 || sd.prim_off + range.y >= b0 + kRefitLeaves;
-                }
-            }
-            if (global) {
-                float4* node = sd.nodes + (size_t)local * kNodeF4;
-                write_slot(node, p & 1, lo, hi);
-                if (atomic_add_acq_rel_gpu(flags + sd.node_off + local, 1u) == 0) break;
-                const float4 n0 = __ldcg(node + 0), n1 = __ldcg(node + 1), n2 = __ldcg(node + 2);
-                lo = make_float4(fmin_(n0.x, n1.x), fmin_(n0.z, n1.z), fmin_(n2.x, n2.z), 0.f);
-                hi = make_float4(fmax_(n0.y, n1.y), fmax_(n0.w, n1.w), fmax_(n2.y, n2.w), 0.f);
-                p = node_parent[sd.node_off + local];
-                continue;
-            }
-            // local: shared memory only; the block writes these nodes' slots at the end
-            float* slot = s_box[k][p & 1];
+    const bool climbs = in && sd.prim_count >= 2;
+    const uint32_t off = sd.prim_off, last = off + sd.prim_count - 1;
+    uint32_t l = g, r = g;
+    int dl = S.delta[tid], dr = S.delta[tid + 1];   // prefixes before and after [l, r]
+    bool go = climbs;                               // still on its way at the end of the local merges
+    if (climbs) {
+        while (l != off || r != last) {             // every pass widens [l, r]
+            const bool left = dr > dl;
+            const uint32_t m = left ? r : l - 1, k = m - b0;   // the merge: between leaf m and m + 1
+            const int d = max(dl, dr);
+            if (!(m >= b0 && k < kMergeLeaves && (int)S.before[k] < d && (int)S.after[k] < d)) break;
+            const uint32_t side = left ? 0u : 1u;
+            float* slot = S.box[k][side];
             slot[0] = lo.x; slot[1] = lo.y; slot[2] = lo.z;
             slot[3] = hi.x; slot[4] = hi.y; slot[5] = hi.z;
+            S.end[k][side] = left ? l : r;
             __threadfence_block();
-            if (atomicAdd(s_flag + k, 1u) == 0) break;
+            if (atomicAdd(&S.flag[k], 1u) == 0u) { go = false; break; }
             __threadfence_block();
-            const float* c0 = s_box[k][0];
-            const float* c1 = s_box[k][1];
+            const float* c0 = S.box[k][0];
+            const float* c1 = S.box[k][1];
             lo = make_float4(fmin_(c0[0], c1[0]), fmin_(c0[1], c1[1]), fmin_(c0[2], c1[2]), 0.f);
             hi = make_float4(fmax_(c0[3], c1[3]), fmax_(c0[4], c1[4]), fmax_(c0[5], c1[5]), 0.f);
-            p = s_parent[k];
+            l = S.end[k][0];
+            r = S.end[k][1];
+            if (l < b0 || r - b0 >= kMergeLeaves || l > m || r <= m) {   // (never for sorted keys)
+                atomicOr(A.status, (uint32_t)LUZ_DEV_KARRAS_RANGE);
+                go = false;
+                break;
+            }
+            dl = S.delta[l - b0];
+            dr = S.delta[r - b0 + 1];
         }
     }
     __syncthreads();
-    // the slots of every node completed in shared memory (both arrivals), one node per
-    // thread at the node of this thread's leaf position
-    if (g < total && s_flag[threadIdx.x] == 2u) {
-        const float* c0 = s_box[threadIdx.x][0];
-        const float* c1 = s_box[threadIdx.x][1];
-        float4* node = sd.nodes + (size_t)(g - sd.prim_off) * kNodeF4;
-        node[0] = make_float4(c0[0], c0[3], c0[1], c0[4]);
-        node[1] = make_float4(c1[0], c1[3], c1[1], c1[4]);
-        node[2] = make_float4(c0[2], c0[5], c1[2], c1[5]);
+    // the nodes completed in shared memory, one per merge position
+    auto put_node = [&](const SegDesc& seg, uint32_t nl, uint32_t nr, uint32_t m, int el, int er, float4 lo0, float4 hi0,
+                        float4 lo1, float4 hi1) {
+        const uint32_t o = seg.prim_off;
+        const bool top = nl == o && nr == o + seg.prim_count - 1;
+        // its own side, and so its index, from the prefixes around it
+        const uint32_t node = top ? 0u : (er > el ? nr : nl) - o;
+        const int c0 = nl == m ? ~(int)(m - o) : (int)(m - o);
+        const int c1 = nr == m + 1 ? ~(int)(m + 1 - o) : (int)(m + 1 - o);
+        float4* q = seg.nodes + (size_t)node * kNodeF4;
+        q[0] = make_float4(lo0.x, hi0.x, lo0.y, hi0.y);
+        q[1] = make_float4(lo1.x, hi1.x, lo1.y, hi1.y);
+        q[2] = make_float4(lo0.z, hi0.z, lo1.z, hi1.z);
+        q[3] = make_float4(__int_as_float(c0), __int_as_float(c1), 0.f, 0.f);
+        if (A.node_parent) {
+            uint32_t* parent = A.node_parent + seg.node_off;
+            if (c0 >= 0) parent[c0] = node << 1;
+            if (c1 >= 0) parent[c1] = (node << 1) | 1u;
+            if (top) parent[0] = 0xFFFFFFFFu;
+        }
+    };
+    if (in && S.flag[tid] == 2u) {   // a merge position lies in the segment of its leaf
+        const uint32_t nl = S.end[tid][0], nr = S.end[tid][1];
+        const float* c0 = S.box[tid][0];
+        const float* c1 = S.box[tid][1];
+        if (nl >= b0 && nr - b0 < kMergeLeaves)
+            put_node(sd, nl, nr, g, S.delta[nl - b0], S.delta[nr - b0 + 1], make_float4(c0[0], c0[1], c0[2], 0.f),
+                     make_float4(c0[3], c0[4], c0[5], 0.f), make_float4(c1[0], c1[1], c1[2], 0.f),
+                     make_float4(c1[3], c1[4], c1[5], 0.f));
     }
+    __syncthreads();   // the block's nodes before its first merge in device memory
+    while (go && (l != off || r != last)) {
+        const bool left = dr > dl;
+        const uint32_t m = left ? r : l - 1;
+        (left ? A.ends[0] : A.ends[1])[m] = left ? make_uint2(l, (uint32_t)(dl + 1)) : make_uint2(r, (uint32_t)(dr + 1));
+        if (atomic_add_acq_rel_gpu(A.flags + m, 1u) == 0u) break;
+        // the sibling's far end and the prefix there, and both that it may be, its leaf and its
+        // node, in flight together
+        const uint32_t sib = (left ? m + 1 : m) - off;
+        const float4* q = sd.nodes + (size_t)min(sib, sd.prim_count - 2u) * kNodeF4;
+        const uint2 far = __ldcg((left ? A.ends[1] : A.ends[0]) + m);
+        const uint32_t oend = far.x;
+        const float4 n0 = __ldcg(q), n1 = __ldcg(q + 1), n2 = __ldcg(q + 2);
+        float4 olo, ohi;
+        leaf_box(sib, olo, ohi);
+        if (oend != sib + off) {
+            olo = make_float4(fmin_(n0.x, n1.x), fmin_(n0.z, n1.z), fmin_(n2.x, n2.z), 0.f);
+            ohi = make_float4(fmax_(n0.y, n1.y), fmax_(n0.w, n1.w), fmax_(n2.y, n2.w), 0.f);
+        }
+        if (left ? oend <= m || oend > last : oend > m || oend < off) {   // (never for sorted keys)
+            atomicOr(A.status, (uint32_t)LUZ_DEV_KARRAS_RANGE);
+            break;
+        }
+        const float4 lo0 = left ? lo : olo, hi0 = left ? hi : ohi, lo1 = left ? olo : lo, hi1 = left ? ohi : hi;
+        if (left) { r = oend; dr = (int)far.y - 1; }
+        else { l = oend; dl = (int)far.y - 1; }
+        put_node(sd, l, r, m, dl, dr, lo0, hi0, lo1, hi1);
+        lo = make_float4(fmin_(lo0.x, lo1.x), fmin_(lo0.y, lo1.y), fmin_(lo0.z, lo1.z), 0.f);
+        hi = make_float4(fmax_(hi0.x, hi1.x), fmax_(hi0.y, hi1.y), fmax_(hi0.z, hi1.z), 0.f);
+    }
+}
+
+// The padded box of a triangle.
+__device__ __forceinline__ void leaf_tri_box(V3 a, V3 b, V3 c, float4& lo, float4& hi) {
+    V3 l, h;
+    tri_box(a, b, c, l, h);
+    const float px = leaf_pad(l.x, h.x), py = leaf_pad(l.y, h.y), pz = leaf_pad(l.z, h.z);
+    lo = make_float4(l.x - px, l.y - py, l.z - pz, 0.f);
+    hi = make_float4(h.x + px, h.y + py, h.z + pz, 0.f);
+}
+
+// The node of a segment without leaves or with one (leaf 0, box [lo, hi]).
+__device__ __forceinline__ void write_single_node(const SegDesc& sd, uint32_t* node_parent, float4 lo, float4 hi) {
+    write_inverted_slot(sd.nodes, 0);
+    write_inverted_slot(sd.nodes, 1);
+    if (sd.prim_count == 1) write_slot(sd.nodes, 0, lo, hi);
+    sd.nodes[3] = make_float4(__int_as_float(sd.prim_count == 1 ? ~0 : kEmptyChild), __int_as_float(kEmptyChild), 0.f, 0.f);
+    if (node_parent) node_parent[sd.node_off] = 0xFFFFFFFFu;
+}
+
+// The nodes of the segments without a leaf (the others' are written with their leaves).
+__global__ void empty_segments_kernel(const SegDesc* segs, int nseg, uint32_t* node_parent) {
+    chain_wait();
+    const int s = blockIdx.x * blockDim.x + threadIdx.x;
+    if (s < nseg && segs[s].prim_count == 0) write_single_node(segs[s], node_parent, float4{}, float4{});
+}
+
+// BLAS: triangles gathered into leaf order, sorted morton/order into the segment's own
+// arrays, and the hierarchy over them.
+__global__ void __launch_bounds__(kMergeLeaves) blas_tree_kernel(const SegDesc* segs, const uint32_t* seg_prim_off, int nseg,
+                                                                 const uint32_t* vals, MergeArgs A) {
+    chain_wait();
+    __shared__ MergeShared S;
+    const MergeSpan span = merge_span(S, A.keys, A.total);
+    const uint32_t g = span.first + threadIdx.x;
+    const bool in = threadIdx.x < span.count;
+    SegDesc sd{};
+    float4 lo = make_float4(0.f, 0.f, 0.f, 0.f), hi = lo;
+    if (in) {
+        sd = segs[find_seg(seg_prim_off, nseg, g)];
+        const uint32_t j = g - sd.prim_off, prim = vals[g] - sd.prim_off;
+        sd.morton[j] = (uint32_t)A.keys[g] & 0x3FFFFFFFu;
+        sd.order[j] = prim;
+        const uint32_t i0 = sd.indices[3 * prim], i1 = sd.indices[3 * prim + 1], i2 = sd.indices[3 * prim + 2];
+        const V3 a = load_pos(sd.vertices, i0), b = load_pos(sd.vertices, i1), c = load_pos(sd.vertices, i2);
+        float4* t = sd.tris + (size_t)j * kTriF4;
+        t[0] = make_float4(a.x, a.y, a.z, __int_as_float((int)prim));
+        t[1] = make_float4(b.x, b.y, b.z, 0.f);
+        t[2] = make_float4(c.x, c.y, c.z, 0.f);
+        leaf_tri_box(a, b, c, lo, hi);
+        if (sd.prim_count == 1) write_single_node(sd, A.node_parent, lo, hi);
+    }
+    const float4* tris = sd.tris;
+    merge_block(S, A, span, sd, in, lo, hi, [tris](uint32_t j, float4& l, float4& h) {
+        const float4* t = tris + (size_t)j * kTriF4;
+        const float4 a = __ldcg(t), b = __ldcg(t + 1), c = __ldcg(t + 2);
+        leaf_tri_box(V3{a.x, a.y, a.z}, V3{b.x, b.y, b.z}, V3{c.x, c.y, c.z}, l, h);
+    });
 }
 
 // ---------------------------------------------------------------- bounding sphere
@@ -474,7 +622,20 @@ __global__ void blas_radius_kernel(const SegDesc* segs, const uint32_t* seg_prim
     const uint32_t full = 0xFFFFFFFFu;
     int s0 = __shfl_sync(full, s, 0);
     bool uniform = __all_sync(full, s == s0 || s < 0);
-    if (uniform) {
+    // one atomic per block where it is of one segment (320 instead of 2560 to one word)
+    __shared__ int s_seg;
+    __shared__ uint32_t s_max;
+    if (threadIdx.x == 0) {
+        s_seg = s0;
+        s_max = 0u;
+    }
+    __syncthreads();
+    if (__syncthreads_and(uniform && (s0 == s_seg || s0 < 0))) {
+        const uint32_t r = __reduce_max_sync(full, r2);
+        if ((threadIdx.x & 31) == 0) atomicMax(&s_max, r);
+        __syncthreads();
+        if (threadIdx.x == 0 && s >= 0) atomicMax((uint32_t*)&root[3].z, s_max);
+    } else if (uniform) {
         uint32_t r = __reduce_max_sync(full, r2);
         float4* root0 = (float4*)__shfl_sync(full, (unsigned long long)root, 0);
         if ((threadIdx.x & 31) == 0 && s0 >= 0) atomicMax((uint32_t*)&root0[3].z, r);
@@ -647,27 +808,49 @@ __global__ void tlas_setup_kernel(uint32_t* bounds, SegDesc* seg, SegDesc value,
     }
 }
 
-__global__ void tlas_morton_kernel(const float4* inst_box, uint32_t n, const uint32_t* seg_bounds,
-                                   unsigned long long* keys, uint32_t* vals) {
+__global__ void __launch_bounds__(256) tlas_morton_kernel(const float4* inst_box, uint32_t n, const uint32_t* seg_bounds,
+                                                          unsigned long long* keys, uint32_t* vals, int passes,
+                                                          uint32_t* hist) {
     chain_wait();
-    uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    float4 l = inst_box[2 * i], h = inst_box[2 * i + 1];
-    V3 cmin, ext;
-    decode_bounds(seg_bounds, cmin, ext);
-    keys[i] = morton30(V3{l.x, l.y, l.z}, V3{h.x, h.y, h.z}, cmin, ext);
-    vals[i] = i;
+    __shared__ uint32_t s_hist[kMaxPasses][kRadix];
+    const BlockHist H{s_hist, passes};
+    H.clear();
+    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < n) {
+        float4 l = inst_box[2 * i], h = inst_box[2 * i + 1];
+        V3 cmin, ext;
+        decode_bounds(seg_bounds, cmin, ext);
+        keys[i] = morton30(V3{l.x, l.y, l.z}, V3{h.x, h.y, h.z}, cmin, ext);
+        vals[i] = i;
+        H.count(keys[i]);
+    }
+    H.add(hist);
 }
 
-
-__global__ void tlas_emit_kernel(const DevInstanceInput* in, const float4* inst_box, uint32_t n,
-                                 const unsigned long long* keys, const uint32_t* vals,
-                                 DevInstance* inst_out, float4* leaf_box, uint32_t* morton_out,
-                                 uint32_t* order_out) {
+// Instance records in leaf order, leaf boxes, sorted codes and order, and the hierarchy
+// over them (seg: the one segment, at least two leaves).
+__global__ void __launch_bounds__(kMergeLeaves) tlas_tree_kernel(const SegDesc* seg, const DevInstanceInput* in_instances,
+                                                                 const float4* inst_box, const uint32_t* vals,
+                                                                 DevInstance* inst_out, float4* leaf_boxes,
+                                                                 uint32_t* morton_out, uint32_t* order_out, MergeArgs A) {
     chain_wait();
-    uint32_t j = blockIdx.x * blockDim.x + threadIdx.x;
-    if (j >= n) return;
-    tlas_emit_one(in, inst_box, j, keys[j], vals[j], inst_out, leaf_box, morton_out, order_out);
+    __shared__ MergeShared S;
+    const MergeSpan span = merge_span(S, A.keys, A.total);
+    const uint32_t g = span.first + threadIdx.x;
+    const bool in = threadIdx.x < span.count;
+    const SegDesc sd = *seg;
+    float4 lo = make_float4(0.f, 0.f, 0.f, 0.f), hi = lo;
+    if (in) {
+        const uint32_t i = vals[g];
+        tlas_emit_leaf(inst_box, g, A.keys[g], i, leaf_boxes, morton_out, order_out);
+        tlas_emit_record(in_instances, g, i, inst_out);
+        lo = inst_box[2 * i];
+        hi = inst_box[2 * i + 1];
+    }
+    merge_block(S, A, span, sd, in, lo, hi, [leaf_boxes](uint32_t j, float4& l, float4& h) {
+        l = __ldcg(leaf_boxes + 2 * j);
+        h = __ldcg(leaf_boxes + 2 * j + 1);
+    });
 }
 
 __global__ void tlas_record_kernel(const DevInstanceInput* in, const uint32_t* order, uint32_t n, DevInstance* inst_out) {
@@ -684,17 +867,24 @@ constexpr uint32_t kTlasLevels = 64;   // above the depth of 30-bit codes split 
 // order, and the digits' offsets are the level table. Every step takes the whole chip
 // (8000 instances: relayout and collapse by one block, level by level, 119 us; these kernels
 // and their sort pass 27).
-__global__ void tlas_depth_kernel(const uint32_t* node_parent, uint32_t m, unsigned long long* keys, uint32_t* vals) {
+__global__ void __launch_bounds__(256) tlas_depth_kernel(const uint32_t* node_parent, uint32_t m, unsigned long long* keys,
+                                                         uint32_t* vals, uint32_t* hist) {
     chain_wait();
+    __shared__ uint32_t s_hist[1][kRadix];
+    const BlockHist H{s_hist, 1};
+    H.clear();
     const uint32_t q = blockIdx.x * blockDim.x + threadIdx.x;
-    if (q >= m) return;
-    uint32_t d = 0, p = node_parent[q];
-    while (p != 0xFFFFFFFFu && d + 1 < kTlasLevels) {
-        ++d;
-        p = node_parent[p >> 1];
+    if (q < m) {
+        uint32_t d = 0, p = node_parent[q];
+        while (p != 0xFFFFFFFFu && d + 1 < kTlasLevels) {
+            ++d;
+            p = node_parent[p >> 1];
+        }
+        keys[q] = d;
+        vals[q] = q;
+        H.count(d);
     }
-    keys[q] = d;
-    vals[q] = q;
+    H.add(hist);
 }
 
 // Level table {L, start_0, ..., start_L}, and the inverse of the order.
@@ -1058,22 +1248,22 @@ static char* carve_sort(char* p, uint32_t n, int passes, SortBuffers& sb) {
     return p;
 }
 
-// Sorts sb.keys[0]/vals[0]; returns the index (0/1) of the buffer holding the result.
+// Clears what a sort counts in (its buffers from hist to tile_counter are consecutive),
+// before the kernel that makes the keys and counts their digits.
+static luz_status clear_sort(luz_ctx* ctx, SortBuffers& sb, int passes) {
+    LUZ_CUDA(ctx, cudaMemsetAsync(sb.hist, 0, (char*)(sb.tile_counter + passes) - (char*)sb.hist, ctx->stream));
+    return LUZ_OK;
+}
+
+// Sorts sb.keys[0]/vals[0], whose digits are counted; returns the index (0/1) of the buffer
+// holding the result. n: at most what sb was carved for.
 static luz_status run_sort(luz_ctx* ctx, SortBuffers& sb, uint32_t n, int passes, int& result) {
-    cudaStream_t st = ctx->stream;
-    LUZ_CUDA(ctx, cudaMemsetAsync(sb.hist, 0, (size_t)passes * 256 * 4, st));
-    LUZ_CUDA(ctx, cudaMemsetAsync(sb.tile_status, 0, (size_t)passes * sb.tiles * 256 * 4, st));
-    LUZ_CUDA(ctx, cudaMemsetAsync(sb.tile_counter, 0, (size_t)passes * 4, st));
-    uint32_t hblocks = std::min<uint32_t>(std::max(1u, cdiv(n, 256 * 16)), (uint32_t)ctx->sm_count * 4);
-    chain(sort_histogram_kernel, hblocks, 256, 0, st, sb.keys[0], n, passes, sb.hist);
-    LUZ_LAUNCHED(ctx, "sort_histogram_kernel");
-    chain(sort_scan_kernel, passes, 256, 0, st, sb.hist, sb.offsets);
-    LUZ_LAUNCHED(ctx, "sort_scan_kernel");
+    const uint32_t tiles = cdiv(n, kSortTile);
     int cur = 0;
     for (int p = 0; p < passes; ++p) {
-        chain(onesweep_pass_kernel, sb.tiles, kSortThreads, 0, st, sb.keys[cur], sb.vals[cur], sb.keys[cur ^ 1], sb.vals[cur ^ 1], n, 8 * p,
-            sb.offsets + p * 256, sb.tile_status + (size_t)p * sb.tiles * 256, sb.tile_counter + p,
-            ctx->d_status);
+        chain(onesweep_pass_kernel, tiles, kSortThreads, 0, ctx->stream, sb.keys[cur], sb.vals[cur], sb.keys[cur ^ 1],
+              sb.vals[cur ^ 1], n, 8 * p, sb.hist + p * 256, sb.offsets + p * 256,
+              sb.tile_status + (size_t)p * sb.tiles * 256, sb.tile_counter + p, ctx->d_status);
         LUZ_LAUNCHED(ctx, "onesweep_pass_kernel");
         cur ^= 1;
     }
@@ -1087,6 +1277,7 @@ luz_status build_blas_batch(luz_ctx* ctx, uint32_t count, const luz_blas_desc* d
     std::vector<SegDesc> segs(count);
     std::vector<uint32_t> prim_off(count), node_off(count);
     uint64_t total_prims = 0, total_nodes = 0, total_verts = 0;
+    bool has_empty = false;
     for (uint32_t s = 0; s < count; ++s) {
         const luz_blas_desc& d = descs[s];
         if (d.index_count % 3 != 0)
@@ -1098,6 +1289,7 @@ luz_status build_blas_batch(luz_ctx* ctx, uint32_t count, const luz_blas_desc* d
             if (d.indices[k] >= d.vertex_count)
                 return set_error(ctx, LUZ_ERR_INVALID, "index out of range of the vertex buffer");
         uint32_t n = d.index_count / 3;
+        has_empty = has_empty || n == 0;
         prim_off[s] = (uint32_t)total_prims;
         node_off[s] = (uint32_t)total_nodes;
         total_prims += n;
@@ -1162,16 +1354,15 @@ luz_status build_blas_batch(luz_ctx* ctx, uint32_t count, const luz_blas_desc* d
         sd.morton = (uint32_t*)(ab + off_mort[s]);
         sd.order = (uint32_t*)(ab + off_ord[s]);
     }
-    // Scratch: segs | prim_off | node_off | bounds | sort | leaf boxes | parents | flags |
-    // 4-wide collapse indices | leaf ranges.
+    // Scratch: segs | prim_off | node_off | bounds | sort | parents | merges' flags and far
+    // ends | 4-wide collapse indices.
     uint32_t N = (uint32_t)total_prims, M = (uint32_t)total_nodes;
     int passes = passes_for((int)count);
     size_t need = align256(count * sizeof(SegDesc)) + 2 * align256(count * 4) +
                   align256(count * 24) + sort_scratch_bytes(std::max(N, 1u), passes) +
-                  align256((size_t)std::max(N, 1u) * 32) + align256((size_t)M * 4) +
-                  align256((size_t)std::max(N, 1u) * 4) + align256((size_t)M * 4) +
+                  align256((size_t)M * 4) + align256((size_t)std::max(N, 1u) * 4) + 2 * align256((size_t)std::max(N, 1u) * 8) +
                   2 * align256((size_t)M * 4) +
-                  align256((size_t)(M / 1024 + 1) * 4) + align256((size_t)M * 8);
+                  align256((size_t)(M / 1024 + 1) * 4);
     luz_status stt = ensure_scratch(ctx, need);
     if (stt != LUZ_OK) { cudaFree(arena->base); delete arena; return stt; }
     char* p = (char*)ctx->d_scratch;
@@ -1181,15 +1372,13 @@ luz_status build_blas_batch(luz_ctx* ctx, uint32_t count, const luz_blas_desc* d
     uint32_t* d_bounds = (uint32_t*)p; p += align256(count * 24);
     SortBuffers sb;
     p = carve_sort(p, std::max(N, 1u), passes, sb);
-    float4* d_leaf_box = (float4*)p; p += align256((size_t)std::max(N, 1u) * 32);
     uint32_t* d_node_parent = (uint32_t*)p; p += align256((size_t)M * 4);
-    uint32_t* d_leaf_parent = (uint32_t*)p; p += align256((size_t)std::max(N, 1u) * 4);
-    uint32_t* d_flags = (uint32_t*)p; p += align256((size_t)M * 4);
+    uint32_t* d_flags = (uint32_t*)p; p += align256((size_t)std::max(N, 1u) * 4);
+    uint2* d_ends[2];
+    for (uint2*& e : d_ends) { e = (uint2*)p; p += align256((size_t)std::max(N, 1u) * 8); }
     uint32_t* d_even = (uint32_t*)p; p += align256((size_t)M * 4);
     uint32_t* d_idx4 = (uint32_t*)p; p += align256((size_t)M * 4);
     uint32_t* d_sums = (uint32_t*)p; p += align256((size_t)(M / 1024 + 1) * 4);
-    uint2* d_range = (uint2*)p; p += align256((size_t)M * 8);
-    for (uint32_t s = 0; s < count; ++s) segs[s].node_range = d_range + node_off[s];
 
     LUZ_CUDA(ctx, cudaMemcpyAsync(d_segs, segs.data(), count * sizeof(SegDesc), cudaMemcpyHostToDevice, st));
     LUZ_CUDA(ctx, cudaMemcpyAsync(d_prim_off, prim_off.data(), count * 4, cudaMemcpyHostToDevice, st));
@@ -1199,34 +1388,28 @@ luz_status build_blas_batch(luz_ctx* ctx, uint32_t count, const luz_blas_desc* d
         for (int k = 0; k < 6; ++k) binit[s * 6 + k] = k < 3 ? 0xFFFFFFFFu : 0u;
     LUZ_CUDA(ctx, cudaMemcpyAsync(d_bounds, binit.data(), count * 24, cudaMemcpyHostToDevice, st));
     LUZ_CUDA(ctx, cudaEventRecord(ctx->build_ev[0], st));   // device pipeline starts here
-    LUZ_CUDA(ctx, cudaMemsetAsync(d_node_parent, 0xFF, (size_t)M * 4, st));
-    LUZ_CUDA(ctx, cudaMemsetAsync(d_leaf_parent, 0xFF, (size_t)std::max(N, 1u) * 4, st));
-    LUZ_CUDA(ctx, cudaMemsetAsync(d_flags, 0, (size_t)M * 4, st));
+    LUZ_CUDA(ctx, cudaMemsetAsync(d_flags, 0, (size_t)std::max(N, 1u) * 4, st));
     if (N > 0) {
-        chain(blas_bounds_kernel, cdiv(N, 256 * kBoundsIters), 256, 0, st, d_segs, d_prim_off, count, N, d_bounds);
+        if ((stt = clear_sort(ctx, sb, passes)) != LUZ_OK) { cudaFree(arena->base); delete arena; return stt; }
+        const uint32_t rows = bounds_rows(N);
+        chain(blas_bounds_kernel, cdiv(N, 256 * rows), 256, 0, st, d_segs, d_prim_off, count, N, rows, d_bounds);
         LUZ_LAUNCHED(ctx, "blas_bounds_kernel");
-        chain(blas_morton_kernel, cdiv(N, 256), 256, 0, st, d_segs, d_prim_off, count, N, d_bounds,
-                                                         sb.keys[0], sb.vals[0]);
+        chain(blas_morton_kernel, morton_blocks(N), 256, 0, st, d_segs, d_prim_off, count, N, d_bounds, sb.keys[0],
+              sb.vals[0], passes, sb.hist);
         LUZ_LAUNCHED(ctx, "blas_morton_kernel");
-    }
-    int res = 0;
-    if (N > 0) {
+        int res = 0;
         stt = run_sort(ctx, sb, N, passes, res);
         if (stt != LUZ_OK) { cudaFree(arena->base); delete arena; return stt; }
+        const MergeArgs A{sb.keys[res], d_node_parent, {d_ends[0], d_ends[1]}, d_flags, ctx->d_status, N};
+        chain(blas_tree_kernel, merge_blocks(N), kMergeLeaves, 0, st, d_segs, d_prim_off, count, sb.vals[res], A);
+        LUZ_LAUNCHED(ctx, "blas_tree_kernel");
     }
-    // Every segment has at least one node; segments with 0 or 1 primitive get their
-    // single node (empty / one leaf) here without reading keys.
-    chain(karras_kernel, cdiv(M, 256), 256, 0, st, d_segs, d_node_off, count, M, sb.keys[res],
-                                                d_node_parent, d_leaf_parent, ctx->d_status);
-    LUZ_LAUNCHED(ctx, "karras_kernel");
+    // Every segment has at least one node, also one without a primitive.
+    if (has_empty) {
+        chain(empty_segments_kernel, cdiv(count, 128), 128, 0, st, d_segs, count, d_node_parent);
+        LUZ_LAUNCHED(ctx, "empty_segments_kernel");
+    }
     if (N > 0) {
-        chain(blas_emit_kernel, cdiv(N, 256), 256, 0, st, d_segs, d_prim_off, count, N, sb.keys[res],
-                                                       sb.vals[res], d_leaf_box);
-        LUZ_LAUNCHED(ctx, "blas_emit_kernel");
-        chain(refit_local_kernel, cdiv(N, kRefitLeaves), kRefitLeaves, 0, st, d_segs, d_prim_off, count, N,
-                                                                           d_leaf_box, d_node_parent, d_leaf_parent,
-                                                                           d_flags);
-        LUZ_LAUNCHED(ctx, "refit_local_kernel");
         chain(blas_radius_kernel, cdiv(N, 256), 256, 0, st, d_segs, d_prim_off, count, N);
         LUZ_LAUNCHED(ctx, "blas_radius_kernel");
     }
@@ -1284,7 +1467,7 @@ static size_t tlas_tmp_bytes(uint32_t cap) {
     return align256((size_t)cap * 32) + align256(24) + sort_scratch_bytes(std::max(cap, 1u), 4) +
            align256((size_t)cap * 32) + align256((size_t)m * 4) + align256((size_t)cap * 4) +
            align256((size_t)m * 4) + align256((size_t)m * 64) + 2 * align256((size_t)m * 4) +
-           align256(sizeof(SegDesc)) + 2 * align256(4);
+           align256(sizeof(SegDesc)) + 2 * align256(4) + 2 * align256((size_t)cap * 8);
 }
 
 luz_status launch_tlas_build(luz_ctx* ctx, luz_tlas* t);
@@ -1345,6 +1528,7 @@ struct TlasScratch {
     SortBuffers sb;
     SegDesc* d_seg;
     uint32_t* d_zero;
+    uint2* ends[2];
 };
 
 static TlasScratch carve_tlas(luz_tlas* t) {
@@ -1370,6 +1554,7 @@ static TlasScratch carve_tlas(luz_tlas* t) {
     a.newidx = (uint32_t*)p; p += align256((size_t)mcap * 4);
     s.d_seg = (SegDesc*)p; p += align256(sizeof(SegDesc));
     s.d_zero = (uint32_t*)p; p += align256(4);
+    for (uint2*& e : s.ends) { e = (uint2*)p; p += align256((size_t)cap * 8); }
     a.inst_out = t->instances;
     a.morton_out = t->morton;
     a.order_out = t->order;
@@ -1404,7 +1589,6 @@ luz_status launch_tlas_kernels(luz_ctx* ctx, luz_tlas* t) {
     SortBuffers& sb = ts.sb;
     float4* leaf_box = A.leaf_box;
     uint32_t* node_parent = A.node_parent;
-    uint32_t* leaf_parent = A.leaf_parent;
     uint32_t* flags = A.flags;
     float4* karras_nodes = A.karras_nodes;
     uint32_t* newidx = A.newidx;
@@ -1446,28 +1630,21 @@ luz_status launch_tlas_kernels(luz_ctx* ctx, luz_tlas* t) {
     // host address that no longer holds them.
     chain(tlas_setup_kernel, 1, 32, 0, st, bounds, d_seg, sd, d_zero);
     LUZ_LAUNCHED(ctx, "tlas_setup_kernel");
-    LUZ_CUDA(ctx, cudaMemsetAsync(node_parent, 0xFF, (size_t)m * 4, st));
-    LUZ_CUDA(ctx, cudaMemsetAsync(leaf_parent, 0xFF, (size_t)n * 4, st));
     LUZ_CUDA(ctx, cudaMemsetAsync(flags, 0, (size_t)m * 4, st));
-
+    luz_status s = clear_sort(ctx, sb, 4);
+    if (s != LUZ_OK) return s;
     chain(tlas_instance_kernel, cdiv(n, 128), 128, 0, st, t->d_input, n, inst_box, t->shade, bounds);
     LUZ_LAUNCHED(ctx, "tlas_instance_kernel");
-    chain(tlas_morton_kernel, cdiv(n, 128), 128, 0, st, inst_box, n, bounds, sb.keys[0], sb.vals[0]);
+    chain(tlas_morton_kernel, cdiv(n, 256), 256, 0, st, inst_box, n, bounds, sb.keys[0], sb.vals[0], 4, sb.hist);
     LUZ_LAUNCHED(ctx, "tlas_morton_kernel");
     int res = 0;
-    luz_status s = run_sort(ctx, sb, n, 4, res);
-    if (s != LUZ_OK) return s;
-    chain(karras_kernel, cdiv(m, 128), 128, 0, st, d_seg, d_zero, 1, m, sb.keys[res], node_parent,
-                                                leaf_parent, ctx->d_status);
-    LUZ_LAUNCHED(ctx, "karras_kernel");
-    chain(tlas_emit_kernel, cdiv(n, 128), 128, 0, st, t->d_input, inst_box, n, sb.keys[res],
-                                                   sb.vals[res], t->instances, leaf_box,
-                                                   t->morton, t->order);
-    LUZ_LAUNCHED(ctx, "tlas_emit_kernel");
-    chain(refit_kernel, cdiv(n, 128), 128, 0, st, d_seg, d_zero, 1, n, leaf_box, node_parent,
-                                               leaf_parent, flags);
-    LUZ_LAUNCHED(ctx, "refit_kernel");
-    chain(tlas_depth_kernel, cdiv(m, 128), 128, 0, st, node_parent, m, sb.keys[0], sb.vals[0]);
+    if ((s = run_sort(ctx, sb, n, 4, res)) != LUZ_OK) return s;
+    const MergeArgs merge{sb.keys[res], node_parent, {ts.ends[0], ts.ends[1]}, flags, ctx->d_status, n};
+    chain(tlas_tree_kernel, merge_blocks(n), kMergeLeaves, 0, st, d_seg, t->d_input, inst_box, sb.vals[res],
+          t->instances, leaf_box, t->morton, t->order, merge);
+    LUZ_LAUNCHED(ctx, "tlas_tree_kernel");
+    if ((s = clear_sort(ctx, sb, 1)) != LUZ_OK) return s;
+    chain(tlas_depth_kernel, cdiv(m, 256), 256, 0, st, node_parent, m, sb.keys[0], sb.vals[0], sb.hist);
     LUZ_LAUNCHED(ctx, "tlas_depth_kernel");
     if ((s = run_sort(ctx, sb, m, 1, res)) != LUZ_OK) return s;
     chain(tlas_newidx_kernel, cdiv(m, 128), 128, 0, st, sb.vals[res], m, sb.offsets, newidx, t->levels);
