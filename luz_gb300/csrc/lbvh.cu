@@ -596,7 +596,7 @@ __global__ void __launch_bounds__(kMergeLeaves) blas_tree_kernel(const SegDesc* 
 
 // Bounding sphere of every BLAS about its root box centre: the largest squared
 // distance of a triangle vertex from the centre, kept as float bits in the root
-// node's spare word n3.z (zero after karras_kernel; positive floats order like their
+// node's spare word n3.z (zero after the hierarchy pass; positive floats order like their
 // bits, so atomicMax on the bits is a float max). Runs after the refit. The TLAS
 // build intersects each instance's transformed root box with the transformed sphere.
 __global__ void blas_radius_kernel(const SegDesc* segs, const uint32_t* seg_prim_off, int nseg,

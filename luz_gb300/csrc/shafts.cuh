@@ -140,8 +140,13 @@ constexpr uint32_t kListAll = 0xFFFFFFFFu;
 constexpr uint32_t kListCapSmall = 15, kListCapLarge = 31;
 inline uint32_t list_cap(uint32_t instances) { return instances > 2048 ? kListCapLarge : kListCapSmall; }
 constexpr uint32_t kSuper = 8;               // patches per block: 16x16 pixels where all are lit
-constexpr uint32_t kSuperLeaves = 128;       // leaves a block's shaft may reach; past it, and past
-constexpr uint32_t kSuperStack = 128;        // its nodes, its groups start at the TLAS root
+// Leaves a block's shaft may reach, and nodes it may have to visit; past either its groups
+// start at the TLAS root. Where the lists are long as well, long shafts pay: 1021x573 over
+// 8000 instances, lists and traversal: 128 leaves 0.79 + 2.42 ms, 250 0.86 + 2.24, 400
+// 0.89 + 2.17, 600 0.93 + 2.13. Over a few hundred instances a block that reaches 128 has
+// groups past their own lists' room: 183x97 over 375 instances 272 us with 128, 281 with 400.
+constexpr uint32_t kSuperLeaves = 400, kSuperLeavesSmall = 128, kSuperStack = 128;
+inline uint32_t super_cap(uint32_t instances) { return instances > 2048 ? kSuperLeaves : kSuperLeavesSmall; }
 constexpr uint32_t kCutsPerPair = 3;         // room for cuts per (light, patch) of a chunk
 // Triangles above which a BLAS is descended: below, the per-ray tests of ray generation
 // against its root cost no more than a cut.
@@ -460,7 +465,7 @@ struct ShaftOut {
     uint32_t vlight_count;
     unsigned long long q0;
     uint32_t cap;                // a multiple of kSuper (0: no shadow rays here)
-    uint32_t list_cap;
+    uint32_t list_cap, super_cap;
     uint32_t* lists;             // kEntryWords per pair
     float4* cuts;                // kCutsPerPair nodes of kNode4F4 per pair
     uint4* active;               // groups to trace: (pair, first slot | samples << 16, patch, -)
@@ -533,7 +538,7 @@ __device__ __forceinline__ void shaft_block(const SceneVis& S, const ShaftOut& A
                     hit = shaft_reaches(s, lo, hi, t0) && ch != kEmptyChild;
                 }
                 const uint32_t lb = __ballot_sync(full, hit && ch < 0), nb = __ballot_sync(full, hit && ch >= 0);
-                if (sn + __popc(lb) > kSuperLeaves || sp + __popc(nb) > kSuperStack) { far = true; break; }
+                if (sn + __popc(lb) > A.super_cap || sp + __popc(nb) > kSuperStack) { far = true; break; }
                 if (hit && ch < 0) super[sn + __popc(lb & lt_mask)] = (uint32_t)~ch;
                 if (hit && ch >= 0) stack[sp + __popc(nb & lt_mask)] = (uint32_t)ch;
                 sn += __popc(lb);

@@ -431,7 +431,7 @@ luz_status launch_visibility(luz_ctx* ctx, luz_frame* f, const luz_tlas* t, int 
         const RayOut R{v.rays_a, v.rays_b, v.rays_c, &n->records};
         const bool shadow = k < shadow_chunks, ao = k < ao_chunks;
         const ShaftOut A{patches, patches + z.patches, f->d_vlights, f->vlight_count, (unsigned long long)k * z.pairs,
-                         shadow ? z.pairs : 0u, cap, v.start_lists, v.cuts, v.active, &n->groups};
+                         shadow ? z.pairs : 0u, cap, super_cap(t->count), v.start_lists, v.cuts, v.active, &n->groups};
         const AoOut O{k * z.ao_patches, ao ? std::min(z.ao_patches, z.patches - k * z.ao_patches) : 0u, cap,
                       f->ao_samples < kAoMinSamples ? 0u : std::min(kAoStepsPerSample * f->ao_samples, kAoSteps),
                       v.start_lists + (size_t)z.pairs * kEntryWords, z.pairs, R};
