@@ -36,11 +36,13 @@ namespace luz {
 // = pixel of the group's patch, over the samples of its virtual light. Separated from
 // traversal so the long arithmetic of light.frag's sampling and the tests against the
 // group's list, the same leaves for all lanes, run on full warps. A ray that enters none
-// of the leaves is unoccluded and leaves no record: bound by issue (0.28 ms for the 5.2 M
-// samples that the shafts of a 1080p frame leave; the traversal that found the same on
-// partly filled warps took 0.28 ms longer).
+// of the leaves is unoccluded and leaves no record. Bound by latency, hence four blocks per
+// SM, and the list of a group held by the lanes: 0.25 ms for the 5.2 M samples that the
+// shafts of a 1080p frame leave (three blocks 0.28, five 0.26; lists read per sample and
+// leaf 0.29), 4K 13.0 -> 10.95 ms; the traversal that found the same on partly filled warps
+// took 0.28 ms longer.
 constexpr uint32_t kRaygenTake = 4;
-__global__ void __launch_bounds__(256, 3) shadow_raygen_kernel(SceneVis S, VisCommon C, Entries E,
+__global__ void __launch_bounds__(256, 4) shadow_raygen_kernel(SceneVis S, VisCommon C, Entries E,
                                                                const uint4* __restrict__ active,
                                                                const uint32_t* __restrict__ active_count,
                                                                uint32_t* tickets, RayOut R) {
@@ -60,6 +62,9 @@ __global__ void __launch_bounds__(256, 3) shadow_raygen_kernel(SceneVis S, VisCo
             const uint32_t first = a.y & 0xFFFFu, samples = a.y >> 16, j = a.z * kPatch + lane;
             const uint32_t* list = E.lists + (size_t)a.x * kEntryWords;
             const uint32_t cnt = __ldg(list);
+            // lane k: leaf k of the list and its cut
+            const bool has = cnt != kListAll && lane < cnt;
+            const uint32_t my_leaf = has ? __ldg(list + 1 + lane) : 0u, my_cut = has ? __ldg(list + kEntryCuts + lane) : 0u;
             for (uint32_t s = 0; s < samples; ++s) {
                 V3 wo{0.f, 0.f, 0.f}, wd{0.f, 0.f, 1.f};
                 float tmin = 0.f, tmax = 0.f;
@@ -76,7 +81,7 @@ __global__ void __launch_bounds__(256, 3) shadow_raygen_kernel(SceneVis S, VisCo
                     set_origin(r, wo);
                     near_planes(r);
                     for (uint32_t k = 0; k < cnt; ++k) {
-                        const uint32_t leaf = __ldg(list + 1 + k), cut = __ldg(list + kEntryCuts + k);
+                        const uint32_t leaf = __shfl_sync(full, my_leaf, k), cut = __shfl_sync(full, my_cut, k);
                         if (ok && leaf_overlaps(r, S.leaf_box, leaf) &&
                             leaf_enters(S.instances + leaf, cut ? E.cuts + (size_t)(cut - 1u) * kNode4F4 : nullptr, wo, wd,
                                         tmin, tmax))
