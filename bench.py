@@ -488,10 +488,9 @@ def batched_uneven(ctx, stream, flush, K, W, count=64, seed=4004, tune=True):
     """count scenes, triangles log-uniform in [1e3, 2e6] from the cube/quad and
     displaced-icosphere generators, resolutions from {256^2, 512^2, 1280x720,
     1920x1080}, 4 AO rays per pixel; one batched BLAS build at creation, then every
-    frame ONE persistent launch (the frame kernel: all TLAS builds, G-buffers, the
-    traversal of every scene's rays and the light passes) replayed as a CUDA graph, its
-    traversal launch shape picked by the autotuner. The staged form (separate launches
-    per scene around one batched traversal launch) is timed beside it."""
+    frame every scene's passes, spread over streams or in one persistent launch as the
+    library's rule has it, replayed as a CUDA graph, its traversal launch shape picked by
+    the autotuner. The form without the frame kernel is timed beside it."""
     import numpy as np
     import torch
 
@@ -548,11 +547,9 @@ def batched_uneven(ctx, stream, flush, K, W, count=64, seed=4004, tune=True):
                         for f, sc in zip(b.frames, scenes))
     traversed = st["rays"] + pixels
     ms = replay_ms()
-    # graph launches counted by the library: one frame kernel per replay when fused
     out.update({"rays_per_replay": rays, "rays_traversed_per_replay": traversed, "ms_per_replay": ms,
                 "grays_per_s": rays / (ms * 1e-3) / 1e9,
-                "graph": ("one CUDA graph per batch frame: a memset of the work counters and ONE persistent "
-                          "frame-kernel launch" if b.fused else "one CUDA graph of staged launches"),
+                "graph": "one CUDA graph per batch frame",
                 "fused": b.fused, "staged_ms_per_replay": staged,
                 "autotuned_shape": tun, "autotune_best_frame_ms": tune_ms})
     b.close()
@@ -643,14 +640,14 @@ def run_ours(args, rank, world, local):
         raise RuntimeError("device status word raised during timing")
 
     # Roofline of the dominant kernel, the traversal (visibility_kernel): algorithmic
-    # bytes per launch = ray records read (32 B per item, written by ray generation) +
-    # hit bits (1/8 B per traversed ray) + 4-wide node visits x 112 B (7 of the 8
+    # bytes per launch = hit bits (1/8 B per ray) + 4-wide node visits x 112 B (7 of the 8
     # float4) + triangle tests x 48 B + instance entries x 80 B, with the visits counted
-    # by the counting build of the same kernel over the same frame. The node and triangle
+    # by the counting build of the same kernel over the same frame (the 48-B records of
+    # the rays that shafts and horizons leave are not counted). The node and triangle
     # loads are served by L1 and L2 (the BVH is read from HBM about once per frame), so
     # the bound is the L2 read bandwidth, measured in this run by L2-only 16-B loads
     # over a 48 MiB buffer on every SM.
-    trav_bytes = (lit * S * 32 + stats["rays"] * 0.125 + (stats["tlas_nodes"] + stats["blas_nodes"]) * 112 +
+    trav_bytes = (stats["rays"] * 0.125 + (stats["tlas_nodes"] + stats["blas_nodes"]) * 112 +
                   stats["tris"] * 48 + stats["instances"] * 80)
     trav_ms = kernel_ms["traversal"]["ms_per_launch"]
     l2_gbs = ctx.probe_l2_read_gbs(48 << 20, 50)
@@ -661,7 +658,7 @@ def run_ours(args, rank, world, local):
                 "frac": achieved / l2_gbs, "traffic": None, "algorithmic_bytes": trav_bytes,
                 "ms_per_launch": trav_ms,
                 "note": "traffic (DRAM bytes per launch) comes from an ncu capture, not from this run; "
-                        "the kernel is issue-bound (about 69 % of issue slots and 13 of 32 lanes per instruction in an ncu capture)",
+                        "the kernel is issue-bound (about 68 % of issue slots and 12 of 32 lanes per instruction in an ncu capture)",
                 "per_ray": {k: stats[k] / max(stats["rays"], 1) for k in
                             ("tlas_nodes", "blas_nodes", "tris", "instances")}}
     # the light pass against HBM: per lit pixel the 32-B surface record, the 16-B record of
@@ -756,11 +753,12 @@ def run_ours(args, rank, world, local):
                              "+ lit pixels x (41 shadow + 16 AO). A shadow ray whose light's term in "
                              "the light pass cannot depend on it (weight max(dot(N, L), 0) = 0 or zero "
                              "unshadowed radiance) is resolved at generation without traversal, the "
-                             "image is unchanged; rays_traversed_per_frame are the rays actually traced.",
+                             "image is unchanged; rays_traversed_per_frame are the others, whether a group's shaft or "
+                             "horizon or a traversal resolves them.",
                 "traversed_grays_per_s": whole_job_rate(world, scene.width * scene.height + stats["rays"], ms),
                 "lit_pixels": lit, "stage_ms": stage_ms, "kernel_ms": kernel_ms,
-                "kernel_ms_note": "gbuffer includes its two tile-list kernels, raygen the near-list check of "
-                                  "the AO rays and the beam-list kernel of the shadow rays",
+                "kernel_ms_note": "gbuffer includes its tile-list kernel, raygen the patches, shafts and horizons "
+                                  "that resolve rays in groups",
                 "blas_build": {"ms": g.blas_build_ms, "device_ms": g.blas_build_device_ms,
                                "triangles": g.blas_prims, "meshes": len(g.blas),
                                "algorithmic_bytes_per_triangle": 248,

@@ -5,7 +5,7 @@
 // unshadowed direct light.
 //
 // BF16 tcgen05 matrix products with FP32 accumulators in tensor memory, operands in
-// shared memory in the K-major no-swizzle core-matrix layout. Inference: a block per
+// shared memory in the no-swizzle core-matrix layout. Inference: a block per
 // SM, warpgroups with a 128-pixel tile each (thread = pixel row). Training: one
 // persistent kernel runs forward, backward and the weight-gradient products over fixed
 // pixel tiles; every block accumulates its weight gradients in tensor memory in a

@@ -6,8 +6,8 @@
 // parameter t lies in the linear blend of the two boxes: a shaft, bounded per axis by two
 // lines in t, and along the patch's mean normal by one more. A box that no t in [0, 1]
 // brings into reach of all seven bounds cannot be touched by any ray of the group.
-// shaft_kernel (one thread per light and patch) descends the TLAS with that test, then
-// the BLAS of each leaf it reaches, and keeps per leaf the up to four nodes of the BLAS
+// A warp per light and block of eight patches descends the TLAS with that test, then four
+// lanes per patch the BLAS of each leaf it reaches, and keeps per leaf the up to four nodes of the BLAS
 // that the shaft still touches as a 4-wide node of their own (a cut). A leaf without any
 // is dropped; a group without leaves has only unoccluded rays: their bits stay 0 and
 // neither a ray record nor a traversal step is spent on them. The normal bound is what

@@ -10,9 +10,10 @@ namespace luz {
 
 const float4* tlas_leaf_boxes(const luz_tlas* t);
 
-// 8x8 pixels per CTA of 64 threads, 16 CTAs per SM (64 registers): measured at
-// 1080p 0.65 ms against 0.75 ms for 16x16-pixel CTAs with the TLAS top staged in
-// shared memory (L1 holds it as well, and the CTAs retire at a finer grain).
+// 8x8 pixels per CTA of 64 threads, 16 CTAs per SM (64 registers): 0.39 ms at 1080p, as with
+// blocks of one warp, 0.393 with 14 CTAs and 0.416 with 20; 16x16-pixel CTAs with the TLAS
+// top staged in shared memory were 15 % slower (L1 holds it as well, and the CTAs retire at
+// a finer grain).
 constexpr uint32_t kGbTile = 8;
 constexpr int kGbMinBlocks = 16;
 
