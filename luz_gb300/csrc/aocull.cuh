@@ -30,7 +30,6 @@ constexpr float kAoFloor = 0x1p-6f;          // horizons start here: lower rays 
 
 struct AoOut {
     uint32_t patch0, patches;    // patches [patch0, patch0 + patches) of the frame (0: no AO here)
-    uint32_t list_cap;
     uint32_t steps;              // node-stack steps of one horizon (0: no horizon)
     uint32_t* lists;             // start lists (kEntryWords), one per patch of the chunk
     uint32_t list0;              // index of the first of them
@@ -198,7 +197,7 @@ __device__ __forceinline__ void ao_patch(const SceneVis& S, const VisCommon& C, 
             if (hit && ch >= 0 && npos < kAoStack) node_st[npos] = (uint32_t)ch;
             leaves += __popc(lb);
             sp += __popc(nb);
-            if (leaves > A.list_cap || sp > kAoStack) { all = true; break; }
+            if (leaves > kListCap || sp > kAoStack) { all = true; break; }
             __syncwarp();
         }
     }

@@ -51,6 +51,7 @@ constexpr int kCutNode = 0x7FFFFFFF;
 struct Entries {
     const uint32_t* lists;       // words per list: kEntryWords
     const float4* cuts;
+    uint32_t cut_cap;            // lists of more leaves have no cuts (shafts.cuh)
 };
 constexpr uint32_t kEntryWords = 64, kEntryCuts = 32;   // words 1..31 leaves, 32..62 cuts (index + 1, 0 none)
 

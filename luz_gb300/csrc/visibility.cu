@@ -83,8 +83,8 @@ __global__ void __launch_bounds__(256, 4) shadow_raygen_kernel(SceneVis S, VisCo
                     for (uint32_t k = 0; k < cnt; ++k) {
                         const uint32_t leaf = __shfl_sync(full, my_leaf, k), cut = __shfl_sync(full, my_cut, k);
                         if (ok && leaf_overlaps(r, S.leaf_box, leaf) &&
-                            leaf_enters(S.instances + leaf, cut ? E.cuts + (size_t)(cut - 1u) * kNode4F4 : nullptr, wo, wd,
-                                        tmin, tmax))
+                            (cnt > E.cut_cap || leaf_enters(S.instances + leaf, cut ? E.cuts + (size_t)(cut - 1u) * kNode4F4 : nullptr, wo, wd,
+                                        tmin, tmax)))
                             mask |= 1u << k;
                     }
                 }
@@ -408,7 +408,6 @@ luz_status launch_visibility(luz_ctx* ctx, luz_frame* f, const luz_tlas* t, int 
     VisCounters* counters = (VisCounters*)v.counters;
     if (!shadow_chunks) LUZ_CUDA(ctx, cudaMemsetAsync(counters, 0, (size_t)z.chunks * sizeof(VisCounters), st));
     if (t->count) S.leaf_box = tlas_leaf_boxes(t);
-    const uint32_t cap = list_cap(t->count);
     if (ctx->raygen_blocks == 0) {   // resident blocks per SM: the persistent grids are one wave
         int a = 0, b = 0;
         LUZ_CUDA(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&a, cull_kernel<true, false>, kCullThreads, 0));
@@ -417,7 +416,7 @@ luz_status launch_visibility(luz_ctx* ctx, luz_frame* f, const luz_tlas* t, int 
         ctx->raygen_blocks = std::max(b, 1);
     }
     const uint32_t sms = (uint32_t)ctx->sm_count;
-    const Entries entries{v.start_lists, v.cuts};
+    const Entries entries{v.start_lists, v.cuts, cut_cap(t->count)};
     prof_begin(ctx, LUZ_KERNEL_RAYGEN);
     PatchRec* patches = (PatchRec*)v.patches;
     if (shadow_chunks) {
@@ -436,8 +435,8 @@ luz_status launch_visibility(luz_ctx* ctx, luz_frame* f, const luz_tlas* t, int 
         const RayOut R{v.rays_a, v.rays_b, v.rays_c, &n->records};
         const bool shadow = k < shadow_chunks, ao = k < ao_chunks;
         const ShaftOut A{patches, patches + z.patches, f->d_vlights, f->vlight_count, (unsigned long long)k * z.pairs,
-                         shadow ? z.pairs : 0u, cap, super_cap(t->count), v.start_lists, v.cuts, v.active, &n->groups};
-        const AoOut O{k * z.ao_patches, ao ? std::min(z.ao_patches, z.patches - k * z.ao_patches) : 0u, cap,
+                         shadow ? z.pairs : 0u, entries.cut_cap, super_cap(t->count), v.start_lists, v.cuts, v.active, &n->groups};
+        const AoOut O{k * z.ao_patches, ao ? std::min(z.ao_patches, z.patches - k * z.ao_patches) : 0u,
                       f->ao_samples < kAoMinSamples ? 0u : std::min(kAoStepsPerSample * f->ao_samples, kAoSteps),
                       v.start_lists + (size_t)z.pairs * kEntryWords, z.pairs, R};
         const uint32_t shaft_work = A.cap / kSuper, max_grid = sms * ctx->cull_blocks;
