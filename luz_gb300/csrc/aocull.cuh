@@ -117,7 +117,7 @@ struct AoShared {
     uint32_t node[kAoStack];
     float e[kAoStack];
     unsigned char slot[kAoStack];        // the nodes' instances
-    float ray[kStageWords][kStageRays];
+    float ray[kStageWords - 1][kStageRays];
 };
 
 // The AO rays of patch A.patch0 + local; called by a whole warp.
@@ -197,7 +197,7 @@ __device__ __forceinline__ void ao_patch(const SceneVis& S, const VisCommon& C, 
             if (hit && ch >= 0 && npos < kAoStack) node_st[npos] = (uint32_t)ch;
             leaves += __popc(lb);
             sp += __popc(nb);
-            if (leaves > kListCap || sp > kAoStack) { all = true; break; }
+            if (leaves > kListShort || sp > kAoStack) { all = true; break; }
             __syncwarp();
         }
     }

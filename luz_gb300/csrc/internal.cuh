@@ -26,7 +26,7 @@ constexpr int kNodeF4 = 4;
 constexpr int kTriF4 = 3;
 constexpr int32_t kEmptyChild = (int32_t)0x80000001;  // child slot with an inverted box
 constexpr int32_t kStackMarker = (int32_t)0x80000000; // two-level stack: back to the TLAS
-constexpr int kStackSize = 128;
+constexpr int kStackSize = 160;
 
 // A 4-wide node (128 B = 8 x float4), the even-depth collapse of the binary tree:
 //   f0 lo.x[4], f1 hi.x[4], f2 lo.y[4], f3 hi.y[4], f4 lo.z[4], f5 hi.z[4],

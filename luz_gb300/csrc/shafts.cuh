@@ -26,8 +26,9 @@ namespace luz {
 
 // ---------------------------------------------------------------- ray records
 // A generated ray that the traversal has to trace: (origin, tMax), (direction, pixel) and
-// (start list, slot, leaves, -): the entries of the list (Entries) that the ray's own
-// tests leave, bit k = leaf k + 1, or all bits for a start at the TLAS root. Slots of the
+// (start list, slot, leaves, more leaves): the entries of the list (Entries) that the ray's
+// own tests leave, bit k = leaf k + 1, or all bits for a start at the TLAS root; of a long
+// list, the second word's bit k = leaf k + 32 and kLongList. Slots of the
 // AO samples follow those of the shadow samples. Warps stage records in shared memory and
 // append them kStageFlush at a time, so one atomic reserves whole lines.
 struct RayOut {
@@ -37,7 +38,8 @@ struct RayOut {
     uint32_t* count;
 };
 constexpr uint32_t kFromRoot = 0xFFFFFFFFu;
-constexpr uint32_t kStageFlush = 64, kStageRays = kStageFlush + 32, kStageWords = 11;
+constexpr uint32_t kStageFlush = 64, kStageRays = kStageFlush + 32, kStageWords = 12;
+constexpr uint32_t kLongList = 0x80000000u;
 
 // Device counters of one chunk, zero before its launches.
 struct VisCounters {
@@ -52,6 +54,8 @@ struct RayStage {
     uint32_t n;
 };
 
+// kMore: with the second word of leaves.
+template <bool kMore = false>
 __device__ __forceinline__ void stage_flush(RayStage& st, const RayOut& R, uint32_t lane) {
     __syncwarp();
     const uint32_t n = min(st.n, kStageFlush);
@@ -62,24 +66,28 @@ __device__ __forceinline__ void stage_flush(RayStage& st, const RayOut& R, uint3
         const size_t at = (size_t)base + k;
         R.a[at] = make_float4(st.w[0][k], st.w[1][k], st.w[2][k], st.w[3][k]);
         R.b[at] = make_float4(st.w[4][k], st.w[5][k], st.w[6][k], st.w[7][k]);
-        R.c[at] = make_uint4(__float_as_uint(st.w[8][k]), __float_as_uint(st.w[9][k]), __float_as_uint(st.w[10][k]), 0u);
+        R.c[at] = make_uint4(__float_as_uint(st.w[8][k]), __float_as_uint(st.w[9][k]), __float_as_uint(st.w[10][k]),
+                             kMore ? __float_as_uint(st.w[kMore ? 11 : 0][k]) : 0u);
     }
     const uint32_t left = st.n - n;   // fewer than 32
-    float keep[kStageWords];
+    constexpr uint32_t rows = kMore ? kStageWords : kStageWords - 1;
+    float keep[rows];
     if (lane < left)
 #pragma unroll
-        for (uint32_t q = 0; q < kStageWords; ++q) keep[q] = st.w[q][kStageFlush + lane];
+        for (uint32_t q = 0; q < rows; ++q) keep[q] = st.w[q][kStageFlush + lane];
     __syncwarp();
     if (lane < left)
 #pragma unroll
-        for (uint32_t q = 0; q < kStageWords; ++q) st.w[q][lane] = keep[q];
+        for (uint32_t q = 0; q < rows; ++q) st.w[q][lane] = keep[q];
     st.n = left;
     __syncwarp();
 }
 
 // Appends the rays of the lanes with `live` set; every lane of the warp calls it.
+template <bool kMore = false>
 __device__ __forceinline__ void stage_rays(RayStage& st, const RayOut& R, uint32_t lane, bool live, V3 o, float tmax,
-                                           V3 d, uint32_t pix, uint32_t list, uint32_t slot, uint32_t leaves) {
+                                           V3 d, uint32_t pix, uint32_t list, uint32_t slot, uint32_t leaves,
+                                           uint32_t more = 0u) {
     const uint32_t m = __ballot_sync(0xFFFFFFFFu, live);
     if (m == 0u) return;
     if (live) {
@@ -89,9 +97,10 @@ __device__ __forceinline__ void stage_rays(RayStage& st, const RayOut& R, uint32
         st.w[8][k] = __uint_as_float(list);
         st.w[9][k] = __uint_as_float(slot);
         st.w[10][k] = __uint_as_float(leaves);
+        if (kMore) st.w[kMore ? 11 : 0][k] = __uint_as_float(more);
     }
     st.n += __popc(m);
-    if (st.n >= kStageFlush) stage_flush(st, R, lane);
+    if (st.n >= kStageFlush) stage_flush<kMore>(st, R, lane);
 }
 
 // The slab test of a TLAS leaf's box for a world-space ray (inverse direction and origin
@@ -133,15 +142,18 @@ __device__ __forceinline__ bool leaf_enters(const DevInstance* __restrict__ I, c
 constexpr uint32_t kPatch = 32;              // lit pixels per patch: one warp of ray generation
 constexpr uint32_t kGroupSamples = 4;        // samples of one light that share a group at most
 // A group's start list (Entries, vis_trace.cuh): word 0 the count (kListAll: start at the
-// TLAS root), then leaves, nearest first, and their cuts.
+// TLAS root), then leaves, nearest first, and their cuts; or a long list's leaves alone.
 constexpr uint32_t kListAll = 0xFFFFFFFFu;
 // Leaves a list may hold before its group falls back to the TLAS root, and leaves up to which
 // a list's leaves get cuts and ray generation tests the way into them: on longer lists a
 // ray's tests end at the leaf boxes. 720p over 201 cubes: lists, generation and traversal
 // 0.473 ms (15 leaves, longer ones at the root 0.479; 31 with cuts and tests 0.498), 512x512
 // over 65 0.110 (0.116), 1080p over 1024 meshes of 81,920 triangles 1.736 (1.735; 1.768). Above
-// 2048 instances the long lists keep both: 1021x573 over 8000 3.02 ms (without 3.03).
-constexpr uint32_t kListCap = 31, kCutCapSmall = 15, kCutCapLarge = 31;
+// 2048 instances lists of up to 31 keep both, and lists of up to 62, unsorted, go without:
+// 1021x573 over 8000 2.86 ms against 3.02 with 31 at most (46: 2.95); below, the room for long
+// lists in ray generation costs what they save (720p 0.454 against 0.444).
+constexpr uint32_t kListCap = 62, kListShort = kEntryCuts - 1, kCutCapSmall = 15, kCutCapLarge = 31;
+inline uint32_t list_cap(uint32_t instances) { return instances > 2048 ? kListCap : kListShort; }
 inline uint32_t cut_cap(uint32_t instances) { return instances > 2048 ? kCutCapLarge : kCutCapSmall; }
 constexpr uint32_t kSuper = 8;               // patches per block: 16x16 pixels where all are lit
 // Leaves a block's shaft may reach, and nodes it may have to visit; past either its groups
@@ -478,7 +490,7 @@ struct ShaftOut {
     uint32_t vlight_count;
     unsigned long long q0;
     uint32_t cap;                // a multiple of kSuper (0: no shadow rays here)
-    uint32_t cut_cap, super_cap;
+    uint32_t list_cap, cut_cap, super_cap;
     uint32_t* lists;             // kEntryWords per pair
     float4* cuts;                // kCutsPerPair nodes of kNode4F4 per pair
     uint4* active;               // groups to trace: (pair, first slot | samples << 16, patch, -)
@@ -563,6 +575,7 @@ __device__ __forceinline__ void shaft_block(const SceneVis& S, const ShaftOut& A
     }
     __syncwarp();
     const uint32_t patch = sb * kSuper + grp, pair = block * kSuper + grp;
+    uint32_t* list = A.lists + (size_t)pair * kEntryWords;
     const PatchRec P = A.patches[min(patch, patches - 1u)];
     const bool eff = patch < patches && !(S.cull && light_has_no_effect(lt, P));
     bool all;
@@ -581,18 +594,20 @@ __device__ __forceinline__ void shaft_block(const SceneVis& S, const ShaftOut& A
             const bool in = shaft_reaches(s, lo, hi, t0) && base + c < sn && eff;
             const uint32_t sub = (__ballot_sync(full, in) >> g4) & 15u;
             const uint32_t pos = cnt + __popc(sub & ((1u << c) - 1u));
-            if (in && pos < kEntryCuts) {
+            if (in && pos < kListShort) {
                 sm.leaf[grp][pos] = leaf;
                 sm.t[grp][pos] = t0;
             }
+            if (in && pos >= kListShort && pos < A.list_cap) list[1 + pos] = leaf;   // a long list's, in place
             cnt += __popc(sub);
         }
     }
-    all = all || cnt > kListCap;
+    all = all || cnt > A.list_cap;
     if (all) cnt = 0;
     __syncwarp();
-    // leaves by their entry parameter, nearest first
-    for (uint32_t i = c; i < cnt; i += 4) {
+    // leaves by their entry parameter, nearest first (long lists as they came)
+    const bool longer = cnt > kListShort;
+    for (uint32_t i = c; i < cnt && !longer; i += 4) {
         const float t = sm.t[grp][i];
         uint32_t rank = 0;
         for (uint32_t k = 0; k < cnt; ++k) rank += sm.t[grp][k] < t || (sm.t[grp][k] == t && k < i);
@@ -601,7 +616,7 @@ __device__ __forceinline__ void shaft_block(const SceneVis& S, const ShaftOut& A
     __syncwarp();
     // The leaves of a long list are entered at their BLAS's root.
     const uint32_t descend = cnt <= A.cut_cap ? cnt : 0u;
-    for (uint32_t i = descend + c; i < cnt; i += 4) sm.t[grp][i] = __uint_as_float(0u);
+    for (uint32_t i = descend + c; i < cnt && !longer; i += 4) sm.t[grp][i] = __uint_as_float(0u);
     // The warp's (patch, leaf) entries, eight at a time: entry e belongs to the group g with
     // first[g] <= e < first[g + 1].
     uint32_t cuts = 0;               // of the warp
@@ -700,23 +715,22 @@ __device__ __forceinline__ void shaft_block(const SceneVis& S, const ShaftOut& A
         if (e < total && c == 0) sm.t[own][i] = __uint_as_float(use ? cut : 0xFFFFFFFFu);
     }
     __syncwarp();
-    uint32_t* list = A.lists + (size_t)pair * kEntryWords;
-    const uint32_t most = __reduce_max_sync(full, cnt);
+    const uint32_t most = min(__reduce_max_sync(full, cnt), kListShort);
     uint32_t kept = 0;
     for (uint32_t base = 0; base < most; base += 4) {
-        const uint32_t cut = base + c < cnt ? __float_as_uint(sm.t[grp][base + c]) : 0xFFFFFFFFu;
+        const uint32_t cut = base + c < min(cnt, kListShort) ? (longer ? 0u : __float_as_uint(sm.t[grp][base + c])) : 0xFFFFFFFFu;
         const bool in = cut != 0xFFFFFFFFu;
         const uint32_t sub = (__ballot_sync(full, in) >> g4) & 15u;
         const uint32_t pos = kept + __popc(sub & ((1u << c) - 1u));
         if (in) {
-            list[1 + pos] = sm.order[grp][base + c];
-            list[kEntryCuts + pos] = cut;
+            list[1 + pos] = longer ? sm.leaf[grp][base + c] : sm.order[grp][base + c];
+            if (!longer) list[kEntryCuts + pos] = cut;
         }
         kept += __popc(sub);
     }
-    if (c == 0) list[0] = all ? kListAll : kept;
+    if (c == 0) list[0] = all ? kListAll : (longer ? cnt : kept);
     // One entry of the active list per surviving pair, one atomic per warp.
-    const bool trace = c == 0 && eff && (all || kept > 0);
+    const bool trace = c == 0 && eff && (all || kept > 0);   // (a long list keeps all)
     const uint32_t m = __ballot_sync(full, trace);
     if (m) {
         uint32_t base = 0;

@@ -46,14 +46,15 @@ constexpr size_t kStackBytes = (size_t)kVisThreads * kSmemStack * 4;
 // Entries of a start list (visibility_kernel): a stacked TLAS leaf ~(kEntryFlag | k) is
 // leaf k of the ray's list, entered at its cut, a 4-wide node outside the BLAS whose
 // children are nodes and triangles of it; kCutNode is that node's index on the way in.
-constexpr uint32_t kEntryFlag = 0x40000000u;   // leaf indices stay below 2^24
+constexpr uint32_t kEntryFlag = 0x40000000u, kEntryLong = 0x20000000u;   // leaf indices stay below 2^24
 constexpr int kCutNode = 0x7FFFFFFF;
 struct Entries {
     const uint32_t* lists;       // words per list: kEntryWords
     const float4* cuts;
     uint32_t cut_cap;            // lists of more leaves have no cuts (shafts.cuh)
 };
-constexpr uint32_t kEntryWords = 64, kEntryCuts = 32;   // words 1..31 leaves, 32..62 cuts (index + 1, 0 none)
+constexpr uint32_t kEntryWords = 64, kEntryCuts = 32;   // words 1..31 leaves, 32..62 cuts (index + 1, 0 none),
+                                                        // or 1..62 leaves (a long list)
 
 // Hot per-lane state (registers).
 struct LaneRay {
@@ -258,7 +259,8 @@ constexpr uint32_t kWaitEntries = 12, kWaitTris = 12, kWaitNodes = 6;
 // ray (kRayStepCap unless a debug cap is set) is charged `steps` per call, so a ray
 // ends after at most step_cap + steps; a ray that reaches it ends unoccluded (shadow)
 // or as a miss (AO) and raises LUZ_DEV_TRAVERSAL_CAP.
-template <bool kStats, bool kStaged, bool kEntries = false>
+// kEntries: 0 no start lists, 1 lists of up to 31 leaves, 2 long lists as well.
+template <bool kStats, bool kStaged, int kEntries = 0>
 __device__ __forceinline__ void run_steps(LaneRay& r, const Cold& c, bool& active, const float4* smem_tlas,
                                           uint32_t staged, const float4* tlas, const DevInstance* insts,
                                           uint32_t* s_stack, int* lstack, uint32_t steps, uint32_t step_cap,
@@ -333,9 +335,9 @@ __device__ __forceinline__ void run_steps(LaneRay& r, const Cold& c, bool& activ
             uint32_t leaf = (uint32_t)~r.node;
             int first = 0;
             if (kEntries && (leaf & kEntryFlag)) {
-                const uint32_t* e = en.lists + (size_t)__float_as_uint(c[kList]) * kEntryWords + (leaf & (kEntryCuts - 1u));
+                const uint32_t* e = en.lists + (size_t)__float_as_uint(c[kList]) * kEntryWords + (leaf & (kEntryWords - 1u));
+                const uint32_t cut = kEntries > 1 && (leaf & kEntryLong) ? 0u : __ldg(e + kEntryCuts - 1);
                 leaf = __ldg(e);
-                const uint32_t cut = __ldg(e + kEntryCuts - 1);
                 if (cut) {
                     first = kCutNode;
                     c[kCut] = __uint_as_float(cut - 1u);

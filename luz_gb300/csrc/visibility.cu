@@ -42,12 +42,14 @@ namespace luz {
 // leaf 0.29), 4K 13.0 -> 10.95 ms; the traversal that found the same on partly filled warps
 // took 0.28 ms longer.
 constexpr uint32_t kRaygenTake = 4;
+// kLong: with lists of more than kListShort leaves.
+template <bool kLong>
 __global__ void __launch_bounds__(256, 4) shadow_raygen_kernel(SceneVis S, VisCommon C, Entries E,
                                                                const uint4* __restrict__ active,
                                                                const uint32_t* __restrict__ active_count,
                                                                uint32_t* tickets, RayOut R) {
     chain_wait();
-    __shared__ float s_ray[8][kStageWords][kStageRays];
+    __shared__ float s_ray[8][kLong ? kStageWords : kStageWords - 1][kStageRays];
     const uint32_t full = 0xFFFFFFFFu;
     const uint32_t lit = *S.lit_count, lane = threadIdx.x & 31, n = *active_count;
     RayStage stage{s_ray[threadIdx.x >> 5], 0u};
@@ -64,7 +66,10 @@ __global__ void __launch_bounds__(256, 4) shadow_raygen_kernel(SceneVis S, VisCo
             const uint32_t cnt = __ldg(list);
             // lane k: leaf k of the list and its cut
             const bool has = cnt != kListAll && lane < cnt;
-            const uint32_t my_leaf = has ? __ldg(list + 1 + lane) : 0u, my_cut = has ? __ldg(list + kEntryCuts + lane) : 0u;
+            const bool longer = kLong && cnt != kListAll && cnt > kListShort;
+            // (of a long list the leaves from the 33rd on in place of the cuts)
+            const uint32_t my_leaf = has ? __ldg(list + 1 + lane) : 0u;
+            const uint32_t my_cut = (longer ? lane + 32 < cnt : has) ? __ldg(list + kEntryCuts + (longer ? 1u : 0u) + lane) : 0u;
             for (uint32_t s = 0; s < samples; ++s) {
                 V3 wo{0.f, 0.f, 0.f}, wd{0.f, 0.f, 1.f};
                 float tmin = 0.f, tmax = 0.f;
@@ -72,7 +77,7 @@ __global__ void __launch_bounds__(256, 4) shadow_raygen_kernel(SceneVis S, VisCo
                 bool record_hit = true;
                 uint32_t pix = 0;
                 const bool ok = j < lit && gen_ray(S, C, first + s, j, wo, wd, tmin, tmax, out, record_hit, pix);
-                uint32_t mask = cnt == kListAll ? kFromRoot : 0u;
+                uint32_t mask = cnt == kListAll ? kFromRoot : 0u, more = 0u;
                 if (cnt != kListAll && __any_sync(full, ok)) {
                     LaneRay r;
                     r.tmin = tmin;
@@ -80,7 +85,14 @@ __global__ void __launch_bounds__(256, 4) shadow_raygen_kernel(SceneVis S, VisCo
                     r.idir = safe_inv(wd);
                     set_origin(r, wo);
                     near_planes(r);
-                    for (uint32_t k = 0; k < cnt; ++k) {
+                    if (longer) {   // leaf boxes alone
+                        more = kLongList;
+                        for (uint32_t k = 0; k < cnt; ++k) {
+                            const uint32_t leaf = __shfl_sync(full, k < 32 ? my_leaf : my_cut, k & 31);
+                            if (ok && leaf_overlaps(r, S.leaf_box, leaf)) (k < 31 ? mask : more) |= 1u << (k < 31 ? k : k - 31);
+                        }
+                    }
+                    for (uint32_t k = 0; k < cnt && !longer; ++k) {
                         const uint32_t leaf = __shfl_sync(full, my_leaf, k), cut = __shfl_sync(full, my_cut, k);
                         if (ok && leaf_overlaps(r, S.leaf_box, leaf) &&
                             (cnt > E.cut_cap || leaf_enters(S.instances + leaf, cut ? E.cuts + (size_t)(cut - 1u) * kNode4F4 : nullptr, wo, wd,
@@ -88,11 +100,11 @@ __global__ void __launch_bounds__(256, 4) shadow_raygen_kernel(SceneVis S, VisCo
                             mask |= 1u << k;
                     }
                 }
-                stage_rays(stage, R, lane, ok && mask != 0u, wo, tmax, wd, pix, a.x, first + s, mask);
+                stage_rays<kLong>(stage, R, lane, ok && (mask | (more & ~kLongList)) != 0u, wo, tmax, wd, pix, a.x, first + s, mask, more);
             }
         }
     }
-    if (stage.n) stage_flush(stage, R, lane);
+    if (stage.n) stage_flush<kLong>(stage, R, lane);
 }
 
 // The rays of a frame that have something to trace (the counting trace's figure: shafts
@@ -118,7 +130,8 @@ __global__ void __launch_bounds__(256) count_rays_kernel(SceneVis S, VisCommon C
 
 // Traversal of one chunk's ray records (one scene; the TLAS top may be staged in shared
 // memory). Shared memory: staged TLAS nodes, then the stacks, then the cold ray state.
-template <bool kStats, bool kStaged>
+// kLong: with lists of more than kListShort leaves.
+template <bool kStats, bool kStaged, bool kLong = true>
 __global__ void __launch_bounds__(kVisThreads, LUZ_VIS_MIN_BLOCKS)
 visibility_kernel(SceneVis S, VisCommon C, Entries E, RayOut R, unsigned long long* stats) {
     chain_wait();
@@ -160,11 +173,16 @@ visibility_kernel(SceneVis S, VisCommon C, Entries E, RayOut R, unsigned long lo
                     // The leaves its tests left, the nearest first: it starts at the nearest,
                     // the others stacked.
                     c[kList] = __uint_as_float(q.x);
-                    r.node = ~(int)(kEntryFlag | (uint32_t)__ffs(q.z));
-                    for (uint32_t m = q.z & (q.z - 1u); m;) {
-                        const uint32_t top = 31u - __clz(m);
-                        m ^= 1u << top;
-                        const int e = ~(int)(kEntryFlag | (top + 1u));
+                    const uint32_t flag = kEntryFlag | (kLong && q.w ? kEntryLong : 0u);
+                    uint32_t lo = q.z, hi = kLong ? q.w & ~kLongList : 0u;
+                    r.node = ~(int)(flag | (lo ? (uint32_t)__ffs(lo) : 31u + (uint32_t)__ffs(hi)));
+                    if (lo) lo &= lo - 1u;
+                    else hi &= hi - 1u;
+                    while (lo | hi) {
+                        uint32_t top;
+                        if (hi) { top = 63u - __clz(hi); hi ^= 1u << (top - 32u); }
+                        else { top = 32u - __clz(lo); lo ^= 1u << (top - 1u); }
+                        const int e = ~(int)(flag | top);
                         if (r.sp < kSmemStack) s_stack[r.sp * 32] = (uint32_t)e;
                         else lstack[r.sp - kSmemStack] = e;
                         ++r.sp;
@@ -173,7 +191,7 @@ visibility_kernel(SceneVis S, VisCommon C, Entries E, RayOut R, unsigned long lo
             }
         }
         if (exhausted && __ballot_sync(full, active) == 0) break;
-        run_steps<kStats, kStaged, true>(r, c, active, smem, staged, S.tlas_nodes, S.instances, s_stack, lstack,
+        run_steps<kStats, kStaged, kLong ? 2 : 1>(r, c, active, smem, staged, S.tlas_nodes, S.instances, s_stack, lstack,
                                          C.steps, C.step_cap, err, cnt, E);
     }
     if (err) atomicOr(C.status, err);
@@ -391,7 +409,7 @@ luz_status launch_visibility(luz_ctx* ctx, luz_frame* f, const luz_tlas* t, int 
     size_t smem = (size_t)staged * kNode4F4 * 16 + kStackBytes + kColdBytes;
     static DeviceSetup setup;   // the traversal kernels' shared-memory limit
     s = device_setup(setup, setup_generation(), smem, [&]() -> luz_status {
-        const void* fns[4] = {(const void*)visibility_kernel<false, false>, (const void*)visibility_kernel<true, false>,
+        const void* fns[5] = {(const void*)visibility_kernel<false, false, false>, (const void*)visibility_kernel<false, false>, (const void*)visibility_kernel<true, false>,
                               (const void*)visibility_kernel<false, true>, (const void*)visibility_kernel<true, true>};
         for (const void* fn : fns)
             LUZ_CUDA(ctx, cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
@@ -411,7 +429,7 @@ luz_status launch_visibility(luz_ctx* ctx, luz_frame* f, const luz_tlas* t, int 
     if (ctx->raygen_blocks == 0) {   // resident blocks per SM: the persistent grids are one wave
         int a = 0, b = 0;
         LUZ_CUDA(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&a, cull_kernel<true, false>, kCullThreads, 0));
-        LUZ_CUDA(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, shadow_raygen_kernel, 256, 0));
+        LUZ_CUDA(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, shadow_raygen_kernel<true>, 256, 0));
         ctx->cull_blocks = std::max(a, 1);
         ctx->raygen_blocks = std::max(b, 1);
     }
@@ -435,7 +453,7 @@ luz_status launch_visibility(luz_ctx* ctx, luz_frame* f, const luz_tlas* t, int 
         const RayOut R{v.rays_a, v.rays_b, v.rays_c, &n->records};
         const bool shadow = k < shadow_chunks, ao = k < ao_chunks;
         const ShaftOut A{patches, patches + z.patches, f->d_vlights, f->vlight_count, (unsigned long long)k * z.pairs,
-                         shadow ? z.pairs : 0u, entries.cut_cap, super_cap(t->count), v.start_lists, v.cuts, v.active, &n->groups};
+                         shadow ? z.pairs : 0u, list_cap(t->count), entries.cut_cap, super_cap(t->count), v.start_lists, v.cuts, v.active, &n->groups};
         const AoOut O{k * z.ao_patches, ao ? std::min(z.ao_patches, z.patches - k * z.ao_patches) : 0u,
                       f->ao_samples < kAoMinSamples ? 0u : std::min(kAoStepsPerSample * f->ao_samples, kAoSteps),
                       v.start_lists + (size_t)z.pairs * kEntryWords, z.pairs, R};
@@ -455,7 +473,7 @@ luz_status launch_visibility(luz_ctx* ctx, luz_frame* f, const luz_tlas* t, int 
             }
         }
         if (shadow) {
-            chain(shadow_raygen_kernel, std::min((z.pairs + 7) / 8, sms * ctx->raygen_blocks), 256, 0, st, S, C, entries, v.active, &n->groups, &n->raygen_tickets, R);
+            chain(A.list_cap > kListShort ? shadow_raygen_kernel<true> : shadow_raygen_kernel<false>, std::min((z.pairs + 7) / 8, sms * ctx->raygen_blocks), 256, 0, st, S, C, entries, v.active, &n->groups, &n->raygen_tickets, R);
             LUZ_LAUNCHED(ctx, "shadow_raygen_kernel");
         }
         prof_end(ctx);
@@ -466,7 +484,8 @@ luz_status launch_visibility(luz_ctx* ctx, luz_frame* f, const luz_tlas* t, int 
         } else {
             prof_begin(ctx, LUZ_KERNEL_TRAVERSAL);
             if (staged) chain(visibility_kernel<false, true>, grid, 256, smem, st, S, C, entries, R, nullptr);
-            else chain(visibility_kernel<false, false>, grid, 256, smem, st, S, C, entries, R, nullptr);
+            else chain(A.list_cap > kListShort ? visibility_kernel<false, false, true> : visibility_kernel<false, false, false>, grid,
+                       256, smem, st, S, C, entries, R, nullptr);
             prof_end(ctx);
             LUZ_LAUNCHED(ctx, "visibility_kernel");
         }
