@@ -64,8 +64,8 @@ __device__ __forceinline__ bool elevation(const float c[3], const float h[3], co
     }
     float r;   // 1 / sqrt(d2) to 2^-22, +inf for 0
     asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(d2));
-    const float num = sup - on;
-    e = num > 0.0f ? fminf(num * (r * scale), 1e9f) : -1.0f;
+    const float num = sup - on;   // NaN where an infinite plane meets a zero of n, or the box has one: no bound
+    e = num <= 0.0f ? -1.0f : fminf(num * (r * scale), 1e9f);
     return d2 <= reach2;
 }
 
