@@ -178,14 +178,16 @@ __device__ __forceinline__ void ao_patch(const SceneVis& S, const VisCommon& C, 
             const uint32_t take = min(sp, 8u);
             sp -= take;
             int ch = kEmptyChild;
-            bool hit = false;
+            bool hit = false, odd = false;
             float e = -1.0f;
             if (g < take) {
                 const float* f = reinterpret_cast<const float*>(S.tlas_nodes + (size_t)node_st[sp + g] * kNode4F4) + ch_i;
                 const float lo[3] = {__ldg(f), __ldg(f + 8), __ldg(f + 16)}, hi[3] = {__ldg(f + 4), __ldg(f + 12), __ldg(f + 20)};
                 ch = __float_as_int(__ldg(f + 24));
                 hit = ch != kEmptyChild && elevation(c, h, nn, on, 1.0f + 0x1p-10f, reach2, lo, hi, e);
+                odd = box_has_nan(lo, hi);
             }
+            if (__any_sync(full, odd)) { all = true; break; }   // its other boxes may not nest: the rays start at the root
             __syncwarp();
             const uint32_t lb = __ballot_sync(full, hit && ch < 0), nb = __ballot_sync(full, hit && ch >= 0);
             const uint32_t lpos = leaves + __popc(lb & lt_mask), npos = sp + __popc(nb & lt_mask);
@@ -215,7 +217,7 @@ __device__ __forceinline__ void ao_patch(const SceneVis& S, const VisCommon& C, 
             const uint4 meta = __ldg(reinterpret_cast<const uint4*>(&I->custom_index));
             use = (meta.y & 0xFFu) != 0 && meta.w > 0;
             AoInstance rec;
-            good = ao_instance(I, leaf, c, h, n, on, reach, rec);
+            good = blas_nests(I) && ao_instance(I, leaf, c, h, n, on, reach, rec);
             if (use && good) sm.inst[lane] = rec;
         }
         if (__any_sync(full, use && !good)) open = false;

@@ -16,6 +16,10 @@
 //
 // The result is that of tracing every ray from the TLAS root: boxes are conservative, and
 // the shaft's boxes are grown past the rounding of the ray origins, ends and transforms.
+// A start below the root also needs every box to lie inside those above it. Unions with a
+// NaN (a vertex or a transform that is none) can lose a box, so that a trace from the root
+// never comes to it: where a NaN is met among the TLAS's boxes, or the mesh has a vertex that
+// is not finite, the rays start at that root instead.
 #pragma once
 #include "raygen.cuh"
 #include "traverse.cuh"
@@ -339,6 +343,16 @@ __device__ __forceinline__ bool make_shaft(Shaft& s, const float c[3], const flo
     return ok && finite3(n) && fabsf(on) <= 1e18f && fabsf(en) <= 1e18f;
 }
 
+__device__ __forceinline__ bool box_has_nan(const float lo[3], const float hi[3]) {
+    const float l = (lo[0] + lo[1]) + lo[2], h = (hi[0] + hi[1]) + hi[2];
+    return l != l || h != h;
+}
+// Whether the boxes of an instance's BLAS nest: its bounding sphere is finite, as every vertex
+// then is (blas_radius_kernel).
+__device__ __forceinline__ bool blas_nests(const DevInstance* __restrict__ I) {
+    return __ldg(&I->sphere.w) < __int_as_float(0x7f800000);
+}
+
 __device__ __forceinline__ float dot_max(const float* lo, const float* hi, const float a[3], const float b[3]) {
     float s = 0.f;   // the largest dot product of a vector in [lo, hi] and one in [a, b]
 #pragma unroll
@@ -557,14 +571,16 @@ __device__ __forceinline__ void shaft_block(const SceneVis& S, const ShaftOut& A
                 const uint32_t take = min(sp, 8u);
                 sp -= take;
                 int ch = kEmptyChild;
-                bool hit = false;
+                bool hit = false, odd = false;
                 if (grp < take) {
                     const float* f = reinterpret_cast<const float*>(S.tlas_nodes + (size_t)stack[sp + grp] * kNode4F4) + c;
                     const float lo[3] = {__ldg(f), __ldg(f + 8), __ldg(f + 16)}, hi[3] = {__ldg(f + 4), __ldg(f + 12), __ldg(f + 20)};
                     ch = __float_as_int(__ldg(f + 24));
                     float t0;
                     hit = shaft_reaches(s, lo, hi, t0) && ch != kEmptyChild;
+                    odd = box_has_nan(lo, hi);
                 }
+                if (__any_sync(full, odd)) { far = true; break; }
                 const uint32_t lb = __ballot_sync(full, hit && ch < 0), nb = __ballot_sync(full, hit && ch >= 0);
                 if (sn + __popc(lb) > A.super_cap || sp + __popc(nb) > kSuperStack) { far = true; break; }
                 if (hit && ch < 0) super[sn + __popc(lb & lt_mask)] = (uint32_t)~ch;
@@ -644,7 +660,7 @@ __device__ __forceinline__ void shaft_block(const SceneVis& S, const ShaftOut& A
             const uint4 meta = __ldg(reinterpret_cast<const uint4*>(&I->custom_index));
             use = (meta.y & 0xFFu) != 0 && meta.w > 0;   // else never hit
             const float4* wp = reinterpret_cast<const float4*>(I->w2o);
-            shaft = use && meta.w > kCutPrims && object_shaft(sm.box[own], __ldg(wp), __ldg(wp + 1), __ldg(wp + 2), so);
+            shaft = use && meta.w > kCutPrims && blas_nests(I) && object_shaft(sm.box[own], __ldg(wp), __ldg(wp + 1), __ldg(wp + 2), so);
             nodes = I->nodes4;
         }
         float lx = inf, hx = -inf, ly = inf, hy = -inf, lz = inf, hz = -inf;   // this lane's slot

@@ -1,4 +1,4 @@
-"""Meshes with a vertex that is infinite: the group bounds (shafts, horizons)
+"""Meshes with a vertex that is infinite or not a number: the group bounds (shafts, horizons)
 leave every hit/miss bit as a trace of each ray from the TLAS root gives it, also for the
 finite triangles that share the boxes above such a vertex."""
 import numpy as np
@@ -9,11 +9,13 @@ from tests.pathutil import bits_mismatch, oracle_frame, oracle_scene
 
 pytestmark = pytest.mark.gpu
 
-INF = np.float32(np.inf)
+INF, NAN = np.float32(np.inf), np.float32(np.nan)
 BAD = {"none": [],
        "inf_x": [[(0, 5, 0), (0, 5, 1), (INF, 5, 0)]],
        "inf_y": [[(0, 0.2, 0), (1, INF, 0), (0, 0.2, 1)]],
-       "inf_all": [[(-INF, 5, 0), (-INF, 5, 1), (-INF, 6, 0)]]}
+       "inf_all": [[(-INF, 5, 0), (-INF, 5, 1), (-INF, 6, 0)]],
+       "nan_last": [[(2, 0.3, 0), (2, 0.3, 1), (NAN, 0.3, 0)], [(-2, 0.4, 2), (-2, 0.4, 1), (0, NAN, NAN)]],
+       "nan_first": [[(NAN, 0.3, 2), (2, 0.3, 1), (1, 0.3, 0)], [(0, NAN, 2), (NAN, 0.4, 1), (-1, 1, NAN)]]}
 
 
 def _quads(y, xs, z0, z1, n, up):
