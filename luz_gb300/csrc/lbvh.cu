@@ -229,13 +229,12 @@ onesweep_pass_kernel(const unsigned long long* __restrict__ kin, const uint32_t*
     __shared__ uint32_t s_vals[kSortTile];
 
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    // Tiles in the order the blocks start, so that a look-back waits only on blocks that run;
-    // a grid that fits the chip at a block per SM needs no order.
-    const bool ordered = gridDim.x > kSortResident;
-    if (ordered && tid == 0) s_tile = atomicAdd(tile_counter, 1u);
+    // Tiles in the order the blocks start, so that a look-back waits only on blocks that run,
+    // however few of them the chip has room for beside other streams' kernels.
+    if (tid == 0) s_tile = atomicAdd(tile_counter, 1u);
     for (int i = tid; i < kSortWarps * kRadix; i += kSortThreads) (&s_warp_hist[0][0])[i] = 0;
     __syncthreads();
-    const uint32_t tile = ordered ? s_tile : blockIdx.x;
+    const uint32_t tile = s_tile;
     const uint32_t base = tile * kSortTile;
 
     unsigned long long key[kSortItems];

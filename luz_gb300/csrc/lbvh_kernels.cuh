@@ -34,7 +34,6 @@ constexpr uint32_t kFlagAggregate = 1u << 30;
 constexpr uint32_t kFlagPrefix = 2u << 30;
 constexpr uint32_t kValueMask = (1u << 30) - 1;
 constexpr uint32_t kLookbackSpinLimit = 1u << 22;
-constexpr uint32_t kSortResident = 128;   // blocks that are resident together on the chip
 constexpr int kLookback = 8;      // tiles a look-back reads at a time
 
 // Rows of 256 primitives one block of blas_bounds_kernel reduces (launch 256 threads and
