@@ -213,7 +213,8 @@ uint64_t luz_ctx_launch_count(const luz_ctx* ctx);
 /* Debug knob, off by default (no counterpart in the reference): the traversal steps a
  * traversed shadow / AO ray may take before the visibility kernel ends it (counted as not
  * occluded, AO: a miss) and raises LUZ_DEV_TRAVERSAL_CAP; 0 restores the library's cap
- * (2^22 steps). For testing that a cap which runs out ends the kernel with a status
+ * (2^22 steps). Counted in eights, a cap below eight ending every ray at once, and looked
+ * at every luz_vis_tuning.steps steps, so a ray may pass it by as many. For testing that a cap which runs out ends the kernel with a status
  * instead of a hang. */
 luz_status luz_ctx_set_debug_step_cap(luz_ctx* ctx, uint32_t steps);
 /* Uses `stream` (a cudaStream_t) for all later work; NULL = the context's own. */

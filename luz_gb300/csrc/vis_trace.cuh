@@ -19,7 +19,7 @@ constexpr int kVisThreads = 256;
 constexpr int kSmemStack = 16;                      // shared-memory stack entries per lane
 constexpr int kLocalStack = kStackSize - kSmemStack;
 constexpr uint32_t kRayStepCap = 1u << 22;
-constexpr uint32_t kMinCharge = 8;                  // a cap below this many steps ends every ray at once
+constexpr uint32_t kStepGrain = 8;                  // steps a cap is counted in
 
 // Ray state that traversal touches only when it enters or leaves a BLAS, tests a
 // triangle or finishes lives in shared memory, one 32-bit field per row of
@@ -255,17 +255,18 @@ constexpr uint32_t kWaitEntries = 12, kWaitTris = 12, kWaitNodes = 6;
 
 // Up to `steps` traversal steps of one lane's ray; clears `active` when it ends.
 // tlas / insts: the scene's TLAS nodes and instances (kernel parameters in the
-// single-scene kernel, the lane's own scene in the batched one). The step cap of a
-// ray (kRayStepCap unless a debug cap is set) is charged `steps` per call, so a ray
-// ends after at most step_cap + steps; a ray that reaches it ends unoccluded (shadow)
-// or as a miss (AO) and raises LUZ_DEV_TRAVERSAL_CAP.
+// single-scene kernel, the lane's own scene in the batched one). A ray's budget counts the
+// steps that it takes itself, not those it waits; it is looked at once per call, and a ray
+// whose next kStepGrain steps are past the cap (kRayStepCap unless a debug cap is set) ends
+// unoccluded (shadow) or as a miss (AO) and raises LUZ_DEV_TRAVERSAL_CAP: after fewer than
+// step_cap + steps of them, and never where it fits the cap in whole grains.
 // kEntries: 0 no start lists, 1 lists of up to 31 leaves, 2 long lists as well.
 template <bool kStats, bool kStaged, int kEntries = 0>
 __device__ __forceinline__ void run_steps(LaneRay& r, const Cold& c, bool& active, const float4* smem_tlas,
                                           uint32_t staged, const float4* tlas, const DevInstance* insts,
                                           uint32_t* s_stack, int* lstack, uint32_t steps, uint32_t step_cap,
                                           uint32_t& err, TraceCounters& cnt, const Entries& en = Entries{}) {
-    if (active && (r.budget += steps) + (steps < kMinCharge ? kMinCharge - steps : 0u) > step_cap) {
+    if (active && (r.budget & ~(kStepGrain - 1u)) + kStepGrain > step_cap) {
         err |= LUZ_DEV_TRAVERSAL_CAP;
         finish_ray(c, active, false);
     }
@@ -282,6 +283,7 @@ __device__ __forceinline__ void run_steps(LaneRay& r, const Cold& c, bool& activ
             // 4-wide node: test the four child boxes, continue with the nearest hit
             // child and push the other hits. Empty slots hold inverted boxes, which
             // no ray overlaps.
+            ++r.budget;
             if (kStats) { if (r.in_blas) cnt.blas_nodes++; else cnt.tlas_nodes++; }
             const float4* np = kStaged ? (r.in_blas ? r.nb : ((uint32_t)r.node < staged ? smem_tlas : tlas)) : r.nb;
             np += (size_t)r.node * kNode4F4;
@@ -331,6 +333,7 @@ __device__ __forceinline__ void run_steps(LaneRay& r, const Cold& c, bool& activ
         } else if (at_leaf && !r.in_blas && do_entries) {
             // Instance leaf: entered unless its mask or BLAS is empty or the ray
             // segment provably misses the BLAS's bounding sphere.
+            ++r.budget;
             if (kStats) cnt.instances++;
             uint32_t leaf = (uint32_t)~r.node;
             int first = 0;
@@ -373,6 +376,7 @@ __device__ __forceinline__ void run_steps(LaneRay& r, const Cold& c, bool& activ
                 pop = true;
             }
         } else if (at_leaf && r.in_blas && do_tris) {
+            ++r.budget;
             if (kStats) cnt.tris++;
             const float4* bt = reinterpret_cast<const float4*>((unsigned long long)__float_as_uint(c[kBtLo]) |
                                                                ((unsigned long long)__float_as_uint(c[kBtHi]) << 32));
