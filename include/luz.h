@@ -510,9 +510,9 @@ void* luz_frame_plane_device_ptr(luz_frame* frame, int32_t plane);
 
 /* ------------------------------------------------------------------ batches
  * Many independent scenes of uneven size as one unit (no counterpart in the
- * reference, which renders one scene per frame). A render takes one of two forms. Scenes
- * of 200,000 pixels and more on average, or up to two scenes of any size, run in lanes:
- * every pass of a scene as the launches of a single frame, the scenes spread over up to
+ * reference, which renders one scene per frame). A render takes one of two forms, the
+ * faster one unless luz_batch_set_fused chooses. Scenes of 200,000 pixels and more on
+ * average, or up to two scenes of any size, run in lanes: every pass of a scene as the launches of a single frame, the scenes spread over up to
  * eight streams that fork from the context's and join it again; a lane's buffers are those
  * of a single frame's trace, for its largest scene. Many small scenes run as ONE
  * persistent launch (the frame kernel) over every scene: the per-frame TLAS builds,
@@ -522,9 +522,8 @@ void* luz_frame_plane_device_ptr(luz_frame* frame, int32_t plane);
  * before them, each wait bounded (LUZ_DEV_BATCH_QUEUE when one gives up). The meshes'
  * BLASes are built before, once, by luz_blas_build_batch (the reference builds them
  * once at load, GPUScene.cpp:108-138). The frame kernel takes scenes of up to 4096
- * instances and 688 lights; a batch with a larger scene always runs in lanes, which
- * luz_batch_set_fused(ctx, b, 0) also selects. Both forms give the same
- * planes bit for bit. Scene constants and instances are uploaded / packed once at
+ * instances and 688 lights; a batch with a larger scene always runs in lanes. Both
+ * forms give the same planes bit for bit. Scene constants and instances are uploaded / packed once at
  * creation (the arrays may be freed after luz_batch_create); luz_batch_capture records
  * a render as one CUDA graph that luz_batch_replay launches; luz_batch_autotune picks
  * the traversal launch shape (ray-batch refill size, steps between refills, CTAs per
@@ -554,10 +553,10 @@ luz_status luz_batch_capture(luz_ctx* ctx, luz_batch* b, int32_t frame_index);
 luz_status luz_batch_replay(luz_ctx* ctx, luz_batch* b);
 luz_status luz_batch_autotune(luz_ctx* ctx, luz_batch* b, uint32_t reps, luz_vis_tuning* chosen,
                               float* best_ms);
-/* on = 1: renders run the frame kernel where it is the faster form (LUZ_ERR_LIMIT when a
- * scene does not fit it); on = 0: lanes. Drops a captured graph. */
+/* on = 1: renders run the frame kernel (LUZ_ERR_LIMIT when a scene does not fit it);
+ * on = 0: lanes. Drops a captured graph where that changes the form. */
 luz_status luz_batch_set_fused(luz_ctx* ctx, luz_batch* b, int32_t on);
-/* 1 unless the batch was set, or is left by its scenes, to lanes alone. */
+/* 1 when the batch renders with the frame kernel. */
 int32_t luz_batch_fused(const luz_batch* b);
 
 /* ------------------------------------------------------------------ denoiser

@@ -583,9 +583,9 @@ class _BorrowedFrame(Frame):
 class Batch:
     """Many scenes rendered as one unit (luz_batch_*): one batched BLAS build over the
     meshes of every scene at creation, then per render every scene's passes spread over
-    a few streams (lanes), or, for many small scenes unless set_fused(False), ONE
-    persistent launch (the frame kernel: every TLAS build, G-buffer, the traversal of all
-    scenes' rays and every light pass); optionally as one CUDA graph."""
+    a few streams (lanes), or, for many small scenes, ONE persistent launch (the frame
+    kernel: every TLAS build, G-buffer, the traversal of all scenes' rays and every light
+    pass); set_fused chooses the form; optionally as one CUDA graph."""
 
     def __init__(self, ctx: "Context", scenes: list[HostScene]):
         self.ctx, self.scenes = ctx, scenes
@@ -638,7 +638,7 @@ class Batch:
 
     @property
     def fused(self) -> bool:
-        """True where the frame kernel may run (it does where it is the faster form)."""
+        """True when renders run the frame kernel."""
         return bool(lib.luz_batch_fused(self._h))
 
     def set_fused(self, on: bool) -> None:

@@ -382,7 +382,7 @@ struct luz_batch {
     int frame_index = 0;
     // frame kernel
     bool fusable = false;            // every scene fits the frame kernel
-    bool fused = false;              // renders run the frame kernel where it is the faster form
+    bool fused = false;              // renders run the frame kernel, else lanes
     luz::FrameScene* d_fs = nullptr;
     uint32_t* d_tile_off = nullptr;
     luz::ClearItem* d_clears = nullptr;
@@ -394,7 +394,6 @@ struct luz_batch {
     std::vector<Lane> lanes;
     std::vector<uint32_t> order, lane_of;   // scenes in launch order; the lane of each scene
     cudaEvent_t fork = nullptr;
-    bool small = false;              // the frame kernel is the faster form
 };
 
 namespace luz {
@@ -449,8 +448,6 @@ static luz_status launch_frame(luz_ctx* ctx, luz_batch* b, bool stats) {
 constexpr uint64_t kLanePixels = 200000;    // mean pixels of a scene from which on the lanes are taken
 constexpr uint32_t kLaneScenes = 2;         // and scenes up to which they always are
 constexpr uint32_t kLanes = 8;
-
-static bool runs_frame_kernel(const luz_batch* b) { return b->fused && b->small; }
 
 static void drop_graph(luz_batch* b) {
     if (b->exec) cudaGraphExecDestroy(b->exec);
@@ -547,7 +544,7 @@ static luz_status launch_lanes(luz_ctx* ctx, luz_batch* b, int frame_index) {
 static luz_status batch_record(luz_ctx* ctx, luz_batch* b, int frame_index, bool stats) {
     luz_status s = set_frame_index(ctx, b, frame_index);
     if (s != LUZ_OK) return s;
-    if (runs_frame_kernel(b)) return launch_frame(ctx, b, stats);
+    if (b->fused) return launch_frame(ctx, b, stats);
     if (!stats) return launch_lanes(ctx, b, frame_index);
     for (size_t i = 0; i < b->frames.size(); ++i) {
         if ((s = launch_tlas_kernels(ctx, b->tlas[i])) != LUZ_OK) return s;
@@ -607,7 +604,6 @@ static luz_status setup_frame_kernel(luz_ctx* ctx, luz_batch* b) {
         e = cudaMemcpy(b->d_clears, clears.data(), clears.size() * sizeof(ClearItem), cudaMemcpyHostToDevice);
     if (e != cudaSuccess) return cuda_error(ctx, e, "batch frame-kernel tables");
     b->fusable = true;
-    b->fused = true;
     return LUZ_OK;
 }
 
@@ -653,10 +649,10 @@ static luz_status batch_create_body(luz_ctx* ctx, uint32_t count, const luz_batc
     if (fs != LUZ_OK) return fail(fs);
     uint64_t pixels = 0;
     for (auto* f : b->frames) pixels += f->pixels;
-    b->small = count > kLaneScenes && pixels < kLanePixels * count;
-    if (!runs_frame_kernel(b) && (fs = reserve_lanes(ctx, b)) != LUZ_OK) {
+    b->fused = b->fusable && count > kLaneScenes && pixels < kLanePixels * count;
+    if (!b->fused && (fs = reserve_lanes(ctx, b)) != LUZ_OK) {
         if (fs != LUZ_ERR_OOM || !b->fusable) return fail(fs);
-        b->small = true;   // no memory for the lanes' traces: the frame kernel needs none
+        b->fused = true;   // no memory for the lanes' traces: the frame kernel needs none
     }
     *out = b;
     return LUZ_OK;
@@ -707,7 +703,7 @@ luz_status luz_batch_capture(luz_ctx* ctx, luz_batch* b, int32_t frame_index) {
         return set_error(ctx, LUZ_ERR_INVALID, "capture needs an explicit stream");
     LUZ_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
     drop_graph(b);
-    if (!runs_frame_kernel(b)) {   // no allocation while recording
+    if (!b->fused) {   // no allocation while recording
         luz_status s = reserve_lanes(ctx, b);
         if (s != LUZ_OK) return s;
     }
@@ -762,7 +758,7 @@ luz_status luz_batch_autotune(luz_ctx* ctx, luz_batch* b, uint32_t reps, luz_vis
                 std::vector<float> ts;
                 for (uint32_t r = 0; r <= reps; ++r) {
                     cudaEventRecord(e0, ctx->stream);
-                    s = runs_frame_kernel(b) ? launch_frame(ctx, b, false) : launch_lanes(ctx, b, b->frame_index);
+                    s = b->fused ? launch_frame(ctx, b, false) : launch_lanes(ctx, b, b->frame_index);
                     if (s != LUZ_OK) return s;
                     cudaEventRecord(e1, ctx->stream);
                     LUZ_CUDA(ctx, cudaEventSynchronize(e1));
@@ -790,9 +786,11 @@ luz_status luz_batch_set_fused(luz_ctx* ctx, luz_batch* b, int32_t on) {
     if (!ctx || !b) return LUZ_ERR_INVALID;
     if (on && !b->fusable)
         return set_error(ctx, LUZ_ERR_LIMIT, "a scene of the batch does not fit the frame kernel");
+    if (!on)
+        if (luz_status s = reserve_lanes(ctx, b); s != LUZ_OK) return s;   // the form stays
     if ((on != 0) != b->fused) drop_graph(b);
     b->fused = on != 0;
-    return runs_frame_kernel(b) ? LUZ_OK : reserve_lanes(ctx, b);
+    return LUZ_OK;
 }
 
 int32_t luz_batch_fused(const luz_batch* b) { return b && b->fused ? 1 : 0; }
