@@ -501,13 +501,14 @@ static luz_status reserve_lanes(luz_ctx* ctx, luz_batch* b) {
         luz_status s = b->lanes.empty() ? make_lanes(ctx, b, count) : LUZ_OK;
         for (uint32_t i = 0; s == LUZ_OK && i < n; ++i) {
             VisScratch& v = b->lanes[b->lane_of[i]].scratch;
-            const VisScratch before = v;
+            const uint32_t moves = v.moves;
             s = reserve_visibility(ctx, b->frames[i], b->tlas[i], v);
-            if (memcmp(&before, &v, sizeof v)) drop_graph(b);   // it holds the buffers' addresses
+            if (v.moves != moves) drop_graph(b);   // it holds the buffers' addresses
         }
         if (s == LUZ_OK) return s;
         cudaGetLastError();
         LUZ_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
+        drop_graph(b);
         drop_lanes(b);
         if (s != LUZ_ERR_OOM || count <= 1) return s;
     }

@@ -190,6 +190,7 @@ struct VisScratch {
     uint4* rays_c = nullptr;
     void* counters = nullptr;             // VisCounters per chunk
     uint32_t patches_cap = 0, lists_cap = 0, pairs_cap = 0, records_cap = 0, chunks_cap = 0;
+    uint32_t moves = 0;                   // times a buffer was freed or replaced
     void release() {
         for (void* p : {patches, (void*)start_lists, (void*)cuts, (void*)active, (void*)rays_a, (void*)rays_b,
                         (void*)rays_c, counters})

@@ -355,6 +355,7 @@ static luz_status ensure_vis_buffers(luz_ctx* ctx, VisScratch& v, const VisSizes
         z.chunks <= v.chunks_cap)
         return LUZ_OK;
     LUZ_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
+    ++v.moves;
     auto again = [&](auto*& p, size_t bytes) -> cudaError_t {
         cudaFree(p);
         p = nullptr;

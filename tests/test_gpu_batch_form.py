@@ -34,3 +34,42 @@ def test_the_chosen_form_renders(sizes, default):
                 assert np.array_equal(fr.read(L.PLANE_LIGHT).view(np.uint32), p.view(np.uint32))
     finally:
         ctx.close()
+
+
+def test_a_recorded_batch_is_dropped_when_its_buffers_move():
+    """A recorded render holds the addresses of the lanes' buffers: renders in between leave it
+    valid, and one whose traces outgrow them drops it, so that a replay is refused."""
+    torch = pytest.importorskip("torch")
+    ctx = L.Context(0)
+    try:
+        ctx.set_stream(torch.cuda.Stream().cuda_stream)
+        ctx.set_blue_noise(L.blue_noise())
+        scenes = [L.HostScene(1, seed=i, width=96, height=64, ao_samples=2) for i in range(2)]
+        b = L.Batch(ctx, scenes)
+        b.set_fused(False)
+        b.render(2)
+        planes = [fr.read(L.PLANE_LIGHT).copy() for fr in b.frames]
+        b.capture(2)
+        for _ in range(3):
+            b.render(2)
+            b.replay()
+        ctx.synchronize()
+        for fr, p in zip(b.frames, planes):
+            assert np.array_equal(fr.read(L.PLANE_LIGHT).view(np.uint32), p.view(np.uint32))
+        more = scenes[0]
+        more.set_sampling(24)
+        b.frames[0].upload(more.block(), more.lights(), more.light_count, more.models(), more.instance_count)
+        b.render(2)
+        ctx.synchronize()
+        with pytest.raises(L.LuzError):
+            b.replay()
+        b.capture(2)
+        b.replay()
+        ctx.synchronize()
+        assert ctx.device_status() == 0
+        g = L.GPUScene(ctx, more)
+        g.render(2)
+        ctx.synchronize()
+        assert np.array_equal(b.frames[0].read(L.PLANE_AO_BITS), g.frame.read(L.PLANE_AO_BITS))
+    finally:
+        ctx.close()
