@@ -527,7 +527,9 @@ void* luz_frame_plane_device_ptr(luz_frame* frame, int32_t plane);
  * creation (the arrays may be freed after luz_batch_create); luz_batch_capture records
  * a render as one CUDA graph that luz_batch_replay launches; luz_batch_autotune picks
  * the traversal launch shape (ray-batch refill size, steps between refills, CTAs per
- * SM) by timing the batch's own launch. */
+ * SM) by timing the batch's own renders, the shape in force and the default among the
+ * candidates. It holds for this batch in its present form, until
+ * luz_ctx_set_vis_tuning is called; single frames keep the context's shape. */
 typedef struct luz_batch luz_batch;
 typedef struct luz_batch_scene {
     const luz_instance* instances;

@@ -394,9 +394,23 @@ struct luz_batch {
     std::vector<Lane> lanes;
     std::vector<uint32_t> order, lane_of;   // scenes in launch order; the lane of each scene
     cudaEvent_t fork = nullptr;
+    // autotuned launch shape: for the form it was timed in, until the context is given another
+    luz::VisTuning tuning{};
+    bool tuned_fused = false;
+    uint32_t tuned_at = 0;
 };
 
 namespace luz {
+
+// The batch's autotuned shape in the context's place, while it holds.
+struct TuningScope {
+    luz_ctx* ctx;
+    VisTuning of_ctx;
+    TuningScope(luz_ctx* c, const luz_batch* b) : ctx(c), of_ctx(c->vis_tuning) {
+        if (b->tuning.set && b->tuned_fused == b->fused && b->tuned_at == c->vis_tuning_changes) c->vis_tuning = b->tuning;
+    }
+    ~TuningScope() { ctx->vis_tuning = of_ctx; }
+};
 
 static luz_status set_frame_index(luz_ctx* ctx, luz_batch* b, int frame_index) {
     // The sampler frame index lives in the per-scene records (fixed inside a graph).
@@ -543,6 +557,7 @@ static luz_status launch_lanes(luz_ctx* ctx, luz_batch* b, int frame_index) {
 
 // stats: every ray traced from its TLAS root by a counting launch, in either form.
 static luz_status batch_record(luz_ctx* ctx, luz_batch* b, int frame_index, bool stats) {
+    const TuningScope scope(ctx, b);
     luz_status s = set_frame_index(ctx, b, frame_index);
     if (s != LUZ_OK) return s;
     if (b->fused) return launch_frame(ctx, b, stats);
@@ -737,45 +752,63 @@ luz_status luz_batch_replay(luz_ctx* ctx, luz_batch* b) {
     return LUZ_OK;
 }
 
-// Times a render of the batch for each candidate shape of the traversal and keeps the fastest (median of `reps` launches). Candidates: refill {8,16,32} x steps
-// {16,32,64} x CTAs per SM {2,3,4}. Drops a captured graph (its shape is stale).
+// Times a render of the batch for each candidate shape of the traversal and keeps the fastest
+// (median of `reps` launches) for the batch's renders in its present form. Candidates: the
+// shape in force and the form's default, so that the choice is never a slower one than either,
+// and refill {8,16,32} x steps {16,32,64} x CTAs per SM {2,3,4}. (The staging size keeps its
+// current value.) Drops a captured graph (its shape is stale).
 luz_status luz_batch_autotune(luz_ctx* ctx, luz_batch* b, uint32_t reps, luz_vis_tuning* chosen, float* best_ms) {
     if (!ctx || !b) return LUZ_ERR_INVALID;
     reps = std::max(reps, 1u);
     drop_graph(b);
     luz_status s = batch_record(ctx, b, b->frame_index, false);   // G-buffers and lit counts in place
     if (s != LUZ_OK) return s;
-    cudaEvent_t e0, e1;
-    LUZ_CUDA(ctx, cudaEventCreate(&e0));
-    LUZ_CUDA(ctx, cudaEventCreate(&e1));
-    const uint32_t refills[] = {8, 16, 32}, steps[] = {16, 32, 64}, ctas[] = {2, 3, 4};
-    const uint32_t base_smem = batch_tuning(ctx).smem_nodes;
-    VisTuning best{0, 0, 0, 0, 0};
+    cudaEvent_t ev[2] = {nullptr, nullptr};
+    const VisTuning of_ctx = ctx->vis_tuning;
+    VisTuning best{};
     float best_t = 3.0e38f;
-    for (uint32_t rf : refills)
-        for (uint32_t sp : steps)
-            for (uint32_t ct : ctas) {
-                ctx->vis_tuning = VisTuning{0, rf, sp, ct, 1};
-                std::vector<float> ts;
-                for (uint32_t r = 0; r <= reps; ++r) {
-                    cudaEventRecord(e0, ctx->stream);
-                    s = b->fused ? launch_frame(ctx, b, false) : launch_lanes(ctx, b, b->frame_index);
-                    if (s != LUZ_OK) return s;
-                    cudaEventRecord(e1, ctx->stream);
-                    LUZ_CUDA(ctx, cudaEventSynchronize(e1));
-                    float ms = 0.f;
-                    cudaEventElapsedTime(&ms, e0, e1);
-                    if (r) ts.push_back(ms);   // the first launch warms up
-                }
-                std::sort(ts.begin(), ts.end());
-                float med = ts[ts.size() / 2];
-                if (med < best_t) { best_t = med; best = ctx->vis_tuning; }
+    auto run = [&]() -> luz_status {
+        for (cudaEvent_t& e : ev) LUZ_CUDA(ctx, cudaEventCreate(&e));
+        std::vector<VisTuning> shapes;
+        {
+            TuningScope scope(ctx, b);
+            shapes.push_back(b->fused ? batch_tuning(ctx) : vis_tuning(ctx));
+            ctx->vis_tuning = VisTuning{};
+            shapes.push_back(b->fused ? batch_tuning(ctx) : vis_tuning(ctx));
+        }
+        for (uint32_t rf : {8, 16, 32})
+            for (uint32_t sp : {16, 32, 64})
+                for (uint32_t ct : {2, 3, 4}) shapes.push_back(VisTuning{0, rf, sp, ct, 1});
+        const uint32_t smem = shapes[0].smem_nodes;
+        for (VisTuning& t : shapes) {
+            t.smem_nodes = smem;
+            t.set = 1;
+            ctx->vis_tuning = t;
+            std::vector<float> ts;
+            for (uint32_t r = 0; r <= reps; ++r) {
+                LUZ_CUDA(ctx, cudaEventRecord(ev[0], ctx->stream));
+                const luz_status l = b->fused ? launch_frame(ctx, b, false) : launch_lanes(ctx, b, b->frame_index);
+                if (l != LUZ_OK) return l;
+                LUZ_CUDA(ctx, cudaEventRecord(ev[1], ctx->stream));
+                LUZ_CUDA(ctx, cudaEventSynchronize(ev[1]));
+                float ms = 0.f;
+                LUZ_CUDA(ctx, cudaEventElapsedTime(&ms, ev[0], ev[1]));
+                if (r) ts.push_back(ms);   // the first launch warms up
             }
-    cudaEventDestroy(e0);
-    cudaEventDestroy(e1);
-    // the single-scene TLAS staging size keeps its current value
-    best.smem_nodes = base_smem;
-    ctx->vis_tuning = best;
+            std::sort(ts.begin(), ts.end());
+            const float med = ts[ts.size() / 2];
+            if (med < best_t) { best_t = med; best = t; }
+        }
+        return LUZ_OK;
+    };
+    s = run();
+    ctx->vis_tuning = of_ctx;
+    for (cudaEvent_t e : ev)
+        if (e) cudaEventDestroy(e);
+    if (s != LUZ_OK) return s;
+    b->tuning = best;
+    b->tuned_fused = b->fused;
+    b->tuned_at = ctx->vis_tuning_changes;
     if (chosen) *chosen = luz_vis_tuning{best.smem_nodes, best.refill, best.steps, best.ctas_per_sm};
     if (best_ms) *best_ms = best_t;
     uint32_t bits = 0;

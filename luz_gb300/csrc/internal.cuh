@@ -128,6 +128,7 @@ struct luz_ctx {
     int raygen_blocks = 0, cull_blocks = 0;   // resident blocks per SM (0: not queried)
     bool registered = false;                    // counted among the process's live contexts
     luz::VisTuning vis_tuning{0, 0, 0, 0, 0};   // set == 0: library defaults
+    uint32_t vis_tuning_changes = 0;            // calls that set it
     uint32_t debug_step_cap = 0;                // traversal steps per ray, 0 = the library's cap
     // device pipeline of the last batched BLAS build (after its host->device copies)
     cudaEvent_t build_ev[2] = {nullptr, nullptr};

@@ -515,12 +515,14 @@ extern "C" luz_status luz_ctx_set_vis_tuning(luz_ctx* ctx, const luz_vis_tuning*
     using namespace luz;
     if (!ctx || !t) return LUZ_ERR_INVALID;
     if (t->smem_nodes == 0 && t->refill == 0 && t->steps == 0 && t->ctas_per_sm == 0) {
+        ++ctx->vis_tuning_changes;
         ctx->vis_tuning = VisTuning{0, 0, 0, 0, 0};
         return LUZ_OK;
     }
     if (t->smem_nodes > 1024 || t->refill < 1 || t->refill > 32 || t->steps < 1 || t->steps > 1024 ||
         t->ctas_per_sm < 1 || t->ctas_per_sm > 16)
         return set_error(ctx, LUZ_ERR_INVALID, "visibility tuning outside its documented ranges");
+    ++ctx->vis_tuning_changes;
     ctx->vis_tuning = VisTuning{t->smem_nodes, t->refill, t->steps, t->ctas_per_sm, 1};
     return LUZ_OK;
 }

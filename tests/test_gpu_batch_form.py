@@ -73,3 +73,34 @@ def test_a_recorded_batch_is_dropped_when_its_buffers_move():
         assert np.array_equal(b.frames[0].read(L.PLANE_AO_BITS), g.frame.read(L.PLANE_AO_BITS))
     finally:
         ctx.close()
+
+
+@pytest.mark.parametrize("fused", [True, False])
+def test_tuning_a_batch_leaves_the_contexts_frames_alone(fused):
+    """The tuned shape is the batch's: the launch shape of single frames, and of other
+    batches, stays what it was; a shape set on the context afterwards holds for all."""
+    ctx = L.Context(0)
+    try:
+        ctx.set_blue_noise(L.blue_noise())
+        scenes = [L.HostScene(1, seed=i, width=80, height=48, ao_samples=2) for i in range(3)]
+        b = L.Batch(ctx, scenes)
+        b.set_fused(fused)
+        before = ctx.vis_tuning()
+        tuned, ms = b.autotune(1)
+        assert ms > 0 and ctx.vis_tuning() == before
+        b.render(2)
+        ctx.synchronize()
+        g = L.GPUScene(ctx, scenes[1])
+        g.render(2)
+        ctx.synchronize()
+        assert ctx.device_status() == 0
+        assert np.array_equal(b.frames[1].read(L.PLANE_LIGHT).view(np.uint32),
+                              g.frame.read(L.PLANE_LIGHT).view(np.uint32))
+        ctx.set_vis_tuning(refill=32, steps=1, ctas_per_sm=1)
+        b.autotune(1)
+        assert ctx.vis_tuning() == {"smem_nodes": 0, "refill": 32, "steps": 1, "ctas_per_sm": 1}
+        b.render(2)
+        ctx.synchronize()
+        assert ctx.device_status() == 0
+    finally:
+        ctx.close()
