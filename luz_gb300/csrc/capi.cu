@@ -572,6 +572,11 @@ static luz_status frame_upload_body(luz_ctx* ctx, luz_frame* f, const luz_scene*
         if (slots > LUZ_MAX_SHADOW_SLOTS)
             return set_error(ctx, LUZ_ERR_LIMIT, "more than LUZ_MAX_SHADOW_SLOTS shadow samples per pixel");
     }
+    // (a recorded copy would read the pinned block as a later upload leaves it)
+    cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
+    LUZ_CUDA(ctx, cudaStreamIsCapturing(ctx->stream, &capturing));
+    if (capturing != cudaStreamCaptureStatusNone)
+        return set_error(ctx, LUZ_ERR_CUDA, "an upload cannot be part of a stream capture");
     const uint32_t shadow_slots = (uint32_t)slots, ao = (uint32_t)scene->ao_num_samples;
     uint32_t cap_shadow = f->shadow_planes_cap, cap_ao = f->ao_planes_cap;
     luz_status s;

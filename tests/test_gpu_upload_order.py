@@ -1,0 +1,102 @@
+"""Scene constants uploaded again and again: each upload is what the work after it reads,
+without waits between and as blocks grow and shrink; during a stream capture an upload is
+refused."""
+import numpy as np
+import pytest
+
+import luz_gb300 as L
+from luz_gb300 import _abi
+
+pytestmark = pytest.mark.gpu
+
+W, H = 72, 40
+
+
+def _block(scene):
+    s = _abi.Scene()
+    s.ambient_light_color[:], s.ambient_light_intensity = [1.0, 1.0, 1.0], 0.0
+    for name in ("proj", "view", "inverse_proj", "inverse_view"):
+        getattr(s, name)[:] = np.eye(4, dtype=np.float32).reshape(-1).tolist()
+    s.cam_pos[:] = [0.0, 3.0, 0.0]
+    s.ao_min, s.ao_max, s.shadow_type = 1e-4, 2.0, L.SHADOW_RAYTRACING
+    s.num_lights = scene
+    return s
+
+
+def _lights(count, intensity):
+    lights = (_abi.Light * max(count, 1))()
+    for i in range(count):
+        lt = lights[i]
+        lt.color[:], lt.intensity, lt.type = [1.0, 0.5, 0.25], intensity / count, L.LIGHT_POINT
+        lt.position[:], lt.direction[:] = [0.0, 5.0, 2.0], [0.0, -1.0, 0.0]
+        lt.num_shadow_samples, lt.shadow_map = 0, -1
+    return lights
+
+
+def _frame(ctx):
+    f = ctx.frame(W, H)
+    f.upload(_block(1), _lights(1, 1.0), 1, None, 0)
+    normal = np.zeros((H, W, 4), np.float32)
+    normal[..., 1] = 1.0
+    f.write(L.PLANE_NORMAL, normal)
+    f.write(L.PLANE_DEPTH, np.full((H, W), 0.5, np.float32))
+    f.write(L.PLANE_ALBEDO, np.full((H, W), 0xFFFFFFFF, np.uint32))
+    f.write(L.PLANE_MATERIAL, np.full((H, W), 0xFFFFFF80, np.uint32))
+    f.write(L.PLANE_EMISSION, np.zeros((H, W), np.uint32))
+    return f
+
+
+def _light(f):
+    return f.read(L.PLANE_LIGHT)[..., :3].copy()
+
+
+def test_uploads_follow_one_another_and_outgrow_their_block():
+    torch = pytest.importorskip("torch")
+    ctx = L.Context(0)
+    try:
+        stream = torch.cuda.Stream()
+        ctx.set_stream(stream.cuda_stream)
+        f = _frame(ctx)
+        f.light_pass()
+        one = _light(f)
+        assert (one > 0).all()
+        frames = [_frame(ctx) for _ in range(4)]
+        with torch.cuda.stream(stream):
+            torch.cuda._sleep(50_000_000)            # the copies queue up behind it
+        for n, intensity in ((1, 2.0), (3, 4.0), (200, 8.0), (2, 16.0), (500, 32.0), (1, 64.0)):
+            models = (_abi.Model * n)()
+            for k, fr in enumerate(frames):
+                fr.upload(_block(n), _lights(n, intensity * 2.0 ** k), n, models, n)
+                fr.light_pass()
+        for k, fr in enumerate(frames):
+            assert np.array_equal(_light(fr), one * np.float32(64.0 * 2.0 ** k))
+        ctx.synchronize()
+        assert ctx.device_status() == 0
+    finally:
+        ctx.close()
+
+
+def test_upload_during_a_capture_is_refused():
+    torch = pytest.importorskip("torch")
+    ctx = L.Context(0)
+    try:
+        stream = torch.cuda.Stream()
+        ctx.set_stream(stream.cuda_stream)
+        f = _frame(ctx)
+        f.light_pass()
+        ctx.synchronize()
+        one = _light(f)
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.stream(stream):
+            graph.capture_begin(capture_error_mode="relaxed")
+            try:
+                with pytest.raises(L.LuzError):
+                    f.upload(_block(1), _lights(1, 2.0), 1, None, 0)
+                f.light_pass()
+            finally:
+                graph.capture_end()
+            graph.replay()
+        ctx.synchronize()
+        assert np.array_equal(_light(f), one)        # the refused upload left nothing behind
+    finally:
+        ctx.close()
