@@ -423,6 +423,12 @@ static luz_status set_frame_index(luz_ctx* ctx, luz_batch* b, int frame_index) {
     return LUZ_OK;
 }
 
+static luz_status constants_ready(luz_ctx* ctx, luz_batch* b) {
+    for (luz_frame* f : b->frames)
+        if (luz_status s = frame_constants_ready(ctx, f); s != LUZ_OK) return s;
+    return LUZ_OK;
+}
+
 // The frame kernel of the batch: the counters cleared, then one persistent launch.
 static luz_status launch_frame(luz_ctx* ctx, luz_batch* b, bool stats) {
     cudaStream_t st = ctx->stream;
@@ -558,7 +564,8 @@ static luz_status launch_lanes(luz_ctx* ctx, luz_batch* b, int frame_index) {
 // stats: every ray traced from its TLAS root by a counting launch, in either form.
 static luz_status batch_record(luz_ctx* ctx, luz_batch* b, int frame_index, bool stats) {
     const TuningScope scope(ctx, b);
-    luz_status s = set_frame_index(ctx, b, frame_index);
+    luz_status s = constants_ready(ctx, b);
+    if (s == LUZ_OK) s = set_frame_index(ctx, b, frame_index);
     if (s != LUZ_OK) return s;
     if (b->fused) return launch_frame(ctx, b, stats);
     if (!stats) return launch_lanes(ctx, b, frame_index);
@@ -747,6 +754,7 @@ luz_status luz_batch_capture(luz_ctx* ctx, luz_batch* b, int32_t frame_index) {
 
 luz_status luz_batch_replay(luz_ctx* ctx, luz_batch* b) {
     if (!ctx || !b || !b->exec) return set_error(ctx, LUZ_ERR_INVALID, "no captured graph");
+    if (luz_status s = constants_ready(ctx, b); s != LUZ_OK) return s;
     LUZ_CUDA(ctx, cudaGraphLaunch(b->exec, ctx->stream));
     ctx->launches++;
     return LUZ_OK;

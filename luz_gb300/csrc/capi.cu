@@ -137,6 +137,18 @@ static luz_status reserve_upload(luz_ctx* ctx, luz_frame* f, uint32_t lights, ui
     return LUZ_OK;
 }
 
+luz_status frame_constants_ready(luz_ctx* ctx, luz_frame* f) {
+    if (!f->upload_ctx || f->upload_ctx == ctx) return LUZ_OK;
+    // (a wait of the host, also while a stream of this thread is capturing)
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+    LUZ_CUDA(ctx, cudaThreadExchangeStreamCaptureMode(&mode));
+    const cudaError_t e = cudaEventSynchronize(f->upload_done);
+    LUZ_CUDA(ctx, cudaThreadExchangeStreamCaptureMode(&mode));
+    if (e != cudaSuccess) return cuda_error(ctx, e, "frame upload");
+    f->upload_ctx = nullptr;
+    return LUZ_OK;
+}
+
 // (Re)allocates *p for at least `need` elements when `cap` is short; cap is updated.
 static luz_status grow(luz_ctx* ctx, void** p, uint32_t& cap, uint32_t need, size_t elem) {
     if (need <= cap && *p) return LUZ_OK;
@@ -628,6 +640,7 @@ static luz_status frame_upload_body(luz_ctx* ctx, luz_frame* f, const luz_scene*
     const size_t bytes = (size_t)((char*)f->d_model_skip + model_count - (char*)f->d_upload);
     LUZ_CUDA(ctx, cudaMemcpyAsync(f->d_upload, h, bytes, cudaMemcpyHostToDevice, ctx->stream));
     LUZ_CUDA(ctx, cudaEventRecord(f->upload_done, ctx->stream));
+    f->upload_ctx = ctx;
     return LUZ_OK;
 }
 

@@ -251,6 +251,7 @@ struct luz_frame {
     void* d_upload = nullptr;          // one block holding the following regions (reserve_upload)
     void* h_upload = nullptr;          // its pinned copy
     cudaEvent_t upload_done = nullptr; // h_upload may be rewritten after this
+    const luz_ctx* upload_ctx = nullptr;   // whose stream the last upload is ordered on (none: it is done)
     luz_scene* d_scene = nullptr;
     luz_light* d_lights = nullptr;
     uint32_t lights_cap = 0, light_count = 0, slots_cap = 0;
@@ -318,6 +319,11 @@ luz_status guarded(luz_ctx* ctx, F&& body) noexcept {
     } while (0)
 
 namespace luz {
+// Before work of ctx that reads the frame's constants: waits for their upload where that is on
+// another context's stream (so that an upload is there for every context when the call has
+// returned, while the uploading one need not wait).
+luz_status frame_constants_ready(luz_ctx* ctx, luz_frame* f);
+
 // Launches a kernel whose launch work overlaps the end of the one before it in the stream:
 // its blocks are scheduled when that one's last block has finished, and the kernel begins
 // with chain_wait, which waits until everything before it in the stream is complete and

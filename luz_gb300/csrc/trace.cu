@@ -554,6 +554,7 @@ luz_status launch_lit_compaction(luz_ctx* ctx, luz_frame* f, bool counted);
 
 // Inputs of the G-buffer pass of frame f over TLAS t.
 luz_status make_gbuf_params(luz_ctx* ctx, luz_frame* f, const luz_tlas* t, GbufParams& G) {
+    if (luz_status s = frame_constants_ready(ctx, f); s != LUZ_OK) return s;
     // 4-wide nodes; node_count (the binary count) bounds the 4-wide count and the
     // nodes4 buffer, so staging that many stays inside it.
     G.tlas_nodes = t->nodes4;
@@ -637,6 +638,7 @@ luz_status launch_lit_compaction(luz_ctx* ctx, luz_frame* f, bool counted) {
 // Rebuilds the lit-pixel list when the planes or scene constants it came from were
 // replaced since the last G-buffer pass (luz_frame_write, luz_frame_upload).
 luz_status ensure_lit_list(luz_ctx* ctx, luz_frame* f) {
+    if (luz_status s = frame_constants_ready(ctx, f); s != LUZ_OK) return s;
     return f->surf_valid ? LUZ_OK : launch_lit_compaction(ctx, f, false);
 }
 

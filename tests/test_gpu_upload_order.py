@@ -1,6 +1,8 @@
 """Scene constants uploaded again and again: each upload is what the work after it reads,
-without waits between and as blocks grow and shrink; during a stream capture an upload is
-refused."""
+without waits between, as blocks grow and shrink and from a context other than the one that
+renders; during a stream capture an upload is refused."""
+import ctypes as C
+
 import numpy as np
 import pytest
 
@@ -74,6 +76,32 @@ def test_uploads_follow_one_another_and_outgrow_their_block():
         assert ctx.device_status() == 0
     finally:
         ctx.close()
+
+
+def test_upload_by_another_context_is_there_when_the_call_returns():
+    torch = pytest.importorskip("torch")
+    loader, ctx = L.Context(0), L.Context(0)
+    try:
+        stream = torch.cuda.Stream()
+        loader.set_stream(stream.cuda_stream)
+        f = _frame(loader)
+        lib, h = L.lib, f.handle
+        loader.synchronize()
+        assert lib.luz_light_pass(ctx.handle, h, 0) == 0
+        ctx.synchronize()
+        one = _light(f)
+        with torch.cuda.stream(stream):
+            torch.cuda._sleep(400_000_000)           # the loader's stream is busy for a while
+        f.upload(_block(1), _lights(1, 2.0), 1, None, 0)
+        assert lib.luz_light_pass(ctx.handle, h, 0) == 0
+        ctx.synchronize()
+        out = np.zeros((H, W, 4), np.float32)
+        assert lib.luz_frame_read(ctx.handle, h, L.PLANE_LIGHT, _abi.ptr(out), C.c_size_t(out.nbytes)) == 0
+        assert np.array_equal(out[..., :3], one * np.float32(2.0))
+        loader.synchronize()
+    finally:
+        ctx.close()
+        loader.close()
 
 
 def test_upload_during_a_capture_is_refused():
