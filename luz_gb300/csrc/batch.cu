@@ -412,10 +412,22 @@ struct TuningScope {
     ~TuningScope() { ctx->vis_tuning = of_ctx; }
 };
 
+// The sampler frame index and the frames' shadow-cull setting in the per-scene records of the
+// frame kernel and the counting trace (fixed inside a graph); whether one changed.
+static bool set_records(luz_batch* b, int frame_index) {
+    bool changed = frame_index != b->frame_index;
+    for (size_t i = 0; i < b->h_scenes.size(); ++i) {
+        SceneVis& s = b->h_scenes[i];
+        const int cull = b->frames[i]->shadow_cull ? 1 : 0;
+        changed = changed || s.cull != cull;
+        s.frame = frame_index;
+        s.cull = cull;
+    }
+    return changed;
+}
+
 static luz_status set_frame_index(luz_ctx* ctx, luz_batch* b, int frame_index) {
-    // The sampler frame index lives in the per-scene records (fixed inside a graph).
-    if (frame_index != b->frame_index) {
-        for (auto& s : b->h_scenes) s.frame = frame_index;
+    if (set_records(b, frame_index)) {
         LUZ_CUDA(ctx, cudaMemcpyAsync(b->d_scenes, b->h_scenes.data(), b->h_scenes.size() * sizeof(SceneVis),
                                       cudaMemcpyHostToDevice, ctx->stream));
         b->frame_index = frame_index;
@@ -731,8 +743,7 @@ luz_status luz_batch_capture(luz_ctx* ctx, luz_batch* b, int32_t frame_index) {
         if (s != LUZ_OK) return s;
     }
     // The frame index is written before capture: the records are then constant.
-    if (frame_index != b->frame_index) {
-        for (auto& s : b->h_scenes) s.frame = frame_index;
+    if (set_records(b, frame_index)) {
         LUZ_CUDA(ctx, cudaMemcpy(b->d_scenes, b->h_scenes.data(), b->h_scenes.size() * sizeof(SceneVis),
                                  cudaMemcpyHostToDevice));
         b->frame_index = frame_index;

@@ -104,3 +104,31 @@ def test_tuning_a_batch_leaves_the_contexts_frames_alone(fused):
         assert ctx.device_status() == 0
     finally:
         ctx.close()
+
+
+@pytest.mark.parametrize("fused", [True, False])
+def test_shadow_cull_of_a_batchs_frame_holds_in_either_form(fused):
+    ctx = L.Context(0)
+    try:
+        ctx.set_blue_noise(L.blue_noise())
+        scenes = [L.HostScene(1, seed=i, width=96, height=64, ao_samples=2) for i in range(3)]
+        b = L.Batch(ctx, scenes)
+        b.set_fused(fused)
+        bits = {}
+        for cull in (True, False, True):
+            for fr in b.frames:
+                fr.set_shadow_cull(cull)
+            b.render(2)
+            ctx.synchronize()
+            for i, (sc, fr) in enumerate(zip(scenes, b.frames)):
+                g = L.GPUScene(ctx, sc)
+                g.frame.set_shadow_cull(cull)
+                g.render(2)
+                ctx.synchronize()
+                got = fr.read(L.PLANE_SHADOW_BITS).copy()
+                assert np.array_equal(got, g.frame.read(L.PLANE_SHADOW_BITS))
+                assert np.array_equal(got, bits.setdefault((i, cull), got))
+            assert ctx.device_status() == 0
+        assert any(not np.array_equal(bits[i, True], bits[i, False]) for i in range(3))
+    finally:
+        ctx.close()
