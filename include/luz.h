@@ -429,7 +429,9 @@ luz_status luz_gbuffer_primary(luz_ctx* ctx, luz_frame* frame, const luz_tlas* t
  * * attenuation is +-0 (outside a spot light's cone, a black light). The light pass
  * output is then the one of tracing every ray, but the exported bit planes are not
  * light.frag's per-ray results for those samples; luz_frame_set_shadow_cull(frame, 0)
- * traces every sample as light.frag does. */
+ * traces every sample as light.frag does. The frame's first trace allocates its ray
+ * buffers, up to 12 GB; frames of more rays, and traces where the device has no room for
+ * as much, go through them in smaller chunks. */
 luz_status luz_trace_visibility(luz_ctx* ctx, luz_frame* frame, const luz_tlas* tlas,
                                 int32_t frame_index);
 /* enable != 0 (the default): leave out the shadow rays of conditions (a) and (b) above;
@@ -512,9 +514,11 @@ void* luz_frame_plane_device_ptr(luz_frame* frame, int32_t plane);
  * Many independent scenes of uneven size as one unit (no counterpart in the
  * reference, which renders one scene per frame). A render takes one of two forms, the
  * faster one unless luz_batch_set_fused chooses. Scenes of 200,000 pixels and more on
- * average, or up to two scenes of any size, run in lanes: every pass of a scene as the launches of a single frame, the scenes spread over up to
- * eight streams that fork from the context's and join it again; a lane's buffers are those
- * of a single frame's trace, for its largest scene. Many small scenes run as ONE
+ * average, or up to two scenes of any size, run in lanes: every pass of a scene as the
+ * launches of a single frame, the scenes spread over up to eight streams that fork from
+ * the context's and join it again; a lane's buffers are those of a single frame's trace,
+ * for its largest scene, all lanes' together those of one frame at most (12 GB). Many
+ * small scenes run as ONE
  * persistent launch (the frame kernel) over every scene: the per-frame TLAS builds,
  * the clearing of the hit/miss planes, the G-buffer passes with their lit-pixel lists,
  * the shadow/AO traversal of all scenes' rays from one work counter, and the light

@@ -504,6 +504,8 @@ static luz_status make_lanes(luz_ctx* ctx, luz_batch* b, uint32_t count) {
     const uint32_t n = (uint32_t)b->frames.size();
     LUZ_CUDA(ctx, cudaEventCreateWithFlags(&b->fork, cudaEventDisableTiming));
     b->lanes.resize(count);
+    for (auto& lane : b->lanes)   // the lanes' traces together take at most what one frame's may
+        for (size_t k = 1; k < count; k *= 2) lane.scratch.ray_chunk /= 2;
     for (size_t k = 1; k < count; ++k) {
         LUZ_CUDA(ctx, cudaStreamCreateWithFlags(&b->lanes[k].stream, cudaStreamNonBlocking));
         LUZ_CUDA(ctx, cudaEventCreateWithFlags(&b->lanes[k].joined, cudaEventDisableTiming));

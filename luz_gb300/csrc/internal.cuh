@@ -33,10 +33,12 @@ constexpr int kStackSize = 160;
 //   f6 child[4] (int bits: >= 0 a 4-wide node, < 0 a leaf ~index, kEmptyChild), f7 0.
 constexpr int kNode4F4 = 8;
 
-// Rays per visibility chunk (shadow, AO): ray generation writes the 48-B records of one
-// chunk at most, the traversal kernel consumes them. A 1080p frame of 41 lights and 16 AO
-// samples fits one chunk even when every pixel is lit and no ray is resolved early.
-constexpr uint32_t kRayChunk = 1u << 27, kAoChunk = 1u << 26;
+// Shadow rays per visibility chunk, and half as many AO rays: ray generation writes the 48-B
+// records of one chunk at most, the traversal kernel consumes them. A 1080p frame of 41 lights
+// and 16 AO samples fits one chunk even when every pixel is lit and no ray is resolved early.
+// The buffers of a whole chunk take up to 12 GB; where the device has no room, chunks are
+// halved down to kRayChunkMin.
+constexpr uint32_t kRayChunk = 1u << 27, kRayChunkMin = 1u << 16;
 
 // One TLAS leaf, in sorted (leaf) order. 96 B, 16-B aligned for vector loads.
 // sphere: the BLAS's bounding sphere in object space, (centre, radius): the root box
@@ -192,11 +194,15 @@ struct VisScratch {
     void* counters = nullptr;             // VisCounters per chunk
     uint32_t patches_cap = 0, lists_cap = 0, pairs_cap = 0, records_cap = 0, chunks_cap = 0;
     uint32_t moves = 0;                   // times a buffer was freed or replaced
+    uint32_t ray_chunk = kRayChunk;       // rays of a chunk at most (a power of two)
     void release() {
         for (void* p : {patches, (void*)start_lists, (void*)cuts, (void*)active, (void*)rays_a, (void*)rays_b,
                         (void*)rays_c, counters})
             if (p) cudaFree(p);
+        const uint32_t m = moves + 1, chunk = ray_chunk;
         *this = VisScratch{};
+        moves = m;
+        ray_chunk = chunk;
     }
 };
 }  // namespace luz

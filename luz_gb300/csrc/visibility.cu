@@ -332,16 +332,17 @@ struct VisSizes {
     uint32_t shadow_chunks, ao_chunks, chunks;
 };
 
+static_assert(((kRayChunkMin / kPatch) >> 2) % kSuper == 0, "chunks of whole blocks of pairs");
 // Chunks over the largest possible counts; what lies past the frame's actual counts
 // returns at once on the device. Without instances no shadow ray has anything to hit.
-static VisSizes vis_sizes(const luz_frame* f, const luz_tlas* t) {
+static VisSizes vis_sizes(const luz_frame* f, const luz_tlas* t, uint32_t ray_chunk) {
     VisSizes z{};
     z.patches = (f->pixels + kPatch - 1) / kPatch;
     z.supers = (z.patches + kSuper - 1) / kSuper;
     const uint32_t shift = f->vlight_shift;
     const unsigned long long max_pairs = t->count > 0 ? (unsigned long long)z.supers * kSuper * f->vlight_count : 0ull;
-    z.pairs = (uint32_t)std::min<unsigned long long>(max_pairs, (kRayChunk / kPatch) >> shift);
-    if (f->ao_samples) z.ao_patches = std::min(z.patches, std::max(kAoChunk / (kPatch * f->ao_samples), 1u));
+    z.pairs = (uint32_t)std::min<unsigned long long>(max_pairs, (ray_chunk / kPatch) >> shift);   // whole blocks
+    if (f->ao_samples) z.ao_patches = std::min(z.patches, std::max(ray_chunk / 2 / (kPatch * f->ao_samples), 1u));
     z.records = ((z.pairs * kPatch) << shift) + z.ao_patches * kPatch * f->ao_samples;
     z.shadow_chunks = z.pairs ? (uint32_t)((max_pairs + z.pairs - 1) / z.pairs) : 0u;
     z.ao_chunks = z.ao_patches ? (z.patches + z.ao_patches - 1) / z.ao_patches : 0u;
@@ -349,7 +350,7 @@ static VisSizes vis_sizes(const luz_frame* f, const luz_tlas* t) {
     return z;
 }
 
-static luz_status ensure_vis_buffers(luz_ctx* ctx, VisScratch& v, const VisSizes& z) {
+static luz_status grow_vis_buffers(luz_ctx* ctx, VisScratch& v, const VisSizes& z) {
     const uint32_t patches = z.patches + z.supers, lists = z.pairs + z.ao_patches;
     if (patches <= v.patches_cap && lists <= v.lists_cap && z.pairs <= v.pairs_cap && z.records <= v.records_cap &&
         z.chunks <= v.chunks_cap)
@@ -392,9 +393,22 @@ static luz_status ensure_vis_buffers(luz_ctx* ctx, VisScratch& v, const VisSizes
     return LUZ_OK;
 }
 
+// The buffers for a trace of f over t, in smaller chunks where there is no memory for larger
+// ones; z: the sizes it then has.
+static luz_status ensure_vis_buffers(luz_ctx* ctx, VisScratch& v, const luz_frame* f, const luz_tlas* t, VisSizes& z) {
+    for (;;) {
+        z = vis_sizes(f, t, v.ray_chunk);
+        const luz_status s = z.chunks ? grow_vis_buffers(ctx, v, z) : LUZ_OK;
+        if (s != LUZ_ERR_OOM || v.ray_chunk <= kRayChunkMin) return s;
+        cudaGetLastError();
+        v.release();   // (the stream is idle: grow_vis_buffers waited for it)
+        v.ray_chunk /= 2;
+    }
+}
+
 luz_status reserve_visibility(luz_ctx* ctx, const luz_frame* f, const luz_tlas* t, VisScratch& scratch) {
-    const VisSizes z = vis_sizes(f, t);
-    return z.chunks ? ensure_vis_buffers(ctx, scratch, z) : LUZ_OK;
+    VisSizes z;
+    return ensure_vis_buffers(ctx, scratch, f, t, z);
 }
 
 luz_status launch_visibility(luz_ctx* ctx, luz_frame* f, const luz_tlas* t, int frame_index,
@@ -418,12 +432,12 @@ luz_status launch_visibility(luz_ctx* ctx, luz_frame* f, const luz_tlas* t, int 
     });
     if (s != LUZ_OK) return s;
     uint32_t grid = (uint32_t)ctx->sm_count * tu.ctas_per_sm;
-    const VisSizes z = vis_sizes(f, t);
+    VisSizes z;
+    if ((s = ensure_vis_buffers(ctx, v, f, t, z)) != LUZ_OK) return s;
     const uint32_t shadow_chunks = z.shadow_chunks, ao_chunks = z.ao_chunks;
     if (d_stats) LUZ_CUDA(ctx, cudaMemsetAsync(d_stats, 0, 5 * sizeof(unsigned long long), st));
     if (!shadow_chunks && (s = clear_visibility(ctx, f)) != LUZ_OK) return s;   // else by patch_kernel
     if (z.chunks == 0) return LUZ_OK;
-    if ((s = ensure_vis_buffers(ctx, v, z)) != LUZ_OK) return s;
     VisCounters* counters = (VisCounters*)v.counters;
     if (!shadow_chunks) LUZ_CUDA(ctx, cudaMemsetAsync(counters, 0, (size_t)z.chunks * sizeof(VisCounters), st));
     if (t->count) S.leaf_box = tlas_leaf_boxes(t);
