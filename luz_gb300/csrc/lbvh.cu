@@ -798,13 +798,10 @@ __global__ void tlas_instance_kernel(const DevInstanceInput* in, uint32_t n, flo
     if (seg_bounds) merge_bounds(have, c, seg_bounds);
 }
 
-__global__ void tlas_setup_kernel(uint32_t* bounds, SegDesc* seg, SegDesc value, uint32_t* zero) {
+__global__ void tlas_setup_kernel(uint32_t* bounds, SegDesc* seg, SegDesc value) {
     chain_wait();
     if (threadIdx.x < 6) bounds[threadIdx.x] = threadIdx.x < 3 ? 0xFFFFFFFFu : 0u;
-    if (threadIdx.x == 0) {
-        *seg = value;
-        *zero = 0;
-    }
+    if (threadIdx.x == 0) *seg = value;
 }
 
 __global__ void __launch_bounds__(256) tlas_morton_kernel(const float4* inst_box, uint32_t n, const uint32_t* seg_bounds,
@@ -1466,7 +1463,7 @@ static size_t tlas_tmp_bytes(uint32_t cap) {
     return align256((size_t)cap * 32) + align256(24) + sort_scratch_bytes(std::max(cap, 1u), 4) +
            align256((size_t)cap * 32) + align256((size_t)m * 4) + align256((size_t)cap * 4) +
            align256((size_t)m * 4) + align256((size_t)m * 64) + 2 * align256((size_t)m * 4) +
-           align256(sizeof(SegDesc)) + 2 * align256(4) + 2 * align256((size_t)cap * 8);
+           align256(sizeof(SegDesc)) + 2 * align256((size_t)cap * 8);
 }
 
 luz_status launch_tlas_build(luz_ctx* ctx, luz_tlas* t);
@@ -1526,7 +1523,6 @@ struct TlasScratch {
     uint32_t* bounds;
     SortBuffers sb;
     SegDesc* d_seg;
-    uint32_t* d_zero;
     uint2* ends[2];
 };
 
@@ -1552,7 +1548,6 @@ static TlasScratch carve_tlas(luz_tlas* t) {
     a.queue = (uint32_t*)p; p += align256((size_t)mcap * 4);
     a.newidx = (uint32_t*)p; p += align256((size_t)mcap * 4);
     s.d_seg = (SegDesc*)p; p += align256(sizeof(SegDesc));
-    s.d_zero = (uint32_t*)p; p += align256(4);
     for (uint2*& e : s.ends) { e = (uint2*)p; p += align256((size_t)cap * 8); }
     a.inst_out = t->instances;
     a.morton_out = t->morton;
@@ -1592,7 +1587,6 @@ luz_status launch_tlas_kernels(luz_ctx* ctx, luz_tlas* t) {
     float4* karras_nodes = A.karras_nodes;
     uint32_t* newidx = A.newidx;
     SegDesc* d_seg = ts.d_seg;
-    uint32_t* d_zero = ts.d_zero;
 
     if (n <= kFusedTlasMax) {
         static DeviceSetup setup;   // the kernel's shared-memory limit
@@ -1624,10 +1618,10 @@ luz_status launch_tlas_kernels(luz_ctx* ctx, luz_tlas* t) {
     sd.prim_count = n;
     sd.node_off = 0;
     sd.nodes = karras_nodes;
-    // Bounds initialiser, segment descriptor and zero offset are written by a kernel from
-    // its parameters: a copy from host memory would, inside a CUDA graph, re-read a
+    // Bounds initialiser and segment descriptor are written by a kernel from its
+    // parameters: a copy from host memory would, inside a CUDA graph, re-read a
     // host address that no longer holds them.
-    chain(tlas_setup_kernel, 1, 32, 0, st, bounds, d_seg, sd, d_zero);
+    chain(tlas_setup_kernel, 1, 32, 0, st, bounds, d_seg, sd);
     LUZ_LAUNCHED(ctx, "tlas_setup_kernel");
     LUZ_CUDA(ctx, cudaMemsetAsync(flags, 0, (size_t)m * 4, st));
     luz_status s = clear_sort(ctx, sb, 4);

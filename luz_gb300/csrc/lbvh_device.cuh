@@ -110,16 +110,15 @@ __device__ __forceinline__ void write_slot(float4* node, int slot, float4 lo, fl
     }
 }
 
-// Leaf g (global index) of segment sd: writes its box into its parent and climbs
-// while it is the second child to arrive. kBlock: every leaf of the tree is handled
-// by one CTA, so block-scope fences order the node writes.
 __device__ __forceinline__ uint32_t atomic_add_acq_rel_gpu(uint32_t* p, uint32_t v) {
     uint32_t old;
     asm volatile("atom.acq_rel.gpu.global.add.u32 %0, [%1], %2;" : "=r"(old) : "l"(p), "r"(v) : "memory");
     return old;
 }
 
-template <bool kBlock>
+// Leaf g (global index) of segment sd, a tree built by one block (block-scope fences order
+// the node writes): writes its box into its parent and climbs while it is the second child
+// to arrive.
 __device__ __forceinline__ void refit_leaf(const SegDesc& sd, uint32_t g, const float4* leaf_box,
                                            const uint32_t* node_parent, const uint32_t* leaf_parent,
                                            uint32_t* flags) {
@@ -132,19 +131,9 @@ __device__ __forceinline__ void refit_leaf(const SegDesc& sd, uint32_t g, const 
         if (p == 0xFFFFFFFFu || local >= node_count) return;
         float4* node = sd.nodes + (size_t)local * kNodeF4;
         write_slot(node, p & 1, lo, hi);
-        uint32_t old;
-        if (kBlock) {
-            __threadfence_block();
-            old = atomicAdd(flags + sd.node_off + local, 1u);
-            if (old == 0) return;
-            __threadfence_block();
-        } else {
-            // One acquire-release atomic instead of two device-wide fences: its release
-            // half publishes this child's slot, its acquire half (for the second
-            // arrival) makes the first child's slot visible to the L2 loads below.
-            old = atomic_add_acq_rel_gpu(flags + sd.node_off + local, 1u);
-            if (old == 0) return;
-        }
+        __threadfence_block();
+        if (atomicAdd(flags + sd.node_off + local, 1u) == 0) return;
+        __threadfence_block();
         float4 n0 = __ldcg(node + 0), n1 = __ldcg(node + 1), n2 = __ldcg(node + 2);
         lo = make_float4(fmin_(n0.x, n1.x), fmin_(n0.z, n1.z), fmin_(n2.x, n2.z), 0.f);
         hi = make_float4(fmax_(n0.y, n1.y), fmax_(n0.w, n1.w), fmax_(n2.y, n2.w), 0.f);
@@ -510,7 +499,7 @@ __device__ __forceinline__ void tlas_build_block(Args A, unsigned long long* s_k
     for (uint32_t j = tid; j < n; j += nt)
         tlas_emit_one(A.in, A.inst_box, j, A.keys[j], A.vals[j], A.inst_out, A.leaf_box, A.morton_out, A.order_out);
     __syncthreads();
-    for (uint32_t g = tid; g < n; g += nt) refit_leaf<true>(sd, g, A.leaf_box, A.node_parent, A.leaf_parent, A.flags);
+    for (uint32_t g = tid; g < n; g += nt) refit_leaf(sd, g, A.leaf_box, A.node_parent, A.leaf_parent, A.flags);
     __syncthreads();
     bfs_relayout_block(A.karras_nodes, A.nodes_out, m, A.queue, A.newidx, A.levels);
     __syncthreads();
