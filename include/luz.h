@@ -526,7 +526,7 @@ void* luz_frame_plane_device_ptr(luz_frame* frame, int32_t plane);
  * before them, each wait bounded (LUZ_DEV_BATCH_QUEUE when one gives up). The meshes'
  * BLASes are built before, once, by luz_blas_build_batch (the reference builds them
  * once at load, GPUScene.cpp:108-138). The frame kernel takes scenes of up to 4096
- * instances and 688 lights; a batch with a larger scene always runs in lanes. Both
+ * instances and 704 lights; a batch with a larger scene always runs in lanes. Both
  * forms give the same planes bit for bit. Scene constants and instances are uploaded / packed once at
  * creation (the arrays may be freed after luz_batch_create); luz_batch_capture records
  * a render as one CUDA graph that luz_batch_replay launches; luz_batch_autotune picks

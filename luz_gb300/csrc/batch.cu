@@ -33,6 +33,7 @@ constexpr uint32_t kClearWords = 16384;               // clear item: 64 KB of a 
 constexpr uint32_t kFrameWaitIters = 1u << 22;        // polls (128 ns apart) before a wait gives up
 constexpr size_t kFrameSmem = kStackBytes + kColdBytes;   // traversal stacks + cold ray state
 constexpr uint32_t kFrameMaxLights = (uint32_t)(kFrameSmem / sizeof(LightRec));
+static_assert(kFrameMaxLights == 704, "luz.h documents the limit");
 static_assert(kVisThreads == kFrameTile * kFrameTile, "a G-buffer item is one pixel per thread");
 static_assert(kFrameSmem >= kFusedTlasMax * sizeof(unsigned long long), "TLAS sort keys fit the shared memory");
 
@@ -272,7 +273,7 @@ __device__ __forceinline__ void frame_trace(const FrameArgs& A, unsigned long lo
 //      planes in 64-KB items, then the G-buffer tiles (each waits for its scene's
 //      TLAS). The CTA that finishes the last prologue item publishes the ray offsets.
 //   2. traversal: after `ready`, the warps of every CTA refill their lanes from one
-//      counter over the rays of all scenes (visibility_batch_kernel's loop); a warp
+//      counter over the rays of all scenes, as visibility_count_kernel does; a warp
 //      that leaves the loop adds the items it took to `resolved`.
 //   3. light passes: 256 lit pixels per item, after every ray item is resolved.
 template <bool kStats>

@@ -6,7 +6,7 @@
 // guarantee, or a host that owns every device allocation through its own pool. This
 // entry point serves them: the caller passes its own device buffers for the inputs
 // and outputs, and every temporary of the build (sort keys and values, tile state,
-// leaf boxes, parent links, refit flags) lives in one file-scope device array of
+// the merges' far ends and flags) lives in one file-scope device array of
 // fixed size. Nothing here calls cudaMalloc, cudaFree or an allocating library
 // routine.
 //
