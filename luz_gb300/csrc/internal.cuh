@@ -179,30 +179,18 @@ struct luz_tlas {
 };
 
 namespace luz {
-// Buffers of one trace, grown on demand: of a chunk (shafts.cuh) the patch bounds, start
-// lists per (virtual light, patch) and per AO patch, the lists' cuts, the shadow groups to
-// trace and the ray records (RayOut, structure of arrays), and the chunks' counters. A
+// Memory of one trace's buffers (VisBuffers, visibility.cu), one block that grows on demand. A
 // frame has its own; traces that run one after the other can share one.
 struct VisScratch {
-    void* patches = nullptr;
-    uint32_t* start_lists = nullptr;
-    float4* cuts = nullptr;
-    uint4* active = nullptr;
-    float4* rays_a = nullptr;
-    float4* rays_b = nullptr;
-    uint4* rays_c = nullptr;
-    void* counters = nullptr;             // VisCounters per chunk
-    uint32_t patches_cap = 0, lists_cap = 0, pairs_cap = 0, records_cap = 0, chunks_cap = 0;
-    uint32_t moves = 0;                   // times a buffer was freed or replaced
+    void* block = nullptr;
+    size_t bytes = 0;
+    uint32_t moves = 0;                   // times the block was freed or replaced
     uint32_t ray_chunk = kRayChunk;       // rays of a chunk at most (a power of two)
     void release() {
-        for (void* p : {patches, (void*)start_lists, (void*)cuts, (void*)active, (void*)rays_a, (void*)rays_b,
-                        (void*)rays_c, counters})
-            if (p) cudaFree(p);
-        const uint32_t m = moves + 1, chunk = ray_chunk;
-        *this = VisScratch{};
-        moves = m;
-        ray_chunk = chunk;
+        if (block) cudaFree(block);
+        block = nullptr;
+        bytes = 0;
+        ++moves;
     }
 };
 }  // namespace luz

@@ -24,6 +24,7 @@
 // which keeps the kernel at 64 registers and 4 CTAs per SM without spills.
 #include <algorithm>
 #include <cstring>
+#include <type_traits>
 
 #include "aocull.cuh"
 #include "shafts.cuh"
@@ -350,58 +351,55 @@ static VisSizes vis_sizes(const luz_frame* f, const luz_tlas* t, uint32_t ray_ch
     return z;
 }
 
-static luz_status grow_vis_buffers(luz_ctx* ctx, VisScratch& v, const VisSizes& z) {
-    const uint32_t patches = z.patches + z.supers, lists = z.pairs + z.ao_patches;
-    if (patches <= v.patches_cap && lists <= v.lists_cap && z.pairs <= v.pairs_cap && z.records <= v.records_cap &&
-        z.chunks <= v.chunks_cap)
-        return LUZ_OK;
-    LUZ_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
-    ++v.moves;
-    auto again = [&](auto*& p, size_t bytes) -> cudaError_t {
-        cudaFree(p);
-        p = nullptr;
-        return bytes ? cudaMalloc((void**)&p, bytes) : cudaSuccess;
+// A trace's buffers: of a chunk (shafts.cuh) the patch bounds (the patches', then their
+// blocks'), start lists per (virtual light, patch) and per AO patch, the lists' cuts, the
+// shadow groups to trace and the ray records (RayOut), and the chunks' counters.
+struct VisBuffers {
+    PatchRec* patches;
+    uint32_t* start_lists;
+    float4* cuts;
+    uint4* active;
+    float4* rays_a;
+    float4* rays_b;
+    uint4* rays_c;
+    VisCounters* counters;
+    size_t bytes;
+};
+static VisBuffers carve_vis(void* block, const VisSizes& z) {
+    VisBuffers b{};
+    auto take = [&](auto*& p, size_t count) {
+        p = reinterpret_cast<std::remove_reference_t<decltype(p)>>((uintptr_t)block + b.bytes);
+        b.bytes += (count * sizeof(*p) + 255) & ~(size_t)255;
     };
-    if (patches > v.patches_cap) {   // the patches, then their blocks
-        v.patches_cap = 0;
-        LUZ_CUDA(ctx, again(v.patches, (size_t)patches * sizeof(PatchRec)));
-        v.patches_cap = patches;
-    }
-    if (lists > v.lists_cap) {
-        v.lists_cap = 0;
-        LUZ_CUDA(ctx, again(v.start_lists, (size_t)lists * kEntryWords * 4));
-        v.lists_cap = lists;
-    }
-    if (z.pairs > v.pairs_cap) {
-        v.pairs_cap = 0;
-        LUZ_CUDA(ctx, again(v.cuts, (size_t)z.pairs * kCutsPerPair * kNode4F4 * sizeof(float4)));
-        LUZ_CUDA(ctx, again(v.active, (size_t)z.pairs * sizeof(uint4)));
-        v.pairs_cap = z.pairs;
-    }
-    if (z.records > v.records_cap) {
-        v.records_cap = 0;
-        LUZ_CUDA(ctx, again(v.rays_a, (size_t)z.records * sizeof(float4)));
-        LUZ_CUDA(ctx, again(v.rays_b, (size_t)z.records * sizeof(float4)));
-        LUZ_CUDA(ctx, again(v.rays_c, (size_t)z.records * sizeof(uint4)));
-        v.records_cap = z.records;
-    }
-    if (z.chunks > v.chunks_cap) {
-        v.chunks_cap = 0;
-        LUZ_CUDA(ctx, again(v.counters, (size_t)z.chunks * sizeof(VisCounters)));
-        v.chunks_cap = z.chunks;
-    }
-    return LUZ_OK;
+    take(b.patches, (size_t)z.patches + z.supers);
+    take(b.start_lists, ((size_t)z.pairs + z.ao_patches) * kEntryWords);
+    take(b.cuts, (size_t)z.pairs * kCutsPerPair * kNode4F4);
+    take(b.active, z.pairs);
+    take(b.rays_a, z.records);
+    take(b.rays_b, z.records);
+    take(b.rays_c, z.records);
+    take(b.counters, z.chunks);
+    return b;
 }
 
-// The buffers for a trace of f over t, in smaller chunks where there is no memory for larger
-// ones; z: the sizes it then has.
+// The block for a trace of f over t, in smaller chunks where there is no memory for larger
+// ones; z: the sizes it then has. One allocation: a new frame object's first frame at 640x360
+// takes 297 us, with one per buffer 490 (its second 190); at 4K 2665 and 2985 (2450).
 static luz_status ensure_vis_buffers(luz_ctx* ctx, VisScratch& v, const luz_frame* f, const luz_tlas* t, VisSizes& z) {
     for (;;) {
         z = vis_sizes(f, t, v.ray_chunk);
-        const luz_status s = z.chunks ? grow_vis_buffers(ctx, v, z) : LUZ_OK;
-        if (s != LUZ_ERR_OOM || v.ray_chunk <= kRayChunkMin) return s;
+        const size_t need = z.chunks ? carve_vis(nullptr, z).bytes : 0;
+        if (need <= v.bytes) return LUZ_OK;
+        LUZ_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
+        v.release();
+        const cudaError_t e = cudaMalloc(&v.block, need);
+        if (e == cudaSuccess) {
+            v.bytes = need;
+            return LUZ_OK;
+        }
+        v.block = nullptr;
+        if (e != cudaErrorMemoryAllocation || v.ray_chunk <= kRayChunkMin) return cuda_error(ctx, e, "trace buffers");
         cudaGetLastError();
-        v.release();   // (the stream is idle: grow_vis_buffers waited for it)
         v.ray_chunk /= 2;
     }
 }
@@ -438,7 +436,8 @@ luz_status launch_visibility(luz_ctx* ctx, luz_frame* f, const luz_tlas* t, int 
     if (d_stats) LUZ_CUDA(ctx, cudaMemsetAsync(d_stats, 0, 5 * sizeof(unsigned long long), st));
     if (!shadow_chunks && (s = clear_visibility(ctx, f)) != LUZ_OK) return s;   // else by patch_kernel
     if (z.chunks == 0) return LUZ_OK;
-    VisCounters* counters = (VisCounters*)v.counters;
+    const VisBuffers buf = carve_vis(v.block, z);
+    VisCounters* counters = buf.counters;
     if (!shadow_chunks) LUZ_CUDA(ctx, cudaMemsetAsync(counters, 0, (size_t)z.chunks * sizeof(VisCounters), st));
     if (t->count) S.leaf_box = tlas_leaf_boxes(t);
     if (ctx->raygen_blocks == 0) {   // resident blocks per SM: the persistent grids are one wave
@@ -449,9 +448,9 @@ luz_status launch_visibility(luz_ctx* ctx, luz_frame* f, const luz_tlas* t, int 
         ctx->raygen_blocks = std::max(b, 1);
     }
     const uint32_t sms = (uint32_t)ctx->sm_count;
-    const Entries entries{v.start_lists, v.cuts, cut_cap(t->count)};
+    const Entries entries{buf.start_lists, buf.cuts, cut_cap(t->count)};
     prof_begin(ctx, LUZ_KERNEL_RAYGEN);
-    PatchRec* patches = (PatchRec*)v.patches;
+    PatchRec* patches = buf.patches;
     if (shadow_chunks) {
         chain(patch_kernel, std::min(z.supers, sms * 8), kSuper * 32, 0, st, S, patches, patches + z.patches, counters,
                                                                           z.chunks);
@@ -465,13 +464,13 @@ luz_status launch_visibility(luz_ctx* ctx, luz_frame* f, const luz_tlas* t, int 
         if (k) prof_begin(ctx, LUZ_KERNEL_RAYGEN);
         VisCounters* n = counters + k;
         C.work_counter = &n->traversed;
-        const RayOut R{v.rays_a, v.rays_b, v.rays_c, &n->records};
+        const RayOut R{buf.rays_a, buf.rays_b, buf.rays_c, &n->records};
         const bool shadow = k < shadow_chunks, ao = k < ao_chunks;
         const ShaftOut A{patches, patches + z.patches, f->d_vlights, f->vlight_count, (unsigned long long)k * z.pairs,
-                         shadow ? z.pairs : 0u, list_cap(t->count), entries.cut_cap, super_cap(t->count), v.start_lists, v.cuts, v.active, &n->groups};
+                         shadow ? z.pairs : 0u, list_cap(t->count), entries.cut_cap, super_cap(t->count), buf.start_lists, buf.cuts, buf.active, &n->groups};
         const AoOut O{k * z.ao_patches, ao ? std::min(z.ao_patches, z.patches - k * z.ao_patches) : 0u,
                       f->ao_samples < kAoMinSamples ? 0u : std::min(kAoStepsPerSample * f->ao_samples, kAoSteps),
-                      v.start_lists + (size_t)z.pairs * kEntryWords, z.pairs, R};
+                      buf.start_lists + (size_t)z.pairs * kEntryWords, z.pairs, R};
         const uint32_t shaft_work = A.cap / kSuper, max_grid = sms * ctx->cull_blocks;
         auto cull_grid = [&](uint32_t warps) { return std::min((warps + kCullWarps - 1) / kCullWarps, max_grid); };
         if (shadow && ao && f->pixels <= kCullTogether) {
@@ -488,7 +487,7 @@ luz_status launch_visibility(luz_ctx* ctx, luz_frame* f, const luz_tlas* t, int 
             }
         }
         if (shadow) {
-            chain(A.list_cap > kListShort ? shadow_raygen_kernel<true> : shadow_raygen_kernel<false>, std::min((z.pairs + 7) / 8, sms * ctx->raygen_blocks), 256, 0, st, S, C, entries, v.active, &n->groups, &n->raygen_tickets, R);
+            chain(A.list_cap > kListShort ? shadow_raygen_kernel<true> : shadow_raygen_kernel<false>, std::min((z.pairs + 7) / 8, sms * ctx->raygen_blocks), 256, 0, st, S, C, entries, buf.active, &n->groups, &n->raygen_tickets, R);
             LUZ_LAUNCHED(ctx, "shadow_raygen_kernel");
         }
         prof_end(ctx);
