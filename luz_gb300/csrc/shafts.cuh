@@ -155,7 +155,12 @@ constexpr uint32_t kListAll = 0xFFFFFFFFu;
 // over 65 0.110 (0.116), 1080p over 1024 meshes of 81,920 triangles 1.736 (1.735; 1.768). Above
 // 2048 instances lists of up to 31 keep both, and lists of up to 62, unsorted, go without:
 // 1021x573 over 8000 2.86 ms against 3.02 with 31 at most (46: 2.95); below, the room for long
-// lists in ray generation costs what they save (720p 0.454 against 0.444).
+// lists in ray generation costs what they save (720p 0.454 against 0.444). The line at 2048
+// was drawn between scenes of 1024 and 8000 instances. Traces of 720p frames, us, long lists
+// (with super_cap's and cut_cap's larger values) and short: 1900 instances of 1280 triangles
+// 403 / 388, of 81,920 400 / 373, cubes 716 / 654; 3000: 667 / 661, 802 / 791, 709 / 612; 4096:
+// 861 / 858, 948 / 941, 718 / 640; 8000: 1842 / 1900, 2283 / 2376, 850 / 773. So up to 4096 the
+// short ones would be faster by up to 14 %, and above it they are only where meshes are small.
 constexpr uint32_t kListCap = 62, kListShort = kEntryCuts - 1, kCutCapSmall = 15, kCutCapLarge = 31;
 inline uint32_t list_cap(uint32_t instances) { return instances > 2048 ? kListCap : kListShort; }
 inline uint32_t cut_cap(uint32_t instances) { return instances > 2048 ? kCutCapLarge : kCutCapSmall; }
