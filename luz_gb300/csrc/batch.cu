@@ -472,12 +472,15 @@ static luz_status launch_frame(luz_ctx* ctx, luz_batch* b, bool stats) {
     return LUZ_OK;
 }
 
-// The frame kernel starts every ray at its TLAS root and traces the G-buffer without tile
-// lists, but is one launch: it stays the faster form for many small scenes. kLanes = 8 is the
-// number of streams that the device takes work from at once. Renders, us, frame kernel and
-// lanes: 12 scenes of 256x256 196 / 235, 64 510 / 981, 12 of 512x512 376 / 360, 40 793 / 729,
-// 12 of 1280x720 813 / 553; few scenes are faster in lanes at any size, a lane each: 2 of
-// 64x64 325 / 193, 2 of 256x256 94 / 81.
+// The form that a batch starts with. The frame kernel starts every ray at its TLAS root and
+// traces the G-buffer without tile lists, but is one launch: it is the faster form for many
+// small scenes. kLanes = 8 is the number of streams that the device takes work from at once.
+// Renders, us, frame kernel and lanes: 12 scenes of 256x256 196 / 235, 64 510 / 981, 12 of
+// 512x512 376 / 360, 40 793 / 729, 12 of 1280x720 813 / 553; few scenes are faster in lanes at
+// any size, a lane each: 2 of 64x64 325 / 193, 2 of 256x256 94 / 81. The lines are drawn for
+// those scenes. Over 2000 to 10,000 triangles and 4 AO rays the lanes gain earlier: 4 of
+// 128x128 448 / 315, 8 548 / 420, 11 607 / 599, 16 725 / 744; 11 of 256x256 1227 / 1125, 16 of
+// 400x400 3376 / 2758 (luz_batch_set_fused chooses).
 constexpr uint64_t kLanePixels = 200000;    // mean pixels of a scene from which on the lanes are taken
 constexpr uint32_t kLaneScenes = 2;         // and scenes up to which they always are
 constexpr uint32_t kLanes = 8;
