@@ -110,9 +110,9 @@ static luz_status reserve_upload(luz_ctx* ctx, luz_frame* f, uint32_t lights, ui
     const size_t scene = region(sizeof(luz_scene)), light = region((size_t)nl * sizeof(luz_light)),
                  first = region((size_t)nl * 4), slot = region((size_t)ns * 4),
                  vlight = region((size_t)ns * 4), model = region((size_t)nm * sizeof(luz_model)), skip = region(nm);
-    // the old block stays in place until the new one is there
+    // the old block stays in place until the new one is there (a new frame has none to wait for)
     if (!f->upload_done) LUZ_CUDA(ctx, cudaEventCreateWithFlags(&f->upload_done, cudaEventDisableTiming));
-    LUZ_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
+    if (f->d_upload) LUZ_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
     void *dev = nullptr, *host = nullptr;
     LUZ_CUDA(ctx, cudaMalloc(&dev, bytes));
     if (cudaError_t e = cudaMallocHost(&host, bytes); e != cudaSuccess) {

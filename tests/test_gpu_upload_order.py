@@ -128,3 +128,23 @@ def test_upload_during_a_capture_is_refused():
         assert np.array_equal(_light(f), one)        # the refused upload left nothing behind
     finally:
         ctx.close()
+
+
+def test_a_frame_is_created_while_the_stream_is_busy():
+    torch = pytest.importorskip("torch")
+    ctx = L.Context(0)
+    try:
+        stream = torch.cuda.Stream()
+        ctx.set_stream(stream.cuda_stream)
+        _frame(ctx)
+        ctx.synchronize()
+        busy = torch.cuda.Event()
+        with torch.cuda.stream(stream):
+            torch.cuda._sleep(1_000_000_000)         # half a second
+            busy.record()
+        f = ctx.frame(W, H)
+        f.upload(_block(1), _lights(1, 1.0), 1, None, 0)
+        assert not busy.query()                      # neither call waited for the stream
+        ctx.synchronize()
+    finally:
+        ctx.close()
