@@ -197,9 +197,9 @@ __device__ __forceinline__ void start_ray(LaneRay& r, const Cold& c, const Scene
     c[kOutHi] = __uint_as_float((uint32_t)(oa >> 32));
     c[kOutBits] = __uint_as_float((pix & 31u) | (record_hit ? 32u : 0u));
     r.tmin = tmin;
-    r.tmax = tmax;
     r.idir = safe_inv(wd);
     set_origin(r, wo);
+    r.tmax = has_axis(r.on, wd) ? tmax : -1.0f;   // (offsets that overflow on every axis: no box)
     near_planes(r);
     c[kWiX] = r.idir.x; c[kWiY] = r.idir.y; c[kWiZ] = r.idir.z;
     c[kWnX] = r.on.x; c[kWnY] = r.on.y; c[kWnZ] = r.on.z;
@@ -372,6 +372,7 @@ __device__ __forceinline__ void run_steps(LaneRay& r, const Cold& c, bool& activ
                 ++r.sp;
                 r.in_blas = true;
                 r.node = first;
+                pop = !has_axis(r.on, od);   // left at once, else it could come to empty slots
             } else {
                 pop = true;
             }
