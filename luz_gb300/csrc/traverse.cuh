@@ -125,12 +125,12 @@ __device__ __forceinline__ bool sphere_misses(V3 o, V3 d, float tmin, float tmax
     return q2 > r * r;
 }
 
-// Whether a ray (o, d) has an axis on which its plane distances are numbers. Without one (an
-// instance's transform that is singular or not finite) every box is overlapped, also the
-// inverted boxes of empty child slots, and no triangle is hit (the test's t is a NaN).
-__device__ __forceinline__ bool has_axis(V3 o, V3 d) {
-    return fminf(fminf(fabsf(o.x) + fabsf(d.x), fabsf(o.y) + fabsf(d.y)), fabsf(o.z) + fabsf(d.z)) <
-           __int_as_float(0x7f800000);
+// Whether an object-space ray can hit anything: one that is not finite (an instance's
+// transform is singular or not finite) hits no triangle, the test's t being a NaN, but
+// overlaps any number of boxes, with a NaN on every axis also the inverted ones of empty
+// child slots.
+__device__ __forceinline__ bool finite_ray(V3 o, V3 d) {
+    return ((fabsf(o.x) + fabsf(o.y)) + (fabsf(o.z) + fabsf(d.x))) + (fabsf(d.y) + fabsf(d.z)) < __int_as_float(0x7f800000);
 }
 
 __device__ __forceinline__ int dir_signs(V3 idir) {
@@ -251,11 +251,11 @@ __device__ __forceinline__ bool trace_ray(const TlasView& T, V3 wo, V3 wd, float
                 take = skip[meta.x] != 1;
                 tested = skip[meta.x] == 2;
             }
-            // Skipped too when the segment provably misses the BLAS's bounding sphere, or
-            // without an axis to tell its boxes by.
+            // Skipped too when the segment provably misses the BLAS's bounding sphere, or the
+            // transform leaves no ray.
             const float m[12] = {r0.x, r0.y, r0.z, r0.w, r1.x, r1.y, r1.z, r1.w, r2.x, r2.y, r2.z, r2.w};
             const V3 oo = xform_point(m, wo), od = xform_dir(m, wd);
-            if (take && has_axis(oo, od) && !sphere_misses(oo, od, tmin, tmax, sph)) {
+            if (take && finite_ray(oo, od) && !sphere_misses(oo, od, tmin, tmax, sph)) {
                 if (sp >= kStackSize) { err |= LUZ_DEV_STACK_OVERFLOW; return false; }
                 stack[sp++] = kStackMarker;
                 o = oo;

@@ -109,6 +109,12 @@ __device__ __forceinline__ bool slab_ordered(float nx, float fx, float ny, float
     return tn * kSlabShrink <= tf;
 }
 
+// Whether an axis is left to tell boxes by: where the offsets of a finite ray overflow on all
+// three, the plane distances are NaNs and the ray overlaps the inverted boxes of empty slots.
+__device__ __forceinline__ bool has_axis(const LaneRay& r) {
+    return fminf(fminf(fabsf(r.on.x), fabsf(r.on.y)), fabsf(r.on.z)) < __int_as_float(0x7f800000);
+}
+
 // The ray of item (slot, j) of scene S (light.frag:86-135): world origin and
 // direction, t range, output word and whether a hit (shadow) or a miss (AO) is
 // recorded. Returns false when there is nothing to trace; the miss (AO) has then
@@ -199,7 +205,7 @@ __device__ __forceinline__ void start_ray(LaneRay& r, const Cold& c, const Scene
     r.tmin = tmin;
     r.idir = safe_inv(wd);
     set_origin(r, wo);
-    r.tmax = has_axis(r.on, wd) ? tmax : -1.0f;   // (offsets that overflow on every axis: no box)
+    r.tmax = has_axis(r) ? tmax : -1.0f;   // (without: no box)
     near_planes(r);
     c[kWiX] = r.idir.x; c[kWiY] = r.idir.y; c[kWiZ] = r.idir.z;
     c[kWnX] = r.on.x; c[kWnY] = r.on.y; c[kWnZ] = r.on.z;
@@ -331,8 +337,8 @@ __device__ __forceinline__ void run_steps(LaneRay& r, const Cold& c, bool& activ
                 pop = true;
             }
         } else if (at_leaf && !r.in_blas && do_entries) {
-            // Instance leaf: entered unless its mask or BLAS is empty or the ray
-            // segment provably misses the BLAS's bounding sphere.
+            // Instance leaf: entered unless its mask or BLAS is empty, its transform leaves
+            // no ray or the segment provably misses the BLAS's bounding sphere.
             ++r.budget;
             if (kStats) cnt.instances++;
             uint32_t leaf = (uint32_t)~r.node;
@@ -352,7 +358,7 @@ __device__ __forceinline__ void run_steps(LaneRay& r, const Cold& c, bool& activ
             float4 q0 = __ldg(wp), q1 = __ldg(wp + 1), q2 = __ldg(wp + 2), sph = __ldg(&I->sphere);
             float m[12] = {q0.x, q0.y, q0.z, q0.w, q1.x, q1.y, q1.z, q1.w, q2.x, q2.y, q2.z, q2.w};
             const V3 od = xform_dir(m, c.wd()), oo = xform_point(m, c.wo());
-            if ((meta.y & 0xFFu) != 0 && meta.w > 0 && !sphere_misses(oo, od, r.tmin, r.tmax, sph)) {
+            if ((meta.y & 0xFFu) != 0 && meta.w > 0 && finite_ray(oo, od) && !sphere_misses(oo, od, r.tmin, r.tmax, sph)) {
                 c[kOdX] = od.x;
                 c[kOdY] = od.y;
                 c[kOdZ] = od.z;
@@ -372,7 +378,7 @@ __device__ __forceinline__ void run_steps(LaneRay& r, const Cold& c, bool& activ
                 ++r.sp;
                 r.in_blas = true;
                 r.node = first;
-                pop = !has_axis(r.on, od);   // left at once, else it could come to empty slots
+                pop = !has_axis(r);   // (without: left at once)
             } else {
                 pop = true;
             }

@@ -79,3 +79,21 @@ def test_frames_without_the_bad_instances(cfg, kw, kind):
         assert ctx.device_status() == 0
     finally:
         ctx.close()
+
+
+def test_many_bad_instances_of_a_large_mesh_cost_a_ray_nothing():
+    """A row of zeros beside rows of NaN leaves boxes to overlap along a plane of the mesh: were
+    they walked, a ray over many such instances would run into its step cap."""
+    ctx = L.Context(0)
+    try:
+        s = _Scene(2, seed=3, width=48, height=32, meshes=2, instances=4000, subdivisions=6)
+        s.kind, s.bad = "inf", np.arange(1, 4000, 2)
+        s.set_sampling(2, ao_max=3.0)
+        g = L.GPUScene(ctx, s)
+        g.render(1)
+        ctx.synchronize()
+        assert ctx.device_status() == 0
+        st = g.frame.trace_stats(g.tlas, 1)
+        assert st["rays"] > 0 and st["blas_nodes"] < 500 * st["rays"]
+    finally:
+        ctx.close()
