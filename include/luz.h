@@ -517,8 +517,8 @@ void* luz_frame_plane_device_ptr(luz_frame* frame, int32_t plane);
  * average, or up to two scenes of any size, run in lanes: every pass of a scene as the
  * launches of a single frame, the scenes spread over up to eight streams that fork from
  * the context's and join it again; a lane's buffers are those of a single frame's trace,
- * for its largest scene, all lanes' together those of one frame at most (12 GB). Many
- * small scenes run as ONE
+ * for its largest scene, all lanes' together an eighth of the device's memory at most.
+ * Many small scenes run as ONE
  * persistent launch (the frame kernel) over every scene: the per-frame TLAS builds,
  * the clearing of the hit/miss planes, the G-buffer passes with their lit-pixel lists,
  * the shadow/AO traversal of all scenes' rays from one work counter, and the light

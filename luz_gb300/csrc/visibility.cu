@@ -382,13 +382,18 @@ static VisBuffers carve_vis(void* block, const VisSizes& z) {
     return b;
 }
 
+size_t visibility_bytes(const luz_frame* f, const luz_tlas* t, uint32_t ray_chunk) {
+    const VisSizes z = vis_sizes(f, t, ray_chunk);
+    return z.chunks ? carve_vis(nullptr, z).bytes : 0;
+}
+
 // The block for a trace of f over t, in smaller chunks where there is no memory for larger
 // ones; z: the sizes it then has. One allocation: a new frame object's first frame at 640x360
 // takes 297 us, with one per buffer 490 (its second 190); at 4K 2665 and 2985 (2450).
 static luz_status ensure_vis_buffers(luz_ctx* ctx, VisScratch& v, const luz_frame* f, const luz_tlas* t, VisSizes& z) {
     for (;;) {
         z = vis_sizes(f, t, v.ray_chunk);
-        const size_t need = z.chunks ? carve_vis(nullptr, z).bytes : 0;
+        const size_t need = visibility_bytes(f, t, v.ray_chunk);
         if (need <= v.bytes) return LUZ_OK;
         LUZ_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
         v.release();

@@ -46,6 +46,8 @@ const float4* tlas_leaf_boxes(const luz_tlas* t);
 luz_status clear_visibility(luz_ctx* ctx, luz_frame* f);
 // Allocates what the traces of frame f over t need from the scratch.
 luz_status reserve_visibility(luz_ctx* ctx, const luz_frame* f, const luz_tlas* t, VisScratch& scratch);
+// Bytes of it where a chunk has `ray_chunk` rays at most.
+size_t visibility_bytes(const luz_frame* f, const luz_tlas* t, uint32_t ray_chunk);
 luz_status launch_visibility(luz_ctx* ctx, luz_frame* f, const luz_tlas* t, int frame_index, unsigned long long* d_stats,
                              VisScratch& scratch);
 luz_status launch_visibility_count(luz_ctx* ctx, const SceneVis* d_scenes, uint32_t n, unsigned long long* d_offsets,

@@ -71,11 +71,11 @@ def test_chunks_shrink_to_the_memory_there_is():
         ctx.close()
 
 
-def test_lanes_share_the_memory_of_one_frames_trace():
+def test_lanes_take_an_eighth_of_the_memory_at_most():
     torch = pytest.importorskip("torch")
     ctx = L.Context(0)
     try:
-        before, _ = torch.cuda.mem_get_info()
+        before, total = torch.cuda.mem_get_info()
         s = L.HostScene(1, seed=8, width=128, height=72, point_lights=1023)
         s.set_sampling(4, light_samples=16)
         b = L.Batch(ctx, [s] * 8)                    # 7 GB a scene in whole chunks
@@ -83,6 +83,6 @@ def test_lanes_share_the_memory_of_one_frames_trace():
         b.render(1)
         ctx.synchronize()
         assert ctx.device_status() == 0
-        assert before - torch.cuda.mem_get_info()[0] < 12 << 30
+        assert before - torch.cuda.mem_get_info()[0] < total // 8 + (1 << 30)
     finally:
         ctx.close()
