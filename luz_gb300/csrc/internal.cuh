@@ -179,17 +179,19 @@ struct luz_tlas {
 };
 
 namespace luz {
-// Memory of one trace's buffers (VisBuffers, visibility.cu), one block that grows on demand. A
-// frame has its own; traces that run one after the other can share one.
+// Memory of one trace's buffers (VisBuffers, visibility.cu), grown on demand: one block, or up
+// to four small ones. A frame has its own; traces that run one after the other can share one.
 struct VisScratch {
-    void* block = nullptr;
-    size_t bytes = 0;
-    uint32_t moves = 0;                   // times the block was freed or replaced
+    void* block[4] = {};
+    size_t bytes[4] = {};
+    uint32_t moves = 0;                   // times the blocks were freed or replaced
     uint32_t ray_chunk = kRayChunk;       // rays of a chunk at most (a power of two)
     void release() {
-        if (block) cudaFree(block);
-        block = nullptr;
-        bytes = 0;
+        for (int k = 0; k < 4; ++k) {
+            if (block[k]) cudaFree(block[k]);
+            block[k] = nullptr;
+            bytes[k] = 0;
+        }
         ++moves;
     }
 };

@@ -359,52 +359,70 @@ struct VisBuffers {
     uint32_t* start_lists;
     float4* cuts;
     uint4* active;
+    VisCounters* counters;
     float4* rays_a;
     float4* rays_b;
     uint4* rays_c;
-    VisCounters* counters;
-    size_t bytes;
+    size_t bytes[4];   // of the scratch's blocks: all but the rays, the rays' three arrays
 };
-static VisBuffers carve_vis(void* block, const VisSizes& z) {
+static VisBuffers carve_vis(const VisScratch& v, const VisSizes& z) {
     VisBuffers b{};
-    auto take = [&](auto*& p, size_t count) {
-        p = reinterpret_cast<std::remove_reference_t<decltype(p)>>((uintptr_t)block + b.bytes);
-        b.bytes += (count * sizeof(*p) + 255) & ~(size_t)255;
+    uintptr_t at = (uintptr_t)v.block[0];
+    auto take = [&](auto*& p, size_t count, int k) {
+        if (k && v.block[k]) at = (uintptr_t)v.block[k];   // (else after the arrays before it)
+        p = reinterpret_cast<std::remove_reference_t<decltype(p)>>(at);
+        const size_t n = (count * sizeof(*p) + 255) & ~(size_t)255;
+        b.bytes[k] += n;
+        at += n;
     };
-    take(b.patches, (size_t)z.patches + z.supers);
-    take(b.start_lists, ((size_t)z.pairs + z.ao_patches) * kEntryWords);
-    take(b.cuts, (size_t)z.pairs * kCutsPerPair * kNode4F4);
-    take(b.active, z.pairs);
-    take(b.rays_a, z.records);
-    take(b.rays_b, z.records);
-    take(b.rays_c, z.records);
-    take(b.counters, z.chunks);
+    take(b.patches, (size_t)z.patches + z.supers, 0);
+    take(b.start_lists, ((size_t)z.pairs + z.ao_patches) * kEntryWords, 0);
+    take(b.cuts, (size_t)z.pairs * kCutsPerPair * kNode4F4, 0);
+    take(b.active, z.pairs, 0);
+    take(b.counters, z.chunks, 0);
+    take(b.rays_a, z.records, 1);
+    take(b.rays_b, z.records, 2);
+    take(b.rays_c, z.records, 3);
     return b;
 }
 
+static size_t total_bytes(const size_t (&n)[4]) { return n[0] + n[1] + n[2] + n[3]; }
+
 size_t visibility_bytes(const luz_frame* f, const luz_tlas* t, uint32_t ray_chunk) {
     const VisSizes z = vis_sizes(f, t, ray_chunk);
-    return z.chunks ? carve_vis(nullptr, z).bytes : 0;
+    return z.chunks ? total_bytes(carve_vis(VisScratch{}, z).bytes) : 0;
 }
 
-// The block for a trace of f over t, in smaller chunks where there is no memory for larger
+// The blocks for a trace of f over t, in smaller chunks where there is no memory for larger
 // ones; z: the sizes it then has. One allocation: a new frame object's first frame at 640x360
-// takes 297 us, with one per buffer 490 (its second 190); at 4K 2665 and 2985 (2450).
+// takes 297 us, with one per buffer 490 (its second 190); at 4K 2665 and 2985 (2450). Up to
+// kVisPooled four: cudaMalloc serves those out of what it holds (frames of 96x64 made and
+// dropped in turn, first frame and preparation: 1090 us, with one block 1285).
+constexpr size_t kVisPooled = 1 << 20;
 static luz_status ensure_vis_buffers(luz_ctx* ctx, VisScratch& v, const luz_frame* f, const luz_tlas* t, VisSizes& z) {
     for (;;) {
         z = vis_sizes(f, t, v.ray_chunk);
-        const size_t need = visibility_bytes(f, t, v.ray_chunk);
-        if (need <= v.bytes) return LUZ_OK;
+        if (!z.chunks) return LUZ_OK;
+        size_t need[4];
+        memcpy(need, carve_vis(VisScratch{}, z).bytes, sizeof need);
+        bool fits = true, pooled = true;
+        if (!v.block[1]) fits = total_bytes(need) <= v.bytes[0];
+        for (int k = 0; k < 4; ++k) {
+            fits = fits && (!v.block[1] || need[k] <= v.bytes[k]);
+            pooled = pooled && need[k] <= kVisPooled;
+        }
+        if (fits) return LUZ_OK;
         LUZ_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
         v.release();
-        const cudaError_t e = cudaMalloc(&v.block, need);
-        if (e == cudaSuccess) {
-            v.bytes = need;
-            return LUZ_OK;
+        cudaError_t e = cudaSuccess;
+        for (int k = 0; k < (pooled ? 4 : 1) && e == cudaSuccess; ++k) {
+            v.bytes[k] = pooled ? need[k] : total_bytes(need);
+            e = cudaMalloc(&v.block[k], std::max<size_t>(v.bytes[k], 256));
         }
-        v.block = nullptr;
-        if (e != cudaErrorMemoryAllocation || v.ray_chunk <= kRayChunkMin) return cuda_error(ctx, e, "trace buffers");
+        if (e == cudaSuccess) return LUZ_OK;
         cudaGetLastError();
+        v.release();
+        if (e != cudaErrorMemoryAllocation || v.ray_chunk <= kRayChunkMin) return cuda_error(ctx, e, "trace buffers");
         v.ray_chunk /= 2;
     }
 }
@@ -441,7 +459,7 @@ luz_status launch_visibility(luz_ctx* ctx, luz_frame* f, const luz_tlas* t, int 
     if (d_stats) LUZ_CUDA(ctx, cudaMemsetAsync(d_stats, 0, 5 * sizeof(unsigned long long), st));
     if (!shadow_chunks && (s = clear_visibility(ctx, f)) != LUZ_OK) return s;   // else by patch_kernel
     if (z.chunks == 0) return LUZ_OK;
-    const VisBuffers buf = carve_vis(v.block, z);
+    const VisBuffers buf = carve_vis(v, z);
     VisCounters* counters = buf.counters;
     if (!shadow_chunks) LUZ_CUDA(ctx, cudaMemsetAsync(counters, 0, (size_t)z.chunks * sizeof(VisCounters), st));
     if (t->count) S.leaf_box = tlas_leaf_boxes(t);
